@@ -741,11 +741,10 @@ int tg_set_level1_galerkin_fast(int32_t on);
  * arithmetic either way.  Applies to solvers created afterwards. */
 int tg_set_coarse_fused(int32_t on);
 /* Schedule of the FP32 fine operator (the mixed form's fine level).  kind 0:
- * the pencil kernel; kind 1: the column-blocked kernel with tile shape `shape`
- * (0 <= shape < 8: Y x W element rows per thread x warps per CTA of 4x4, 6x4,
- * 3x4, 2x8 for shapes 0-3, the same tiles with the x and y components in
- * paired FP32 instructions for shapes 4-7) and `kz` >= 8 element layers per
- * CTA.  The setting overrides the per-grid, per-mode table (apply, residual,
+ * one element row per thread (the FP64 form's schedule, its tile chosen by a
+ * cost model); kind 1: two element rows per thread in paired FP32 instructions,
+ * with 2, 3, 4, 5, 6, 8, 10 or 12 warps per CTA for `shape` 0 .. 7 and `kz` >= 8
+ * node layers per CTA.  The setting overrides the per-grid, per-mode table (apply, residual,
  * smoothing; measured on the first large mixed job of a grid) for every later
  * FP32 launch in the process; kind < 0 clears it.  Results of every schedule
  * agree to FP32 rounding. */

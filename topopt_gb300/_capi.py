@@ -951,9 +951,8 @@ def kernel_launches() -> int:
 
 
 SCHED_PENCIL, SCHED_COLUMN = 0, 1
-# (element rows per thread, warps per CTA, x/y in paired FP32 instructions)
-FP32_SHAPES = [(4, 4, False), (6, 4, False), (3, 4, False), (2, 8, False),
-               (4, 4, True), (6, 4, True), (3, 4, True), (2, 8, True)]
+# (element rows per thread, warps per CTA, rows in paired FP32 instructions)
+FP32_SHAPES = [(2, w, True) for w in (2, 3, 4, 5, 6, 8, 10, 12)]
 
 
 APPLY_L1_STENCIL, APPLY_L1_TC = 3, 4

@@ -60,7 +60,7 @@ __device__ __forceinline__ int dwrap(int a, int n) {
 // order, so the fields are deterministic.
 __global__ void k_homog_cell(const uint8_t* __restrict__ tags, int ncell, int nx, int ny, int nz,
                              double E, double kdiag, CornerLoads cl, double* __restrict__ ef,
-                             uint8_t* __restrict__ kept, double* __restrict__ invd,
+                             uint8_t* __restrict__ kn, double* __restrict__ invd,
                              double* __restrict__ F) {
   const int64_t np = int64_t(nx) * ny * nz, nd = 3 * np;
   const int64_t total = np * ncell;
@@ -86,10 +86,10 @@ __global__ void k_homog_cell(const uint8_t* __restrict__ tags, int ncell, int nx
 #pragma unroll
         for (int c = 0; c < 3; ++c) f[J][c] += cl.fe[J][a][c];
     }
+    const bool kk = cnt > 0 && p > 0;  // node 0 pinned, untouched DOFs pinned
+    kn[q] = kk ? 7 : 0;
     for (int c = 0; c < 3; ++c) {
       const int64_t d = 3 * p + c;
-      const bool kk = cnt > 0 && d >= 3;  // node 0 pinned, untouched DOFs pinned
-      kept[cell * nd + d] = kk;
       invd[cell * nd + d] = kk ? 1.0 / (kdiag * E * double(cnt)) : 0.0;
 #pragma unroll
       for (int J = 0; J < 6; ++J) F[(cell * 6 + J) * nd + d] = kk ? f[J][c] : 0.0;
@@ -395,8 +395,8 @@ struct Batch {
     const int Pop = periodic_op_blocks<T>(nx, ny, nz);
     int host_nact = B;
     for (int k = 0; k < max_it && host_nact > 0; ++k) {
-      launch_periodic_op<T>(kApply, nx, ny, nz, mc, ef, kept, Pv, nullptr, nullptr, T(0), Tv,
-                            ppap.p, B, nrhs, s);
+      launch_periodic_op<T>(kApply, nx, ny, nz, mc, ef, kept, Pv, nullptr, Tv, ppap.p, B, nrhs,
+                            act.p, s);
       k_bsum<<<wb(), 256, 0, s>>>(ppap.p, Pop, B, pap.p, nullptr, nullptr);
       TG_LAUNCH_CHECK();
       k_b_xr<T><<<g2(), kT, 0, s>>>(X, R, Pv, Tv, invd, nd, nrhs, absn.p, pap.p, act.p, prr.p,
@@ -519,7 +519,7 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
     dtags.alloc(size_t(ncell * np));
     TG_CUDA(cudaMemcpyAsync(dtags.p, tags, size_t(ncell * np), cudaMemcpyHostToDevice, s));
     ef.alloc(size_t(ncell * np));
-    kept.alloc(size_t(ncell * nd));
+    kept.alloc(size_t(ncell * np));
     invd.alloc(size_t(ncell * nd));
     F.alloc(size_t(ncell * 6 * nd));
     for (DBuf<double>* v : {&Bv, &X, &R}) v->alloc(size_t(B) * size_t(nd));
@@ -582,8 +582,8 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
       for (int ref = 0;; ++ref) {
         // r = b - A x (FP64) -- the first residual is b itself (x = 0).
         if (ref > 0)
-          launch_periodic_op<double>(kResidual, nx, ny, nz, bt.mc, ef.p, kept.p, X.p, Bv.p,
-                                     nullptr, 0.0, R.p, nullptr, B, nrhs, s);
+          launch_periodic_op<double>(kResidual, nx, ny, nz, bt.mc, ef.p, kept.p, X.p, Bv.p, R.p,
+                                     nullptr, B, nrhs, bt.run.p, s);
         k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
         TG_LAUNCH_CHECK();
         k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, bt.rr.p, nullptr, nullptr);

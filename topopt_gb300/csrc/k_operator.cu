@@ -17,13 +17,15 @@
 // FP64 at roughly 1/64 of its FP32 rate.  The result equals Ke u to rounding
 // (checked against the oracle's dense Ke in the tests).
 //
-// Scheduling: x-pencils marching in z (see k_fine_op below): element outputs are
-// combined along x by warp shuffles, along y through shared memory and along z
-// in registers, so each node is finished exactly once without atomics and the
-// per-node summation order is fixed -- the apply is deterministic run to run.
+// Scheduling: warps march in z over node columns (k_fine_march below), sharing
+// the transforms between neighbouring elements; each node is finished exactly
+// once, without atomics, in a fixed summation order -- the apply is
+// deterministic run to run.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <cmath>
 #include <type_traits>
 
 #include "tg_df.h"
@@ -47,7 +49,7 @@ ModalConsts ModalConsts::make(double nu, double h) {
 
 template <class T>
 struct ModalT {
-  T L0, L1, M0, M1, M02, M12, LM2;  // per unit modulus; M02 = 2*M0, LM2 = L2 + 4*M2
+  T L0, L1, M0, M1, M02, LM2;  // per unit modulus; M02 = 2*M0, LM2 = L2 + 4*M2
 };
 
 // Storage (T) to compute (C) and back: the identity, except that a double is
@@ -65,6 +67,10 @@ __device__ __forceinline__ C load_c(T v) {
   return cvt<C>(v);
 }
 template <>
+__device__ __forceinline__ df load_c<df, double>(double v) {
+  return df_split(v);
+}
+template <>
 __device__ __forceinline__ float load_c<float, float>(float v) {
   return v;
 }
@@ -74,14 +80,6 @@ __device__ __forceinline__ double store_t(df v) { return df_to_double(v); }
 __device__ __forceinline__ bool nonzero(float v) { return v != 0.0f; }
 __device__ __forceinline__ bool nonzero(double v) { return v != 0.0; }
 __device__ __forceinline__ bool nonzero(df v) { return df_nonzero(v); }
-__device__ __forceinline__ float shfl_up(float v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-__device__ __forceinline__ double shfl_up(double v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-__device__ __forceinline__ float shfl_down(float v, int d) {
-  return __shfl_down_sync(0xffffffffu, v, d);
-}
-__device__ __forceinline__ double shfl_down(double v, int d) {
-  return __shfl_down_sync(0xffffffffu, v, d);
-}
 template <class C>
 __host__ __device__ __forceinline__ C czero() {
   return cvt<C>(0.0);
@@ -95,7 +93,6 @@ ModalT<T> to_modal(const ModalConsts& c) {
   m.M0 = cvt<T>(c.M[0]);
   m.M1 = cvt<T>(c.M[1]);
   m.M02 = cvt<T>(2.0 * c.M[0]);
-  m.M12 = cvt<T>(2.0 * c.M[1]);
   m.LM2 = cvt<T>(c.L[2] + 4.0 * c.M[2]);
   return m;
 }
@@ -104,219 +101,28 @@ ModalT<T> to_modal(const ModalConsts& c) {
 __device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
 
-// Forward Walsh transform of one component: v[idx], idx = sx | sy<<1 | sz<<2
-// with s = 1 on the + side, becomes the unnormalised mode coefficients
-// 8*m[mask], mask bit i set when axis i is in the monomial.
-template <class T>
-__device__ __forceinline__ void walsh_fwd(T (&v)[8]) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      const T lo = v[i], hi = v[i | b];
-      v[i] = hi + lo;
-      v[i | b] = hi - lo;
-    }
-  }
-}
-
-// Inverse (unnormalised) transform: corner values from mode coefficients.
-template <class T>
-__device__ __forceinline__ void walsh_inv(T (&w)[8]) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      const T lo = w[i], hi = w[i | b];
-      w[i] = lo - hi;
-      w[i | b] = lo + hi;
-    }
-  }
-}
-
-// out = f * Ke * u for one element; u and out indexed [corner idx][comp].
-template <class T>
-__device__ __forceinline__ void modal_apply(const ModalT<T>& mc, T f, T (&ux)[8], T (&uy)[8],
-                                            T (&uz)[8]) {
-  walsh_fwd(ux);
-  walsh_fwd(uy);
-  walsh_fwd(uz);
-  const T L0 = mc.L0 * f, L1 = mc.L1 * f, M0 = mc.M0 * f, M1 = mc.M1 * f;
-  const T M02 = mc.M02 * f, M12 = mc.M12 * f, LM2 = mc.LM2 * f;
-  T gx[8], gy[8], gz[8];
-  // |T| = 0: the constant-gradient block.
-  {
-    const T Ltr = L0 * (ux[1] + uy[2] + uz[4]);
-    gx[1] = mad(M02, ux[1], Ltr);
-    gy[2] = mad(M02, uy[2], Ltr);
-    gz[4] = mad(M02, uz[4], Ltr);
-    const T txy = M0 * (uy[1] + ux[2]);
-    const T txz = M0 * (uz[1] + ux[4]);
-    const T tyz = M0 * (uz[2] + uy[4]);
-    gy[1] = txy; gz[1] = txz;
-    gx[2] = txy; gz[2] = tyz;
-    gx[4] = txz; gy[4] = tyz;
-  }
-  // |T| = 1: gradients linear along one axis; modes 3, 5, 6 each get two terms.
-  {
-    const T Ltr = L1 * (uy[3] + uz[5]);  // T = {x}: rows y (mode 3), z (mode 5)
-    const T t = M1 * (uz[3] + uy[5]);
-    gx[3] = M1 * ux[3];
-    gy[3] = mad(M12, uy[3], Ltr);
-    gz[3] = t;
-    gx[5] = M1 * ux[5];
-    gy[5] = t;
-    gz[5] = mad(M12, uz[5], Ltr);
-  }
-  {
-    const T Ltr = L1 * (ux[3] + uz[6]);  // T = {y}: rows x (mode 3), z (mode 6)
-    const T t = M1 * (uz[3] + ux[6]);
-    gx[3] = gx[3] + mad(M12, ux[3], Ltr);
-    gy[3] = mad(M1, uy[3], gy[3]);
-    gz[3] = gz[3] + t;
-    gx[6] = t;
-    gy[6] = M1 * uy[6];
-    gz[6] = mad(M12, uz[6], Ltr);
-  }
-  {
-    const T Ltr = L1 * (ux[5] + uy[6]);  // T = {z}: rows x (mode 5), y (mode 6)
-    const T t = M1 * (uy[5] + ux[6]);
-    gx[5] = gx[5] + mad(M12, ux[5], Ltr);
-    gy[5] = gy[5] + t;
-    gz[5] = mad(M1, uz[5], gz[5]);
-    gx[6] = gx[6] + t;
-    gy[6] = gy[6] + mad(M12, uy[6], Ltr);
-    gz[6] = mad(M1, uz[6], gz[6]);
-  }
-  // |T| = 2: the trilinear mode.
-  gx[7] = LM2 * ux[7];
-  gy[7] = LM2 * uy[7];
-  gz[7] = LM2 * uz[7];
-  gx[0] = gy[0] = gz[0] = czero<T>();
-  walsh_inv(gx);
-  walsh_inv(gy);
-  walsh_inv(gz);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    ux[i] = gx[i];
-    uy[i] = gy[i];
-    uz[i] = gz[i];
-  }
-}
-
-// ---- the same element operator with the x and y components packed ----
-// Blackwell's paired FP32 instructions (FADD2/FMUL2/FFMA2) operate on a float2
-// as one instruction.  The Walsh transforms treat x and y identically, so they
-// run on (x, y) pairs; the isotropic "stress" block mixes components and stays
-// scalar.  Same operations per component as modal_apply, same rounding.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);  // a - b, one rounding
-}
-__device__ __forceinline__ void walsh_fwd2(float2 (&v)[8]) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      const float2 lo = v[i], hi = v[i | b];
-      v[i] = add2(hi, lo);
-      v[i | b] = sub2(hi, lo);
-    }
-  }
-}
-__device__ __forceinline__ void walsh_inv2(float2 (&w)[8]) {
-#pragma unroll
-  for (int b = 1; b < 8; b <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i & b) continue;
-      const float2 lo = w[i], hi = w[i | b];
-      w[i] = sub2(lo, hi);
-      w[i | b] = add2(lo, hi);
-    }
-  }
-}
-__device__ __forceinline__ void modal_apply_xy(const ModalT<float>& mc, float f, float2 (&uxy)[8],
-                                               float (&uz)[8]) {
-  walsh_fwd2(uxy);
-  walsh_fwd(uz);
-  const float L0 = mc.L0 * f, L1 = mc.L1 * f, M0 = mc.M0 * f, M1 = mc.M1 * f;
-  const float M02 = mc.M02 * f, M12 = mc.M12 * f, LM2 = mc.LM2 * f;
-  float2 g[8];
-  float gz[8];
-  {
-    const float Ltr = L0 * (uxy[1].x + uxy[2].y + uz[4]);
-    g[1].x = mad(M02, uxy[1].x, Ltr);
-    g[2].y = mad(M02, uxy[2].y, Ltr);
-    gz[4] = mad(M02, uz[4], Ltr);
-    const float txy = M0 * (uxy[1].y + uxy[2].x);
-    const float txz = M0 * (uz[1] + uxy[4].x);
-    const float tyz = M0 * (uz[2] + uxy[4].y);
-    g[1].y = txy; gz[1] = txz;
-    g[2].x = txy; gz[2] = tyz;
-    g[4].x = txz; g[4].y = tyz;
-  }
-  {
-    const float Ltr = L1 * (uxy[3].y + uz[5]);
-    const float t = M1 * (uz[3] + uxy[5].y);
-    g[3].x = M1 * uxy[3].x;
-    g[3].y = mad(M12, uxy[3].y, Ltr);
-    gz[3] = t;
-    g[5].x = M1 * uxy[5].x;
-    g[5].y = t;
-    gz[5] = mad(M12, uz[5], Ltr);
-  }
-  {
-    const float Ltr = L1 * (uxy[3].x + uz[6]);
-    const float t = M1 * (uz[3] + uxy[6].x);
-    g[3].x = g[3].x + mad(M12, uxy[3].x, Ltr);
-    g[3].y = mad(M1, uxy[3].y, g[3].y);
-    gz[3] = gz[3] + t;
-    g[6].x = t;
-    g[6].y = M1 * uxy[6].y;
-    gz[6] = mad(M12, uz[6], Ltr);
-  }
-  {
-    const float Ltr = L1 * (uxy[5].x + uxy[6].y);
-    const float t = M1 * (uxy[5].y + uxy[6].x);
-    g[5].x = g[5].x + mad(M12, uxy[5].x, Ltr);
-    g[5].y = g[5].y + t;
-    gz[5] = mad(M1, uz[5], gz[5]);
-    g[6].x = g[6].x + t;
-    g[6].y = g[6].y + mad(M12, uxy[6].y, Ltr);
-    gz[6] = mad(M1, uz[6], gz[6]);
-  }
-  g[7] = __fmul2_rn(make_float2(LM2, LM2), uxy[7]);
-  gz[7] = LM2 * uz[7];
-  g[0] = make_float2(0.0f, 0.0f);
-  gz[0] = 0.0f;
-  walsh_inv2(g);
-  walsh_inv(gz);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    uxy[i] = g[i];
-    uz[i] = gz[i];
-  }
-}
-
 struct GridDev {
   int nx, ny, nz, nnx, nny, nnz;
 };
 
 // Batched periodic applies (homogenization): system bi of the batch reads x, b,
-// y at bi * sx and the cell fields (factors, kept mask, inverse diagonal) of
-// cell bi / nrhs.  On the torus nodes and elements coincide (nnx == nx ...).
+// y at bi * sx and the cell fields (factors, kept bits) of cell bi / nrhs.  On the torus nodes and elements coincide (nnx == nx ...).
+// Systems whose entry of `run` is not 1 are skipped: their y and partials stay.
 struct BatchDev {
-  int nrhs, nzc;         // systems per cell; z-chunks per system
-  int64_t sx, se, sk;    // strides: DOF vectors, element factors, per-cell DOF fields
+  int nrhs;         // systems per cell
+  int64_t sx, se;   // strides: DOF vectors; a cell's element factors and kept bits
+  const int* run;   // null: every system
 };
 
 __device__ __forceinline__ int wrap_index(int a, int n) {
   a %= n;
   return a < 0 ? a + n : a;
+}
+// The same for -1 <= a <= n + 1 without a division (n = 1 wraps twice).
+__device__ __forceinline__ int wrap_near(int a, int n) {
+  a = a < 0 ? a + n : a;
+  a = a >= n ? a - n : a;
+  return a >= n ? a - n : a;
 }
 
 __device__ __forceinline__ double block_sum(double v) {
@@ -337,768 +143,853 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;  // valid in thread 0
 }
 
-// Pencil geometry.  A CTA is PY warps.  Lane l of warp w evaluates the elements
-// (ex, ey, ez) with ex = 31*bx - 1 + l and ey = (PY-1)*by - 1 + w for KZ+1
-// consecutive element layers, marching upward in z.  Contributions are combined
-//   along x by a warp shuffle (an element's +x corners belong to the next lane),
-//   along y through shared memory (a warp's +y corners belong to the next warp),
-//   along z in registers (a layer's +z corners wait for the next step),
-// so lane l >= 1 of warp w >= 1 finishes node (ex, ey, ez) once element layers
-// ez-1 and ez are in.  Lane 0, warp 0 and the first element layer are the halo:
-// recomputed, never written.  One __syncthreads per element layer, no atomics,
-// and a fixed summation order per node (x, then y, then z), so the result is
-// deterministic run to run.
-template <class T>
-struct Pencil;
+// ---------------------------------------------------------------------------
+// The element operator in the modal basis, shared between neighbours.
+//
+// A trilinear element's modes are a tensor product, so the transform of an
+// element is the z-difference and z-sum of the xy-modes of its two faces, and a
+// face's xy-modes are y-sums and y-differences of the x-sums and x-differences
+// of its two node rows.  Marching in z, a face is transformed once and serves
+// the element above and the element below; with several element rows per thread
+// a node row is x-transformed once for the rows on both sides.  The inverse runs
+// the same way back: the top face of one element layer and the bottom face of
+// the next are added as xy-modes, so y- and x-inverse, the exchange between
+// lanes and the hand-over between warps happen once per node layer.  Per element
+// and layer that is about 141 operations (x 12 forward, 6 back; y 12 and 12; z
+// 21 and 30; 39 for the stress; 9 for combining), against 217 when every element
+// transforms its own 24 values and combines 24 results, with half the shuffles.
+
+// V: the type the element rows of a thread are carried in -- two rows packed in
+// a float2 (Blackwell's paired FP32 instructions), or one row as float, double
+// or double-float.
+template <class V>
+struct RowsOf;
 template <>
-struct Pencil<double> {
-  static constexpr int PY = 8, KZ = 16, MINB = 2;
-};
-#ifndef TG_PENCIL_F32_PY
-#define TG_PENCIL_F32_PY 8
-#endif
-#ifndef TG_PENCIL_F32_KZ
-#define TG_PENCIL_F32_KZ 16
-#endif
-#ifndef TG_PENCIL_F32_MINB
-#define TG_PENCIL_F32_MINB 3
-#endif
-template <>
-struct Pencil<float> {
-  static constexpr int PY = TG_PENCIL_F32_PY, KZ = TG_PENCIL_F32_KZ, MINB = TG_PENCIL_F32_MINB;
+struct RowsOf<float2> {
+  using S = float;
+  static constexpr int R = 2, kMaxWarps = 12;
 };
 template <>
-struct Pencil<df> {
-  static constexpr int PY = 8, KZ = 16, MINB = 2;
+struct RowsOf<float> {
+  using S = float;
+  static constexpr int R = 1, kMaxWarps = 12;
+};
+template <>
+struct RowsOf<double> {
+  using S = double;
+  static constexpr int R = 1, kMaxWarps = 12;
+};
+template <>
+struct RowsOf<df> {
+  using S = df;
+  static constexpr int R = 1, kMaxWarps = 12;
 };
 
-template <class T, bool PER = false>
-__device__ __forceinline__ void load_node(const GridDev& g, const T* __restrict__ x, int a, int b,
-                                          int c, T (&v)[3]) {
-  if (PER) {
-    a = wrap_index(a, g.nnx);
-    b = wrap_index(b, g.nny);
-    c = wrap_index(c, g.nnz);
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) {
+  return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);  // a - b, one rounding
+}
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vmad(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+template <class S>
+__device__ __forceinline__ S vadd(S a, S b) { return a + b; }
+template <class S>
+__device__ __forceinline__ S vsub(S a, S b) { return a - b; }
+template <class S>
+__device__ __forceinline__ S vmul(S a, S b) { return a * b; }
+template <class S>
+__device__ __forceinline__ S vmad(S a, S b, S c) { return mad(a, b, c); }
+template <class S>
+__device__ __forceinline__ S vneg(S a) { return -a; }
+template <class V, class S>
+__device__ __forceinline__ V vset(S a) {
+  if constexpr (RowsOf<V>::R == 2)
+    return make_float2(a, a);
+  else
+    return a;
+}
+
+// The modes' stresses of unit-modulus constants times f, in place.  Index bits
+// 1, 2, 4: the mode is linear in x, y, z.  Mode 0 (rigid translation) is not
+// read, and has no stress.  M0 = 3 M1 merges the two gradient blocks that
+// modes 3, 5 and 6 belong to: e.g. mode 3 of u_x gets M1 from T = {x} and 2 M1
+// from T = {y}, and the three shears of those modes share one sum.
+template <class V, class S>
+__device__ __forceinline__ void modal_stress(const ModalT<S>& mc, V f, V (&ux)[8], V (&uy)[8],
+                                             V (&uz)[8]) {
+  const V m0 = vmul(vset<V>(mc.M0), f), m02 = vmul(vset<V>(mc.M02), f);
+  const V l0 = vmul(vset<V>(mc.L0), f);
+  {
+    const V tr = vmul(l0, vadd(vadd(ux[1], uy[2]), uz[4]));
+    ux[1] = vmad(m02, ux[1], tr);
+    uy[2] = vmad(m02, uy[2], tr);
+    uz[4] = vmad(m02, uz[4], tr);
+    ux[2] = uy[1] = vmul(m0, vadd(uy[1], ux[2]));
+    ux[4] = uz[1] = vmul(m0, vadd(uz[1], ux[4]));
+    uy[4] = uz[2] = vmul(m0, vadd(uz[2], uy[4]));
   }
-  if (PER || (a >= 0 && a < g.nnx && b >= 0 && b < g.nny && c >= 0 && c < g.nnz)) {
-    const T* p = x + 3 * ((int64_t(c) * g.nny + b) * g.nnx + a);
-    v[0] = p[0];
-    v[1] = p[1];
-    v[2] = p[2];
+  const V l1 = vmul(vset<V>(mc.L1), f), m1 = vmul(vset<V>(mc.M1), f);
+  {
+    const V tx = vmul(l1, vadd(uy[3], uz[5]));
+    const V ty = vmul(l1, vadd(ux[3], uz[6]));
+    const V tz = vmul(l1, vadd(ux[5], uy[6]));
+    ux[3] = vmad(m0, ux[3], ty);
+    uy[3] = vmad(m0, uy[3], tx);
+    ux[5] = vmad(m0, ux[5], tz);
+    uz[5] = vmad(m0, uz[5], tx);
+    uy[6] = vmad(m0, uy[6], tz);
+    uz[6] = vmad(m0, uz[6], ty);
+    const V sh = vmul(m1, vadd(vadd(uz[3], uy[5]), ux[6]));
+    uz[3] = vmad(m1, uz[3], sh);
+    uy[5] = vmad(m1, uy[5], sh);
+    ux[6] = vmad(m1, ux[6], sh);
+  }
+  const V lm2 = vmul(vset<V>(mc.LM2), f);
+  ux[7] = vmul(lm2, ux[7]);
+  uy[7] = vmul(lm2, uy[7]);
+  uz[7] = vmul(lm2, uz[7]);
+}
+
+// xy-modes of a face from its node rows' own and right-neighbour values.
+template <class V, class S>
+__device__ __forceinline__ void face_modes(const S (&a)[RowsOf<V>::R + 1], const S (&b)[RowsOf<V>::R + 1],
+                                           V (&F)[4]) {
+  if constexpr (RowsOf<V>::R == 2) {
+    const float2 a01 = make_float2(a[0], a[1]), b01 = make_float2(b[0], b[1]);
+    const float2 s01 = vadd(b01, a01), d01 = vsub(b01, a01);
+    const float2 s12 = make_float2(s01.y, b[2] + a[2]), d12 = make_float2(d01.y, b[2] - a[2]);
+    F[0] = vadd(s12, s01);
+    F[1] = vadd(d12, d01);
+    F[2] = vsub(s12, s01);
+    F[3] = vsub(d12, d01);
   } else {
-    v[0] = v[1] = v[2] = T(0);
+    const S s0 = b[0] + a[0], d0 = b[0] - a[0], s1 = b[1] + a[1], d1 = b[1] - a[1];
+    F[0] = s1 + s0;
+    F[1] = d1 + d0;
+    F[2] = s1 - s0;
+    F[3] = d1 - d0;
   }
 }
 
-// Raw loads of layer c for the lane's own column: nodes (ex, ey, c), (ex, ey+1, c)
-// and, for lane 31, (ex+1, ey, c), (ex+1, ey+1, c).  Issued one step ahead so
-// their latency overlaps the current layer's arithmetic.
-template <class T, bool PER = false>
-__device__ __forceinline__ void load_raw(const GridDev& g, const T* __restrict__ x, int ex, int ey,
-                                         int c, int lane, T (&r)[2][2][3]) {
-  load_node<T, PER>(g, x, ex, ey, c, r[0][0]);
-  load_node<T, PER>(g, x, ex, ey + 1, c, r[1][0]);
-  if (lane == 31) {
-    load_node<T, PER>(g, x, ex + 1, ey, c, r[0][1]);
-    load_node<T, PER>(g, x, ex + 1, ey + 1, c, r[1][1]);
-  }
+__device__ __forceinline__ float shfl_at(float v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ double shfl_at(double v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+__device__ __forceinline__ df shfl_at(df v, int l) {
+  return df(__shfl_sync(0xffffffffu, v.hi, l), __shfl_sync(0xffffffffu, v.lo, l));
 }
 
-// The same loads for the non-periodic grid with the column's x/y validity
-// (m[yb][xb]) and base offset hoisted out of the z march: layer c adds
-// 3*c*nnx*nny to the offset and tests only its own z range.
-template <class T, class C>
-__device__ __forceinline__ void load_raw_np(const T* __restrict__ x, int64_t o, int snx, bool vc,
-                                            const bool (&m)[2][2], int lane, C (&r)[2][2][3]) {
-#pragma unroll
-  for (int yb = 0; yb < 2; ++yb)
-#pragma unroll
-    for (int xb = 0; xb < 2; ++xb) {
-      if (xb == 1 && lane != 31) continue;
-      const bool ok = vc && m[yb][xb];
-      const T* p = x + (o + yb * snx + 3 * xb);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) r[yb][xb][k] = ok ? load_c<C>(p[k]) : czero<C>();
-    }
+// Tiling.  A CTA is W warps; lanes run along x, thread rows along y, the march
+// along z.
+//   x: the node columns of all the y strips are numbered in one sequence (strip
+//      by strip), and a warp owns kOwn consecutive ones, so no lane idles at a
+//      row's end; lane 0 is the halo column on the left, and with 30 owned
+//      columns lane 31 only supplies its values (FP64 owns 31: lane 31 loads its
+//      right neighbour itself, a load its arithmetic hides).
+//      At a strip's end the next lane belongs to another strip: the element
+//      column there lies past the grid, its factor is 0.
+//      Periodic cells of at most 32 columns: a row is a group of nx lanes with
+//      no halo, 32 / nx rows side by side in a warp.
+//   y: a warp evaluates R element rows; the node row between two warps is
+//      finished by the lower one, the upper warp's share handed over as x-modes
+//      through shared memory (one barrier per layer).  A CTA finishes W R - 1
+//      node rows.
+//   z: KZ node layers per CTA, and one more element layer below.
+// Every node is finished once, by one thread, in an order that does not depend
+// on the tiling: results are deterministic, and the same under every schedule.
+//
+// Two packed rows (FP32): what a step reads -- the next node layer's three rows,
+// the element factors, the right-hand side and the inverse diagonal -- is copied
+// to shared memory kDepth layers ahead (cp.async, each warp its own copy, so
+// only the warp waits).  One layer ahead in registers left 38 % of the issue
+// slots to DRAM latency (74 us on 256x128x128): 12 warps of 160 registers keep
+// 14 KB per SM in flight, and the latency times the bandwidth needs three times
+// that.  Copies are of consecutive words; rows and layers past the grid are read
+// from its edge, since the elements there have factor 0.
+//
+// Measured per launch, one element at a time -> this kernel: FP32 apply on
+// 256x128x128 71.8 -> 51.3 us (119 MB; issue-bound, 2.4 of 4 instructions per
+// cycle), on 60x20x20 38 -> 5; FP64 apply on 256x128x128 2,340 -> 1,393 us (FP64
+// units busy), on 60x36x28 258 -> 43, on 24x8x8 133 -> 14 (two layers of ~150
+// FP64 instructions at 64 cycles).
+constexpr int kDepth = 3;       // layers copied ahead
+constexpr int kRowWords = 96;  // a copied row: 32 nodes x 3 components
+
+// Words of one layer's copies of one warp: 3 rows of x, 2 rows of factors, and 2
+// rows each of b and the inverse diagonal where the mode reads them.
+template <int MODE>
+__host__ __device__ constexpr int slot_words() {
+  return 3 * kRowWords + 64 + (MODE != kApply ? 2 * kRowWords : 0) +
+         (MODE == kSmooth ? 2 * kRowWords : 0);
 }
 
-// Completes a layer: v[yb][xb][comp] for nodes (ex + xb, ey + yb); the +x nodes
-// come from the next lane (lane 31 loaded its own).
-template <class T>
-__device__ __forceinline__ void finish_layer(int lane, const T (&r)[2][2][3], T (&v)[2][2][3]) {
-#pragma unroll
-  for (int yb = 0; yb < 2; ++yb)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      v[yb][0][k] = r[yb][0][k];
-      const T nb = shfl_down(r[yb][0][k], 1);
-      v[yb][1][k] = lane == 31 ? r[yb][1][k] : nb;
-    }
+// base (the same for every lane) + an unsigned byte offset: one address operand.
+template <class P>
+__device__ __forceinline__ P* at(P* base, unsigned bytes) {
+  using B = typename std::conditional<std::is_const<P>::value, const char, char>::type;
+  return reinterpret_cast<P*>(reinterpret_cast<B*>(base) + bytes);
+}
+__device__ __forceinline__ void copy_word(unsigned dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_word_or_zero(unsigned dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait_ahead() {  // all but the newest kDepth - 1 groups are in
+  asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
 }
 
-// PER: the periodic (torus) grid of a batch of systems (BatchDev); nodes and
-// elements wrap around, so every element exists and the halo lanes read the
-// opposite face.  The non-periodic instantiations compile the PER branches away.
-template <class T, int PY, int KZ, int MINB, int MODE, bool PER = false, class C = T>
-__global__ void __launch_bounds__(32 * PY, MINB) k_fine_op(GridDev g, ModalT<C> mc,
-                                                     const T* __restrict__ ef,
-                                                     const uint8_t* __restrict__ kept,
-                                                     const T* __restrict__ x, const T* __restrict__ b,
-                                                     const T* __restrict__ invdiag, T omega,
-                                                     T* __restrict__ y, double* __restrict__ dot_part,
-                                                     BatchDev bd = BatchDev{}) {
-  __shared__ C sy[2][PY][6][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int ex = blockIdx.x * 31 - 1 + lane;
-  const int ey = blockIdx.y * (PY - 1) - 1 + w;
-  int k0 = blockIdx.z * KZ;
-  if (PER) {
-    const int bi = blockIdx.z / bd.nzc, cell = bi / bd.nrhs;
-    k0 = (blockIdx.z - bi * bd.nzc) * KZ;
+template <class V, class T, int MODE, bool PER>
+__global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
+    k_fine_march(GridDev g, ModalT<typename RowsOf<V>::S> mc, int KZ, int nss,
+                 const T* __restrict__ ef, const uint8_t* __restrict__ kn,
+                 const T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ invdiag,
+                 T omega, T* __restrict__ y, double* __restrict__ dot_part, int guard,
+                 BatchDev bd) {
+  using S = typename RowsOf<V>::S;
+  constexpr int R = RowsOf<V>::R;
+  constexpr bool kXtra = !PER && std::is_same<S, double>::value;  // lane 31 loads its neighbour
+  constexpr int kOwn = kXtra ? 31 : 30;
+  extern __shared__ __align__(16) unsigned char march_smem[];
+  S* const xs = reinterpret_cast<S*>(march_smem);  // [2][W][6][32]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int rows = W * R - 1;
+  if constexpr (PER) {
+    const int bi = blockIdx.z, cell = bi / bd.nrhs;
+    if (bd.run != nullptr && bd.run[bi] != 1) return;  // uniform over the CTA
     x += bi * bd.sx;
     y += bi * bd.sx;
     if (b) b += bi * bd.sx;
     ef += cell * bd.se;
-    if (kept) kept += cell * bd.sk;
-    if (invdiag) invdiag += cell * bd.sk;
+    if (kn) kn += cell * bd.se;
   }
-  const bool own_xy = lane >= 1 && w >= 1 && ex < g.nnx && ey < g.nny;
-  const bool exy_ok = PER || (ex >= 0 && ex < g.nx && ey >= 0 && ey < g.ny);
-  const int64_t exy = PER ? int64_t(wrap_index(ey, g.ny)) * g.nx + wrap_index(ex, g.nx)
-                          : int64_t(ey) * g.nx + ex;
-  // Non-periodic: hoisted column validity and running offsets (nodes: o_x,
-  // outputs: o_y, element factors: o_e).
-  const int64_t plane3 = 3 * int64_t(g.nnx) * g.nny, eplane = int64_t(g.nx) * g.ny;
-  const int snx = 3 * g.nnx;
-  const bool vx0 = ex >= 0 && ex < g.nnx, vx1 = ex + 1 < g.nnx;
-  const bool vy0 = ey >= 0 && ey < g.nny, vy1 = ey + 1 < g.nny;
-  const bool msk[2][2] = {{vx0 && vy0, vx1 && vy0}, {vx0 && vy1, vx1 && vy1}};
-  const int64_t oxy = 3 * (int64_t(ey) * g.nnx + ex);
-  C cur[2][2][3], nxt[2][2][3], raw[2][2][3];
+  // This lane's element column ex, strip ss, and the lanes its x neighbours are in.
+  int ex, ss, rl, ll;
+  bool own_x;
   if constexpr (PER) {
-    load_raw<T, PER>(g, x, ex, ey, k0 - 1, lane, raw);
-  } else {
-    load_raw_np(x, oxy + (k0 - 1) * plane3, snx, k0 - 1 >= 0 && k0 - 1 < g.nnz, msk, lane, raw);
-  }
-  finish_layer(lane, raw, cur);
-  if constexpr (PER)
-    load_raw<T, PER>(g, x, ex, ey, k0, lane, raw);
-  else
-    load_raw_np(x, oxy + k0 * plane3, snx, k0 < g.nnz, msk, lane, raw);
-  C pend[3] = {czero<C>(), czero<C>(), czero<C>()};
-  C dsum = czero<C>();  // this thread's share of x.y: a few dozen nodes, then FP64 across the CTA
-#pragma unroll 1
-  for (int s = 0; s <= KZ; ++s) {
-    const int ez = k0 - 1 + s;
-    finish_layer(lane, raw, nxt);
-    if (s < KZ) {
-      if constexpr (PER)
-        load_raw<T, PER>(g, x, ex, ey, ez + 2, lane, raw);
-      else
-        load_raw_np(x, oxy + (ez + 2) * plane3, snx, ez + 2 < g.nnz, msk, lane, raw);
-    }
-    C ux[8], uy[8], uz[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int xb = c & 1, yb = (c >> 1) & 1, zb = c >> 2;
-      ux[c] = zb ? nxt[yb][xb][0] : cur[yb][xb][0];
-      uy[c] = zb ? nxt[yb][xb][1] : cur[yb][xb][1];
-      uz[c] = zb ? nxt[yb][xb][2] : cur[yb][xb][2];
-    }
-    C f;
-    if constexpr (PER)
-      f = load_c<C>(ef[int64_t(wrap_index(ez, g.nz)) * g.ny * g.nx + exy]);
-    else
-      f = (exy_ok && ez >= 0 && ez < g.nz) ? load_c<C>(ef[ez * eplane + exy]) : czero<C>();
-    if (nonzero(f)) {
-      modal_apply(mc, f, ux, uy, uz);
+    if (g.nx <= 32) {
+      const int ng = 32 / g.nx, gi = lane / g.nx;
+      ex = lane - gi * g.nx;
+      ss = blockIdx.x * ng + gi;
+      own_x = gi < ng && ss < nss;
+      rl = own_x ? gi * g.nx + (ex + 1 == g.nx ? 0 : ex + 1) : lane;
+      ll = own_x ? gi * g.nx + (ex == 0 ? g.nx - 1 : ex - 1) : lane;
+      if (!own_x) ss = 0;
     } else {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) ux[c] = uy[c] = uz[c] = czero<C>();
+      const int nseg = (g.nx + kOwn - 1) / kOwn, seg = blockIdx.x % nseg;
+      ss = blockIdx.x / nseg;
+      const int c = seg * kOwn - 1 + lane;
+      own_x = lane >= 1 && lane <= kOwn && c < g.nx;
+      ex = wrap_index(c, g.nx);
+      rl = lane < 31 ? lane + 1 : lane;
+      ll = lane > 0 ? lane - 1 : lane;
     }
-    // x: add the previous lane's +x corners to this lane's -x corners.
-    C L[2][2][3];  // [yb][zb][comp] at node x = ex
+  } else {
+    const int q = blockIdx.x * kOwn - 1 + lane;
+    ss = q > 0 ? q / g.nnx : 0;
+    ex = q - ss * g.nnx;
+    own_x = lane >= 1 && lane <= kOwn && ss < nss;
+    rl = lane < 31 ? lane + 1 : lane;
+    ll = lane > 0 ? lane - 1 : lane;
+  }
+  const int ey0 = ss * rows - 1 + w * R;  // element rows ey0 .. ey0+R-1, node rows ey0 .. ey0+R
+  const bool vx = PER || (ex >= 0 && ss < nss);
+  const int plane = g.nnx * g.nny, eplane = g.nx * g.ny;
+  int no[R + 1];  // the nodes' indexes within a layer
+  bool rv[R + 1], rown[R + 1];
 #pragma unroll
-    for (int yb = 0; yb < 2; ++yb)
+  for (int i = 0; i <= R; ++i) {
+    const int yr = ey0 + i;
+    rv[i] = vx && (PER || (yr >= 0 && yr < g.nny));
+    rown[i] = own_x && i >= 1 && (i < R || w < W - 1) && yr < g.nny;
+    no[i] = g.nnx * (PER ? wrap_index(yr, g.nny) : yr) + ex;
+  }
+  int eo[R];
+  bool ev[R];
 #pragma unroll
-      for (int zb = 0; zb < 2; ++zb) {
-        const int c0 = (yb << 1) | (zb << 2);
-        L[yb][zb][0] = ux[c0] + shfl_up(ux[c0 | 1], 1);
-        L[yb][zb][1] = uy[c0] + shfl_up(uy[c0 | 1], 1);
-        L[yb][zb][2] = uz[c0] + shfl_up(uz[c0 | 1], 1);
+  for (int j = 0; j < R; ++j) {
+    const int er = ey0 + j;
+    ev[j] = vx && (PER || (ex < g.nx && er >= 0 && er < g.ny));
+    eo[j] = (PER ? wrap_index(er, g.ny) : er) * g.nx + ex;
+  }
+  const int z0 = blockIdx.y * KZ;
+
+  // Copied rows: word 32 j + lane of a row is component (32 j + lane) % 3 of the
+  // lane (32 j + lane) / 3's node, whose strip and clamped (wrapped) row give the
+  // word's offset within a layer.
+  constexpr bool kPipe = R == 2;
+  constexpr int kSlot = kPipe ? slot_words<MODE>() : 0;
+  float* const mine = reinterpret_cast<float*>(xs + 2 * W * 192) + w * (kDepth + 1) * kSlot;
+  const unsigned mine_s = static_cast<unsigned>(__cvta_generic_to_shared(mine));
+  unsigned eb[R];  // bytes; and the bytes to copy: 4, or 0 for an absent element
+  int eok[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    eb[j] = ev[j] ? 4u * unsigned(eo[j]) : 0u;
+    eok[j] = ev[j] ? 4 : 0;
+  }
+  unsigned wo[kPipe ? 3 : 1][kPipe ? 3 : 1];  // bytes
+  if constexpr (kPipe) {
+    const int yc0 = PER ? 0 : ey0;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int word = 32 * j + lane, m = word / 3, k = word - 3 * m;
+      const int exm = __shfl_sync(0xffffffffu, PER ? ex : min(max(ex, 0), g.nnx - 1), m);
+      const int ym = __shfl_sync(0xffffffffu, PER ? ss * rows - 1 + w * R : yc0, m);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const int yr = PER ? wrap_index(ym + i, g.nny) : min(max(ym + i, 0), g.nny - 1);
+        wo[j][i] = 4u * unsigned(3 * (g.nnx * yr + exm) + k);
       }
-    // y: hand the +y corners to the next warp through shared memory.
-    const int buf = s & 1;
+    }
+  }
+  // The copies of step s: node layer ez + 1, factors, b and diagonal of layer ez.
+  auto copy_step = [&](int s) {
+    if constexpr (kPipe) {
+      const int ez = z0 - 1 + s;
+      if (s <= KZ && ez <= g.nnz - 1) {
+        const unsigned st = mine_s + (unsigned(s) % (kDepth + 1)) * (4u * kSlot) + 4u * lane;
+        const float* xl =
+            x + 3 * (plane * (PER ? wrap_near(ez + 1, g.nnz) : min(ez + 1, g.nnz - 1)));
 #pragma unroll
-    for (int zb = 0; zb < 2; ++zb)
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) sy[buf][w][zb * 3 + k][lane] = L[1][zb][k];
-    __syncthreads();
-    C N[2][3];
+          for (int j = 0; j < 3; ++j)
+            copy_word(st + 4 * (i * kRowWords + 32 * j), at(xl, wo[j][i]));
+        const bool vc = PER || (ez >= 0 && ez < g.nz);
+        const float* el = ef + eplane * (PER ? wrap_near(ez, g.nz) : (vc ? ez : 0));
 #pragma unroll
-    for (int zb = 0; zb < 2; ++zb)
+        for (int j = 0; j < 2; ++j)
+          copy_word_or_zero(st + 4 * (3 * kRowWords + 32 * j), at(el, eb[j]), vc ? eok[j] : 0);
+        if (MODE != kApply && s >= 1) {
+          const float *bl = b + 3 * plane * ez, *dl = invdiag + 3 * plane * ez;
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        N[zb][k] = L[0][zb][k] + (w >= 1 ? sy[buf][w - 1][zb * 3 + k][lane] : czero<C>());
-    // z: node layer ez is complete (element layers ez-1 and ez).
-    if (s >= 1 && own_xy && ez < g.nnz) {
-      const int64_t d0 = oxy + ez * plane3;
-      C node_dot = czero<C>();  // x.y over the node's 3 DOFs, accumulated in FP64 below
+          for (int i = 1; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+              const unsigned d = st + 4 * (3 * kRowWords + 64 + (i - 1) * kRowWords + 32 * j);
+              copy_word(d, at(bl, wo[j][i]));
+              if (MODE == kSmooth) copy_word(d + 8 * kRowWords, at(dl, wo[j][i]));
+            }
+        }
+      }
+      copy_commit();
+    }
+  };
+
+  auto load_layer = [&](int c, S (&r)[R + 1][3], S (&e)[R + 1][3]) {
+    const bool vc = PER || (c >= 0 && c < g.nnz);
+    const int o = plane * (PER ? wrap_near(c, g.nnz) : c);
+#pragma unroll
+    for (int i = 0; i <= R; ++i)
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const int64_t d = d0 + k;
-        const bool kk = kept == nullptr || kept[d] != 0;
-        const C ax = pend[k] + N[0][k];
+        r[i][k] = (vc && rv[i]) ? load_c<S>(x[3 * (o + no[i]) + k]) : czero<S>();
+        if constexpr (kXtra)
+          e[i][k] = (lane == 31 && vc && rv[i] && ex + 1 < g.nnx) ? load_c<S>(x[3 * (o + no[i]) + 3 + k])
+                                                                   : czero<S>();
+      }
+  };
+  auto load_f = [&](int c, S (&f)[R]) {
+    const bool vc = PER || (c >= 0 && c < g.nz);
+    const int o = eplane * (PER ? wrap_near(c, g.nz) : c);
+#pragma unroll
+    for (int j = 0; j < R; ++j) f[j] = (vc && ev[j]) ? load_c<S>(ef[o + eo[j]]) : czero<S>();
+  };
+  auto face = [&](const S (&r)[R + 1][3], const S (&e)[R + 1][3], V (&F)[3][4]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      S a[R + 1], nb[R + 1];
+#pragma unroll
+      for (int i = 0; i <= R; ++i) {
+        a[i] = r[i][k];
+        nb[i] = shfl_at(r[i][k], rl);
+        if constexpr (kXtra) nb[i] = lane == 31 ? e[i][k] : nb[i];
+      }
+      face_modes<V, S>(a, nb, F[k]);
+    }
+  };
+
+  // The first chunk of a bounded grid has no element layer below it.
+  const int s0 = (!PER && z0 == 0) ? 1 : 0;
+  S raw[R + 1][3], rext[R + 1][3], keep[R + 1][3];
+  V Fc[3][4], pend[3][4];
+  load_layer(z0 - 1 + s0, raw, rext);
+  face(raw, rext, Fc);
+#pragma unroll
+  for (int i = 0; i <= R; ++i)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) keep[i][k] = raw[i][k];
+  S fn[R];
+  if constexpr (kPipe) {
+#pragma unroll 1
+    for (int q = 0; q < kDepth; ++q) copy_step(s0 + q);
+  } else {
+    load_layer(z0 + s0, raw, rext);
+    load_f(z0 - 1 + s0, fn);
+  }
+  unsigned kbn[R + 1];  // kept bits of the owned rows, requested a step ahead
+  auto load_kb = [&](int s, unsigned (&kb)[R + 1]) {
+    const int ez = z0 - 1 + s;
+#pragma unroll
+    for (int i = 1; i <= R; ++i)
+      kb[i] = kn == nullptr
+                  ? 7u
+                  : (s >= 1 && ez < g.nnz && rown[i] ? unsigned(*at(kn + plane * ez, unsigned(no[i]))) : 0u);
+  };
+  load_kb(s0, kbn);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) pend[k][m] = vset<V>(czero<S>());
+  S dsum = czero<S>();
+
+  // Two steps per pass: this layer's faces become the last layer's without moves.
+#pragma unroll(kPipe ? 2 : 1)
+  for (int s = s0; s <= KZ; ++s) {
+    const int ez = z0 - 1 + s;
+    if (ez > g.nnz - 1) break;  // uniform: the last chunk ends with the grid
+    const bool out_z = s >= 1;
+    const int oz = plane * ez;
+    unsigned kb[R + 1];
+#pragma unroll
+    for (int i = 1; i <= R; ++i) kb[i] = kbn[i];
+    if (s < KZ) load_kb(s + 1, kbn);
+    T bv[R + 1][3], dv[R + 1][3];
+    V f;
+    V Fn[3][4];
+    S knext[R + 1][3];
+    const float* st = nullptr;
+    if constexpr (kPipe) {
+      copy_wait_ahead();
+      __syncwarp();  // every lane's words of this step are in, and the last step's are read
+      copy_step(s + kDepth);
+      st = mine + (s % (kDepth + 1)) * kSlot;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        S a[3], nb[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          a[i] = st[i * kRowWords + 3 * lane + k];
+          nb[i] = st[i * kRowWords + 3 * rl + k];
+        }
+        face_modes<V, S>(a, nb, Fn[k]);
+#pragma unroll
+        for (int i = 1; i < 3; ++i) knext[i][k] = a[i];
+      }
+      f = make_float2(st[3 * kRowWords + lane], st[3 * kRowWords + 32 + lane]);
+    } else {
+      // Requested now, used at the end of the step: right-hand side and inverse
+      // diagonal; and the layer after the next.
+#pragma unroll
+      for (int i = 1; i <= R; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const bool ok = out_z && rown[i];
+          bv[i][k] = (MODE != kApply && ok) ? b[3 * (oz + no[i]) + k] : T(0);
+          dv[i][k] = (MODE == kSmooth && ok) ? invdiag[3 * (oz + no[i]) + k] : T(0);
+        }
+      f = fn[0];
+      face(raw, rext, Fn);
+#pragma unroll
+      for (int i = 1; i <= R; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) knext[i][k] = raw[i][k];
+      if (s < KZ) {
+        load_layer(ez + 2, raw, rext);
+        load_f(ez + 1, fn);
+      }
+    }
+    // z: element modes from the two faces (mode 0 is never used).
+    V u[3][8];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      u[k][0] = vset<V>(czero<S>());
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        if (m > 0) u[k][m] = vadd(Fn[k][m], Fc[k][m]);
+        u[k][m | 4] = vsub(Fn[k][m], Fc[k][m]);
+      }
+    }
+    modal_stress<V, S>(mc, f, u[0], u[1], u[2]);
+    if (guard) {
+      // Values at a node of absent elements only must not reach its neighbours
+      // whatever they are (0 times an infinity or NaN is not 0).
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int m = 1; m < 8; ++m) {
+          if constexpr (R == 2) {
+            u[k][m].x = f.x != 0.0f ? u[k][m].x : 0.0f;
+            u[k][m].y = f.y != 0.0f ? u[k][m].y : 0.0f;
+          } else {
+            u[k][m] = nonzero(f) ? u[k][m] : czero<S>();
+          }
+        }
+    }
+    // Back in z: this layer's bottom face completes node layer ez, its top face
+    // waits; then y.
+    V lo[3][2], up[3][2];  // x-modes of the thread's element rows' lower and upper node rows
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      V P[4];
+      P[0] = vsub(pend[k][0], u[k][4]);
+      pend[k][0] = u[k][4];
+#pragma unroll
+      for (int m = 1; m < 4; ++m) {
+        P[m] = vadd(pend[k][m], vsub(u[k][m], u[k][m | 4]));
+        pend[k][m] = vadd(u[k][m], u[k][m | 4]);
+      }
+      lo[k][0] = vsub(P[0], P[2]);
+      lo[k][1] = vsub(P[1], P[3]);
+      up[k][0] = vadd(P[0], P[2]);
+      up[k][1] = vadd(P[1], P[3]);
+    }
+    S* const buf = xs + (s & 1) * (W * 192);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        if constexpr (R == 2)
+          buf[w * 192 + (2 * k + m) * 32 + lane] = lo[k][m].x;
+        else
+          buf[w * 192 + (2 * k + m) * 32 + lane] = lo[k][m];
+      }
+    // Writes node row i of layer ez from its x-modes r[k][2].
+    auto finish = [&](int i, const S (&r)[3][2]) {
+      S nd = czero<S>();
+      T* const yl = at(y + 3 * int64_t(oz), unsigned(3 * sizeof(T)) * unsigned(no[i]));
+      if constexpr (kPipe) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float* q = st + 3 * kRowWords + 64 + (i - 1) * kRowWords + 3 * lane + k;
+          bv[i][k] = MODE != kApply ? q[0] : 0.0f;
+          dv[i][k] = MODE == kSmooth ? q[2 * kRowWords] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const S right = r[k][0] + r[k][1];
+        const S ax = (r[k][0] - r[k][1]) + shfl_at(right, ll);
+        if (!(out_z && rown[i])) continue;
+        const bool kk = ((kb[i] >> k) & 1u) != 0u;
         T out;
         if constexpr (MODE == kApply) {
           out = kk ? store_t(ax) : T(0);
-          node_dot = node_dot + cur[0][0][k] * load_c<C>(out);
+          nd = nd + keep[i][k] * load_c<S>(out);
         } else if constexpr (MODE == kResidual) {
-          // Residual in the storage type: a double-float sum is rounded to FP64 once.
-          out = kk ? T(b[d] - store_t(ax)) : T(0);
+          out = kk ? T(bv[i][k] - store_t(ax)) : T(0);
         } else {
-          out = kk ? T(store_t(cur[0][0][k]) + omega * invdiag[d] * (b[d] - store_t(ax))) : T(0);
+          out = kk ? T(store_t(keep[i][k]) + omega * dv[i][k] * (bv[i][k] - store_t(ax))) : T(0);
+          nd = nd + load_c<S>(bv[i][k]) * load_c<S>(out);
         }
-        y[d] = out;
+        yl[k] = out;
       }
-      if constexpr (MODE == kApply) dsum = dsum + node_dot;
+      if constexpr (MODE != kResidual) dsum = dsum + nd;
+    };
+    if constexpr (R == 2) {
+      S r1[3][2];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) r1[k][m] = up[k][m].x + lo[k][m].y;
+      finish(1, r1);
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) pend[k] = N[1][k];
-#pragma unroll
-    for (int yb = 0; yb < 2; ++yb)
-#pragma unroll
-      for (int xb = 0; xb < 2; ++xb)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) cur[yb][xb][k] = nxt[yb][xb][k];
-  }
-  if (MODE == kApply && dot_part != nullptr) {
-    const double sum = block_sum(double(store_t(dsum)));
-    if (threadIdx.x == 0)
-      dot_part[(int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = sum;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Column-blocked FP32 operator (the mixed form's fine level).
-//
-// The pencil kernel above spends most of its issue slots on moving node values
-// between lanes and warps and recomputes 37% of its element slots as halo.  This
-// schedule keeps more of the combine in registers:
-//   * lanes run along x: lane l evaluates the element column ex = x0 - 1 + l and
-//     finishes node column ex (lanes 1..30; lane 0 and lane 31 are halo);
-//   * each thread marches a column of Y element rows in y: the y-combine of two
-//     consecutive element rows is a register add inside the thread, and an
-//     element's inputs share the node row with the element below it;
-//   * W warps stack in y; the node row between two warps is finished by the
-//     lower warp with the upper warp's contribution handed over through shared
-//     memory (one __syncthreads per element layer), so a CTA recomputes one
-//     element row of halo in y, not one per warp;
-//   * the CTA marches KZ element layers in z (KZ chosen per grid so the chunks
-//     divide the node layers evenly), completing node layers in registers.
-// Per node the summation order is fixed (y inside the thread, then x across
-// lanes, then the warp hand-over, then z), so the apply is deterministic.
-// Node values of layer ez+2 are loaded while layer ez is evaluated.
-template <int Y, int W>
-struct ColShape {
-  static constexpr int kRows = W * Y - 1;  // node rows a CTA finishes
-  static constexpr int kMinB = 12 / W > 0 ? 12 / W : 1;  // ~12 resident warps per SM
-};
-
-template <int Y, int W, int MODE, bool PK>
-__global__ void __launch_bounds__(32 * W, (ColShape<Y, W>::kMinB))
-    k_fine_op_col(GridDev g, ModalT<float> mc, int KZ, const float* __restrict__ ef,
-                  const uint8_t* __restrict__ kept, const uint8_t* __restrict__ kn,
-                  const float* __restrict__ x, const float* __restrict__ b,
-                  const float* __restrict__ invdiag, float omega, float* __restrict__ y,
-                  double* __restrict__ dot_part) {
-  __shared__ float xs[2][W][6][32];
-  // Smoothing with dot_part set: partial b . y as well (the PCG's r . z).
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int ex = blockIdx.x * 30 - 1 + lane;
-  const int ey0 = blockIdx.y * ColShape<Y, W>::kRows - 1 + w * Y;  // element rows ey0 .. ey0+Y-1
-  const int z0 = blockIdx.z * KZ;
-  const int64_t plane = int64_t(g.nnx) * g.nny, eplane = int64_t(g.nx) * g.ny;
-  const bool vx = ex >= 0 && ex < g.nnx;
-  const bool own_x = lane >= 1 && lane <= 30 && ex < g.nnx;
-  bool rv[Y + 1];
-#pragma unroll
-  for (int i = 0; i <= Y; ++i) rv[i] = vx && ey0 + i >= 0 && ey0 + i < g.nny;
-  bool ev[Y];
-#pragma unroll
-  for (int j = 0; j < Y; ++j) ev[j] = ex >= 0 && ex < g.nx && ey0 + j >= 0 && ey0 + j < g.ny;
-  // Node rows i = 1..Y of the column are this thread's (row Y only below the
-  // top warp); row 0 belongs to the warp below.
-  bool ro[Y + 1];
-#pragma unroll
-  for (int i = 0; i <= Y; ++i) ro[i] = own_x && i >= 1 && (i < Y || w < W - 1) && ey0 + i < g.nny;
-  const int64_t col = int64_t(ey0) * g.nnx + ex;  // node (ex, ey0) in a layer
-  const int64_t ecol = int64_t(ey0) * g.nx + ex;   // element (ex, ey0) in a layer
-
-  auto load_layer = [&](int c, float (&r)[Y + 1][3]) {
-    const bool vc = c >= 0 && c < g.nnz;
-    const float* p = x + 3 * (int64_t(c) * plane + col);
-#pragma unroll
-    for (int i = 0; i <= Y; ++i)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) r[i][k] = (vc && rv[i]) ? p[3 * i * g.nnx + k] : 0.0f;
-  };
-  // Element factors of layer c (0 outside the grid).
-  auto load_f = [&](int c, float (&f)[Y]) {
-    const bool vc = c >= 0 && c < g.nz;
-#pragma unroll
-    for (int j = 0; j < Y; ++j)
-      f[j] = (vc && ev[j]) ? ef[int64_t(c) * eplane + ecol + int64_t(j) * g.nx] : 0.0f;
-  };
-  // Kept bits of the owned node rows of layer c (bit k: DOF k kept; all kept
-  // without a mask).
-  auto load_kb = [&](int c, unsigned (&kb)[Y + 1]) {
-    const bool vc = c >= 0 && c < g.nnz;
-#pragma unroll
-    for (int i = 1; i <= Y; ++i)
-      kb[i] = kn == nullptr ? 7u
-                            : ((vc && ro[i]) ? unsigned(kn[int64_t(c) * plane + col + int64_t(i) * g.nnx])
-                                             : 0u);
-  };
-
-  float cur[Y + 1][3], nxt[Y + 1][3], raw[Y + 1][3];
-  load_layer(z0 - 1, cur);
-  load_layer(z0, nxt);
-  float fn[Y];
-  load_f(z0 - 1, fn);
-  unsigned kbn[Y + 1];
-  load_kb(z0 - 1, kbn);
-  float pend[Y + 1][3];
-#pragma unroll
-  for (int i = 0; i <= Y; ++i) pend[i][0] = pend[i][1] = pend[i][2] = 0.0f;
-  float dsum = 0.0f;
-
-  // The right-hand side and inverse diagonal of node row i, layer c (smoothing
-  // and residual modes), requested an element ahead of their use.
-  auto load_bd = [&](int i, int c, float (&bv)[3], float (&dv)[3]) {
-    const bool ok = c >= 0 && c < g.nnz && ro[i];
-    const int64_t d0 = 3 * (int64_t(c) * plane + col + int64_t(i) * g.nnx);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      bv[k] = (MODE != kApply && ok) ? b[d0 + k] : 0.0f;
-      dv[k] = (MODE == kSmooth && ok) ? invdiag[d0 + k] : 0.0f;
-    }
-  };
-  // Writes node row i of layer ez from its finished sum ax.
-  auto emit = [&](int i, int ez, unsigned kb, const float (&ax)[3], const float (&bv)[3],
-                  const float (&dv)[3]) {
-    const int64_t d0 = 3 * (int64_t(ez) * plane + col + int64_t(i) * g.nnx);
-    float nd = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int64_t d = d0 + k;
-      const bool kk = kn != nullptr ? ((kb >> k) & 1u) != 0u : (kept == nullptr || kept[d] != 0);
-      float out;
-      if constexpr (MODE == kApply) {
-        out = kk ? ax[k] : 0.0f;
-        nd = fmaf(cur[i][k], out, nd);
-      } else if constexpr (MODE == kResidual) {
-        out = kk ? bv[k] - ax[k] : 0.0f;
-      } else {
-        out = kk ? cur[i][k] + omega * dv[k] * (bv[k] - ax[k]) : 0.0f;
-        nd = fmaf(bv[k], out, nd);
-      }
-      y[d] = out;
-    }
-    if constexpr (MODE != kResidual) dsum += nd;
-  };
-
-#pragma unroll 1
-  for (int s = 0; s <= KZ; ++s) {
-    const int ez = z0 - 1 + s;
-    if (s < KZ) load_layer(ez + 2, raw);
-    float f[Y];
-    unsigned kb[Y + 1];
-#pragma unroll
-    for (int j = 0; j < Y; ++j) f[j] = fn[j];
-#pragma unroll
-    for (int i = 1; i <= Y; ++i) kb[i] = kbn[i];
-    if (s < KZ) {
-      load_f(ez + 1, fn);
-      load_kb(ez + 1, kbn);
-    }
-    const bool out_z = s >= 1 && ez < g.nnz;
-    float bv[3], dv[3];
-    load_bd(1, out_z ? ez : -1, bv, dv);
-    // x + 1 node values of the element's lower row (cur, nxt layers).
-    float c1[3], n1[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      c1[k] = shfl_down(cur[0][k], 1);
-      n1[k] = shfl_down(nxt[0][k], 1);
-    }
-    float C[2][2][3];  // the previous element's +y corners [cx][cz][comp]
-#pragma unroll
-    for (int j = 0; j < Y; ++j) {
-      float c1u[3], n1u[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        c1u[k] = shfl_down(cur[j + 1][k], 1);
-        n1u[k] = shfl_down(nxt[j + 1][k], 1);
-      }
-      // corner c = xb | yb << 1 | zb << 2
-      float ux[8] = {cur[j][0], c1[0], cur[j + 1][0], c1u[0], nxt[j][0], n1[0], nxt[j + 1][0], n1u[0]};
-      float uy[8] = {cur[j][1], c1[1], cur[j + 1][1], c1u[1], nxt[j][1], n1[1], nxt[j + 1][1], n1u[1]};
-      float uz[8] = {cur[j][2], c1[2], cur[j + 1][2], c1u[2], nxt[j][2], n1[2], nxt[j + 1][2], n1u[2]};
-      if (f[j] != 0.0f) {
-        if constexpr (PK) {
-          float2 uxy[8];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) uxy[c] = make_float2(ux[c], uy[c]);
-          modal_apply_xy(mc, f[j], uxy, uz);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            ux[c] = uxy[c].x;
-            uy[c] = uxy[c].y;
-          }
-        } else {
-          modal_apply(mc, f[j], ux, uy, uz);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) ux[c] = uy[c] = uz[c] = 0.0f;
-      }
-      // Node row j: the previous element's +y corners and this element's -y
-      // corners, then the x-combine with the lane below.
-      float T[2][2][3];
-#pragma unroll
-      for (int cx = 0; cx < 2; ++cx)
-#pragma unroll
-        for (int cz = 0; cz < 2; ++cz) {
-          const int c0 = cx | (cz << 2), c1i = cx | 2 | (cz << 2);
-          T[cx][cz][0] = j > 0 ? C[cx][cz][0] + ux[c0] : ux[c0];
-          T[cx][cz][1] = j > 0 ? C[cx][cz][1] + uy[c0] : uy[c0];
-          T[cx][cz][2] = j > 0 ? C[cx][cz][2] + uz[c0] : uz[c0];
-          C[cx][cz][0] = ux[c1i];
-          C[cx][cz][1] = uy[c1i];
-          C[cx][cz][2] = uz[c1i];
-        }
-      float N[2][3];
-#pragma unroll
-      for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) N[cz][k] = T[0][cz][k] + shfl_up(T[1][cz][k], 1);
-      if (j == 0) {
-#pragma unroll
-        for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) xs[s & 1][w][cz * 3 + k][lane] = N[cz][k];
-      } else {
-        float ax[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          ax[k] = pend[j][k] + N[0][k];
-          pend[j][k] = N[1][k];
-        }
-        if (out_z && ro[j]) emit(j, ez, kb[j], ax, bv, dv);
-        load_bd(j + 1, out_z ? ez : -1, bv, dv);
-      }
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        c1[k] = c1u[k];
-        n1[k] = n1u[k];
-      }
-    }
-    // Node row Y: this thread's top element's +y corners and the next warp's
-    // bottom element's -y corners (through shared memory).
-    float NY[2][3];
-#pragma unroll
-    for (int cz = 0; cz < 2; ++cz)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) NY[cz][k] = C[0][cz][k] + shfl_up(C[1][cz][k], 1);
     __syncthreads();
     if (w < W - 1) {
-      float ax[3];
+      S r2[3][2];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        ax[k] = pend[Y][k] + (NY[0][k] + xs[s & 1][w + 1][k][lane]);
-        pend[Y][k] = NY[1][k] + xs[s & 1][w + 1][3 + k][lane];
-      }
-      if (out_z && ro[Y]) emit(Y, ez, kb[Y], ax, bv, dv);
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const S hi = buf[(w + 1) * 192 + (2 * k + m) * 32 + lane];
+          if constexpr (R == 2)
+            r2[k][m] = up[k][m].y + hi;
+          else
+            r2[k][m] = up[k][m] + hi;
+        }
+      finish(R, r2);
     }
 #pragma unroll
-    for (int i = 0; i <= Y; ++i)
+    for (int k = 0; k < 3; ++k)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        cur[i][k] = nxt[i][k];
-        nxt[i][k] = raw[i][k];
+      for (int m = 0; m < 4; ++m) Fc[k][m] = Fn[k][m];
+#pragma unroll
+    for (int i = 1; i <= R; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) keep[i][k] = knext[i][k];
+  }
+  if constexpr (MODE != kResidual) {
+    if (dot_part != nullptr) {
+      const double sum = block_sum(double(store_t(dsum)));
+      if (threadIdx.x == 0)
+        dot_part[(int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = sum;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ schedules
+namespace {
+
+struct MarchTile {
+  int W, kz;  // warps per CTA, node layers per CTA
+};
+
+// SM cycles of one warp step (a layer of R element rows): kBusy while the SM's
+// pipes are full, kChain for a warp that has them to itself, kStart to launch a
+// CTA and load its first layers.  FP64: a warp instruction takes 64 cycles on its
+// scheduler whatever its active lanes, 19 when four schedulers share the SM's
+// units (measured), and a step has about 150.
+template <class V>
+struct StepCost;
+template <>
+struct StepCost<float2> {
+  static constexpr double kBusy = 150.0, kChain = 900.0, kStart = 3000.0;
+};
+template <>
+struct StepCost<float> {
+  static constexpr double kBusy = 110.0, kChain = 800.0, kStart = 3000.0;
+};
+template <>
+struct StepCost<double> {
+  static constexpr double kBusy = 2900.0, kChain = 9600.0, kStart = 4000.0;
+};
+template <>
+struct StepCost<df> {
+  static constexpr double kBusy = 650.0, kChain = 6000.0, kStart = 4000.0;
+};
+constexpr int kSms = 152;
+
+template <class V>
+dim3 march_grid(int nnx, int nny, int nnz, int nsys, bool per, const MarchTile& t) {
+  constexpr int R = RowsOf<V>::R;
+  const int rows = t.W * R - 1, nss = (nny + rows - 1) / rows;
+  int64_t gx;
+  if (!per) {
+    const int own = std::is_same<V, double>::value ? 31 : 30;
+    gx = (int64_t(nnx) * nss + own - 1) / own;
+  } else if (nnx <= 32) {
+    gx = (nss + 32 / nnx - 1) / (32 / nnx);
+  } else {
+    gx = int64_t(nss) * ((nnx + 29) / 30);
+  }
+  return dim3(unsigned(gx), unsigned((nnz + t.kz - 1) / t.kz), unsigned(nsys));
+}
+
+// The tile with the least modelled time.  CTAs spread over the SMs and follow
+// one another as they end, so the fullest SM runs ceil(CTAs / SMs) of them, as
+// many together as its registers hold; a CTA's march takes kz + 1 steps.  Small
+// grids get short marches over many SMs, large ones long marches with little
+// halo and no nearly empty last round.
+template <class V>
+double march_cost(const MarchTile& t, const dim3& d) {
+  using C = StepCost<V>;
+  const int64_t ctas = int64_t(d.x) * d.y * d.z;
+  const double res = std::max(1, RowsOf<V>::kMaxWarps / t.W);
+  const double per_sm = double((ctas + kSms - 1) / kSms), rounds = std::ceil(per_sm / res);
+  return std::max(per_sm * t.W * (t.kz + 1) * C::kBusy, rounds * (t.kz + 1) * C::kChain) +
+         rounds * C::kStart;
+}
+
+template <class V>
+MarchTile march_tile(int nnx, int nny, int nnz, int nsys, bool per) {
+  MarchTile best{4, 8};
+  double best_cost = 1e300;
+  for (int W : {2, 3, 4, 5, 6, 8, 10, 12}) {
+    if (W > RowsOf<V>::kMaxWarps) break;
+    for (int target : {1, 2, 3, 4, 6, 8, 11, 16, 22, 32, 43, 64}) {
+      const int chunks = (nnz + target - 1) / target;
+      const MarchTile t{W, (nnz + chunks - 1) / chunks};
+      const double c = march_cost<V>(t, march_grid<V>(nnx, nny, nnz, nsys, per, t));
+      if (c < best_cost) {
+        best_cost = c;
+        best = t;
       }
+      if (target >= nnz) break;
+    }
   }
-  if (MODE != kResidual && dot_part != nullptr) {
-    const double sum = block_sum(double(dsum));
-    if (threadIdx.x == 0)
-      dot_part[(int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = sum;
+  return best;
+}
+
+template <class V, class T, int MODE, bool PER>
+void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalConsts& c,
+                  const T* ef, const uint8_t* kn, const T* x, const T* b, const T* invdiag,
+                  T omega, T* y, double* dot_part, const BatchDev& bd, cudaStream_t s) {
+  using S = typename RowsOf<V>::S;
+  const dim3 grid = march_grid<V>(gd.nnx, gd.nny, gd.nnz, nsys, PER, t);
+  const int rows = t.W * RowsOf<V>::R - 1, nss = (gd.nny + rows - 1) / rows;
+  const size_t smem = size_t(2) * t.W * 192 * sizeof(S) +
+                      (RowsOf<V>::R == 2 ? size_t(t.W) * (kDepth + 1) * slot_words<MODE>() * 4 : 0);
+  if constexpr (RowsOf<V>::R == 2) {
+    // More than the default 48 KB: once per process and mode (any thread may be
+    // first; the attribute is the same).
+    static std::atomic<bool> done{false};
+    if (!done.load()) {
+      constexpr int most = RowsOf<V>::kMaxWarps * (2 * 192 + (kDepth + 1) * slot_words<MODE>()) * 4;
+      TG_CUDA(cudaFuncSetAttribute(k_fine_march<V, T, MODE, PER>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      done.store(true);
+    }
   }
+  // Only the public apply takes values at nodes of absent elements; within the
+  // solver (a kept mask) they are zeros.
+  const int guard = kn == nullptr ? 1 : 0;
+  k_fine_march<V, T, MODE, PER><<<grid, 32 * t.W, smem, s>>>(
+      gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b, invdiag, omega, y, dot_part, guard, bd);
+  TG_LAUNCH_CHECK();
 }
 
-// Tile shapes of the column kernel (Y element rows per thread, W warps per CTA)
-// and the z-chunk target; the shape is picked per grid (fine_op_col_shape).
-struct ColCfg {
-  int shape;  // index into kColShapes
-  int kz;     // element layers per CTA
-};
-struct ColShapeDesc {
-  int Y, W;
-};
-constexpr ColShapeDesc kColShapes[] = {{4, 4}, {6, 4}, {3, 4}, {2, 8}};
-constexpr int kNumColShapes = 8;  // shapes 4..7: the same tiles with the packed (x, y) arithmetic
-
-static dim3 col_grid(const Grid& g, const ColCfg& c) {
-  const ColShapeDesc d = kColShapes[c.shape % 4];
-  const int rows = d.W * d.Y - 1;
-  return dim3((g.nnx + 29) / 30, (g.nny + rows - 1) / rows, (g.nnz + c.kz - 1) / c.kz);
+template <class V, class T>
+void launch_march_mode(int mode, const Grid& g, const MarchTile& t, const ModalConsts& c,
+                       const T* ef, const uint8_t* kn, const T* x, const T* b, const T* invdiag,
+                       T omega, T* y, double* dot_part, int* nblocks_out, cudaStream_t s) {
+  const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
+  if (nblocks_out) {
+    const dim3 d = march_grid<V>(g.nnx, g.nny, g.nnz, 1, false, t);
+    *nblocks_out = int(d.x * d.y);
+  }
+  if (mode == kApply)
+    launch_march<V, T, kApply, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot_part,
+                                      BatchDev{}, s);
+  else if (mode == kResidual)
+    launch_march<V, T, kResidual, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, nullptr,
+                                         BatchDev{}, s);
+  else
+    launch_march<V, T, kSmooth, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot_part,
+                                       BatchDev{}, s);
 }
 
-template <class T>
-static dim3 pencil_grid(const Grid& g) {
-  using P = Pencil<T>;
-  return dim3((g.nnx + 30) / 31, (g.nny + P::PY - 2) / (P::PY - 1), (g.nnz + P::KZ - 1) / P::KZ);
-}
+// Warps per CTA of the FP32 tile shapes (two packed element rows per thread).
+constexpr int kShapeWarps[] = {2, 3, 4, 5, 6, 8, 10, 12};
+constexpr int kNumShapes = 8;
+constexpr int kTunedMinKz = 8;  // shortest z-chunk of a stored or forced FP32 schedule
 
-// Smallest z-chunk the column schedule uses: bounds the partial-sum count.
-constexpr int kColMinKz = 8;
+int blocks_of(const dim3& d) { return int(d.x * d.y); }
+}  // namespace
 
 int fine_op_blocks(const Grid& g, bool fp64) {
-  const dim3 d = fp64 ? pencil_grid<double>(g) : pencil_grid<float>(g);
-  int n = int(d.x * d.y * d.z);
-  if (!fp64)
-    for (int sh = 0; sh < kNumColShapes; ++sh) {
-      const dim3 c = col_grid(g, ColCfg{sh, kColMinKz});
-      n = std::max(n, int(c.x * c.y * c.z));
-    }
+  if (fp64)
+    return blocks_of(march_grid<double>(g.nnx, g.nny, g.nnz, 1, false,
+                                        march_tile<double>(g.nnx, g.nny, g.nnz, 1, false)));
+  int n = std::max(blocks_of(march_grid<float2>(g.nnx, g.nny, g.nnz, 1, false,
+                                                march_tile<float2>(g.nnx, g.nny, g.nnz, 1, false))),
+                   blocks_of(march_grid<float>(g.nnx, g.nny, g.nnz, 1, false,
+                                               march_tile<float>(g.nnx, g.nny, g.nnz, 1, false))));
+  for (int W : kShapeWarps)
+    n = std::max(n, blocks_of(march_grid<float2>(g.nnx, g.nny, g.nnz, 1, false,
+                                                 MarchTile{W, kTunedMinKz})));
   return n;
 }
 
-// z-chunk length: chunks of at most `target` element layers that divide the
-// node layers evenly (fewest chunks, then the shortest chunk that covers).
-static int even_kz(int nnz, int target) {
-  const int chunks = std::max(1, (nnz + target - 1) / target);
-  return std::max(kColMinKz, (nnz + chunks - 1) / chunks);
-}
-
 FineSchedule default_fine_schedule(const Grid& g) {
+  const MarchTile t = march_tile<float2>(g.nnx, g.nny, g.nnz, 1, false);
   FineSchedule s;
   s.kind = FineSchedule::kColumn;
-  s.shape = 0;
-  s.kz = even_kz(g.nnz, 32);
+  s.shape = int(std::find(kShapeWarps, kShapeWarps + kNumShapes, t.W) - kShapeWarps);
+  s.kz = t.kz;
   return s;
 }
 
-int fine_schedule_shapes() { return kNumColShapes; }
+int fine_schedule_shapes() { return kNumShapes; }
 
 bool fine_schedule_valid(const FineSchedule& s) {
   if (s.kind == FineSchedule::kPencil) return true;
-  return s.kind == FineSchedule::kColumn && s.shape >= 0 && s.shape < kNumColShapes &&
-         s.kz >= kColMinKz && s.kz <= 4096;
-}
-
-template <int Y, int W, int MODE, bool PK>
-static void launch_col(const Grid& g, const ColCfg& cc, const ModalConsts& c, const float* ef,
-                       const uint8_t* kept, const uint8_t* kn, const float* x, const float* b,
-                       const float* invdiag, float omega, float* y, double* dot_part,
-                       cudaStream_t s) {
-  const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
-  k_fine_op_col<Y, W, MODE, PK><<<col_grid(g, cc), 32 * W, 0, s>>>(
-      gd, to_modal<float>(c), cc.kz, ef, kept, kn, x, b, invdiag, omega, y, dot_part);
-  TG_LAUNCH_CHECK();
-}
-
-template <int MODE>
-static void launch_col_shape(const Grid& g, const ColCfg& cc, const ModalConsts& c,
-                             const float* ef, const uint8_t* kept, const uint8_t* kn,
-                             const float* x, const float* b, const float* invdiag, float omega,
-                             float* y, double* dot_part, cudaStream_t s) {
-  switch (cc.shape) {
-    case 0:
-      launch_col<4, 4, MODE, false>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 1:
-      launch_col<6, 4, MODE, false>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 2:
-      launch_col<3, 4, MODE, false>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 3:
-      launch_col<2, 8, MODE, false>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 4:
-      launch_col<4, 4, MODE, true>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 5:
-      launch_col<6, 4, MODE, true>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case 6:
-      launch_col<3, 4, MODE, true>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    default:
-      launch_col<2, 8, MODE, true>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-  }
-}
-
-template <class T, int MODE>
-static void launch_mode(const Grid& g, const ModalConsts& c, const T* ef, const uint8_t* kept,
-                        const T* x, const T* b, const T* invdiag, T omega, T* y,
-                        double* dot_part, cudaStream_t s) {
-  using P = Pencil<T>;
-  const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
-  k_fine_op<T, P::PY, P::KZ, P::MINB, MODE><<<pencil_grid<T>(g), 32 * P::PY, 0, s>>>(
-      gd, to_modal<T>(c), ef, kept, x, b, invdiag, omega, y, dot_part);
-  TG_LAUNCH_CHECK();
+  return s.kind == FineSchedule::kColumn && s.shape >= 0 && s.shape < kNumShapes &&
+         s.kz >= kTunedMinKz && s.kz <= 4096;
 }
 
 template <class T>
-void launch_fine_op(int mode, const Grid& g, const ModalConsts& c, const T* ef,
-                    const uint8_t* kept, const T* x, const T* b, const T* invdiag, T omega,
-                    T* y, double* dot_part, int* nblocks_out, cudaStream_t s,
-                    const uint8_t* kn) {
+void launch_fine_op(int mode, const Grid& g, const ModalConsts& c, const T* ef, const uint8_t* kn,
+                    const T* x, const T* b, const T* invdiag, T omega, T* y, double* dot_part,
+                    int* nblocks_out, cudaStream_t s) {
   if constexpr (std::is_same<T, float>::value) {
-    launch_fine_op_sched(fine_schedule_for(g, mode), mode, g, c, ef, kept, x, b, invdiag, omega, y,
-                         dot_part, nblocks_out, s, kn);
-    return;
-  }
-  if (nblocks_out) {
-    const dim3 d = pencil_grid<T>(g);
-    *nblocks_out = int(d.x * d.y * d.z);
-  }
-  switch (mode) {
-    case kApply:
-      launch_mode<T, kApply>(g, c, ef, kept, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case kResidual:
-      launch_mode<T, kResidual>(g, c, ef, kept, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    default:
-      launch_mode<T, kSmooth>(g, c, ef, kept, x, b, invdiag, omega, y, dot_part, s);
+    launch_fine_op_sched(fine_schedule_for(g, mode), mode, g, c, ef, kn, x, b, invdiag, omega, y,
+                         dot_part, nblocks_out, s);
+  } else {
+    launch_march_mode<double, double>(mode, g, march_tile<double>(g.nnx, g.nny, g.nnz, 1, false),
+                                      c, ef, kn, x, b, invdiag, omega, y, dot_part, nblocks_out,
+                                      s);
   }
 }
 
 // The FP32 operator under an explicit schedule (the autotuner times candidates
 // through this without touching the process-wide table).
 void launch_fine_op_sched(const FineSchedule& fs, int mode, const Grid& g, const ModalConsts& c,
-                          const float* ef, const uint8_t* kept, const float* x, const float* b,
+                          const float* ef, const uint8_t* kn, const float* x, const float* b,
                           const float* invdiag, float omega, float* y, double* dot_part,
-                          int* nblocks_out, cudaStream_t s, const uint8_t* kn) {
-  using T = float;
-  {
-    if (fs.kind == FineSchedule::kColumn) {
-      const ColCfg cc{fs.shape, fs.kz};
-      if (nblocks_out) {
-        const dim3 d = col_grid(g, cc);
-        *nblocks_out = int(d.x * d.y * d.z);
-      }
-      if (mode == kApply)
-        launch_col_shape<kApply>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      else if (mode == kResidual)
-        launch_col_shape<kResidual>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      else
-        launch_col_shape<kSmooth>(g, cc, c, ef, kept, kn, x, b, invdiag, omega, y, dot_part, s);
-      return;
-    }
-  }
-  // The pencil kernel has no fused b . y: its partials come from a dot kernel.
-  if (nblocks_out) {
-    const dim3 d = pencil_grid<T>(g);
-    *nblocks_out = mode == kSmooth && dot_part != nullptr ? kRedBlocks : int(d.x * d.y * d.z);
-  }
-  switch (mode) {
-    case kApply:
-      launch_mode<T, kApply>(g, c, ef, kept, x, b, invdiag, omega, y, dot_part, s);
-      break;
-    case kResidual:
-      launch_mode<T, kResidual>(g, c, ef, kept, x, b, invdiag, omega, y, nullptr, s);
-      break;
-    default:
-      launch_mode<T, kSmooth>(g, c, ef, kept, x, b, invdiag, omega, y, nullptr, s);
-      if (dot_part != nullptr) launch_dot_partials_f(b, y, g.ndof, dot_part, s);
-  }
+                          int* nblocks_out, cudaStream_t s) {
+  if (fs.kind == FineSchedule::kColumn)
+    launch_march_mode<float2, float>(mode, g, MarchTile{kShapeWarps[fs.shape], fs.kz}, c, ef, kn,
+                                     x, b, invdiag, omega, y, dot_part, nblocks_out, s);
+  else
+    launch_march_mode<float, float>(mode, g, march_tile<float>(g.nnx, g.nny, g.nnz, 1, false), c,
+                                    ef, kn, x, b, invdiag, omega, y, dot_part, nblocks_out, s);
 }
 
 // The FP64 residual y = b - A x evaluated in double-float arithmetic (tg_df.h):
 // FP64 inputs and output, about 48 significant bits inside, on the FP32 pipe.
 void launch_fine_residual_df(const Grid& g, const ModalConsts& c, const double* ef,
-                             const uint8_t* kept, const double* x, const double* b, double* y,
+                             const uint8_t* kn, const double* x, const double* b, double* y,
                              cudaStream_t s) {
-  using P = Pencil<df>;
   const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
-  const dim3 grid((g.nnx + 30) / 31, (g.nny + P::PY - 2) / (P::PY - 1), (g.nnz + P::KZ - 1) / P::KZ);
-  k_fine_op<double, P::PY, P::KZ, P::MINB, kResidual, false, df><<<grid, 32 * P::PY, 0, s>>>(
-      gd, to_modal<df>(c), ef, kept, x, b, nullptr, 0.0, y, nullptr);
-  TG_LAUNCH_CHECK();
+  launch_march<df, double, kResidual, false>(gd, march_tile<df>(g.nnx, g.nny, g.nnz, 1, false), 1,
+                                             c, ef, kn, x, b, nullptr, 0.0, y, nullptr, BatchDev{},
+                                             s);
 }
 
 template void launch_fine_op<double>(int, const Grid&, const ModalConsts&, const double*,
                                      const uint8_t*, const double*, const double*,
                                      const double*, double, double*, double*, int*,
-                                     cudaStream_t, const uint8_t*);
+                                     cudaStream_t);
 template void launch_fine_op<float>(int, const Grid&, const ModalConsts&, const float*,
                                     const uint8_t*, const float*, const float*, const float*,
-                                    float, float*, double*, int*, cudaStream_t,
-                                    const uint8_t*);
+                                    float, float*, double*, int*, cudaStream_t);
 
 // Periodic batched apply: nsys systems on the nx*ny*nz torus; system bi uses
-// x/b/y at bi*ndof and the factors / kept mask / inverse diagonal of cell
-// bi / nrhs.  dot_part (kApply) receives one partial of x.y per CTA, the CTAs of
-// a system contiguous: periodic_op_blocks<T>() per system.
+// x/b/y at bi*ndof and the factors and kept bits of cell bi / nrhs.  dot_part
+// (kApply) receives one partial of x.y per CTA, the CTAs of a system
+// contiguous: periodic_op_blocks<T>() per system.
+namespace {
+template <class T>
+using PerV = typename std::conditional<std::is_same<T, float>::value, float2, double>::type;
+// One tile per cell size, whatever the batch, so that a system's partial sums
+// and with them its iterates do not depend on who else runs: the tile of four
+// cells' worth of strains, between a single cell's and a full GPU's.
+constexpr int kTileSystems = 24;
+template <class T>
+MarchTile periodic_tile(int nx, int ny, int nz) {
+  return march_tile<PerV<T>>(nx, ny, nz, kTileSystems, true);
+}
+}  // namespace
 template <class T>
 int periodic_op_blocks(int nx, int ny, int nz) {
-  using P = Pencil<T>;
-  return ((nx + 30) / 31) * ((ny + P::PY - 2) / (P::PY - 1)) * ((nz + P::KZ - 1) / P::KZ);
+  return blocks_of(march_grid<PerV<T>>(nx, ny, nz, 1, true, periodic_tile<T>(nx, ny, nz)));
 }
 template int periodic_op_blocks<double>(int, int, int);
 template int periodic_op_blocks<float>(int, int, int);
 
-template <class T, int MODE>
-static void launch_periodic_mode(int nx, int ny, int nz, const ModalConsts& c, const T* ef,
-                                 const uint8_t* kept, const T* x, const T* b, const T* invdiag,
-                                 T omega, T* y, double* dot_part, int nsys, int nrhs,
-                                 cudaStream_t s) {
-  using P = Pencil<T>;
-  const GridDev gd{nx, ny, nz, nx, ny, nz};
-  const int nzc = (nz + P::KZ - 1) / P::KZ;
-  const int64_t ndof = 3 * int64_t(nx) * ny * nz, nv = int64_t(nx) * ny * nz;
-  // gridDim.z <= 65535: whole cells per launch.
-  const int cells_per = std::max(1, 65535 / (nzc * nrhs));
-  const int ncell = nsys / nrhs;
-  const int nblk = periodic_op_blocks<T>(nx, ny, nz);
-  for (int c0 = 0; c0 < ncell; c0 += cells_per) {
-    const int nc = std::min(cells_per, ncell - c0);
-    const int64_t s0 = int64_t(c0) * nrhs;
-    const BatchDev bd{nrhs, nzc, ndof, nv, ndof};
-    const dim3 grid((nx + 30) / 31, (ny + P::PY - 2) / (P::PY - 1), nzc * nc * nrhs);
-    k_fine_op<T, P::PY, P::KZ, P::MINB, MODE, true><<<grid, 32 * P::PY, 0, s>>>(
-        gd, to_modal<T>(c), ef + c0 * nv, kept ? kept + c0 * ndof : nullptr, x + s0 * ndof,
-        b ? b + s0 * ndof : nullptr, invdiag ? invdiag + c0 * ndof : nullptr, omega,
-        y + s0 * ndof, dot_part ? dot_part + s0 * nblk : nullptr, bd);
-    TG_LAUNCH_CHECK();
-  }
-}
-
 template <class T>
 void launch_periodic_op(int mode, int nx, int ny, int nz, const ModalConsts& c, const T* ef,
-                        const uint8_t* kept, const T* x, const T* b, const T* invdiag, T omega,
-                        T* y, double* dot_part, int nsys, int nrhs, cudaStream_t s) {
+                        const uint8_t* kn, const T* x, const T* b, T* y, double* dot_part,
+                        int nsys, int nrhs, const int* run, cudaStream_t s) {
+  using V = PerV<T>;
+  const GridDev gd{nx, ny, nz, nx, ny, nz};
+  const int64_t nv = int64_t(nx) * ny * nz;
+  const MarchTile t = periodic_tile<T>(nx, ny, nz);
+  const BatchDev bd{nrhs, 3 * nv, nv, run};
   if (mode == kApply)
-    launch_periodic_mode<T, kApply>(nx, ny, nz, c, ef, kept, x, b, invdiag, omega, y, dot_part,
-                                    nsys, nrhs, s);
-  else if (mode == kResidual)
-    launch_periodic_mode<T, kResidual>(nx, ny, nz, c, ef, kept, x, b, invdiag, omega, y,
-                                       dot_part, nsys, nrhs, s);
+    launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y, dot_part, bd,
+                                     s);
   else
-    launch_periodic_mode<T, kSmooth>(nx, ny, nz, c, ef, kept, x, b, invdiag, omega, y, dot_part,
-                                     nsys, nrhs, s);
+    launch_march<V, T, kResidual, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y, nullptr,
+                                        bd, s);
 }
 template void launch_periodic_op<double>(int, int, int, int, const ModalConsts&, const double*,
-                                         const uint8_t*, const double*, const double*,
-                                         const double*, double, double*, double*, int, int,
-                                         cudaStream_t);
+                                         const uint8_t*, const double*, const double*, double*,
+                                         double*, int, int, const int*, cudaStream_t);
 template void launch_periodic_op<float>(int, int, int, int, const ModalConsts&, const float*,
-                                        const uint8_t*, const float*, const float*, const float*,
-                                        float, float*, double*, int, int, cudaStream_t);
+                                        const uint8_t*, const float*, const float*, float*,
+                                        double*, int, int, const int*, cudaStream_t);
 
 // diag(A) at every DOF = kdiag * (sum of the adjacent element factors), summed
 // in a fixed element order; invdiag = 1/diag on kept DOFs, 0 elsewhere

@@ -203,7 +203,7 @@ __device__ __forceinline__ double to_c<double>(double v) {
 }
 template <>
 __device__ __forceinline__ df to_c<df>(double v) {
-  return df_from(v);
+  return df_split(v);
 }
 __device__ __forceinline__ double from_c(double v) { return v; }
 __device__ __forceinline__ double from_c(df v) { return df_to_double(v); }
@@ -391,10 +391,10 @@ __global__ void k_oc_prepare(const double* __restrict__ x, const double* __restr
       l = (rho_min < xm) ? xm : rho_min;
       h = (xp < 1.0) ? xp : 1.0;
     }
-    sq[e] = df_from(s);
-    lo[e] = df_from(l);
-    hi[e] = df_from(h);
-    dvd[e] = df_from(d);
+    sq[e] = df_split(s);
+    lo[e] = df_split(l);
+    hi[e] = df_split(h);
+    dvd[e] = df_split(d);
   }
 }
 

@@ -365,7 +365,7 @@ Solver::Solver(const FineProblem& fp, const tg_solve_options& opt, cudaStream_t 
       launch_fill<float>(pf_.p, 1.0f, fp.g.ndof, s_);
       launch_fill<float>(t0f_.p, 0.5f, fp.g.ndof, s_);
       launch_fill<float>(t1f_.p, 0.25f, fp.g.ndof, s_);
-      autotune_fine_schedule(fp.g, fp.mc, Ef_.p, fp.kept.p, fp.kept_node.p, pf_.p, apf_.p,
+      autotune_fine_schedule(fp.g, fp.mc, Ef_.p, fp.kept_node.p, pf_.p, apf_.p,
                              part_.p, s_, t0f_.p, t1f_.p);
     }
   }
@@ -714,12 +714,12 @@ double Solver::time_operator(int form, int reps) {
   TG_CUDA(cudaEventRecord(a, s_));
   for (int i = 0; i < reps; ++i) {
     if (fp32)
-      launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept.p, pf_.p, nullptr, nullptr, 0.0f,
-                            apf_.p, nullptr, nullptr, s_, fp_.kept_node.p);
+      launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
+                            apf_.p, nullptr, nullptr, s_);
     else if (form == 2)  // the double-float residual kernel
-      launch_fine_residual_df(g, fp_.mc, E_, fp_.kept.p, p_.p, rhs_.p, ap_.p, s_);
+      launch_fine_residual_df(g, fp_.mc, E_, fp_.kept_node.p, p_.p, rhs_.p, ap_.p, s_);
     else
-      launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept.p, p_.p, nullptr, nullptr, 0.0,
+      launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0,
                              ap_.p, nullptr, nullptr, s_);
   }
   TG_CUDA(cudaEventRecord(b, s_));
@@ -1050,13 +1050,13 @@ double* Solver::vcycle<double>(const double* b, double* bz, bool x0_ready) {
   double* x = t1_.p;
   double* r = t0_.p;
   auto smooth = [&] {
-    launch_fine_op<double>(kSmooth, g, fp_.mc, E_, fp_.kept.p, x, b, invdiag_.p, omega_, r,
+    launch_fine_op<double>(kSmooth, g, fp_.mc, E_, fp_.kept_node.p, x, b, invdiag_.p, omega_, r,
                            nullptr, nullptr, s_);
     std::swap(x, r);
   };
   mg_jacobi_first<double>(b, invdiag_.p, omega_, g.ndof, x, s_);
   for (int k = 1; k < sweeps_; ++k) smooth();
-  launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept.p, x, b, invdiag_.p, omega_, r,
+  launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x, b, invdiag_.p, omega_, r,
                          nullptr, nullptr, s_);
   const FirstStep<double> fs = first_step<double>(1);
   mg_restrict<double>(fd, N.d, r, N.act.p, N.B<double>(), s_, fs);
@@ -1082,15 +1082,15 @@ float* Solver::vcycle<float>(const float* b, double* bz, bool x0_ready) {
   auto smooth = [&](bool last) {
     int nb = 0;
     double* part = last && bz != nullptr ? part_.p : nullptr;
-    launch_fine_op<float>(kSmooth, g, fp_.mc, Ef_.p, fp_.kept.p, x, b, invdiagf_.p, w, r, part,
-                          &nb, s_, fp_.kept_node.p);
+    launch_fine_op<float>(kSmooth, g, fp_.mc, Ef_.p, fp_.kept_node.p, x, b, invdiagf_.p, w, r, part,
+                          &nb, s_);
     if (part != nullptr) launch_sum_partials(part_.p, nb, bz, s_);
     std::swap(x, r);
   };
   if (!x0_ready) mg_jacobi_first<float>(b, invdiagf_.p, w, g.ndof, x, s_);
   for (int k = 1; k < sweeps_; ++k) smooth(false);
-  launch_fine_op<float>(kResidual, g, fp_.mc, Ef_.p, fp_.kept.p, x, b, invdiagf_.p, w, r, nullptr,
-                        nullptr, s_, fp_.kept_node.p);
+  launch_fine_op<float>(kResidual, g, fp_.mc, Ef_.p, fp_.kept_node.p, x, b, invdiagf_.p, w, r, nullptr,
+                        nullptr, s_);
   const FirstStep<float> fs = first_step<float>(1);
   mg_restrict<float>(fd, N.d, r, N.act.p, N.B<float>(), s_, fs);
   float* ec = vcycle_level<float>(1, fs.kind != 0);
@@ -1127,7 +1127,7 @@ bool Solver::mgpcg(double tol, int max_it, bool warm, SolverStats& st) {
   if (!std::isfinite(read_scalar(0))) return false;
   int nb = 0;
   for (int k = 1; k <= max_it; ++k) {
-    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
+    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
                            part_.p, &nb, s_);
     ++fine_matvecs_;
     launch_sum_partials(part_.p, nb, scal_.p + 1, s_);
@@ -1213,8 +1213,8 @@ bool Solver::build_inner_graph() {
       TG_CUDA(cudaMemcpyAsync(scal_.p + 6, scal_.p + 9, sizeof(double), cudaMemcpyDeviceToDevice,
                               s_));
       int nb = 0;
-      launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept.p, pf_.p, nullptr, nullptr, 0.0f,
-                            apf_.p, part_.p, &nb, s_, fp_.kept_node.p);
+      launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
+                            apf_.p, part_.p, &nb, s_);
       launch_sum_partials(part_.p, nb, scal_.p + 7, s_);
       launch_cg_update_r_f(rf_.p, apf_.p, scal_.p + 6, scal_.p + 7, n, part_.p, s_, invdiagf_.p,
                            float(omega_), t1f_.p);
@@ -1257,8 +1257,8 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
   int nb = 0;
   *iters = 0;
   for (int k = 1; k <= max_it; ++k) {
-    launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept.p, pf_.p, nullptr, nullptr, 0.0f,
-                          apf_.p, part_.p, &nb, s_, fp_.kept_node.p);
+    launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
+                          apf_.p, part_.p, &nb, s_);
     ++lowp_matvecs_;
     launch_sum_partials(part_.p, nb, scal_.p + 7, s_);
     // r now; x += alpha p when p is next overwritten or at exit (flush_x), or on
@@ -1320,9 +1320,9 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
 void Solver::refinement_residual() {
   const Grid& g = fp_.g;
   if (df_residual_) {
-    launch_fine_residual_df(g, fp_.mc, E_, fp_.kept.p, x_.p, rhs_.p, r_.p, s_);
+    launch_fine_residual_df(g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, r_.p, s_);
   } else {
-    launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
+    launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
                            nullptr, nullptr, s_);
   }
   ++fine_matvecs_;
@@ -1342,7 +1342,7 @@ bool Solver::mixed_refine(double tol, int max_it, bool warm, SolverStats& st) {
   }
   const double bnorm = std::sqrt(bnorm2), threshold = tol * bnorm;
   if (warm) {
-    launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
+    launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
                            nullptr, nullptr, s_);
     ++fine_matvecs_;
   } else {
@@ -1409,7 +1409,7 @@ bool Solver::jacobi_pcg(double tol, int max_it, bool warm, SolverStats& st) {
   double threshold = tol * tol * rhs2;
   if (threshold < std::numeric_limits<double>::min()) threshold = std::numeric_limits<double>::min();
   if (!warm) launch_fill<double>(x_.p, 0.0, n, s_);
-  launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
+  launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
                          nullptr, nullptr, s_);
   ++fine_matvecs_;
   launch_dot(r_.p, r_.p, n, part_.p, scal_.p + 2, s_);
@@ -1422,7 +1422,7 @@ bool Solver::jacobi_pcg(double tol, int max_it, bool warm, SolverStats& st) {
   launch_sum_partials(part_.p, kRedBlocks, scal_.p + 0, s_);
   int i = 0, nb = 0;
   while (i < maxIters) {
-    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
+    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
                            part_.p, &nb, s_);
     ++fine_matvecs_;
     launch_sum_partials(part_.p, nb, scal_.p + 1, s_);

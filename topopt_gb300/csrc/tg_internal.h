@@ -151,25 +151,25 @@ enum ApplyMode { kApply = 0, kResidual = 1, kSmooth = 2, kCheb = 3 };
 // kResidual of the FP64 operator evaluated in double-float arithmetic (FP32
 // pairs, ~48 significant bits): the refinement residual of the mixed form.
 void launch_fine_residual_df(const Grid& g, const ModalConsts& c, const double* ef,
-                             const uint8_t* kept, const double* x, const double* b, double* y,
+                             const uint8_t* kept_node, const double* x, const double* b, double* y,
                              cudaStream_t s);
 // Fine operator on the full grid, element factors `ef` (0 = no element):
 //   kApply:    y = M A x                 (M = kept mask; dot = sum x.y if dot_part)
 //   kResidual: y = M (b - A x)
 //   kSmooth:   y = x + omega*invdiag*(b - A x)   (invdiag is 0 off the kept set)
-//   kept_node (optional): the kept mask as 3 bits per node, read by the FP32
-//   column schedule instead of kept (one byte per node instead of three).
-//   kSmooth with dot_part (FP32 only): partials of b . y as well.
+//   kept_node: M as one byte per node (bit k: DOF 3n+k kept); null keeps every
+//   DOF, and then x may hold anything at nodes of absent elements.
+//   kSmooth with dot_part: partials of b . y as well.
 template <class T>
 void launch_fine_op(int mode, const Grid& g, const ModalConsts& mc, const T* ef,
-                    const uint8_t* kept, const T* x, const T* b, const T* invdiag, T omega,
-                    T* y, double* dot_part, int* nblocks_out, cudaStream_t s,
-                    const uint8_t* kept_node = nullptr);
+                    const uint8_t* kept_node, const T* x, const T* b, const T* invdiag, T omega,
+                    T* y, double* dot_part, int* nblocks_out, cudaStream_t s);
 int fine_op_blocks(const Grid& g, bool fp64);  // upper bound of the partials any schedule writes
 
-// How the FP32 fine operator is scheduled on a grid (k_operator.cu): the
-// pencil kernel (the FP64 form's schedule) or the column-blocked kernel with
-// one of fine_schedule_shapes() tile shapes and kz element layers per CTA.
+// How the FP32 fine operator is scheduled on a grid (k_operator.cu): two packed
+// element rows per thread (column) with one of fine_schedule_shapes() tile
+// shapes and kz node layers per CTA, or one row per thread (pencil, the FP64
+// form's schedule; its tile is the modelled one).
 struct FineSchedule {
   enum { kPencil = 0, kColumn = 1 };
   int kind = kColumn, shape = 0, kz = 32;
@@ -184,16 +184,16 @@ void set_fine_schedule_override(const FineSchedule* s);  // null clears
 bool fine_schedule_known(const Grid& g);  // in the table, or an override is set
 // The FP32 operator under an explicit schedule.
 void launch_fine_op_sched(const FineSchedule& fs, int mode, const Grid& g, const ModalConsts& c,
-                          const float* ef, const uint8_t* kept, const float* x, const float* b,
-                          const float* invdiag, float omega, float* y, double* dot_part,
-                          int* nblocks_out, cudaStream_t s, const uint8_t* kn);
+                          const float* ef, const uint8_t* kept_node, const float* x,
+                          const float* b, const float* invdiag, float omega, float* y,
+                          double* dot_part, int* nblocks_out, cudaStream_t s);
 // Times every candidate schedule of the FP32 operator on the given buffers
 // (CUDA events on s) for the apply and, with b and invdiag, the residual and
 // smoothing modes; publishes the fastest per mode in the table for g (one sweep
 // at a time; a grid already in the table is not measured again) and returns
 // the apply's.
 FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const float* ef,
-                                    const uint8_t* kept, const uint8_t* kn, const float* x,
+                                    const uint8_t* kept_node, const float* x,
                                     float* y, double* part, cudaStream_t s,
                                     const float* b = nullptr, const float* invdiag = nullptr,
                                     int reps = 3);
@@ -216,8 +216,8 @@ template <class T>
 int periodic_op_blocks(int nx, int ny, int nz);
 template <class T>
 void launch_periodic_op(int mode, int nx, int ny, int nz, const ModalConsts& c, const T* ef,
-                        const uint8_t* kept, const T* x, const T* b, const T* invdiag, T omega,
-                        T* y, double* dot_part, int nsys, int nrhs, cudaStream_t s);
+                        const uint8_t* kept_node, const T* x, const T* b, T* y, double* dot_part,
+                        int nsys, int nrhs, const int* run, cudaStream_t s);
 
 // Jacobi diagonal of the fine operator: diag = kdiag * sum of adjacent factors.
 void launch_fine_invdiag(const Grid& g, double kdiag, const double* ef, const uint8_t* kept,

@@ -63,7 +63,7 @@ bool fine_schedule_known(const Grid& g) {
 }
 
 // The measured sweep: every column tile shape with z-chunks of about 8 .. 33
-// element layers, and the pencil kernel, each launched once untimed and then
+// node layers, and the one-row kernel, each launched once untimed and then
 // timed over `reps` back-to-back launches, for each of the three modes as the
 // mixed solve runs them: the apply with the kept mask and the p.Ap partials,
 // the residual, and the smoothing sweep with its b.y partials (b, invdiag:
@@ -72,7 +72,7 @@ bool fine_schedule_known(const Grid& g) {
 // of every candidate agree to FP32 rounding, so the choice changes timing only.
 // Returns the apply's schedule in the table.
 FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const float* ef,
-                                    const uint8_t* kept, const uint8_t* kn, const float* x,
+                                    const uint8_t* kn, const float* x,
                                     float* y, double* part, cudaStream_t s, const float* b,
                                     const float* invdiag, int reps) {
   std::lock_guard<std::mutex> tune_lock(g_tune_mu);
@@ -106,10 +106,10 @@ FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const 
     FineSchedule best = default_fine_schedule(g);
     float best_ms = 1e30f;
     for (const FineSchedule& c : cands) {
-      launch_fine_op_sched(c, mode, g, mc, ef, kept, x, bb, dd, 0.6f, y, pp, nullptr, s, kn);
+      launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, pp, nullptr, s);
       TG_CUDA(cudaEventRecord(ea, s));
       for (int r = 0; r < reps; ++r)
-        launch_fine_op_sched(c, mode, g, mc, ef, kept, x, bb, dd, 0.6f, y, pp, nullptr, s, kn);
+        launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, pp, nullptr, s);
       TG_CUDA(cudaEventRecord(eb, s));
       TG_CUDA(cudaEventSynchronize(eb));
       float ms = 0.0f;
