@@ -413,7 +413,7 @@ def run_ours(args, world, rank, local, pg):
 def run_op_only(args):
     """Operator launches on a resident job of the benchmark workload (its kept
     mask and element factors), for ncu captures: three launches of the FP32 or
-    FP64 fine operator, or of the level-1 tensor-core operator ("l1tc").  The
+    FP64 fine operator, or of the level-1 matrix-free operator ("l1tc").  The
     FP32 schedule comes from --fp32-schedule (kind,shape,kz), so no autotuning
     launches precede the captured ones."""
     import topopt_gb300 as tg

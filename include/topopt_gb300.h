@@ -80,7 +80,8 @@ typedef enum { TG_PREC_FP64 = 0, TG_PREC_MIXED = 1 } tg_precision;
  * (the mixed form's refinement residual kernel). */
 enum { TG_APPLY_DF = 2 };
 /* tg_job_time_operator only: the level-1 operator of the mixed form's V-cycle,
- * residual mode -- the assembled FP32 stencil or the tensor-core operator. */
+ * residual mode -- the assembled FP32 stencil or the matrix-free operator (the
+ * name is historical: it was a tensor-core kernel). */
 enum { TG_APPLY_L1_STENCIL = 3, TG_APPLY_L1_TC = 4 };
 
 /* Solver knobs.  Zero-initialised means: MG-PCG, FP64, the deepest hierarchy the
@@ -718,18 +719,18 @@ int tg_filter_noalloc(int32_t nx, int32_t ny, int32_t nz, const uint8_t* d_tags,
  * launches timed with CUDA events on the job's stream. */
 int tg_job_time_operator(tg_job* job, int32_t precision, int32_t reps, double* avg_ms);
 /* The level-1 operator of a mixed job's V-cycle on its current design, applied
- * to a seeded vector by the assembled FP32 stencil and by the tensor-core
+ * to a seeded vector by the assembled FP32 stencil and by the matrix-free
  * operator: max |difference| / max |stencil result|. */
 int tg_job_check_level1(tg_job* job, double* rel_diff);
 /* Kernels this library has launched in the process so far. */
 int64_t tg_kernel_launches(void);
 /* Level 1 of the mixed form's V-cycle: on (default) the Galerkin operator is
- * applied on the tensor cores from the fine moduli (tcgen05, TF32 splits to
- * FP32 accuracy); off, as the assembled FP32 node stencil.  Applies to solvers
- * created afterwards. */
+ * applied without a matrix, from the fine moduli (the name is historical: it was
+ * a tensor-core kernel); off, as the assembled FP32 node stencil.  Applies to
+ * solvers created afterwards. */
 int tg_set_level1_tc(int32_t on);
-/* Level 1's Galerkin matrices in the mixed form with level 1 on the tensor
- * cores: on (default) the fast-path elements' matrices (sum_c E_c G_c) come
+/* Level 1's Galerkin matrices in the mixed form with the matrix-free level 1:
+ * on (default) the fast-path elements' matrices (sum_c E_c G_c) come
  * from a bandwidth-bound kernel, the others from the general one; off, all from
  * the general one.  The matrices are bit-identical either way.  Applies to
  * hierarchy builds from then on. */

@@ -959,8 +959,9 @@ APPLY_L1_STENCIL, APPLY_L1_TC = 3, 4
 
 
 def set_level1_tc(on: bool):
-    """Level 1 of the mixed V-cycle on the tensor cores (True, default) or as the
-    assembled FP32 stencil (False), for solvers created afterwards."""
+    """Level 1 of the mixed V-cycle without a matrix, from the fine moduli (True,
+    default), or as the assembled FP32 stencil (False), for solvers created
+    afterwards.  (The name is historical: it was a tensor-core kernel.)"""
     _check(lib().tg_set_level1_tc(int(bool(on))))
 
 
@@ -1155,7 +1156,7 @@ class SimpJob:
         return x, xp
 
     def check_level1(self):
-        """Level-1 operator, tensor cores against the assembled FP32 stencil on a
+        """Level-1 operator, matrix-free against the assembled FP32 stencil on a
         seeded vector: max |difference| / max |stencil result|."""
         d = C.c_double(0.0)
         _check(lib().tg_job_check_level1(self._h, C.byref(d)))

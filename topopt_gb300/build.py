@@ -20,7 +20,7 @@ LIB = os.path.join(HERE, "libtopopt_gb300.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["k_operator.cu", "k_vector.cu", "k_simp.cu", "k_multigrid.cu", "solver.cu", "api.cu",
            "formats.cu", "noalloc.cu", "homog.cu", "server.cu", "k_active.cu", "tune.cu",
-           "k_coarse_tc.cu"]
+           "k_level1.cu"]
 
 
 def nvcc() -> str:

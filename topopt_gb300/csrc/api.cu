@@ -1968,7 +1968,7 @@ int tg_job_check_level1(tg_job* job, double* rel_diff) {
 int64_t tg_kernel_launches(void) { return tg::g_launches.load(); }
 
 int tg_set_level1_tc(int32_t on) {
-  return guarded([&] { set_level1_tc(on != 0); });
+  return guarded([&] { set_level1_matfree(on != 0); });
 }
 
 int tg_set_level1_galerkin_fast(int32_t on) {

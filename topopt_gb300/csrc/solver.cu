@@ -409,7 +409,7 @@ size_t Solver::device_bytes() const {
   for (const DBuf<float>* d : {&Ef_, &invdiagf_, &xf_, &rf_, &zf_, &pf_, &apf_, &t0f_, &t1f_})
     b += d->bytes();
   for (const auto& L : levels_) b += L->bytes();
-  b += spos1_.bytes() + slist1_.bytes() + yspec1_.bytes() + tc_err_.bytes() + chc_.bytes() +
+  b += spos1_.bytes() + slist1_.bytes() + yspec1_.bytes() + act_node1_.bytes() + chc_.bytes() +
        pipart_.bytes();
   return b + cidx_.bytes() + kebf_.bytes() + Gf_.bytes();
 }
@@ -537,8 +537,8 @@ void Solver::build_structure() {
   Gf_.alloc(8 * 576);
   TG_CUDA(cudaMemcpyAsync(kebf_.p, kbf.data(), kebf_.bytes(), cudaMemcpyHostToDevice, s_));
   TG_CUDA(cudaMemcpyAsync(Gf_.p, Gf.data(), Gf_.bytes(), cudaMemcpyHostToDevice, s_));
-  l1_tc_ = mixed_ && level1_tc_enabled();
-  if (l1_tc_) {
+  l1_mf_ = mixed_ && level1_matfree_enabled();
+  if (l1_mf_) {
     // Coarse elements of level 1 off the sum_c E_c G_c fast path.
     const Level& L1 = *levels_[0];
     const MgDims& d = L1.d;
@@ -582,8 +582,12 @@ void Solver::build_structure() {
       TG_CUDA(cudaMemcpyAsync(slist1_.p, slist.data(), slist1_.bytes(), cudaMemcpyHostToDevice,
                               s_));
     }
-    tc_err_.alloc(1);
-    TG_CUDA(cudaMemsetAsync(tc_err_.p, 0, sizeof(int), s_));
+    std::vector<uint8_t> an(size_t(L1.nn));
+    for (size_t n = 0; n < an.size(); ++n)
+      an[n] = uint8_t(L1.act_h[3 * n] | L1.act_h[3 * n + 1] << 1 | L1.act_h[3 * n + 2] << 2);
+    act_node1_.alloc(an.size());
+    TG_CUDA(cudaMemcpyAsync(act_node1_.p, an.data(), an.size(), cudaMemcpyHostToDevice, s_));
+    TG_CUDA(cudaStreamSynchronize(s_));  // an goes out of scope
   }
   // The small levels (from the first one of at most kFusedMaxNodes nodes, below
   // level 1) in one cluster launch, when at least one of them is smoothed and
@@ -604,13 +608,13 @@ void Solver::build_structure() {
   have_mg_ = true;
 }
 
-// Level 1 of the FP32 V-cycle on the tensor cores (mode kResidual or kSmooth):
+// Level 1 of the FP32 V-cycle without its matrix (mode kResidual or kSmooth):
 // L.R = b - A1 x or the smoothed iterate, as the stencil apply would write it.
 void Solver::level1_op(int mode, Level& L, float omega) {
   const Grid& g = fp_.g;
-  mg_level1_tc(mode, dims_of(g.nx, g.ny, g.nz), L.d, Ef_.p, L.act.p, spos1_.p, slist1_.p,
-               nspec1_, L.Ke<float>(), Gf_.p, L.X<float>(), L.B<float>(), L.Dinv<float>(), omega,
-               L.R<float>(), yspec1_.p, tc_err_.p, s_);
+  mg_level1_op(mode, dims_of(g.nx, g.ny, g.nz), L.d, fp_.mc, Ef_.p, act_node1_.p, spos1_.p,
+               slist1_.p, nspec1_, L.Ke<float>(), L.X<float>(), L.B<float>(), L.Dinv<float>(),
+               omega, L.R<float>(), yspec1_.p, s_);
 }
 
 double Solver::read_scalar(int idx) {
@@ -641,8 +645,8 @@ void Solver::level1_stencil() {
 }
 
 double Solver::check_level1() {
-  if (!mixed_ || !l1_tc_ || !have_mg_ || !numeric_ok_)
-    raise(TG_EINVAL, "check_level1: needs a mixed job with the level-1 tensor-core path");
+  if (!mixed_ || !l1_mf_ || !have_mg_ || !numeric_ok_)
+    raise(TG_EINVAL, "check_level1: needs a mixed job with the matrix-free level 1");
   level1_stencil();
   Level& L = *levels_[0];
   const size_t n = size_t(L.ndof);
@@ -661,10 +665,7 @@ double Solver::check_level1() {
   TG_CUDA(cudaStreamSynchronize(s_));
   level1_op(kApply, L, 0.0f);
   TG_CUDA(cudaMemcpyAsync(bq.data(), L.R<float>(), n * sizeof(float), cudaMemcpyDeviceToHost, s_));
-  int tc_err = 0;
-  TG_CUDA(cudaMemcpyAsync(&tc_err, tc_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
   TG_CUDA(cudaStreamSynchronize(s_));
-  if (tc_err) raise(TG_EDEVICE, "level-1 tensor-core operator: MMA completion wait timed out");
   double dmax = 0.0, amax = 0.0;
   for (size_t i = 0; i < n; ++i) {
     dmax = std::max(dmax, std::fabs(double(a[i]) - double(bq[i])));
@@ -680,9 +681,9 @@ double Solver::time_operator(int form, int reps) {
     raise(TG_EINVAL, "time_operator: FP32 operators need a mixed-precision job");
   if (form >= 3) {
     // Level 1 of the FP32 V-cycle, residual mode: form 3 the assembled stencil,
-    // form 4 the tensor-core operator.
+    // form 4 the matrix-free operator.
     if (!have_mg_ || !numeric_ok_) raise(TG_EINVAL, "time_operator: no multigrid hierarchy");
-    if (form == 4 && !l1_tc_) raise(TG_EINVAL, "time_operator: level-1 tensor-core path is off");
+    if (form == 4 && !l1_mf_) raise(TG_EINVAL, "time_operator: the matrix-free level 1 is off");
     if (form == 3) level1_stencil();
     Level& L = *levels_[0];
     launch_fill<float>(L.X<float>(), 1.0f, L.ndof, s_);
@@ -798,14 +799,14 @@ bool Solver::build_numeric() {
     if (l == 0)
       mg_galerkin_level1<T>(fd, L.d, ef, fp_.kept.p, L.act.p, pick<T>(keb_, kebf_),
                             pick<T>(G_, Gf_), L.Ke<T>(), s_,
-                            sizeof(T) == 4 && l1_tc_ && level1_galerkin_fast_enabled()
+                            sizeof(T) == 4 && l1_mf_ && level1_galerkin_fast_enabled()
                                 ? spos1_.p
                                 : nullptr);
     else
       mg_galerkin_coarse<T>(pd, L.d, levels_[l - 1]->Ke<T>(), L.act.p, L.Ke<T>(), s_);
-    // Level 1 on the tensor cores needs only its inverse diagonal; the assembled
+    // The matrix-free level 1 needs only its inverse diagonal; the assembled
     // stencil (275 MB on the 256x128x128 cantilever) is formed on demand (level1_stencil()).
-    const bool diag_only = sizeof(T) == 4 && l == 0 && l1_tc_;
+    const bool diag_only = sizeof(T) == 4 && l == 0 && l1_mf_;
     mg_assemble_stencil<T>(L.d, L.Ke<T>(), L.act.p, diag_only ? nullptr : L.Am<T>(), L.Dinv<T>(),
                            s_);
     if (sizeof(T) == 4 && l == 0) l1_stencil_ok_ = !diag_only;
@@ -954,7 +955,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
   const T w = T(omega_);
   auto op = [&](int mode) {
     if constexpr (sizeof(T) == 4) {
-      if (l == 1 && l1_tc_) {
+      if (l == 1 && l1_mf_) {
         level1_op(mode, L, float(w));
         return;
       }
@@ -1468,15 +1469,6 @@ SolverStats Solver::solve(double tol, int max_it, const double* guess, double* u
       // and an FP32 iteration costs about 1/6 of the FP64 retry's.
       if (warm) seed();
       solved = mixed_refine(tol, std::min(cap, 3 * budget_), warm, st);
-    }
-    if (mixed_ && l1_tc_) {
-      // A tensor-core completion wait that ran out is a device error, not a
-      // solver verdict.
-      int tc_err = 0;
-      TG_CUDA(cudaMemcpyAsync(&tc_err, tc_err_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
-      TG_CUDA(cudaStreamSynchronize(s_));
-      if (tc_err)
-        raise(TG_EDEVICE, "level-1 tensor-core operator: MMA completion wait timed out");
     }
     if (mixed_ && !solved) st.mixed_fallback = true;
     if (!solved && (!mixed_ || build_numeric<double>())) {

@@ -197,10 +197,10 @@ FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const 
                                     float* y, double* part, cudaStream_t s,
                                     const float* b = nullptr, const float* invdiag = nullptr,
                                     int reps = 3);
-// Whether the mixed form's V-cycle applies its level-1 operator on the tensor
-// cores (k_coarse_tc.cu) instead of the assembled FP32 stencil; on by default.
-bool level1_tc_enabled();
-void set_level1_tc(bool on);
+// Whether the mixed form's V-cycle applies its level-1 operator without a matrix
+// (k_level1.cu) instead of the assembled FP32 stencil; on by default.
+bool level1_matfree_enabled();
+void set_level1_matfree(bool on);
 // Whether the hierarchy build forms level 1's fast-path Galerkin matrices with
 // the bandwidth-bound kernel (bit-identical to the general one); on by default.
 bool level1_galerkin_fast_enabled();

@@ -6,6 +6,8 @@
 
 namespace tg {
 
+struct ModalConsts;
+
 // Entries per node of a stored coarse stencil: the self block and the 13 forward
 // neighbour blocks, 3x3 each (the backward blocks are their transposes).
 constexpr int kStencilEntries = 14 * 9;
@@ -24,7 +26,7 @@ struct MgDims {
 };
 
 // spos (FP32, optional): per coarse element, < 0 on the fast path (sum_c f_c G_c;
-// the level-1 tensor-core operator's special-element positions), where a
+// the level-1 operator's special-element positions), where a
 // bandwidth-bound kernel forms the matrix.
 template <class T>
 void mg_galerkin_level1(const MgDims& fd, const MgDims& cd, const T* ef, const uint8_t* fact,
@@ -136,17 +138,15 @@ struct FusedCoarse {
 int fused_coarse_blocks();
 void mg_coarse_vcycle_fused(const FusedCoarse& fc, cudaStream_t s);
 
-// The FP32 level-1 Galerkin operator on the tensor cores (k_coarse_tc.cu):
+// The FP32 level-1 Galerkin operator without an assembled matrix (k_level1.cu):
 // y = A1 x (kApply), b - A1 x (kResidual) or x + omega D^-1 (b - A1 x) (kSmooth),
-// masked by act, from the fine FP32 factors ef and the 8 child blocks G (FP32,
-// [8][576] corner-bit order).  The nspec coarse elements off the fast path
+// masked by act_node (bit k: DOF 3n+k active), from the fine FP32 factors ef and
+// the fine element's modal constants.  The nspec coarse elements off the fast path
 // (slist; spos[ce] = position in slist or -1) are applied from their stored
-// matrices Kel by a pre-pass into yspec (nspec x 24).  A wait that runs out
-// sets *err.
-void mg_level1_tc(int mode, const MgDims& fd, const MgDims& cd, const float* ef,
-                  const uint8_t* act, const int* spos, const int* slist, int nspec,
-                  const float* Kel, const float* G, const float* x, const float* b,
-                  const float* invdiag, float omega, float* y, float* yspec, int* err,
-                  cudaStream_t s);
+// matrices Kel by a pre-pass into yspec (nspec x 24).
+void mg_level1_op(int mode, const MgDims& fd, const MgDims& cd, const ModalConsts& c,
+                  const float* ef, const uint8_t* act_node, const int* spos, const int* slist,
+                  int nspec, const float* Kel, const float* x, const float* b,
+                  const float* invdiag, float omega, float* y, float* yspec, cudaStream_t s);
 
 }  // namespace tg

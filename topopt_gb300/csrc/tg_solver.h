@@ -72,7 +72,7 @@ class Solver {
   // form: 0 FP64, 1 FP32, 2 the double-float residual kernel.
   double time_operator(int form, int reps);
   // Level 1 of the FP32 V-cycle applied to a seeded vector by the assembled
-  // stencil and by the tensor-core operator: max |difference| / max |stencil|.
+  // stencil and by the matrix-free operator: max |difference| / max |stencil|.
   double check_level1();
   size_t device_bytes() const;
   int levels() const { return int(levels_.size()) + 1; }
@@ -148,15 +148,15 @@ class Solver {
   std::unique_ptr<InnerGraph> ig_;
   bool ig_failed_ = false, use_graph_ = true;
   DBuf<int> istate_;           // [0] iterations done, [1] budget, [2] breakdown
-  // Level 1 of the FP32 V-cycle on the tensor cores: per coarse element, 1 when
-  // its matrix is not sum_c E_c G_c (a Dirichlet or untouched fine DOF in a
-  // solid child, an inactive coarse DOF or a half element) and the stored
-  // matrix is applied instead; the kernel's timeout flag.
-  bool l1_tc_ = false;
+  // Level 1 of the FP32 V-cycle without its matrix: the coarse elements whose
+  // matrix is not the children's sum (a Dirichlet or untouched fine DOF in a
+  // solid child, an inactive coarse DOF or a half element), applied from their
+  // stored matrices; the level's activity as 3 bits per node.
+  bool l1_mf_ = false;
   int nspec1_ = 0;
   DBuf<int> spos1_, slist1_;  // per coarse element: position in slist1_ or -1
   DBuf<float> yspec1_;        // their outputs, nspec1_ x 24
-  DBuf<int> tc_err_;  // a tensor-core completion wait that ran out
+  DBuf<uint8_t> act_node1_;
   // The small levels of the FP32 V-cycle in one cluster launch.
   size_t fused_level_ = 0;  // first level of the fused cluster launch (0: none)
   bool l1_stencil_ok_ = true;  // the FP32 level-1 stencil is assembled (not only its diagonal)

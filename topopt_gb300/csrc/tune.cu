@@ -130,10 +130,10 @@ FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const 
 }
 
 namespace {
-std::atomic<bool> g_level1_tc{true};
+std::atomic<bool> g_level1_matfree{true};
 }
-bool level1_tc_enabled() { return g_level1_tc.load(); }
-void set_level1_tc(bool on) { g_level1_tc.store(on); }
+bool level1_matfree_enabled() { return g_level1_matfree.load(); }
+void set_level1_matfree(bool on) { g_level1_matfree.store(on); }
 namespace {
 std::atomic<bool> g_level1_galerkin_fast{true};
 }
