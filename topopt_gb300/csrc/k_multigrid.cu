@@ -325,23 +325,30 @@ __device__ __forceinline__ double cheb_dir(double c0, double dprev, double c1, d
   return __fma_rn(c0, dprev, __dmul_rn(c1, res));
 }
 
-// u = a0 x0 + a1 x1 + a2 x2 with one rounding pattern (a product, then two
-// fused multiply-adds) in every kernel that evaluates a stencil term.
-__device__ __forceinline__ float dot3(float a0, float x0, float a1, float x1, float a2, float x2) {
-  return __fmaf_rn(a2, x2, __fmaf_rn(a1, x1, __fmul_rn(a0, x0)));
+// s plus one stencil block's row times x, in one rounding pattern in every kernel
+// that evaluates it.  FP32: the block's sum first (a product, two fused
+// multiply-adds), then one addition, so the blocks' sums do not wait for one
+// another.  FP64, where each operation takes 64 cycles of the scheduler's unit
+// whatever waits: three fused multiply-adds onto s, a quarter fewer.
+__device__ __forceinline__ float add_block(float s, float a0, float x0, float a1, float x1,
+                                           float a2, float x2, bool on) {
+  const float u = __fmaf_rn(a2, x2, __fmaf_rn(a1, x1, __fmul_rn(a0, x0)));
+  return __fadd_rn(s, on ? u : 0.0f);
 }
-__device__ __forceinline__ double dot3(double a0, double x0, double a1, double x1, double a2,
-                                       double x2) {
-  return __fma_rn(a2, x2, __fma_rn(a1, x1, __dmul_rn(a0, x0)));
+__device__ __forceinline__ double add_block(double s, double a0, double x0, double a1, double x1,
+                                            double a2, double x2, bool on) {
+  const double t = __fma_rn(a2, x2, __fma_rn(a1, x1, __fma_rn(a0, x0, s)));
+  return on ? t : s;
 }
 
 // Part `part` (0..3) of row r of node (a, bb, c) of a stored symmetric stencil
 // times x.  The row is the self block (term 0) plus, for j = 1..13, forward
 // block j (neighbour n + off_j) and the transposed forward block of neighbour
-// n - off_j; part q sums the terms j = q, q + 4, ... in increasing j (part 0
-// starts from the self term), and the row is ((p0 + p1) + p2) + p3.  Four
+// n - off_j; part q accumulates the terms j = q, q + 4, ... in increasing j (part
+// 0 starts from the self term), and the row is ((p0 + p1) + p2) + p3.  Four
 // parts let four threads share a row on the small levels, where a row's ~160
-// loads in one thread are a chain of dependent memory round trips.
+// loads in one thread are a chain of dependent memory round trips -- and, in
+// FP64, its 81 multiply-adds a chain of 64 cycles each.
 template <class T, bool COH>
 __device__ __forceinline__ T stencil_part(const MgDims& d, const T* __restrict__ A, const T* x,
                                           int a, int bb, int c, int r, int part) {
@@ -351,8 +358,8 @@ __device__ __forceinline__ T stencil_part(const MgDims& d, const T* __restrict__
   const T* An = A + n + int64_t(3 * r) * nn;  // row r of the self block
   T s = T(0);
   if (part == 0)
-    s = dot3(An[0], vload<T, COH>(x + 3 * n), An[nn], vload<T, COH>(x + 3 * n + 1), An[2 * nn],
-             vload<T, COH>(x + 3 * n + 2));
+    s = add_block(T(0), An[0], vload<T, COH>(x + 3 * n), An[nn], vload<T, COH>(x + 3 * n + 1),
+                  An[2 * nn], vload<T, COH>(x + 3 * n + 2), true);
 #pragma unroll
   for (int j = 1; j < 14; ++j) {
     if ((j & 3) != part) continue;
@@ -367,12 +374,10 @@ __device__ __forceinline__ T stencil_part(const MgDims& d, const T* __restrict__
     const int64_t p = bin ? n - off : n;
     const T* Af = An + int64_t(j * 9) * nn;
     const T* Ab = A + int64_t(j * 9 + r) * nn + p;
-    const T u = dot3(Af[0], vload<T, COH>(x + 3 * m), Af[nn], vload<T, COH>(x + 3 * m + 1),
-                     Af[2 * nn], vload<T, COH>(x + 3 * m + 2));
-    const T v = dot3(Ab[0], vload<T, COH>(x + 3 * p), Ab[3 * nn], vload<T, COH>(x + 3 * p + 1),
-                     Ab[6 * nn], vload<T, COH>(x + 3 * p + 2));
-    s += fin ? u : T(0);
-    s += bin ? v : T(0);
+    s = add_block(s, Af[0], vload<T, COH>(x + 3 * m), Af[nn], vload<T, COH>(x + 3 * m + 1),
+                  Af[2 * nn], vload<T, COH>(x + 3 * m + 2), fin);
+    s = add_block(s, Ab[0], vload<T, COH>(x + 3 * p), Ab[3 * nn], vload<T, COH>(x + 3 * p + 1),
+                  Ab[6 * nn], vload<T, COH>(x + 3 * p + 2), bin);
   }
   return s;
 }
@@ -444,27 +449,34 @@ __global__ void __launch_bounds__(kStencilThreads) k_stencil_op(MgDims d, const 
   y[dof] = out;
 }
 
-// The FP32 stencil kernels on small levels: four threads per (node, row), one
+// The stencil kernels on small levels: four threads per (node, row), one
 // part of the row each (stencil_part), combined in shared memory in the order
 // stencil_row uses, so both kernels give the same bits.  384 threads: 32
 // consecutive nodes x 3 rows x 4 parts.  The update's vector reads are issued
 // before the row's, so they overlap.
 constexpr int kSplitThreads = 384;
-constexpr int64_t kSplitMaxNodes = 16384;
+// Up to here the four threads win.  FP32, bound by memory latency: 3.1-3.6 us
+// against 6.4-7.5 on 225 to 9,537 nodes, 14.8 against 14.1 on 70,785.  FP64, bound
+// by its units: 7-10 us against 21 on 225 to 4,225 nodes, 19-26 against 30 on
+// 30,625.
+template <class T>
+constexpr int64_t split_max_nodes() {
+  return sizeof(T) == 8 ? 100000 : 16384;
+}
 
-template <int MODE>
+template <class T, int MODE>
 __global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
-    MgDims d, const float* __restrict__ A, const uint8_t* __restrict__ act,
-    const float* __restrict__ x, const float* __restrict__ b, const float* __restrict__ invdiag,
-    float omega, float* __restrict__ y, ChebStep ch) {
-  __shared__ float parts[3][3][32];
+    MgDims d, const T* __restrict__ A, const uint8_t* __restrict__ act,
+    const T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ invdiag,
+    T omega, T* __restrict__ y, ChebStep ch) {
+  __shared__ T parts[3][3][32];
   const int t = threadIdx.x, q = t / 96, r = (t / 32) % 3, lane = t & 31;
   const int64_t n = int64_t(blockIdx.x) * 32 + lane;
   const bool valid = n < int64_t(d.nnx) * d.nny * d.nnz;
   const int64_t dof = 3 * n + r;
-  float* dir = static_cast<float*>(ch.dir_);
+  T* dir = static_cast<T*>(ch.dir_);
   bool ac = false;
-  float xv = 0.0f, bv = 0.0f, dv = 0.0f, dprev = 0.0f;
+  T xv = T(0), bv = T(0), dv = T(0), dprev = T(0);
   if (q == 0 && valid) {
     ac = act[dof] != 0;
     if (MODE == kSmooth || MODE == kCheb) xv = x[dof];
@@ -472,19 +484,19 @@ __global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
     if (MODE == kSmooth || MODE == kCheb) dv = invdiag[dof];
     if (MODE == kCheb && ch.step > 0) dprev = dir[dof];
   }
-  float p = 0.0f;
+  T p = T(0);
   if (valid) {
     int a, bb, c;
     node_abc(d, n, a, bb, c);
-    p = stencil_part<float, false>(d, A, x, a, bb, c, r, q);
+    p = stencil_part<T, false>(d, A, x, a, bb, c, r, q);
   }
   if (q > 0) parts[q - 1][r][lane] = p;
   __syncthreads();
   if (q != 0 || !valid) return;
-  const float s = ((p + parts[0][r][lane]) + parts[1][r][lane]) + parts[2][r][lane];
-  float dnew;
-  const float out = stencil_update<float, MODE>(ac, s, xv, bv, dv, omega, ch.coef, ch.step,
-                                                ac ? dprev : 0.0f, dnew);
+  const T s = ((p + parts[0][r][lane]) + parts[1][r][lane]) + parts[2][r][lane];
+  T dnew;
+  const T out = stencil_update<T, MODE>(ac, s, xv, bv, dv, omega, ch.coef, ch.step,
+                                                ac ? dprev : T(0), dnew);
   if (MODE == kCheb) dir[dof] = dnew;
   y[dof] = out;
 }
@@ -556,71 +568,49 @@ __global__ void k_jacobi_first(const T* __restrict__ b, const T* __restrict__ in
 __device__ __forceinline__ bool tail_node(int i, int Ef, int align) {
   return align && (Ef & 1) && i == Ef;
 }
-// Weight of fine node i (= 2N + d) in coarse node N along one axis.
+// Weights of the fine nodes 2N - 1, 2N, 2N + 1 in coarse node N along one axis, 0
+// beyond the grid.
 template <class T>
-__device__ __forceinline__ T axis_w(int i, int N, int d, int Ef, int align) {
-  if (tail_node(i, Ef, align)) return N == (Ef + 1) / 2 ? T(1) : T(0);
-  return d == 0 ? T(1) : T(0.5);
+__device__ __forceinline__ void axis_weights(int N, int Ef, int nf, int align, T (&w)[3]) {
+#pragma unroll
+  for (int d = -1; d <= 1; ++d) {
+    const int i = 2 * N + d;
+    T v = d == 0 ? T(1) : T(0.5);
+    if (tail_node(i, Ef, align)) v = N == (Ef + 1) / 2 ? T(1) : T(0);
+    w[d + 1] = i >= 0 && i < nf ? v : T(0);
+  }
 }
 
-// Restriction R = P^T: coarse node N gathers the (up to 27) fine nodes
-// 2N + delta, delta in {-1,0,1}^3, weight prod(1 or 1/2).  Inactive coarse DOFs
-// get 0; fine residuals are already 0 on inactive fine DOFs.  One thread per
-// coarse node on a 3D grid (x fastest), 32-bit index arithmetic.
-// The restricted residual at coarse node (a, b, c): s[k] = sum of the (up to 27)
-// fine nodes' component k times their weights, in a fixed order.
+// Restriction R = P^T at component k of coarse node (a, b, c): the (up to 27) fine
+// nodes 2N + delta, summed axis by axis -- 39 operations, where a weight product
+// per fine node takes 108.  A fine node beyond the grid has weight 0 and is read
+// at its clamped place.  Fine residuals are already 0 on inactive fine DOFs.
 template <class T, bool COH>
-__device__ __forceinline__ void restrict_node(const MgDims& fd, const MgDims& cd, const T* rf,
-                                              int a, int b, int c, T (&s)[3]) {
-  s[0] = s[1] = s[2] = T(0);
+__device__ __forceinline__ T restrict_dof(const MgDims& fd, const MgDims& cd, const T* rf, int a,
+                                          int b, int c, int k) {
+  T wx[3], wy[3], wz[3];
+  axis_weights<T>(a, fd.ex, fd.nnx, cd.align, wx);
+  axis_weights<T>(b, fd.ey, fd.nny, cd.align, wy);
+  axis_weights<T>(c, fd.ez, fd.nnz, cd.align, wz);
+  int ox[3];
 #pragma unroll
-  for (int dz = -1; dz <= 1; ++dz) {
-    const int k = 2 * c + dz;
-    if (k < 0 || k >= fd.nnz) continue;
-    const T wz = axis_w<T>(k, c, dz, fd.ez, cd.align);
+  for (int d = 0; d < 3; ++d) ox[d] = 3 * min(max(2 * a + d - 1, 0), fd.nnx - 1) + k;
+  T sz = T(0);
 #pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int j = 2 * b + dy;
-      if (j < 0 || j >= fd.nny) continue;
-      const T wy = axis_w<T>(j, b, dy, fd.ey, cd.align) * wz;
+  for (int dz = 0; dz < 3; ++dz) {
+    const int z = min(max(2 * c + dz - 1, 0), fd.nnz - 1);
+    T sy = T(0);
 #pragma unroll
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int i = 2 * a + dx;
-        if (i < 0 || i >= fd.nnx) continue;
-        const T w = axis_w<T>(i, a, dx, fd.ex, cd.align) * wy;
-        const T* q = rf + 3 * ((int64_t(k) * fd.nny + j) * fd.nnx + i);
-        s[0] += w * vload<T, COH>(q);
-        s[1] += w * vload<T, COH>(q + 1);
-        s[2] += w * vload<T, COH>(q + 2);
-      }
+    for (int dy = 0; dy < 3; ++dy) {
+      const int y = min(max(2 * b + dy - 1, 0), fd.nny - 1);
+      const T* row = rf + 3 * (int64_t(z) * fd.nny + y) * fd.nnx;
+      const T sx = fma(wx[2], vload<T, COH>(row + ox[2]),
+                       fma(wx[1], vload<T, COH>(row + ox[1]), wx[0] * vload<T, COH>(row + ox[0])));
+      sy = fma(wy[dy], sx, sy);
     }
+    sz = fma(wz[dz], sy, sz);
   }
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) k_restrict(MgDims fd, MgDims cd, const T* __restrict__ rf,
-                                                  const uint8_t* __restrict__ cact,
-                                                  T* __restrict__ bc, FirstStep<T> first) {
-  const int a = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y * 8 + threadIdx.y, c = blockIdx.z;
-  if (a >= cd.nnx || b >= cd.nny) return;
-  T s[3];
-  restrict_node<T, false>(fd, cd, rf, a, b, c, s);
-  const int64_t n = (int64_t(c) * cd.nny + b) * cd.nnx + a;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int64_t dof = 3 * n + k;
-    const bool ac = cact[dof] != 0;
-    const T bv = ac ? s[k] : T(0);
-    bc[dof] = bv;
-    if (first.kind == 1) {
-      first.x[dof] = first.omega * first.dinv[dof] * bv;
-    } else if (first.kind == 2) {
-      T dnew;
-      first.x[dof] = stencil_update<T, kCheb>(ac, T(0), T(0), bv, first.dinv[dof], T(0),
-                                              first.coef, 0, T(0), dnew);
-      first.chd[dof] = dnew;
-    }
-  }
+  return sz;
 }
 
 // The prolonged correction at fine node (a, b, c): per axis one coarse node
@@ -658,8 +648,56 @@ __device__ __forceinline__ void prolong_node(const MgDims& fd, const MgDims& cd,
   }
 }
 
+// The restriction runs a thread per DOF, consecutive threads on consecutive DOFs
+// of a coarse node layer (blockIdx.y): its reads are half-full lines instead of a
+// node's 12 bytes of every 24, and in FP64 three threads share what one did at 64
+// cycles an instruction (25x25x49 coarse nodes: 19.2 -> 10.5 us; FP32 on
+// 65x33x33: 8.7 -> 6.8, 129x65x65 unchanged at 25).  The row of an entry comes
+// from a multiplication by the row length's reciprocal (n < 2^31: exact).
+struct RowDiv {
+  unsigned len, mul, shift;
+};
+RowDiv row_div(int nnx) {
+  RowDiv r{unsigned(3 * nnx), 0, 0};
+  while ((1ull << r.shift) < r.len) ++r.shift;
+  r.mul = unsigned(((1ull << 32) * ((1ull << r.shift) - r.len)) / r.len + 1);
+  return r;
+}
+__device__ __forceinline__ unsigned row_of(const RowDiv& r, unsigned n) {
+  return (__umulhi(r.mul, n) + n) >> r.shift;
+}
+constexpr int kRestrictThreads = 128;
+
+// Right-hand side of the coarse level (inactive DOFs 0), and its first smoothing
+// step from zero.
+template <class T>
+__global__ void __launch_bounds__(kRestrictThreads) k_restrict(MgDims fd, MgDims cd, RowDiv rd,
+                                                               const T* __restrict__ rf,
+                                                               const uint8_t* __restrict__ cact,
+                                                               T* __restrict__ bc,
+                                                               FirstStep<T> first) {
+  const unsigned id = blockIdx.x * unsigned(kRestrictThreads) + threadIdx.x;
+  const int c = blockIdx.y;
+  if (id >= rd.len * unsigned(cd.nny)) return;
+  const int b = int(row_of(rd, id)), e = int(id - unsigned(b) * rd.len), a = e / 3, k = e - 3 * a;
+  const int64_t dof = int64_t(c) * rd.len * cd.nny + id;
+  const bool ac = cact[dof] != 0;
+  const T s = restrict_dof<T, false>(fd, cd, rf, a, b, c, k);
+  const T bv = ac ? s : T(0);
+  bc[dof] = bv;
+  if (first.kind == 1) {
+    first.x[dof] = first.omega * first.dinv[dof] * bv;
+  } else if (first.kind == 2) {
+    T dnew;
+    first.x[dof] = stencil_update<T, kCheb>(ac, T(0), T(0), bv, first.dinv[dof], T(0), first.coef,
+                                            0, T(0), dnew);
+    first.chd[dof] = dnew;
+  }
+}
+
 // Prolongation + correction: x_f += P e_c on active fine DOFs.  One thread per
-// fine node on a 3D grid.
+// fine node on a 3D grid: a thread per DOF repeats the node's index arithmetic and
+// took 79 us against 33 on 257x129x129 nodes.
 template <class T>
 __global__ void __launch_bounds__(256) k_prolong_add(MgDims fd, MgDims cd,
                                                      const T* __restrict__ ec,
@@ -963,22 +1001,22 @@ void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, co
                    const T* b, const T* invdiag, T omega, T* y, cudaStream_t s,
                    ChebStep ch) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
-  if constexpr (sizeof(T) == 4) {
-    if (nn <= kSplitMaxNodes) {
-      const unsigned ns = unsigned((nn + 31) / 32);
-      if (mode == kApply)
-        k_stencil_split<kApply><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-      else if (mode == kResidual)
-        k_stencil_split<kResidual><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
-                                                                ch);
-      else if (mode == kCheb)
-        k_stencil_split<kCheb><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-      else
-        k_stencil_split<kSmooth><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
+  if (nn <= split_max_nodes<T>()) {
+    const unsigned ns = unsigned((nn + 31) / 32);
+    if (mode == kApply)
+      k_stencil_split<T, kApply><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
                                                               ch);
-      TG_LAUNCH_CHECK();
-      return;
-    }
+    else if (mode == kResidual)
+      k_stencil_split<T, kResidual><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega,
+                                                                 y, ch);
+    else if (mode == kCheb)
+      k_stencil_split<T, kCheb><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
+                                                             ch);
+    else
+      k_stencil_split<T, kSmooth><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
+                                                               ch);
+    TG_LAUNCH_CHECK();
+    return;
   }
   const int64_t items = (nn + 31) / 32 * 96;
   const unsigned nb = unsigned((items + kStencilThreads - 1) / kStencilThreads);
@@ -1035,8 +1073,8 @@ void mg_jacobi_first(const T* b, const T* invdiag, T omega, int64_t n, T* x, cud
 template <class T>
 void mg_restrict(const MgDims& fd, const MgDims& cd, const T* rf, const uint8_t* cact, T* bc,
                  cudaStream_t s, FirstStep<T> first) {
-  const dim3 grid((cd.nnx + 31) / 32, (cd.nny + 7) / 8, cd.nnz);
-  k_restrict<T><<<grid, dim3(32, 8), 0, s>>>(fd, cd, rf, cact, bc, first);
+  const dim3 grid((3 * cd.nnx * cd.nny + kRestrictThreads - 1) / kRestrictThreads, cd.nnz);
+  k_restrict<T><<<grid, kRestrictThreads, 0, s>>>(fd, cd, row_div(cd.nnx), rf, cact, bc, first);
   TG_LAUNCH_CHECK();
 }
 
@@ -1129,7 +1167,7 @@ TG_INST(float)
 // thousand DOFs whose cost is its latency.  Here every step of the same
 // V-cycle is a phase of one kernel -- a
 // cluster-stride loop with the arithmetic and summation order of the separate
-// kernels (stencil_row, restrict_node, prolong_node, the coarsest inverse) --
+// kernels (stencil_row, restrict_dof, prolong_node, the coarsest inverse) --
 // and phases are separated by the cluster's hardware barrier (release/acquire
 // at cluster scope, no spin loop).  The restriction into a level and that
 // level's first smoothing step (from a zero iterate, so it needs no operator)
@@ -1225,12 +1263,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_coarse_vcycle(FusedCoarse 
     for (int64_t n = tid; n < nn; n += nthreads) {
       int a, b, c;
       node_abc(C.d, n, a, b, c);
-      float s[3];
-      restrict_node<float, true>(F.d, C.d, rf, a, b, c, s);
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const int64_t dof = 3 * n + k;
-        const float bv = C.act[dof] ? s[k] : 0.0f;
+        const float s = restrict_dof<float, true>(F.d, C.d, rf, a, b, c, k);
+        const float bv = C.act[dof] ? s : 0.0f;
         C.b[dof] = bv;
         if (!smoothed) continue;
         if (fc.cheb_m > 0) {
