@@ -115,6 +115,79 @@ __device__ __forceinline__ double bred(double v, double* sh) {
   return s;
 }
 
+// Running sums of r.r and r.(D^-1 r).  FP64 data: FP64.  FP32 data: each product
+// exact as a value and its rounding error (one FMA), accumulated as an unevaluated
+// FP32 pair (Knuth's TwoSum; the errors in the low part), about 2^-46 relative.
+// Alpha and beta, rounded to FP32, and the iteration counts come out the same as
+// from FP64 sums, whose five instructions per DOF on units 58 times slower took
+// twice the operator's time (24 systems of 32^3: 34 us against 17).
+template <class T>
+struct RrRz;
+template <>
+struct RrRz<double> {
+  double a = 0.0, b = 0.0;
+  __device__ __forceinline__ void add(double v, double iv) {
+    a += v * v;
+    b += v * (iv * v);
+  }
+  // The block's sums into prr, prz[0].
+  __device__ __forceinline__ void store(double* prr, double* prz, double* sh) const {
+    const double ta = bred(a, sh), tb = bred(b, sh);
+    if (threadIdx.x == 0) {
+      *prr = ta;
+      *prz = tb;
+    }
+  }
+};
+template <>
+struct RrRz<float> {
+  float ah = 0.0f, al = 0.0f, bh = 0.0f, bl = 0.0f;
+  __device__ __forceinline__ void add(float v, float iv) {
+    const float p = __fmul_rn(v, v), pe = __fmaf_rn(v, v, -p);
+    const df s = two_sum(ah, p);
+    ah = s.hi;
+    al = __fadd_rn(al, __fadd_rn(s.lo, pe));
+    const float q = __fmul_rn(iv, v), qe = __fmaf_rn(iv, v, -q);
+    const float m = __fmul_rn(q, v), me = __fmaf_rn(qe, v, __fmaf_rn(q, v, -m));
+    const df t = two_sum(bh, m);
+    bh = t.hi;
+    bl = __fadd_rn(bl, __fadd_rn(t.lo, me));
+  }
+  // Across the warp as pairs too (an FP64 addition holds its scheduler 64 cycles),
+  // then one FP64 sum over the warps.
+  __device__ __forceinline__ void store(double* prr, double* prz, double* sh) const {
+    df a = quick_two_sum(ah, al), b = quick_two_sum(bh, bl);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a = a + df(__shfl_down_sync(0xffffffffu, a.hi, o), __shfl_down_sync(0xffffffffu, a.lo, o));
+      b = b + df(__shfl_down_sync(0xffffffffu, b.hi, o), __shfl_down_sync(0xffffffffu, b.lo, o));
+    }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) {
+      sh[wid] = df_to_double(a);
+      sh[kT / 32 + wid] = df_to_double(b);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      double t = 0.0;
+      for (int q = 0; q < kT / 32; ++q) t += sh[threadIdx.x * (kT / 32) + q];
+      *(threadIdx.x == 0 ? prr : prz) = t;
+    }
+  }
+};
+
+// f(index, count) over this CTA's share of a system's nd DOFs: runs of four when
+// they can be read 16 bytes at a time (FP32, nd a multiple of 4), else single DOFs.
+template <class T, class F4, class F1>
+__device__ __forceinline__ void share(int64_t nd, F4&& f4, F1&& f1) {
+  const int64_t t0 = blockIdx.x * int64_t(kT) + threadIdx.x, st = int64_t(gridDim.x) * kT;
+  if (sizeof(T) == 4 && (nd & 3) == 0) {
+    for (int64_t q = t0; q < (nd >> 2); q += st) f4(q);
+  } else {
+    for (int64_t d = t0; d < nd; d += st) f1(d);
+  }
+}
+
 // rr = r.r, rz = r.(D^-1 r) per system.
 template <class T>
 __global__ void k_b_rr_rz(const T* __restrict__ R, const T* __restrict__ invd, int64_t nd,
@@ -123,18 +196,19 @@ __global__ void k_b_rr_rz(const T* __restrict__ R, const T* __restrict__ invd, i
   const int bi = blockIdx.y, P = gridDim.x;
   const T* r = R + bi * nd;
   const T* iv = invd + (bi / nrhs) * nd;
-  double a = 0.0, b = 0.0;
-  for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd; d += int64_t(P) * kT) {
-    const double v = double(r[d]);
-    a += v * v;
-    b += v * (double(iv[d]) * v);
-  }
-  a = bred(a, sh);
-  b = bred(b, sh);
-  if (threadIdx.x == 0) {
-    prr[int64_t(bi) * P + blockIdx.x] = a;
-    prz[int64_t(bi) * P + blockIdx.x] = b;
-  }
+  RrRz<T> acc;
+  for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd; d += int64_t(P) * kT)
+    acc.add(r[d], iv[d]);
+  acc.store(prr + int64_t(bi) * P + blockIdx.x, prz + int64_t(bi) * P + blockIdx.x, sh);
+}
+
+// Sum of n partials by one warp, in a fixed order; valid in lane 0.
+__device__ __forceinline__ double warp_partials(const double* __restrict__ part, int n) {
+  double s = 0.0;
+  for (int q = threadIdx.x & 31; q < n; q += 32) s += part[q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  return s;
 }
 
 // One warp per system: out[bi] = sum of its P partials, in order.
@@ -216,85 +290,141 @@ __global__ void k_b_init(int B, const double* __restrict__ rr, const double* __r
   act[bi] = (b2 > 0.0 && !(b2 < t)) ? 1 : 0;
 }
 
-// x += alpha p, r -= alpha t for iterating systems (alpha = absNew / p.Ap), with
-// the partials of r.r and r.(D^-1 r) of the updated residual.
+// One CG iteration after the operator is two launches; each CTA sums the partials
+// it needs itself (a few dozen, by one warp, in a fixed order), so no launch only
+// adds numbers up.  A launch of a few microseconds for each of the sums, the
+// scalars and the counter had been a third of an iteration.
+
+// x += alpha p, r -= alpha t for iterating systems (alpha = absNew / p.Ap, p.Ap the
+// sum of the operator's npap partials, kept in pap), with the partials of r.r and
+// r.(D^-1 r) of the updated residual.
 template <class T>
-__global__ void k_b_xr(T* __restrict__ X, T* __restrict__ R, const T* __restrict__ Pv,
-                       const T* __restrict__ Tv, const T* __restrict__ invd, int64_t nd, int nrhs,
-                       const double* __restrict__ absn, const double* __restrict__ pap,
-                       const int* __restrict__ act, double* __restrict__ prr,
-                       double* __restrict__ prz) {
+__global__ void __launch_bounds__(kT) k_b_xr(T* __restrict__ X, T* __restrict__ R,
+                                             const T* __restrict__ Pv, const T* __restrict__ Tv,
+                                             const T* __restrict__ invd, int64_t nd, int nrhs,
+                                             const double* __restrict__ absn,
+                                             const double* __restrict__ ppap, int npap,
+                                             double* __restrict__ pap,
+                                             const int* __restrict__ act,
+                                             double* __restrict__ prr, double* __restrict__ prz) {
   __shared__ double sh[32];
+  __shared__ double s_pa;
   const int bi = blockIdx.y, P = gridDim.x;
-  double a = 0.0, b = 0.0;
-  if (act[bi] == 1) {
-    const double pa = pap[bi];
-    const T alpha = T(pa > 0.0 ? absn[bi] / pa : 0.0);
-    const T* iv = invd + (bi / nrhs) * nd;
-    T* x = X + bi * nd;
-    T* r = R + bi * nd;
-    const T* p = Pv + bi * nd;
-    const T* t = Tv + bi * nd;
-    for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd; d += int64_t(P) * kT) {
-      x[d] += alpha * p[d];
-      const T v = r[d] - alpha * t[d];
-      r[d] = v;
-      const double vd = double(v);
-      a += vd * vd;
-      b += vd * (double(iv[d]) * vd);
+  if (act[bi] != 1) return;  // uniform over the CTA; its partials are not read
+  if (threadIdx.x < 32) {
+    const double v = warp_partials(ppap + int64_t(bi) * npap, npap);
+    if (threadIdx.x == 0) {
+      s_pa = v;
+      if (blockIdx.x == 0) pap[bi] = v;
     }
   }
-  a = bred(a, sh);
-  b = bred(b, sh);
-  if (threadIdx.x == 0) {
-    prr[int64_t(bi) * P + blockIdx.x] = a;
-    prz[int64_t(bi) * P + blockIdx.x] = b;
-  }
+  __syncthreads();
+  const double pa = s_pa;
+  const T alpha = T(pa > 0.0 ? absn[bi] / pa : 0.0);
+  const T* iv = invd + (bi / nrhs) * nd;
+  T* x = X + bi * nd;
+  T* r = R + bi * nd;
+  const T* p = Pv + bi * nd;
+  const T* t = Tv + bi * nd;
+  RrRz<T> acc;
+  share<T>(
+      nd,
+      [&](int64_t q) {
+        float4 xv = reinterpret_cast<float4*>(x)[q], rv = reinterpret_cast<float4*>(r)[q];
+        const float4 pv = reinterpret_cast<const float4*>(p)[q],
+                     tv = reinterpret_cast<const float4*>(t)[q],
+                     dv = reinterpret_cast<const float4*>(iv)[q];
+        const float al = float(alpha);
+        xv.x += al * pv.x; xv.y += al * pv.y; xv.z += al * pv.z; xv.w += al * pv.w;
+        rv.x -= al * tv.x; rv.y -= al * tv.y; rv.z -= al * tv.z; rv.w -= al * tv.w;
+        reinterpret_cast<float4*>(x)[q] = xv;
+        reinterpret_cast<float4*>(r)[q] = rv;
+        acc.add(T(rv.x), T(dv.x));
+        acc.add(T(rv.y), T(dv.y));
+        acc.add(T(rv.z), T(dv.z));
+        acc.add(T(rv.w), T(dv.w));
+      },
+      [&](int64_t d) {
+        x[d] += alpha * p[d];
+        const T v = r[d] - alpha * t[d];
+        r[d] = v;
+        acc.add(v, iv[d]);
+      });
+  acc.store(prr + int64_t(bi) * P + blockIdx.x, prz + int64_t(bi) * P + blockIdx.x, sh);
 }
 
-// The scalar step of every iterating system: stop at the threshold (this
-// iteration not counted, as Eigen), else beta = rz / absNew, absNew = rz, one
-// more iteration, and stop at the budget.  nact counts the systems still iterating.
-__global__ void k_b_scalars(int B, const double* __restrict__ rr, const double* __restrict__ rz,
-                            const double* __restrict__ thr, const double* __restrict__ pap,
-                            int max_it, int* __restrict__ act, int* __restrict__ it,
-                            double* __restrict__ absn, double* __restrict__ beta,
-                            int* __restrict__ nact) {
-  const int bi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bi >= B || act[bi] != 1) return;
-  if (!(pap[bi] > 0.0)) {
-    act[bi] = 2;  // breakdown: p.Ap <= 0
-    return;
-  }
-  if (rr[bi] < thr[bi]) {
-    act[bi] = 0;
-    return;
-  }
-  beta[bi] = rz[bi] / absn[bi];
-  absn[bi] = rz[bi];
-  const int n = it[bi] + 1;
-  it[bi] = n;
-  if (n >= max_it) {
-    act[bi] = 2;
-    return;
-  }
-  atomicAdd(nact, 1);
-}
-
-// p = D^-1 r + beta p for iterating systems.
+// The scalar step of every iterating system, by each of its CTAs: stop at the
+// threshold (this iteration not counted, as Eigen), else beta = rz / absNew, absNew
+// = rz, one more iteration, and stop at the budget; then p = D^-1 r + beta p.  The
+// state (act, absNew, it) is read from one buffer and written, by CTA 0, to the
+// other, so that no CTA reads what another has updated.  nact counts the systems still
+// iterating.
 template <class T>
-__global__ void k_b_p(T* __restrict__ Pv, const T* __restrict__ R, const T* __restrict__ invd,
-                      int64_t nd, int nrhs, const double* __restrict__ beta,
-                      const int* __restrict__ act) {
+__global__ void __launch_bounds__(kT) k_b_p(T* __restrict__ Pv, const T* __restrict__ R,
+                                            const T* __restrict__ invd, int64_t nd, int nrhs,
+                                            const double* __restrict__ prr,
+                                            const double* __restrict__ prz, int np,
+                                            const double* __restrict__ thr,
+                                            const double* __restrict__ pap, int max_it,
+                                            const int* __restrict__ act_in,
+                                            int* __restrict__ act_out,
+                                            const double* __restrict__ absn_in,
+                                            double* __restrict__ absn_out,
+                                            const int* __restrict__ it_in, int* __restrict__ it_out,
+                                            double* __restrict__ rr_out,
+                                            int* __restrict__ nact) {
+  __shared__ double s_rz;
+  __shared__ int s_act;
   const int bi = blockIdx.y;
-  if (act[bi] != 1) return;
-  const T bt = T(beta[bi]);
+  const int a0 = act_in[bi];
+  if (a0 != 1) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      act_out[bi] = a0;
+      it_out[bi] = it_in[bi];
+      rr_out[bi] = 0.0;
+    }
+    return;
+  }
+  if (threadIdx.x < 32) {
+    const double rr = warp_partials(prr + int64_t(bi) * np, np);
+    const double rz = warp_partials(prz + int64_t(bi) * np, np);
+    if (threadIdx.x == 0) {
+      int a = 1;
+      if (!(pap[bi] > 0.0))
+        a = 2;  // breakdown: p.Ap <= 0
+      else if (rr < thr[bi])
+        a = 0;
+      const int n = it_in[bi] + (a == 1 ? 1 : 0);
+      if (a == 1 && n >= max_it) a = 2;
+      s_rz = rz;
+      s_act = a;
+      if (blockIdx.x == 0) {
+        rr_out[bi] = rr;
+        act_out[bi] = a;
+        absn_out[bi] = rz;
+        it_out[bi] = n;
+        if (a == 1) atomicAdd(nact, 1);
+      }
+    }
+  }
+  __syncthreads();
+  if (s_act != 1) return;
+  const T bt = T(s_rz / absn_in[bi]);
   const T* iv = invd + (bi / nrhs) * nd;
   T* p = Pv + bi * nd;
   const T* r = R + bi * nd;
-  for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd;
-       d += int64_t(gridDim.x) * kT)
-    p[d] = iv[d] * r[d] + bt * p[d];
+  share<T>(
+      nd,
+      [&](int64_t q) {
+        float4 pv = reinterpret_cast<float4*>(p)[q];
+        const float4 rv = reinterpret_cast<const float4*>(r)[q],
+                     dv = reinterpret_cast<const float4*>(iv)[q];
+        const float b = float(bt);
+        pv.x = dv.x * rv.x + b * pv.x; pv.y = dv.y * rv.y + b * pv.y;
+        pv.z = dv.z * rv.z + b * pv.z; pv.w = dv.w * rv.w + b * pv.w;
+        reinterpret_cast<float4*>(p)[q] = pv;
+      },
+      [&](int64_t d) { p[d] = iv[d] * r[d] + bt * p[d]; });
 }
 
 // Mixed form: X64 += |r| * X32 for the systems that ran.
@@ -356,24 +486,29 @@ struct Batch {
   ModalConsts mc;
   const uint8_t* kept;
   cudaStream_t s;
-  DBuf<double> prr, prz, ppap, rr, rz, pap, thr, rhs2, absn, beta, rn;
-  DBuf<int> act, it, nact, run, nrun;
+  DBuf<double> prr, prz, ppap, rr, rz, pap, thr, rhs2, absn, rn;
+  DBuf<int> act, it, nact, run, nrun;  // absn, act and it: two buffers of B, used in turn
   int64_t iterations_total = 0;
   int iterations_max = 0;
-  void init(int B_, int64_t nd_, int P_) {
-    B = B_;
+  const int* act_last = nullptr;  // the state pcg() ended with
+  void init(int systems, int64_t nd_, int P_) {
     nd = nd_;
     P = P_;
+    B = systems;
     const int Pop = std::max(periodic_op_blocks<double>(nx, ny, nz),
                              periodic_op_blocks<float>(nx, ny, nz));
     prr.alloc(size_t(B) * P);
     prz.alloc(size_t(B) * P);
     ppap.alloc(size_t(B) * Pop);
-    for (DBuf<double>* d : {&rr, &rz, &pap, &thr, &rhs2, &absn, &beta, &rn}) d->alloc(size_t(B));
-    for (DBuf<int>* d : {&act, &it, &run}) d->alloc(size_t(B));
-    nact.alloc(1);
+    for (DBuf<double>* d : {&rr, &rz, &pap, &thr, &rhs2, &rn}) d->alloc(size_t(B));
+    absn.alloc(size_t(2 * B));
+    act.alloc(size_t(2 * B));
+    it.alloc(size_t(2 * B));
+    run.alloc(size_t(B));
+    nact.alloc(kCheck);
     nrun.alloc(1);
   }
+  static constexpr int kCheck = 8;  // iterations between the host's looks at nact
   dim3 g2() const { return dim3(static_cast<unsigned>(P), static_cast<unsigned>(B)); }
   int sb() const { return (B + 255) / 256; }
   int wb() const { return (B * 32 + 255) / 256; }
@@ -393,30 +528,29 @@ struct Batch {
     k_b_init<<<sb(), 256, 0, s>>>(B, rr.p, rz.p, tol, runp, act.p, it.p, thr.p, rhs2.p, absn.p);
     TG_LAUNCH_CHECK();
     const int Pop = periodic_op_blocks<T>(nx, ny, nz);
-    int host_nact = B;
-    for (int k = 0; k < max_it && host_nact > 0; ++k) {
+    int host_nact = B, k = 0;
+    for (; k < max_it && host_nact > 0; ++k) {
+      const size_t in = size_t(k & 1) * size_t(B), out = size_t((k + 1) & 1) * size_t(B);
+      const int slot = k % kCheck;
+      if (slot == 0) TG_CUDA(cudaMemsetAsync(nact.p, 0, kCheck * sizeof(int), s));
       launch_periodic_op<T>(kApply, nx, ny, nz, mc, ef, kept, Pv, nullptr, Tv, ppap.p, B, nrhs,
-                            act.p, s);
-      k_bsum<<<wb(), 256, 0, s>>>(ppap.p, Pop, B, pap.p, nullptr, nullptr);
+                            act.p + in, s);
+      k_b_xr<T><<<g2(), kT, 0, s>>>(X, R, Pv, Tv, invd, nd, nrhs, absn.p + in, ppap.p, Pop, pap.p,
+                                    act.p + in, prr.p, prz.p);
       TG_LAUNCH_CHECK();
-      k_b_xr<T><<<g2(), kT, 0, s>>>(X, R, Pv, Tv, invd, nd, nrhs, absn.p, pap.p, act.p, prr.p,
-                                    prz.p);
+      k_b_p<T><<<g2(), kT, 0, s>>>(Pv, R, invd, nd, nrhs, prr.p, prz.p, P, thr.p, pap.p, max_it,
+                                   act.p + in, act.p + out, absn.p + in, absn.p + out, it.p + in,
+                                   it.p + out, rr.p, nact.p + slot);
       TG_LAUNCH_CHECK();
-      k_bsum<<<wb(), 256, 0, s>>>(prr.p, P, B, rr.p, prz.p, rz.p);
-      TG_LAUNCH_CHECK();
-      TG_CUDA(cudaMemsetAsync(nact.p, 0, sizeof(int), s));
-      k_b_scalars<<<sb(), 256, 0, s>>>(B, rr.p, rz.p, thr.p, pap.p, max_it, act.p, it.p, absn.p,
-                                       beta.p, nact.p);
-      TG_LAUNCH_CHECK();
-      k_b_p<T><<<g2(), kT, 0, s>>>(Pv, R, invd, nd, nrhs, beta.p, act.p);
-      TG_LAUNCH_CHECK();
-      if ((k & 7) == 7) {
-        TG_CUDA(cudaMemcpyAsync(&host_nact, nact.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+      if (slot == kCheck - 1) {
+        TG_CUDA(cudaMemcpyAsync(&host_nact, nact.p + slot, sizeof(int), cudaMemcpyDeviceToHost, s));
         TG_CUDA(cudaStreamSynchronize(s));
       }
     }
+    act_last = act.p + size_t(k & 1) * size_t(B);
     std::vector<int> hit(static_cast<size_t>(B));
-    TG_CUDA(cudaMemcpyAsync(hit.data(), it.p, sizeof(int) * B, cudaMemcpyDeviceToHost, s));
+    TG_CUDA(cudaMemcpyAsync(hit.data(), it.p + size_t(k & 1) * size_t(B), sizeof(int) * B,
+                            cudaMemcpyDeviceToHost, s));
     TG_CUDA(cudaStreamSynchronize(s));
     int mx = 0;
     for (int v : hit) {
@@ -514,73 +648,88 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
     bt.mc = ModalConsts::make(poisson, spacing);
     bt.mc.kdiag = ke[0];
     bt.s = s;
+    // All cells together: solving them a group at a time, so that a group's CG
+    // vectors stay in L2, measured slower (32 cells of 32^3: 109 ms in groups of 8,
+    // 96 in groups of 16, 80 at once) -- the launches of a group are too short to
+    // fill the GPU.
+    const bool mixed = precision == TG_PREC_MIXED;
     DBuf<uint8_t> dtags, kept;
     DBuf<double> ef, invd, F, Bv, X, R, Pv, Tv;
+    DBuf<float> eff32, invd32, Xf, Rf, Pf, Tf;
     dtags.alloc(size_t(ncell * np));
-    TG_CUDA(cudaMemcpyAsync(dtags.p, tags, size_t(ncell * np), cudaMemcpyHostToDevice, s));
     ef.alloc(size_t(ncell * np));
     kept.alloc(size_t(ncell * np));
     invd.alloc(size_t(ncell * nd));
     F.alloc(size_t(ncell * 6 * nd));
     for (DBuf<double>* v : {&Bv, &X, &R}) v->alloc(size_t(B) * size_t(nd));
-    const int nb_cell = int(std::min<int64_t>((ncell * np + kT - 1) / kT, 152 * 64));
-    k_homog_cell<<<nb_cell, kT, 0, s>>>(dtags.p, ncell, nx, ny, nz, youngs_modulus, bt.mc.kdiag,
-                                         cl, ef.p, kept.p, invd.p, F.p);
-    TG_LAUNCH_CHECK();
+    if (mixed) {
+      eff32.alloc(size_t(ncell * np));
+      invd32.alloc(size_t(ncell * nd));
+      for (DBuf<float>* v : {&Xf, &Rf, &Pf, &Tf}) v->alloc(size_t(B) * size_t(nd));
+    } else {
+      Pv.alloc(size_t(B) * size_t(nd));
+      Tv.alloc(size_t(B) * size_t(nd));
+    }
     bt.kept = kept.p;
-    const int P = int(std::max<int64_t>(1, std::min<int64_t>(64, (nd + kT * 8 - 1) / (kT * 8))));
+    // CTAs per system of the vector kernels: 12 DOFs a thread up to 16 CTAs, then 24,
+    // so that the two block sums weigh little (32^3: 16 against 48 CTAs, 80 ms
+    // against 121) and a single small cell still has a few CTAs (12^3: 4.4 ms
+    // with two per system, 5.0 with one).
+    const int64_t per12 = (nd + 12 * kT - 1) / (12 * kT), per24 = (nd + 24 * kT - 1) / (24 * kT);
+    const int P = int(std::min<int64_t>(64, std::max(std::min<int64_t>(16, per12), per24)));
     bt.init(B, nd, P);
     DBuf<int> djl(static_cast<size_t>(B));
     std::vector<int> jl_sys(static_cast<size_t>(B));
     for (int bi = 0; bi < B; ++bi) jl_sys[size_t(bi)] = jl[size_t(bi % nrhs)];
     TG_CUDA(cudaMemcpyAsync(djl.p, jl_sys.data(), sizeof(int) * B, cudaMemcpyHostToDevice, s));
-    k_b_start<<<bt.g2(), kT, 0, s>>>(F.p, djl.p, nd, nrhs, Bv.p, X.p, R.p);
-    TG_LAUNCH_CHECK();
+    DBuf<double> thr_o(static_cast<size_t>(B)), b2(static_cast<size_t>(B));
+    DBuf<double> pfx(size_t(B) * 6 * P), fx(size_t(B) * 6);
+    std::vector<double> hb2(static_cast<size_t>(B)), hthr(static_cast<size_t>(B)),
+        hrr(static_cast<size_t>(B)), hfx(static_cast<size_t>(B) * 6);
+    std::vector<int> hact(static_cast<size_t>(B));
     TG_CUDA(cudaStreamSynchronize(s));
     inf.t_setup_ms = now_ms() - t0;
     const double ts = now_ms();
     bool all_ok = true;
-    if (precision == TG_PREC_FP64) {
-      Pv.alloc(size_t(B) * size_t(nd));
-      Tv.alloc(size_t(B) * size_t(nd));
+    const double vol = double(np) * spacing * spacing * spacing;
+    TG_CUDA(cudaMemcpyAsync(dtags.p, tags, size_t(ncell * np), cudaMemcpyHostToDevice, s));
+    const int nb_cell = int(std::min<int64_t>((ncell * np + kT - 1) / kT, 152 * 64));
+    k_homog_cell<<<nb_cell, kT, 0, s>>>(dtags.p, ncell, nx, ny, nz, youngs_modulus, bt.mc.kdiag, cl,
+                                         ef.p, kept.p, invd.p, F.p);
+    TG_LAUNCH_CHECK();
+    k_b_start<<<bt.g2(), kT, 0, s>>>(F.p, djl.p, nd, nrhs, Bv.p, X.p, R.p);
+    TG_LAUNCH_CHECK();
+    if (!mixed) {
       bt.pcg<double>(X.p, R.p, Pv.p, Tv.p, ef.p, invd.p, tolerance, max_it, nullptr, nullptr);
-      std::vector<double> hrr(static_cast<size_t>(B)), hb2(static_cast<size_t>(B));
-      std::vector<int> hact(static_cast<size_t>(B));
       TG_CUDA(cudaMemcpyAsync(hrr.data(), bt.rr.p, sizeof(double) * B, cudaMemcpyDeviceToHost, s));
       TG_CUDA(cudaMemcpyAsync(hb2.data(), bt.rhs2.p, sizeof(double) * B, cudaMemcpyDeviceToHost, s));
-      TG_CUDA(cudaMemcpyAsync(hact.data(), bt.act.p, sizeof(int) * B, cudaMemcpyDeviceToHost, s));
+      TG_CUDA(cudaMemcpyAsync(hact.data(), bt.act_last, sizeof(int) * B, cudaMemcpyDeviceToHost, s));
       TG_CUDA(cudaStreamSynchronize(s));
       for (int bi = 0; bi < B; ++bi)
-        if (!(hact[size_t(bi)] == 0 &&
-              (hb2[size_t(bi)] == 0.0 || std::sqrt(hrr[size_t(bi)] / hb2[size_t(bi)]) <= tolerance)))
+        if (!(hact[size_t(bi)] == 0 && (hb2[size_t(bi)] == 0.0 ||
+                                        std::sqrt(hrr[size_t(bi)] / hb2[size_t(bi)]) <= tolerance)))
           all_ok = false;
     } else {
       // FP64 refinement around FP32 inner solves (relative 1e-3 each).
-      DBuf<float> eff32, invd32, Xf, Rf, Pf, Tf;
-      eff32.alloc(size_t(ncell * np));
-      invd32.alloc(size_t(ncell * nd));
-      for (DBuf<float>* v : {&Xf, &Rf, &Pf, &Tf}) v->alloc(size_t(B) * size_t(nd));
       k_to_f32<<<nb_cell, kT, 0, s>>>(ef.p, eff32.p, ncell * np);
       TG_LAUNCH_CHECK();
       k_to_f32<<<nb_cell, kT, 0, s>>>(invd.p, invd32.p, ncell * nd);
       TG_LAUNCH_CHECK();
-      DBuf<double> thr_o(static_cast<size_t>(B)), b2(static_cast<size_t>(B));
       // |b|^2 and the outer threshold tol^2 |b|^2.
       k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
       TG_LAUNCH_CHECK();
       k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, b2.p, nullptr, nullptr);
       TG_LAUNCH_CHECK();
-      std::vector<double> hb2(static_cast<size_t>(B)), hthr(static_cast<size_t>(B));
       TG_CUDA(cudaMemcpyAsync(hb2.data(), b2.p, sizeof(double) * B, cudaMemcpyDeviceToHost, s));
       TG_CUDA(cudaStreamSynchronize(s));
       for (int bi = 0; bi < B; ++bi)
         hthr[size_t(bi)] = std::max(tolerance * tolerance * hb2[size_t(bi)], DBL_MIN);
       TG_CUDA(cudaMemcpyAsync(thr_o.p, hthr.data(), sizeof(double) * B, cudaMemcpyHostToDevice, s));
-      std::vector<double> hrr(static_cast<size_t>(B));
       const int max_ref = 30;
-      int budget = max_it;
+      int budget = max_it, refinements = 0;
       for (int ref = 0;; ++ref) {
-        // r = b - A x (FP64) -- the first residual is b itself (x = 0).
+        // r = b - A x (FP64) -- the first residual is b itself (x = 0); later, of
+        // the systems the last inner solve ran for (the others' is current).
         if (ref > 0)
           launch_periodic_op<double>(kResidual, nx, ny, nz, bt.mc, ef.p, kept.p, X.p, Bv.p, R.p,
                                      nullptr, B, nrhs, bt.run.p, s);
@@ -599,12 +748,13 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
           all_ok = false;
           break;
         }
-        ++inf.refinements;
+        ++refinements;
         budget -= bt.pcg<float>(Xf.p, Rf.p, Pf.p, Tf.p, eff32.p, invd32.p, 1e-3, budget, bt.run.p,
                                 R.p);
         k_b_correct<<<bt.g2(), kT, 0, s>>>(X.p, Xf.p, bt.rn.p, bt.run.p, nd);
         TG_LAUNCH_CHECK();
       }
+      inf.refinements = std::max(inf.refinements, refinements);
       // Converged: every final FP64 residual below its threshold (NaN fails).
       TG_CUDA(cudaMemcpyAsync(hrr.data(), bt.rr.p, sizeof(double) * B, cudaMemcpyDeviceToHost, s));
       TG_CUDA(cudaStreamSynchronize(s));
@@ -612,23 +762,13 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
         if (!(hrr[size_t(bi)] < hthr[size_t(bi)]) && hb2[size_t(bi)] > 0.0) all_ok = false;
     }
     // CH from F_I . chi_J.
-    DBuf<double> pfx(size_t(B) * 6 * P), fx(size_t(B) * 6);
-    {
-      const dim3 g(static_cast<unsigned>(P), static_cast<unsigned>(B), 6u);
-      k_b_fx<<<g, kT, 0, s>>>(F.p, X.p, nd, nrhs, pfx.p);
-      TG_LAUNCH_CHECK();
-      k_bsum<<<(B * 6 * 32 + 255) / 256, 256, 0, s>>>(pfx.p, P, B * 6, fx.p, nullptr, nullptr);
-      TG_LAUNCH_CHECK();
-    }
-    std::vector<double> hfx(static_cast<size_t>(B) * 6);
+    const dim3 g(static_cast<unsigned>(P), static_cast<unsigned>(B), 6u);
+    k_b_fx<<<g, kT, 0, s>>>(F.p, X.p, nd, nrhs, pfx.p);
+    TG_LAUNCH_CHECK();
+    k_bsum<<<(B * 6 * 32 + 255) / 256, 256, 0, s>>>(pfx.p, P, B * 6, fx.p, nullptr, nullptr);
+    TG_LAUNCH_CHECK();
     TG_CUDA(cudaMemcpyAsync(hfx.data(), fx.p, sizeof(double) * B * 6, cudaMemcpyDeviceToHost, s));
     TG_CUDA(cudaStreamSynchronize(s));
-    inf.t_solve_ms = now_ms() - ts;
-    inf.systems = B;
-    inf.iterations_max = bt.iterations_max;
-    inf.iterations_total = bt.iterations_total;
-    inf.converged = all_ok ? 1 : 0;
-    const double vol = double(np) * spacing * spacing * spacing;
     for (int c = 0; c < ncell; ++c) {
       double* ch = ch_out + int64_t(c) * 36;
       std::fill(ch, ch + 36, 0.0);
@@ -639,6 +779,11 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
               (double(nsolid[size_t(c)]) * c0[I][J] - hfx[size_t(bi) * 6 + I]) / vol;
       }
     }
+    inf.t_solve_ms = now_ms() - ts;
+    inf.systems = B;
+    inf.iterations_max = bt.iterations_max;
+    inf.iterations_total = bt.iterations_total;
+    inf.converged = all_ok ? 1 : 0;
   } catch (const Error& e) {
     set_last_error(e.what());
     rc = e.code;

@@ -52,12 +52,14 @@ struct GridDev {
 };
 
 // Batched periodic applies (homogenization): system bi of the batch reads x, b,
-// y at bi * sx and the cell fields (factors, kept bits) of cell bi / nrhs.  On the torus nodes and elements coincide (nnx == nx ...).
+// y at bi * sx and the cell fields (factors, kept bits) of cell bi / nrhs.  On the
+// torus nodes and elements coincide (nnx == nx ...).
 // Systems whose entry of `run` is not 1 are skipped: their y and partials stay.
 struct BatchDev {
   int nrhs;         // systems per cell
   int64_t sx, se;   // strides: DOF vectors; a cell's element factors and kept bits
   const int* run;   // null: every system
+  int flat;         // rows numbered in one sequence of nx + 2 columns (periodic_flat)
 };
 
 __device__ __forceinline__ int wrap_index(int a, int n) {
@@ -114,8 +116,10 @@ __device__ __forceinline__ double block_sum(double v) {
 //      right neighbour itself, a load its arithmetic hides).
 //      At a strip's end the next lane belongs to another strip: the element
 //      column there lies past the grid, its factor is 0.
-//      Periodic cells of at most 32 columns: a row is a group of nx lanes with
-//      no halo, 32 / nx rows side by side in a warp.
+//      Periodic cells: a row is a group of nx lanes with no halo, 32 / nx rows
+//      side by side in a warp (nx 8, 16, 32 fill it); where that leaves more lanes
+//      idle than two halo columns per row do (nx 17-26, or above 32), rows of
+//      nx + 2 columns are numbered in one sequence as above.
 //   y: a warp evaluates R element rows; the node row between two warps is
 //      finished by the lower one, the upper warp's share handed over as x-modes
 //      through shared memory (one barrier per layer).  A CTA finishes W R - 1
@@ -175,7 +179,15 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
   int ex, ss, rl, ll;
   bool own_x;
   if constexpr (PER) {
-    if (g.nx <= 32) {
+    rl = lane < 31 ? lane + 1 : lane;
+    ll = lane > 0 ? lane - 1 : lane;
+    if (bd.flat) {
+      const int len = g.nx + 2, q = blockIdx.x * kOwn - 1 + lane;
+      ss = q > 0 ? q / len : 0;
+      const int c = q - ss * len;  // 0: the left halo, 1 .. nx: owned, nx + 1: the right neighbour
+      own_x = lane >= 1 && lane <= kOwn && ss < nss && c >= 1 && c <= g.nx;
+      ex = wrap_index(c - 1, g.nx);
+    } else {
       const int ng = 32 / g.nx, gi = lane / g.nx;
       ex = lane - gi * g.nx;
       ss = blockIdx.x * ng + gi;
@@ -183,14 +195,6 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
       rl = own_x ? gi * g.nx + (ex + 1 == g.nx ? 0 : ex + 1) : lane;
       ll = own_x ? gi * g.nx + (ex == 0 ? g.nx - 1 : ex - 1) : lane;
       if (!own_x) ss = 0;
-    } else {
-      const int nseg = (g.nx + kOwn - 1) / kOwn, seg = blockIdx.x % nseg;
-      ss = blockIdx.x / nseg;
-      const int c = seg * kOwn - 1 + lane;
-      own_x = lane >= 1 && lane <= kOwn && c < g.nx;
-      ex = wrap_index(c, g.nx);
-      rl = lane < 31 ? lane + 1 : lane;
-      ll = lane > 0 ? lane - 1 : lane;
     }
   } else {
     const int q = blockIdx.x * kOwn - 1 + lane;
@@ -568,6 +572,12 @@ struct StepCost<df> {
 };
 constexpr int kSms = 152;
 
+// Whether a periodic row of nx columns uses more of a warp's lanes in one sequence
+// of nx + 2 columns (30 of 32 lanes own one) than in groups of nx lanes.
+bool periodic_flat(int nx) {
+  return nx > 32 || 30 * nx > (nx + 2) * nx * (32 / nx);
+}
+
 template <class V>
 dim3 march_grid(int nnx, int nny, int nnz, int nsys, bool per, const MarchTile& t) {
   constexpr int R = RowsOf<V>::R;
@@ -576,10 +586,10 @@ dim3 march_grid(int nnx, int nny, int nnz, int nsys, bool per, const MarchTile& 
   if (!per) {
     const int own = std::is_same<V, double>::value ? 31 : 30;
     gx = (int64_t(nnx) * nss + own - 1) / own;
-  } else if (nnx <= 32) {
-    gx = (nss + 32 / nnx - 1) / (32 / nnx);
+  } else if (periodic_flat(nnx)) {
+    gx = (int64_t(nnx + 2) * nss + 29) / 30;
   } else {
-    gx = int64_t(nss) * ((nnx + 29) / 30);
+    gx = (nss + 32 / nnx - 1) / (32 / nnx);
   }
   return dim3(unsigned(gx), unsigned((nnz + t.kz - 1) / t.kz), unsigned(nsys));
 }
@@ -784,7 +794,7 @@ void launch_periodic_op(int mode, int nx, int ny, int nz, const ModalConsts& c, 
   const GridDev gd{nx, ny, nz, nx, ny, nz};
   const int64_t nv = int64_t(nx) * ny * nz;
   const MarchTile t = periodic_tile<T>(nx, ny, nz);
-  const BatchDev bd{nrhs, 3 * nv, nv, run};
+  const BatchDev bd{nrhs, 3 * nv, nv, run, periodic_flat(nx) ? 1 : 0};
   if (mode == kApply)
     launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y, dot_part, bd,
                                      s);
