@@ -1506,7 +1506,7 @@ int tg_matfree_apply(const tg_grid* grid, double E, double nu, const double* you
       launch_copy_d2f(ff.p, df.p, g.nv, cs.s);
       launch_copy_d2f(fu.p, du.p, g.ndof, cs.s);
       launch_fine_op<float>(kApply, g, mc, ff.p, nullptr, fu.p, nullptr, nullptr, 0.0f, fy.p,
-                            nullptr, nullptr, cs.s);
+                            SumOut{}, cs.s);
       std::vector<float> hy(size_t(g.ndof));
       TG_CUDA(cudaMemcpyAsync(hy.data(), fy.p, fy.bytes(), cudaMemcpyDeviceToHost, cs.s));
       TG_CUDA(cudaStreamSynchronize(cs.s));
@@ -1524,7 +1524,7 @@ int tg_matfree_apply(const tg_grid* grid, double E, double nu, const double* you
       return;
     }
     launch_fine_op<double>(kApply, g, mc, df.p, nullptr, du.p, nullptr, nullptr, 0.0, dy.p,
-                           nullptr, nullptr, cs.s);
+                           SumOut{}, cs.s);
     TG_CUDA(cudaMemcpyAsync(y, dy.p, dy.bytes(), cudaMemcpyDeviceToHost, cs.s));
     TG_CUDA(cudaStreamSynchronize(cs.s));
   });

@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <utility>
 
 namespace tg {
 
@@ -403,6 +404,7 @@ __device__ __forceinline__ T stencil_update(bool active, T s, T xv, T bv, T dv, 
   if (!active) return T(0);
   if (MODE == kApply) return s;
   if (MODE == kResidual) return bv - s;
+  if (MODE == kDinvA) return dv * s;
   if (MODE == kCheb) {
     // Chebyshev step (Saad, Iterative Methods, Alg. 12.1): d_k = rho_k rho_{k-1}
     // d_{k-1} + (2 rho_k / delta) D^-1 (b - A x_k), d_0 = D^-1 (b - A x_0) / theta,
@@ -442,8 +444,9 @@ __global__ void __launch_bounds__(kStencilThreads) k_stencil_op(MgDims d, const 
   const bool ac = act[dof] != 0;
   T dnew;
   const T out = stencil_update<T, MODE>(
-      ac, s, (MODE == kSmooth || MODE == kCheb) ? x[dof] : T(0), MODE != kApply ? b[dof] : T(0),
-      (MODE == kSmooth || MODE == kCheb) ? invdiag[dof] : T(0), omega, ch.coef, ch.step,
+      ac, s, (MODE == kSmooth || MODE == kCheb) ? x[dof] : T(0),
+      MODE != kApply && MODE != kDinvA ? b[dof] : T(0),
+      (MODE == kSmooth || MODE == kCheb || MODE == kDinvA) ? invdiag[dof] : T(0), omega, ch.coef, ch.step,
       (MODE == kCheb && ch.step > 0 && ac) ? dir[dof] : T(0), dnew);
   if (MODE == kCheb) dir[dof] = dnew;
   y[dof] = out;
@@ -480,8 +483,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
   if (q == 0 && valid) {
     ac = act[dof] != 0;
     if (MODE == kSmooth || MODE == kCheb) xv = x[dof];
-    if (MODE != kApply) bv = b[dof];
-    if (MODE == kSmooth || MODE == kCheb) dv = invdiag[dof];
+    if (MODE != kApply && MODE != kDinvA) bv = b[dof];
+    if (MODE == kSmooth || MODE == kCheb || MODE == kDinvA) dv = invdiag[dof];
     if (MODE == kCheb && ch.step > 0) dprev = dir[dof];
   }
   T p = T(0);
@@ -501,8 +504,11 @@ __global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
   y[dof] = out;
 }
 
-// Power iteration for lambda_max(D^-1 A) of one stencil level: v on the
-// active DOFs from a fixed hash, then w = D^-1 A v, v = w / |w|; |w| -> lam.
+// Power iteration for lambda_max(D^-1 A) of one stencil level: v on the active
+// DOFs from a fixed hash, then w = D^-1 A v, v = w; |w| / |v| of the last step ->
+// lam.  Not normalised on the way: lambda is a few units, so ten steps stay far
+// inside FP32's range, and a step is one launch instead of five (0.5 ms of a
+// 256x128x128 hierarchy build's small dependent launches).
 template <class T>
 __global__ void k_pi_init(const uint8_t* __restrict__ act, int64_t n, T* __restrict__ v) {
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
@@ -512,23 +518,10 @@ __global__ void k_pi_init(const uint8_t* __restrict__ act, int64_t n, T* __restr
     v[i] = act[i] ? T(0.5) + T(h & 0xffff) * T(1.0 / 65536.0) : T(0);
   }
 }
-template <class T>
-__global__ void k_pi_dinv(T* __restrict__ w, const T* __restrict__ invdiag, int64_t n) {
-  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * kThreads)
-    w[i] *= invdiag[i];
-}
-template <class T>
-__global__ void k_pi_scale(T* __restrict__ v, const T* __restrict__ w,
-                           const double* __restrict__ nrm2, int64_t n) {
-  const double q = nrm2[0] > 0.0 ? 1.0 / sqrt(nrm2[0]) : 0.0;
-  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * kThreads)
-    v[i] = T(q) * w[i];
-}
 __global__ void k_pi_lambda(const double* __restrict__ nrm2, double safety,
                             double* __restrict__ lam) {
-  if (threadIdx.x == 0) lam[0] = safety * sqrt(nrm2[0] > 0.0 ? nrm2[0] : 1.0);
+  if (threadIdx.x == 0)
+    lam[0] = safety * (nrm2[0] > 0.0 && nrm2[1] > 0.0 ? sqrt(nrm2[1] / nrm2[0]) : 1.0);
 }
 
 // Chebyshev coefficients on [lmax / ratio, lmax]: theta, delta the interval's
@@ -1009,6 +1002,9 @@ void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, co
     else if (mode == kResidual)
       k_stencil_split<T, kResidual><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega,
                                                                  y, ch);
+    else if (mode == kDinvA)
+      k_stencil_split<T, kDinvA><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
+                                                              ch);
     else if (mode == kCheb)
       k_stencil_split<T, kCheb><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
                                                              ch);
@@ -1025,6 +1021,8 @@ void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, co
     k_stencil_op<T, kApply><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
   else if (mode == kResidual)
     k_stencil_op<T, kResidual><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
+  else if (mode == kDinvA)
+    k_stencil_op<T, kDinvA><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
   else if (mode == kCheb)
     k_stencil_op<T, kCheb><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
   else
@@ -1038,31 +1036,21 @@ void mg_cheb_table(const double* lam, double ratio, int m, float* coef, cudaStre
   TG_LAUNCH_CHECK();
 }
 
-template <class T>
-void mg_lambda_max(const MgDims& d, const T* A, const uint8_t* act, const T* invdiag, T* v,
-                   T* w, int iters, double safety, double* part, double* nrm2, double* lam,
-                   cudaStream_t s) {
+void mg_lambda_max(const MgDims& d, const float* A, const uint8_t* act, const float* invdiag,
+                   float* v, float* w, int iters, double safety, double* part, double* nrm2,
+                   unsigned* count, double* lam, cudaStream_t s) {
   const int64_t n = 3 * int64_t(d.nnx) * d.nny * d.nnz;
-  const int nbk = nblk(n);
-  k_pi_init<T><<<nbk, kThreads, 0, s>>>(act, n, v);
+  k_pi_init<float><<<nblk(n), kThreads, 0, s>>>(act, n, v);
   TG_LAUNCH_CHECK();
   for (int it = 0; it < iters; ++it) {
-    mg_stencil_op<T>(kApply, d, A, act, v, nullptr, nullptr, T(0), w, s);
-    k_pi_dinv<T><<<nbk, kThreads, 0, s>>>(w, invdiag, n);
-    TG_LAUNCH_CHECK();
-    if constexpr (sizeof(T) == 4)
-      launch_dot_f(w, w, n, part, nrm2, s);
-    else
-      launch_dot(w, w, n, part, nrm2, s);
-    k_pi_scale<T><<<nbk, kThreads, 0, s>>>(v, w, nrm2, n);
-    TG_LAUNCH_CHECK();
+    if (it == iters - 1) launch_dot_f(v, v, n, SumOut{part, nrm2, count}, s);
+    mg_stencil_op<float>(kDinvA, d, A, act, v, nullptr, invdiag, 0.0f, w, s);
+    std::swap(v, w);
   }
+  launch_dot_f(v, v, n, SumOut{part, nrm2 + 1, count}, s);
   k_pi_lambda<<<1, 32, 0, s>>>(nrm2, safety, lam);
   TG_LAUNCH_CHECK();
 }
-template void mg_lambda_max<float>(const MgDims&, const float*, const uint8_t*, const float*,
-                                   float*, float*, int, double, double*, double*, double*,
-                                   cudaStream_t);
 
 template <class T>
 void mg_jacobi_first(const T* b, const T* invdiag, T omega, int64_t n, T* x, cudaStream_t s) {

@@ -30,6 +30,7 @@
 
 #include "tg_internal.h"
 #include "tg_march.h"
+#include "tg_reduce.h"
 
 namespace tg {
 
@@ -71,24 +72,6 @@ __device__ __forceinline__ int wrap_near(int a, int n) {
   a = a < 0 ? a + n : a;
   a = a >= n ? a - n : a;
   return a >= n ? a - n : a;
-}
-
-__device__ __forceinline__ double block_sum(double v) {
-  __shared__ double red[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-    s = lane < nw ? red[lane] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  }
-  return s;  // valid in thread 0
 }
 
 // ---------------------------------------------------------------------------
@@ -156,7 +139,7 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
     k_fine_march(GridDev g, ModalT<typename RowsOf<V>::S> mc, int KZ, int nss,
                  const T* __restrict__ ef, const uint8_t* __restrict__ kn,
                  const T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ invdiag,
-                 T omega, T* __restrict__ y, double* __restrict__ dot_part, int guard,
+                 T omega, T* __restrict__ y, SumOut dot, int guard,
                  BatchDev bd) {
   using S = typename RowsOf<V>::S;
   constexpr int R = RowsOf<V>::R;
@@ -532,11 +515,10 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
       for (int k = 0; k < 3; ++k) keep[i][k] = knext[i][k];
   }
   if constexpr (MODE != kResidual) {
-    if (dot_part != nullptr) {
-      const double sum = block_sum(double(store_t(dsum)));
-      if (threadIdx.x == 0)
-        dot_part[(int64_t(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = sum;
-    }
+    if (dot.part != nullptr)
+      grid_sum(double(store_t(dsum)), dot,
+               int((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x),
+               int(gridDim.x * gridDim.y));
   }
 }
 
@@ -632,7 +614,7 @@ MarchTile march_tile(int nnx, int nny, int nnz, int nsys, bool per) {
 template <class V, class T, int MODE, bool PER>
 void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalConsts& c,
                   const T* ef, const uint8_t* kn, const T* x, const T* b, const T* invdiag,
-                  T omega, T* y, double* dot_part, const BatchDev& bd, cudaStream_t s) {
+                  T omega, T* y, const SumOut& dot, const BatchDev& bd, cudaStream_t s) {
   using S = typename RowsOf<V>::S;
   const dim3 grid = march_grid<V>(gd.nnx, gd.nny, gd.nnz, nsys, PER, t);
   const int rows = t.W * RowsOf<V>::R - 1, nss = (gd.nny + rows - 1) / rows;
@@ -653,27 +635,23 @@ void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalCo
   // solver (a kept mask) they are zeros.
   const int guard = kn == nullptr ? 1 : 0;
   k_fine_march<V, T, MODE, PER><<<grid, 32 * t.W, smem, s>>>(
-      gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b, invdiag, omega, y, dot_part, guard, bd);
+      gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b, invdiag, omega, y, dot, guard, bd);
   TG_LAUNCH_CHECK();
 }
 
 template <class V, class T>
 void launch_march_mode(int mode, const Grid& g, const MarchTile& t, const ModalConsts& c,
                        const T* ef, const uint8_t* kn, const T* x, const T* b, const T* invdiag,
-                       T omega, T* y, double* dot_part, int* nblocks_out, cudaStream_t s) {
+                       T omega, T* y, const SumOut& dot, cudaStream_t s) {
   const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
-  if (nblocks_out) {
-    const dim3 d = march_grid<V>(g.nnx, g.nny, g.nnz, 1, false, t);
-    *nblocks_out = int(d.x * d.y);
-  }
   if (mode == kApply)
-    launch_march<V, T, kApply, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot_part,
+    launch_march<V, T, kApply, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot,
                                       BatchDev{}, s);
   else if (mode == kResidual)
-    launch_march<V, T, kResidual, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, nullptr,
+    launch_march<V, T, kResidual, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, SumOut{},
                                          BatchDev{}, s);
   else
-    launch_march<V, T, kSmooth, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot_part,
+    launch_march<V, T, kSmooth, false>(gd, t, 1, c, ef, kn, x, b, invdiag, omega, y, dot,
                                        BatchDev{}, s);
 }
 
@@ -718,15 +696,14 @@ bool fine_schedule_valid(const FineSchedule& s) {
 
 template <class T>
 void launch_fine_op(int mode, const Grid& g, const ModalConsts& c, const T* ef, const uint8_t* kn,
-                    const T* x, const T* b, const T* invdiag, T omega, T* y, double* dot_part,
-                    int* nblocks_out, cudaStream_t s) {
+                    const T* x, const T* b, const T* invdiag, T omega, T* y, const SumOut& dot,
+                    cudaStream_t s) {
   if constexpr (std::is_same<T, float>::value) {
     launch_fine_op_sched(fine_schedule_for(g, mode), mode, g, c, ef, kn, x, b, invdiag, omega, y,
-                         dot_part, nblocks_out, s);
+                         dot, s);
   } else {
     launch_march_mode<double, double>(mode, g, march_tile<double>(g.nnx, g.nny, g.nnz, 1, false),
-                                      c, ef, kn, x, b, invdiag, omega, y, dot_part, nblocks_out,
-                                      s);
+                                      c, ef, kn, x, b, invdiag, omega, y, dot, s);
   }
 }
 
@@ -734,14 +711,14 @@ void launch_fine_op(int mode, const Grid& g, const ModalConsts& c, const T* ef, 
 // through this without touching the process-wide table).
 void launch_fine_op_sched(const FineSchedule& fs, int mode, const Grid& g, const ModalConsts& c,
                           const float* ef, const uint8_t* kn, const float* x, const float* b,
-                          const float* invdiag, float omega, float* y, double* dot_part,
-                          int* nblocks_out, cudaStream_t s) {
+                          const float* invdiag, float omega, float* y, const SumOut& dot,
+                          cudaStream_t s) {
   if (fs.kind == FineSchedule::kColumn)
     launch_march_mode<float2, float>(mode, g, MarchTile{kShapeWarps[fs.shape], fs.kz}, c, ef, kn,
-                                     x, b, invdiag, omega, y, dot_part, nblocks_out, s);
+                                     x, b, invdiag, omega, y, dot, s);
   else
     launch_march_mode<float, float>(mode, g, march_tile<float>(g.nnx, g.nny, g.nnz, 1, false), c,
-                                    ef, kn, x, b, invdiag, omega, y, dot_part, nblocks_out, s);
+                                    ef, kn, x, b, invdiag, omega, y, dot, s);
 }
 
 // The FP64 residual y = b - A x evaluated in double-float arithmetic (tg_df.h):
@@ -751,17 +728,16 @@ void launch_fine_residual_df(const Grid& g, const ModalConsts& c, const double* 
                              cudaStream_t s) {
   const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
   launch_march<df, double, kResidual, false>(gd, march_tile<df>(g.nnx, g.nny, g.nnz, 1, false), 1,
-                                             c, ef, kn, x, b, nullptr, 0.0, y, nullptr, BatchDev{},
+                                             c, ef, kn, x, b, nullptr, 0.0, y, SumOut{}, BatchDev{},
                                              s);
 }
 
 template void launch_fine_op<double>(int, const Grid&, const ModalConsts&, const double*,
                                      const uint8_t*, const double*, const double*,
-                                     const double*, double, double*, double*, int*,
-                                     cudaStream_t);
+                                     const double*, double, double*, const SumOut&, cudaStream_t);
 template void launch_fine_op<float>(int, const Grid&, const ModalConsts&, const float*,
                                     const uint8_t*, const float*, const float*, const float*,
-                                    float, float*, double*, int*, cudaStream_t);
+                                    float, float*, const SumOut&, cudaStream_t);
 
 // Periodic batched apply: nsys systems on the nx*ny*nz torus; system bi uses
 // x/b/y at bi*ndof and the factors and kept bits of cell bi / nrhs.  dot_part
@@ -796,11 +772,11 @@ void launch_periodic_op(int mode, int nx, int ny, int nz, const ModalConsts& c, 
   const MarchTile t = periodic_tile<T>(nx, ny, nz);
   const BatchDev bd{nrhs, 3 * nv, nv, run, periodic_flat(nx) ? 1 : 0};
   if (mode == kApply)
-    launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y, dot_part, bd,
-                                     s);
+    launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
+                                     SumOut{dot_part}, bd, s);
   else
-    launch_march<V, T, kResidual, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y, nullptr,
-                                        bd, s);
+    launch_march<V, T, kResidual, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
+                                        SumOut{}, bd, s);
 }
 template void launch_periodic_op<double>(int, int, int, int, const ModalConsts&, const double*,
                                          const uint8_t*, const double*, const double*, double*,

@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "tg_internal.h"
+#include "tg_reduce.h"
 
 namespace tg {
 
@@ -61,14 +62,12 @@ __device__ __forceinline__ double block_max256(double v) {
 // dozen terms) and in FP64 across threads and blocks: on GB300 an FP64 multiply
 // per element would make these streaming kernels FP64-pipe-bound.
 template <class T>
-__global__ void k_dot(const T* __restrict__ a, const T* __restrict__ b, int64_t n,
-                      double* __restrict__ part) {
+__global__ void k_dot(const T* __restrict__ a, const T* __restrict__ b, int64_t n, SumOut o) {
   T t = T(0);
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * kThreads)
     t += a[i] * b[i];
-  const double s = block_sum256(double(t));
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(double(t), o, int(blockIdx.x), int(gridDim.x));
 }
 
 // One block: out = sum of n partials, fixed order.
@@ -86,27 +85,28 @@ __global__ void k_max_partials(const double* __restrict__ part, int n, double* _
   if (threadIdx.x == 0) *out = s;
 }
 
-// x += alpha p; r -= alpha Ap with alpha = rz / pAp; partial r.r (FP64 sums).
-// The FP64 PCG's update; the FP32 inner PCG runs it as two kernels below.
-template <class T>
-__global__ void k_cg_update_xr(T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                               const T* __restrict__ ap, const double* __restrict__ rz,
-                               const double* __restrict__ pap, int64_t n,
-                               double* __restrict__ part) {
+// x += alpha p; r -= alpha Ap with alpha = rz / pAp; sum of r.r (FP64).  With x0
+// set, also x0 = omega invdiag .* r.  The FP64 PCG's update; the FP32 inner PCG
+// runs it as two kernels below.
+__global__ void k_cg_update_xr(double* __restrict__ x, double* __restrict__ r,
+                               const double* __restrict__ p, const double* __restrict__ ap,
+                               const double* __restrict__ rz, const double* __restrict__ pap,
+                               int64_t n, const double* __restrict__ invdiag, double omega,
+                               double* __restrict__ x0, SumOut o) {
   // A non-positive or non-finite pAp is a breakdown the host reports; leave the
   // iterate untouched so the last good x survives.
   const double pp = *pap;
-  const T a = T((pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0);
-  T t = T(0);
+  const double a = (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
+  double t = 0.0;
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * kThreads) {
     x[i] += a * p[i];
-    const T ri = r[i] - a * ap[i];
+    const double ri = r[i] - a * ap[i];
     r[i] = ri;
+    if (x0 != nullptr) x0[i] = omega * invdiag[i] * ri;
     t += ri * ri;
   }
-  const double s = block_sum256(double(t));
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(t, o, int(blockIdx.x), int(gridDim.x));
 }
 
 // The FP32 inner PCG's update in two kernels (alpha as k_cg_update_xr forms it,
@@ -121,9 +121,8 @@ __device__ __forceinline__ float cg_alpha_f(const double* rz, const double* pap)
 // sweep from zero, as k_jacobi_first computes it).
 __global__ void k_cg_update_r_f(float* __restrict__ r, const float* __restrict__ ap,
                                 const double* __restrict__ rz, const double* __restrict__ pap,
-                                int64_t n, double* __restrict__ part,
-                                const float* __restrict__ invdiag, float omega,
-                                float* __restrict__ x0) {
+                                int64_t n, const float* __restrict__ invdiag, float omega,
+                                float* __restrict__ x0, SumOut o) {
   const float af = cg_alpha_f(rz, pap);
   const int64_t n4 = n >> 2;
   float4* r4 = reinterpret_cast<float4*>(r);
@@ -152,8 +151,7 @@ __global__ void k_cg_update_r_f(float* __restrict__ r, const float* __restrict__
     t += ri * ri;
     if (x0 != nullptr) x0[i] = omega * invdiag[i] * ri;
   }
-  const double s = block_sum256(double(t));
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(double(t), o, int(blockIdx.x), int(gridDim.x));
 }
 __global__ void k_cg_update_x_f(float* __restrict__ x, const float* __restrict__ p,
                                 const double* __restrict__ rz, const double* __restrict__ pap,
@@ -174,10 +172,9 @@ __global__ void k_cg_update_x_f(float* __restrict__ x, const float* __restrict__
     x[i] += af * p[i];
 }
 
-// z = invdiag .* r (Jacobi preconditioner); partial r.z.
+// z = invdiag .* r (Jacobi preconditioner); sum of r.z.
 __global__ void k_scale_mask(double* __restrict__ z, const double* __restrict__ r,
-                             const double* __restrict__ invdiag, int64_t n,
-                             double* __restrict__ part) {
+                             const double* __restrict__ invdiag, int64_t n, SumOut o) {
   double s = 0.0;
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * kThreads) {
@@ -185,8 +182,7 @@ __global__ void k_scale_mask(double* __restrict__ z, const double* __restrict__ 
     z[i] = zi;
     s += r[i] * zi;
   }
-  s = block_sum256(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  grid_sum(s, o, int(blockIdx.x), int(gridDim.x));
 }
 
 // p = z + beta p, beta = rz_new / rz_old.
@@ -326,25 +322,19 @@ double fma_probe_tflops(bool fp64) {
   return best;
 }
 
-void launch_dot(const double* a, const double* b, int64_t n, double* part, double* out,
-                cudaStream_t s) {
-  k_dot<double><<<kRedBlocks, kThreads, 0, s>>>(a, b, n, part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials<<<1, kThreads, 0, s>>>(part, kRedBlocks, out);
+// Four elements a thread up to the full grid: a small vector's sum is not spread
+// over 608 blocks that the last one waits for.
+int red_blocks(int64_t n) {
+  return int(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + 4 * kThreads - 1) / (4 * kThreads))));
+}
+
+void launch_dot(const double* a, const double* b, int64_t n, const SumOut& o, cudaStream_t s) {
+  k_dot<double><<<red_blocks(n), kThreads, 0, s>>>(a, b, n, o);
   TG_LAUNCH_CHECK();
 }
 
-void launch_dot_f(const float* a, const float* b, int64_t n, double* part, double* out,
-                  cudaStream_t s) {
-  k_dot<float><<<kRedBlocks, kThreads, 0, s>>>(a, b, n, part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials<<<1, kThreads, 0, s>>>(part, kRedBlocks, out);
-  TG_LAUNCH_CHECK();
-}
-
-void launch_dot_partials_f(const float* a, const float* b, int64_t n, double* part,
-                           cudaStream_t s) {
-  k_dot<float><<<kRedBlocks, kThreads, 0, s>>>(a, b, n, part);
+void launch_dot_f(const float* a, const float* b, int64_t n, const SumOut& o, cudaStream_t s) {
+  k_dot<float><<<red_blocks(n), kThreads, 0, s>>>(a, b, n, o);
   TG_LAUNCH_CHECK();
 }
 
@@ -353,39 +343,36 @@ void launch_sum_partials(const double* part, int n, double* out, cudaStream_t s)
   TG_LAUNCH_CHECK();
 }
 
-template <class T>
-void launch_cg_update_xr(T* x, T* r, const T* p, const T* ap, const double* rz,
-                         const double* pap, int64_t n, double* rr_part, cudaStream_t s) {
-  k_cg_update_xr<T><<<kRedBlocks, kThreads, 0, s>>>(x, r, p, ap, rz, pap, n, rr_part);
+void launch_cg_update_xr(double* x, double* r, const double* p, const double* ap,
+                         const double* rz, const double* pap, int64_t n, const SumOut& rr,
+                         cudaStream_t s, const double* invdiag, double omega, double* x0) {
+  k_cg_update_xr<<<red_blocks(n), kThreads, 0, s>>>(x, r, p, ap, rz, pap, n, invdiag, omega, x0,
+                                                    rr);
   TG_LAUNCH_CHECK();
 }
-template void launch_cg_update_xr<double>(double*, double*, const double*, const double*,
-                                          const double*, const double*, int64_t, double*,
-                                          cudaStream_t);
 
 void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const double* pap,
-                          int64_t n, double* rr_part, cudaStream_t s, const float* invdiag,
+                          int64_t n, const SumOut& rr, cudaStream_t s, const float* invdiag,
                           float omega, float* x0) {
-  k_cg_update_r_f<<<kRedBlocks, kThreads, 0, s>>>(r, ap, rz, pap, n, rr_part, invdiag, omega,
-                                                  x0);
+  k_cg_update_r_f<<<red_blocks(n), kThreads, 0, s>>>(r, ap, rz, pap, n, invdiag, omega, x0, rr);
   TG_LAUNCH_CHECK();
 }
 void launch_cg_update_x_f(float* x, const float* p, const double* rz, const double* pap,
                           int64_t n, cudaStream_t s) {
-  k_cg_update_x_f<<<kRedBlocks, kThreads, 0, s>>>(x, p, rz, pap, n);
+  k_cg_update_x_f<<<red_blocks(n), kThreads, 0, s>>>(x, p, rz, pap, n);
   TG_LAUNCH_CHECK();
 }
 
 void launch_scale_mask(double* z, const double* r, const double* invdiag, int64_t n,
-                       double* rz_part, cudaStream_t s) {
-  k_scale_mask<<<kRedBlocks, kThreads, 0, s>>>(z, r, invdiag, n, rz_part);
+                       const SumOut& rz, cudaStream_t s) {
+  k_scale_mask<<<red_blocks(n), kThreads, 0, s>>>(z, r, invdiag, n, rz);
   TG_LAUNCH_CHECK();
 }
 
 template <class T>
 void launch_cg_update_p(T* p, const T* z, const double* rz_new, const double* rz_old, int64_t n,
                         cudaStream_t s) {
-  k_cg_update_p<T><<<kRedBlocks, kThreads, 0, s>>>(p, z, rz_new, rz_old, n);
+  k_cg_update_p<T><<<red_blocks(n), kThreads, 0, s>>>(p, z, rz_new, rz_old, n);
   TG_LAUNCH_CHECK();
 }
 template void launch_cg_update_p<double>(double*, const double*, const double*, const double*,

@@ -350,6 +350,8 @@ Solver::Solver(const FineProblem& fp, const tg_solve_options& opt, cudaStream_t 
                       152 * 32});
   part_.alloc(size_t(part_n_));
   scal_.alloc(32);
+  cnt_.alloc(kSumSlots);  // the sums' counters: zero, and left zero by every sum
+  TG_CUDA(cudaMemsetAsync(cnt_.p, 0, cnt_.bytes(), s));
   h_scal_ = static_cast<double*>(pinned_scalars(32 * sizeof(double)));
   istate_.alloc(4);
   h_ist_ = static_cast<int*>(pinned_scalars(4 * sizeof(int)));
@@ -372,11 +374,12 @@ Solver::Solver(const FineProblem& fp, const tg_solve_options& opt, cudaStream_t 
   if (opt.solver == TG_SOLVER_MGCG) build_structure();
 }
 
-struct Solver::InnerGraph {
+struct Solver::LoopGraph {
+  const double* E = nullptr;  // the element factors the body reads (FP64 loops)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int64_t body_launches = 0;  // kernels per body execution
-  ~InnerGraph() {
+  ~LoopGraph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
   }
@@ -384,6 +387,8 @@ struct Solver::InnerGraph {
 
 Solver::~Solver() {
   ig_.reset();
+  ig64_.reset();
+  igj_.reset();
   for (size_t i = 0; i < pi_streams_.size(); ++i) {
     cudaStreamSynchronize(pi_streams_[i]);
     cudaStreamDestroy(pi_streams_[i]);
@@ -631,8 +636,8 @@ void Solver::read_scalars(int idx0, int n, double* out) {
 }
 
 void Solver::apply_unmasked(const double* E, const double* x, double* y) {
-  launch_fine_op<double>(kApply, fp_.g, fp_.mc, E, nullptr, x, nullptr, nullptr, 0.0, y, nullptr,
-                         nullptr, s_);
+  launch_fine_op<double>(kApply, fp_.g, fp_.mc, E, nullptr, x, nullptr, nullptr, 0.0, y,
+                         SumOut{}, s_);
 }
 
 // The assembled FP32 level-1 stencil, formed from the level's element matrices
@@ -716,12 +721,12 @@ double Solver::time_operator(int form, int reps) {
   for (int i = 0; i < reps; ++i) {
     if (fp32)
       launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
-                            apf_.p, nullptr, nullptr, s_);
+                            apf_.p, SumOut{}, s_);
     else if (form == 2)  // the double-float residual kernel
       launch_fine_residual_df(g, fp_.mc, E_, fp_.kept_node.p, p_.p, rhs_.p, ap_.p, s_);
     else
       launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0,
-                             ap_.p, nullptr, nullptr, s_);
+                             ap_.p, SumOut{}, s_);
   }
   TG_CUDA(cudaEventRecord(b, s_));
   TG_CUDA(cudaEventSynchronize(b));
@@ -815,13 +820,17 @@ bool Solver::build_numeric() {
   if (sizeof(T) == 4 && cheb_m_ > 0) {
     // lambda_max(D^-1 A) of every smoothed level >= 2 for its Chebyshev smoother.
     // The levels' power iterations are independent chains of small launches
-    // (10 steps of 5 each); they run side by side, one stream per level, each
+    // (10 steps); they run side by side, one stream per level, each
     // with its own partials, and rejoin the solver's stream.
     const size_t nlev = levels_.size();
     if (!lam_.p) lam_.alloc(nlev + 1);
     if (!chc_.p) chc_.alloc(kChebCoefStride * (nlev + 1));
-    constexpr size_t kPiStride = size_t(kRedBlocks) + 8;  // partials, then the norm
-    if (!pipart_.p) pipart_.alloc((nlev + 1) * kPiStride);
+    constexpr size_t kPiStride = size_t(kRedBlocks) + 8;  // partials, then the two norms
+    if (!pipart_.p) {
+      pipart_.alloc((nlev + 1) * kPiStride);
+      picnt_.alloc(nlev + 1);
+      TG_CUDA(cudaMemsetAsync(picnt_.p, 0, picnt_.bytes(), s_));
+    }
     ensure_pi_streams(nlev);
     TG_CUDA(cudaEventRecord(pi_fork_, s_));
     for (size_t li = 1; li + 1 < nlev; ++li) {
@@ -830,9 +839,9 @@ bool Solver::build_numeric() {
       cudaStream_t ls = pi_streams_[li];
       double* part = pipart_.p + li * kPiStride;
       TG_CUDA(cudaStreamWaitEvent(ls, pi_fork_, 0));
-      mg_lambda_max<float>(L.d, L.Am<float>(), L.act.p, L.Dinv<float>(), L.X<float>(),
-                           L.R<float>(), cheb_iters_, cheb_safety_, part, part + kRedBlocks,
-                           lam_.p + li, ls);
+      mg_lambda_max(L.d, L.Am<float>(), L.act.p, L.Dinv<float>(), L.X<float>(), L.R<float>(),
+                    cheb_iters_, cheb_safety_, part, part + kRedBlocks, picnt_.p + li,
+                    lam_.p + li, ls);
       mg_cheb_table(lam_.p + li, cheb_ratio_, cheb_m_, chc_.p + kChebCoefStride * li, ls);
       TG_CUDA(cudaEventRecord(pi_events_[li], ls));
       TG_CUDA(cudaStreamWaitEvent(s_, pi_events_[li], 0));
@@ -1042,147 +1051,57 @@ float* Solver::fused_coarse_vcycle() {
   return cheb_m_ > 0 ? fc.L[0].xp : fc.L[0].xq;
 }
 
-template <>
-double* Solver::vcycle<double>(const double* b, double* bz, bool x0_ready) {
-  if (bz != nullptr || x0_ready) raise(TG_EINVAL, "vcycle<double>: no fused b.z or first sweep");
-  const Grid& g = fp_.g;
-  Level& N = *levels_[0];
-  const MgDims fd = dims_of(g.nx, g.ny, g.nz);
-  double* x = t1_.p;
-  double* r = t0_.p;
-  auto smooth = [&] {
-    launch_fine_op<double>(kSmooth, g, fp_.mc, E_, fp_.kept_node.p, x, b, invdiag_.p, omega_, r,
-                           nullptr, nullptr, s_);
-    std::swap(x, r);
-  };
-  mg_jacobi_first<double>(b, invdiag_.p, omega_, g.ndof, x, s_);
-  for (int k = 1; k < sweeps_; ++k) smooth();
-  launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x, b, invdiag_.p, omega_, r,
-                         nullptr, nullptr, s_);
-  const FirstStep<double> fs = first_step<double>(1);
-  mg_restrict<double>(fd, N.d, r, N.act.p, N.B<double>(), s_, fs);
-  double* ec = vcycle_level<double>(1, fs.kind != 0);
-  mg_prolong_add<double>(fd, N.d, ec, fp_.kept.p, x, s_);
-  for (int k = 0; k < sweeps_; ++k) smooth();
-  fine_matvecs_ += 2 * sweeps_;
-  return x;
-}
-
-template <>
 // With bz set, b . z of the returned z is summed into *bz (device): the last
 // smoothing sweep accumulates it while it writes z.  With x0_ready the first
-// sweep from zero, omega D^-1 b, is already in t1f_ (the PCG's r update wrote
-// it).
-float* Solver::vcycle<float>(const float* b, double* bz, bool x0_ready) {
+// sweep from zero, omega D^-1 b, is already in t1_ / t1f_ (the PCG's r update
+// wrote it).
+template <class T>
+T* Solver::vcycle(const T* b, double* bz, bool x0_ready) {
   const Grid& g = fp_.g;
   Level& N = *levels_[0];
   const MgDims fd = dims_of(g.nx, g.ny, g.nz);
-  float* x = t1f_.p;
-  float* r = t0f_.p;
-  const float w = float(omega_);
+  T *x, *r;
+  const T *ef, *dinv;
+  if constexpr (sizeof(T) == 4) {
+    x = t1f_.p;
+    r = t0f_.p;
+    ef = Ef_.p;
+    dinv = invdiagf_.p;
+  } else {
+    x = t1_.p;
+    r = t0_.p;
+    ef = E_;
+    dinv = invdiag_.p;
+  }
+  const T w = T(omega_);
   auto smooth = [&](bool last) {
-    int nb = 0;
-    double* part = last && bz != nullptr ? part_.p : nullptr;
-    launch_fine_op<float>(kSmooth, g, fp_.mc, Ef_.p, fp_.kept_node.p, x, b, invdiagf_.p, w, r, part,
-                          &nb, s_);
-    if (part != nullptr) launch_sum_partials(part_.p, nb, bz, s_);
+    launch_fine_op<T>(kSmooth, g, fp_.mc, ef, fp_.kept_node.p, x, b, dinv, w, r,
+                      last && bz != nullptr ? SumOut{part_.p, bz, cnt_.p + 3} : SumOut{}, s_);
     std::swap(x, r);
   };
-  if (!x0_ready) mg_jacobi_first<float>(b, invdiagf_.p, w, g.ndof, x, s_);
+  if (!x0_ready) mg_jacobi_first<T>(b, dinv, w, g.ndof, x, s_);
   for (int k = 1; k < sweeps_; ++k) smooth(false);
-  launch_fine_op<float>(kResidual, g, fp_.mc, Ef_.p, fp_.kept_node.p, x, b, invdiagf_.p, w, r, nullptr,
-                        nullptr, s_);
-  const FirstStep<float> fs = first_step<float>(1);
-  mg_restrict<float>(fd, N.d, r, N.act.p, N.B<float>(), s_, fs);
-  float* ec = vcycle_level<float>(1, fs.kind != 0);
-  mg_prolong_add<float>(fd, N.d, ec, fp_.kept.p, x, s_);
+  launch_fine_op<T>(kResidual, g, fp_.mc, ef, fp_.kept_node.p, x, b, dinv, w, r, SumOut{}, s_);
+  const FirstStep<T> fs = first_step<T>(1);
+  mg_restrict<T>(fd, N.d, r, N.act.p, N.B<T>(), s_, fs);
+  T* ec = vcycle_level<T>(1, fs.kind != 0);
+  mg_prolong_add<T>(fd, N.d, ec, fp_.kept.p, x, s_);
   for (int k = 0; k < sweeps_; ++k) smooth(k == sweeps_ - 1);
-  lowp_matvecs_ += 2 * sweeps_;
+  (sizeof(T) == 4 ? lowp_matvecs_ : fine_matvecs_) += 2 * sweeps_;
   return x;
 }
 
-// ------------------------------------------------------------------ MG-PCG
-// mf_mgpcg (multigrid.cpp:1211-1313): stop at ||r|| <= tol ||b||, breakdown when
-// pAp <= 0 or non-finite, x finite at exit.
-bool Solver::mgpcg(double tol, int max_it, bool warm, SolverStats& st) {
-  const Grid& g = fp_.g;
-  const int64_t n = g.ndof;
-  launch_dot(rhs_.p, rhs_.p, n, part_.p, scal_.p + 4, s_);
-  const double bnorm2 = read_scalar(4);
-  st.iterations = 0;
-  st.residual = 0.0;
-  if (!(bnorm2 > 0.0)) {
-    launch_fill<double>(x_.p, 0.0, n, s_);
-    return true;
-  }
-  const double bnorm = std::sqrt(bnorm2), threshold = tol * bnorm;
-  if (warm) {
-    refinement_residual();
-  } else {
-    launch_fill<double>(x_.p, 0.0, n, s_);
-    TG_CUDA(cudaMemcpyAsync(r_.p, rhs_.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s_));
-  }
-  double* z = vcycle<double>(r_.p);
-  TG_CUDA(cudaMemcpyAsync(p_.p, z, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s_));
-  launch_dot(r_.p, z, n, part_.p, scal_.p + 0, s_);
-  if (!std::isfinite(read_scalar(0))) return false;
-  int nb = 0;
-  for (int k = 1; k <= max_it; ++k) {
-    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
-                           part_.p, &nb, s_);
-    ++fine_matvecs_;
-    launch_sum_partials(part_.p, nb, scal_.p + 1, s_);
-    launch_cg_update_xr<double>(x_.p, r_.p, p_.p, ap_.p, scal_.p + 0, scal_.p + 1, n, part_.p, s_);
-    launch_sum_partials(part_.p, kRedBlocks, scal_.p + 2, s_);
-    double sc[2];
-    read_scalars(1, 2, sc);
-    const double pap = sc[0], rr = sc[1];
-    if (!(pap > 0.0) || !std::isfinite(pap)) return false;
-    st.iterations = k;
-    const double rn = std::sqrt(rr);
-    st.residual = rn / bnorm;
-    if (rn <= threshold) {
-      launch_dot(x_.p, x_.p, n, part_.p, scal_.p + 5, s_);
-      return std::isfinite(read_scalar(5));
-    }
-    z = vcycle<double>(r_.p);
-    launch_dot(r_.p, z, n, part_.p, scal_.p + 3, s_);
-    launch_cg_update_p<double>(p_.p, z, scal_.p + 3, scal_.p + 0, n, s_);
-    TG_CUDA(cudaMemcpyAsync(scal_.p + 0, scal_.p + 3, sizeof(double), cudaMemcpyDeviceToDevice, s_));
-  }
-  return false;
-}
-
-// FP32 inner MG-PCG on the unit-norm residual held in zf_; solution in xf_.
-// FP64 dot products; stops at relative residual rel_tol or max_it.
-// The decision at the end of one graph-resident inner PCG iteration, exactly the
-// host loop's: breakdown (p.Ap <= 0 or not finite) stops without counting the
-// iteration; otherwise it is counted and the loop continues while
-// ||r|| > thr and the budget allows.  scal[7] = p.Ap, scal[8] = r.r,
-// scal[11] = thr; st[0] = iterations done, st[1] = budget, st[2] = breakdown.
-__global__ void k_inner_cond(cudaGraphConditionalHandle h, const double* __restrict__ scal,
-                             int* __restrict__ st) {
-  const double pap = scal[7], rr = scal[8], thr = scal[11];
-  if (!(pap > 0.0) || !isfinite(pap)) {
-    st[2] = 1;
-    cudaGraphSetConditional(h, 0u);
-    return;
-  }
-  const int k = st[0] + 1;
-  st[0] = k;
-  cudaGraphSetConditional(h, (!(sqrt(rr) <= thr) && k < st[1]) ? 1u : 0u);
-}
-
-// Captures iterations 2.. of inner_pcg<float> into a WHILE conditional node.
-// All pointers the body uses (fine vectors, level buffers, scalars) live as
-// long as the solver, so the graph is built once and replayed for every inner
-// solve.  On any capture error the solver keeps the host-driven loop.
-bool Solver::build_inner_graph() {
-  if (ig_failed_) return false;
-  if (ig_) return true;
-  const Grid& g = fp_.g;
-  const int64_t n = g.ndof;
-  auto ig = std::make_unique<InnerGraph>();
+// Captures a PCG loop's iterations 2.. into a WHILE conditional node; body
+// records one iteration, whose last kernel takes the loop's decision (LoopCond).
+// All pointers a body uses (fine vectors, level buffers, scalars; E is checked
+// again by the caller) live as long as the solver, so a graph is built once and
+// replayed for every solve.  On any capture error the solver keeps the
+// host-driven loop.
+template <class Body>
+bool Solver::capture_loop(std::unique_ptr<LoopGraph>& slot, Body&& record) {
+  if (graph_failed_) return false;
+  auto ig = std::make_unique<LoopGraph>();
+  ig->E = E_;
   bool ok = cudaGraphCreate(&ig->graph, 0) == cudaSuccess;
   cudaGraphConditionalHandle h{};
   cudaGraph_t body = nullptr;
@@ -1204,24 +1123,10 @@ bool Solver::build_inner_graph() {
                                        cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
     const int64_t l0 = kernel_launch_count();
-    const int64_t m0 = lowp_matvecs_;
+    const int64_t m0 = lowp_matvecs_, f0 = fine_matvecs_;
     bool cap_ok = true;
     try {
-      pending_x_ = true;  // every body execution starts with the last one's x update
-      float* z = vcycle<float>(rf_.p, scal_.p + 9, true);
-      flush_x();
-      launch_cg_update_p<float>(pf_.p, z, scal_.p + 9, scal_.p + 6, n, s_);
-      TG_CUDA(cudaMemcpyAsync(scal_.p + 6, scal_.p + 9, sizeof(double), cudaMemcpyDeviceToDevice,
-                              s_));
-      int nb = 0;
-      launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
-                            apf_.p, part_.p, &nb, s_);
-      launch_sum_partials(part_.p, nb, scal_.p + 7, s_);
-      launch_cg_update_r_f(rf_.p, apf_.p, scal_.p + 6, scal_.p + 7, n, part_.p, s_, invdiagf_.p,
-                           float(omega_), t1f_.p);
-      launch_sum_partials(part_.p, kRedBlocks, scal_.p + 8, s_);
-      k_inner_cond<<<1, 1, 0, s_>>>(h, scal_.p, istate_.p);
-      TG_LAUNCH_CHECK();
+      record(h);
     } catch (const Error&) {
       cap_ok = false;
     }
@@ -1232,42 +1137,156 @@ bool Solver::build_inner_graph() {
     ig->body_launches = kernel_launch_count() - l0;
     add_kernel_launches(-ig->body_launches);  // captured, not launched
     lowp_matvecs_ = m0;
+    fine_matvecs_ = f0;
     ok = cap_ok && end_ok;
   }
   if (ok) ok = cudaGraphInstantiate(&ig->exec, ig->graph, 0) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();  // clear a capture error; the host loop runs instead
-    ig_failed_ = true;
+    graph_failed_ = true;
     return false;
   }
-  ig_ = std::move(ig);
+  slot = std::move(ig);
   return true;
 }
 
+// Runs a captured loop from iteration `first` (done so far) with at most `most`:
+// one launch, one read-back of the state and the last scalars [1], [2].
+void Solver::run_loop(const LoopGraph& ig, double thr, int first, int most, int* done,
+                      int* broke) {
+  h_scal_[11] = thr;
+  h_ist_[0] = first;
+  h_ist_[1] = most;
+  h_ist_[2] = 0;
+  TG_CUDA(cudaMemcpyAsync(scal_.p + 11, h_scal_ + 11, sizeof(double), cudaMemcpyHostToDevice, s_));
+  TG_CUDA(cudaMemcpyAsync(istate_.p, h_ist_, 3 * sizeof(int), cudaMemcpyHostToDevice, s_));
+  TG_CUDA(cudaGraphLaunch(ig.exec, s_));
+  if (pending_x_) flush_x();  // the FP32 loop's last x update
+  TG_CUDA(cudaMemcpyAsync(h_ist_, istate_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s_));
+  TG_CUDA(cudaMemcpyAsync(h_scal_ + 1, scal_.p + 1, 2 * sizeof(double), cudaMemcpyDeviceToHost, s_));
+  TG_CUDA(cudaStreamSynchronize(s_));
+  *done = h_ist_[0];
+  *broke = h_ist_[2];
+}
+
+// ------------------------------------------------------------------ MG-PCG
+// mf_mgpcg (multigrid.cpp:1211-1313): stop at ||r|| <= tol ||b||, breakdown when
+// pAp <= 0 or non-finite, x finite at exit.
+bool Solver::mgpcg(double tol, int max_it, bool warm, SolverStats& st) {
+  const Grid& g = fp_.g;
+  const int64_t n = g.ndof;
+  launch_dot(rhs_.p, rhs_.p, n, sum_to(4, 0), s_);
+  const double bnorm2 = read_scalar(4);
+  st.iterations = 0;
+  st.residual = 0.0;
+  if (!(bnorm2 > 0.0)) {
+    launch_fill<double>(x_.p, 0.0, n, s_);
+    return true;
+  }
+  const double bnorm = std::sqrt(bnorm2), threshold = tol * bnorm;
+  if (warm) {
+    refinement_residual();
+  } else {
+    launch_fill<double>(x_.p, 0.0, n, s_);
+    TG_CUDA(cudaMemcpyAsync(r_.p, rhs_.p, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+  }
+  double* z = vcycle<double>(r_.p, scal_.p + 0);
+  TG_CUDA(cudaMemcpyAsync(p_.p, z, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s_));
+  if (!std::isfinite(read_scalar(0))) return false;
+  // p.Ap into scal_[1] (and rz_new, scal_[3], into rz, scal_[0], where the loop
+  // goes on from it), then the update with r.r into scal_[2] and the next
+  // V-cycle's first sweep into t1_.
+  auto apply_update = [&](bool next, const LoopCond& cond) {
+    SumOut pap = sum_to(1, 1), rr = sum_to(2, 2);
+    if (next) {
+      pap.copy_from = scal_.p + 3;
+      pap.copy_to = scal_.p + 0;
+    }
+    rr.cond = cond;
+    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0,
+                           ap_.p, pap, s_);
+    launch_cg_update_xr(x_.p, r_.p, p_.p, ap_.p, scal_.p + 0, scal_.p + 1, n, rr, s_, invdiag_.p,
+                        omega_, t1_.p);
+  };
+  auto next_p = [&] {
+    double* zn = vcycle<double>(r_.p, scal_.p + 3, true);
+    launch_cg_update_p<double>(p_.p, zn, scal_.p + 3, scal_.p + 0, n, s_);
+  };
+  auto finish = [&](double rr) {
+    st.residual = std::sqrt(rr) / bnorm;
+    if (!(std::sqrt(rr) <= threshold)) return false;
+    launch_dot(x_.p, x_.p, n, sum_to(5, 0), s_);
+    return std::isfinite(read_scalar(5));
+  };
+  for (int k = 1; k <= max_it; ++k) {
+    if (k > 1) next_p();
+    apply_update(k > 1, LoopCond{});
+    ++fine_matvecs_;
+    double sc[2];
+    read_scalars(1, 2, sc);
+    if (!(sc[0] > 0.0) || !std::isfinite(sc[0])) return false;
+    st.iterations = k;
+    st.residual = std::sqrt(sc[1]) / bnorm;
+    if (std::sqrt(sc[1]) <= threshold) return finish(sc[1]);
+    if (k == 1 && max_it > 1 && use_graph_) {
+      // Iterations 2.. on the device: one graph launch, one read-back.
+      if (ig64_ && ig64_->E != E_) ig64_.reset();
+      if (ig64_ || capture_loop(ig64_, [&](cudaGraphConditionalHandle h) {
+            next_p();
+            apply_update(true, LoopCond{h, scal_.p + 1, scal_.p + 11, istate_.p});
+          })) {
+        int done = 0, broke = 0;
+        run_loop(*ig64_, threshold, 1, max_it, &done, &broke);
+        const int64_t runs = int64_t(done - 1) + broke;  // body executions
+        add_kernel_launches(runs * ig64_->body_launches);
+        fine_matvecs_ += (2 * sweeps_ + 1) * runs;
+        st.iterations = done;
+        return finish(h_scal_[2]) && !broke;
+      }
+    }
+  }
+  return false;
+}
+
+// FP32 inner MG-PCG on the unit-norm residual held in zf_; solution in xf_.
+// FP64 dot products; stops at relative residual rel_tol or max_it.
 template <>
 bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* iters) {
   const Grid& g = fp_.g;
   const int64_t n = g.ndof;
   launch_fill<float>(xf_.p, 0.0f, n, s_);
   TG_CUDA(cudaMemcpyAsync(rf_.p, zf_.p, size_t(n) * sizeof(float), cudaMemcpyDeviceToDevice, s_));
-  launch_dot_f(rf_.p, rf_.p, n, part_.p, scal_.p + 10, s_);
+  launch_dot_f(rf_.p, rf_.p, n, sum_to(10, 0), s_);
   float* z = vcycle<float>(rf_.p, scal_.p + 6);
   TG_CUDA(cudaMemcpyAsync(pf_.p, z, size_t(n) * sizeof(float), cudaMemcpyDeviceToDevice, s_));
   const double b2 = read_scalar(10);
   const double thr = rel_tol * std::sqrt(b2);
-  int nb = 0;
-  *iters = 0;
-  for (int k = 1; k <= max_it; ++k) {
+  // p.Ap into scal_[7] (and rz_new, scal_[9], into rz, scal_[6]), then r with r.r
+  // into scal_[8].  x += alpha p when p is next overwritten or at exit (flush_x),
+  // or on the side stream beside the next V-cycle's coarse levels (fork_x).
+  auto apply_update = [&](bool next, const LoopCond& cond) {
+    SumOut pap = sum_to(7, 1), rr = sum_to(8, 2);
+    if (next) {
+      pap.copy_from = scal_.p + 9;
+      pap.copy_to = scal_.p + 6;
+    }
+    rr.cond = cond;
     launch_fine_op<float>(kApply, g, fp_.mc, Ef_.p, fp_.kept_node.p, pf_.p, nullptr, nullptr, 0.0f,
-                          apf_.p, part_.p, &nb, s_);
-    ++lowp_matvecs_;
-    launch_sum_partials(part_.p, nb, scal_.p + 7, s_);
-    // r now; x += alpha p when p is next overwritten or at exit (flush_x), or on
-    // the side stream beside the next V-cycle's coarse levels (fork_x).
-    launch_cg_update_r_f(rf_.p, apf_.p, scal_.p + 6, scal_.p + 7, n, part_.p, s_, invdiagf_.p,
+                          apf_.p, pap, s_);
+    launch_cg_update_r_f(rf_.p, apf_.p, scal_.p + 6, scal_.p + 7, n, rr, s_, invdiagf_.p,
                          float(omega_), t1f_.p);
     pending_x_ = true;
-    launch_sum_partials(part_.p, kRedBlocks, scal_.p + 8, s_);
+  };
+  auto next_p = [&] {
+    float* zn = vcycle<float>(rf_.p, scal_.p + 9, true);
+    flush_x();
+    launch_cg_update_p<float>(pf_.p, zn, scal_.p + 9, scal_.p + 6, n, s_);
+  };
+  *iters = 0;
+  for (int k = 1; k <= max_it; ++k) {
+    if (k > 1) next_p();
+    apply_update(k > 1, LoopCond{});
+    ++lowp_matvecs_;
     double sc[2];
     read_scalars(7, 2, sc);
     if (!(sc[0] > 0.0) || !std::isfinite(sc[0])) {  // breakdown: alpha = 0, x and r untouched
@@ -1280,21 +1299,16 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
       flush_x();
       return true;
     }
-    if (k == 1 && max_it > 1 && use_graph_ && build_inner_graph()) {
+    if (k == 1 && max_it > 1 && use_graph_ &&
+        (ig_ || capture_loop(ig_, [&](cudaGraphConditionalHandle h) {
+           pending_x_ = true;  // every body execution starts with the last one's x update
+           next_p();
+           apply_update(true, LoopCond{h, scal_.p + 7, scal_.p + 11, istate_.p});
+         }))) {
       // Iterations 2.. on the device: one graph launch, one read-back.
-      h_scal_[11] = thr;
-      h_ist_[0] = 1;
-      h_ist_[1] = max_it;
-      h_ist_[2] = 0;
-      TG_CUDA(cudaMemcpyAsync(scal_.p + 11, h_scal_ + 11, sizeof(double), cudaMemcpyHostToDevice,
-                              s_));
-      TG_CUDA(cudaMemcpyAsync(istate_.p, h_ist_, 3 * sizeof(int), cudaMemcpyHostToDevice, s_));
-      TG_CUDA(cudaGraphLaunch(ig_->exec, s_));
-      pending_x_ = true;  // the last body execution's x update
-      flush_x();
-      TG_CUDA(cudaMemcpyAsync(h_ist_, istate_.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, s_));
-      TG_CUDA(cudaStreamSynchronize(s_));
-      const int done = h_ist_[0], broke = h_ist_[2];
+      int done = 0, broke = 0;
+      pending_x_ = true;  // the last body execution's x update, run behind the graph
+      run_loop(*ig_, thr, 1, max_it, &done, &broke);
       const int64_t runs = int64_t(done - 1) + broke;  // body executions
       add_kernel_launches(runs * ig_->body_launches);
       lowp_matvecs_ += 3 * runs;
@@ -1302,13 +1316,8 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
       if (broke) ++st.inner_breakdowns;
       return true;
     }
-    z = vcycle<float>(rf_.p, scal_.p + 9, true);
-    flush_x();
-    launch_cg_update_p<float>(pf_.p, z, scal_.p + 9, scal_.p + 6, n, s_);
-    TG_CUDA(cudaMemcpyAsync(scal_.p + 6, scal_.p + 9, sizeof(double), cudaMemcpyDeviceToDevice, s_));
   }
   flush_x();
-  (void)st;
   return true;
 }
 
@@ -1324,7 +1333,7 @@ void Solver::refinement_residual() {
     launch_fine_residual_df(g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, r_.p, s_);
   } else {
     launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
-                           nullptr, nullptr, s_);
+                           SumOut{}, s_);
   }
   ++fine_matvecs_;
 }
@@ -1333,7 +1342,7 @@ bool Solver::mixed_refine(double tol, int max_it, bool warm, SolverStats& st) {
   mixed_partial_ = false;
   const Grid& g = fp_.g;
   const int64_t n = g.ndof;
-  launch_dot(rhs_.p, rhs_.p, n, part_.p, scal_.p + 4, s_);
+  launch_dot(rhs_.p, rhs_.p, n, sum_to(4, 0), s_);
   const double bnorm2 = read_scalar(4);
   st.iterations = 0;
   st.residual = 0.0;
@@ -1344,7 +1353,7 @@ bool Solver::mixed_refine(double tol, int max_it, bool warm, SolverStats& st) {
   const double bnorm = std::sqrt(bnorm2), threshold = tol * bnorm;
   if (warm) {
     launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
-                           nullptr, nullptr, s_);
+                           SumOut{}, s_);
     ++fine_matvecs_;
   } else {
     launch_fill<double>(x_.p, 0.0, n, s_);
@@ -1360,7 +1369,7 @@ bool Solver::mixed_refine(double tol, int max_it, bool warm, SolverStats& st) {
   int total_inner = 0;
   double rn0 = -1.0;
   for (int ref = 0; ref <= max_ref; ++ref) {
-    launch_dot(r_.p, r_.p, n, part_.p, scal_.p + 5, s_);
+    launch_dot(r_.p, r_.p, n, sum_to(5, 0), s_);
     const double rr = read_scalar(5);
     const double rn = std::sqrt(rr);
     st.residual = rn / bnorm;
@@ -1399,7 +1408,7 @@ bool Solver::jacobi_pcg(double tol, int max_it, bool warm, SolverStats& st) {
   const Grid& g = fp_.g;
   const int64_t n = g.ndof;
   const int maxIters = max_it > 0 ? max_it : int(std::min<int64_t>(2 * fp_.ng, 1 << 30));
-  launch_dot(rhs_.p, rhs_.p, n, part_.p, scal_.p + 4, s_);
+  launch_dot(rhs_.p, rhs_.p, n, sum_to(4, 0), s_);
   const double rhs2 = read_scalar(4);
   st.iterations = 0;
   st.residual = 0.0;
@@ -1411,35 +1420,57 @@ bool Solver::jacobi_pcg(double tol, int max_it, bool warm, SolverStats& st) {
   if (threshold < std::numeric_limits<double>::min()) threshold = std::numeric_limits<double>::min();
   if (!warm) launch_fill<double>(x_.p, 0.0, n, s_);
   launch_fine_op<double>(kResidual, g, fp_.mc, E_, fp_.kept_node.p, x_.p, rhs_.p, nullptr, 0.0, r_.p,
-                         nullptr, nullptr, s_);
+                         SumOut{}, s_);
   ++fine_matvecs_;
-  launch_dot(r_.p, r_.p, n, part_.p, scal_.p + 2, s_);
+  launch_dot(r_.p, r_.p, n, sum_to(2, 0), s_);
   double rr = read_scalar(2);
   if (rr < threshold) {
     st.residual = std::sqrt(rr / rhs2);
     return st.residual <= tol;
   }
-  launch_scale_mask(p_.p, r_.p, invdiag_.p, n, part_.p, s_);
-  launch_sum_partials(part_.p, kRedBlocks, scal_.p + 0, s_);
-  int i = 0, nb = 0;
+  launch_scale_mask(p_.p, r_.p, invdiag_.p, n, sum_to(0, 3), s_);
+  auto apply_update = [&](bool next, const LoopCond& cond) {
+    SumOut pap = sum_to(1, 1), r2 = sum_to(2, 2);
+    if (next) {
+      pap.copy_from = scal_.p + 3;
+      pap.copy_to = scal_.p + 0;
+    }
+    r2.cond = cond;
+    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0,
+                           ap_.p, pap, s_);
+    launch_cg_update_xr(x_.p, r_.p, p_.p, ap_.p, scal_.p + 0, scal_.p + 1, n, r2, s_);
+  };
+  auto next_p = [&] {
+    launch_scale_mask(z_.p, r_.p, invdiag_.p, n, sum_to(3, 3), s_);
+    launch_cg_update_p<double>(p_.p, z_.p, scal_.p + 3, scal_.p + 0, n, s_);
+  };
+  int i = 0;
   while (i < maxIters) {
-    launch_fine_op<double>(kApply, g, fp_.mc, E_, fp_.kept_node.p, p_.p, nullptr, nullptr, 0.0, ap_.p,
-                           part_.p, &nb, s_);
+    if (i > 0) next_p();
+    apply_update(i > 0, LoopCond{});
     ++fine_matvecs_;
-    launch_sum_partials(part_.p, nb, scal_.p + 1, s_);
-    launch_cg_update_xr<double>(x_.p, r_.p, p_.p, ap_.p, scal_.p + 0, scal_.p + 1, n, part_.p, s_);
-    launch_sum_partials(part_.p, kRedBlocks, scal_.p + 2, s_);
     rr = read_scalar(2);
     if (rr < threshold) break;
-    launch_scale_mask(z_.p, r_.p, invdiag_.p, n, part_.p, s_);
-    launch_sum_partials(part_.p, kRedBlocks, scal_.p + 3, s_);
-    launch_cg_update_p<double>(p_.p, z_.p, scal_.p + 3, scal_.p + 0, n, s_);
-    TG_CUDA(cudaMemcpyAsync(scal_.p + 0, scal_.p + 3, sizeof(double), cudaMemcpyDeviceToDevice, s_));
     ++i;
+    if (i == 1 && maxIters > 1 && use_graph_) {
+      if (igj_ && igj_->E != E_) igj_.reset();
+      if (igj_ || capture_loop(igj_, [&](cudaGraphConditionalHandle h) {
+            next_p();
+            apply_update(true, LoopCond{h, nullptr, scal_.p + 11, istate_.p});
+          })) {
+        int broke = 0;
+        run_loop(*igj_, threshold, 1, maxIters, &i, &broke);
+        rr = h_scal_[2];
+        const int64_t runs = int64_t(i - 1) + (rr < threshold ? 1 : 0);
+        add_kernel_launches(runs * igj_->body_launches);
+        fine_matvecs_ += runs;
+        break;
+      }
+    }
   }
   st.iterations = i;
   st.residual = std::sqrt(rr / rhs2);
-  launch_dot(x_.p, x_.p, n, part_.p, scal_.p + 5, s_);
+  launch_dot(x_.p, x_.p, n, sum_to(5, 0), s_);
   const bool finite = std::isfinite(read_scalar(5));
   return st.residual <= tol && finite;
 }

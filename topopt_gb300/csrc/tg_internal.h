@@ -146,7 +146,26 @@ struct ModalConsts {
 };
 
 // ---------------------------------------------------------------- operator
-enum ApplyMode { kApply = 0, kResidual = 1, kSmooth = 2, kCheb = 3 };
+enum ApplyMode { kApply = 0, kResidual = 1, kSmooth = 2, kCheb = 3, kDinvA = 4 };
+
+// Where a sum over a grid of CTAs goes: one partial per CTA into part, and, with
+// count (a zero that the launch leaves zero), the total into out by the CTA that
+// ends last, which then also copies *copy_from to *copy_to and takes a
+// graph-resident loop's decision (tg_reduce.h).
+struct LoopCond {
+  cudaGraphConditionalHandle h{};
+  const double* pap = nullptr;  // null: Jacobi-PCG
+  const double* thr = nullptr;
+  int* st = nullptr;            // null: no loop
+};
+struct SumOut {
+  double* part = nullptr;
+  double* out = nullptr;
+  unsigned* count = nullptr;
+  const double* copy_from = nullptr;
+  double* copy_to = nullptr;
+  LoopCond cond{};
+};
 
 // kResidual of the FP64 operator evaluated in double-float arithmetic (FP32
 // pairs, ~48 significant bits): the refinement residual of the mixed form.
@@ -154,16 +173,16 @@ void launch_fine_residual_df(const Grid& g, const ModalConsts& c, const double* 
                              const uint8_t* kept_node, const double* x, const double* b, double* y,
                              cudaStream_t s);
 // Fine operator on the full grid, element factors `ef` (0 = no element):
-//   kApply:    y = M A x                 (M = kept mask; dot = sum x.y if dot_part)
+//   kApply:    y = M A x                 (M = kept mask; dot: sum x.y if dot.part)
 //   kResidual: y = M (b - A x)
 //   kSmooth:   y = x + omega*invdiag*(b - A x)   (invdiag is 0 off the kept set)
 //   kept_node: M as one byte per node (bit k: DOF 3n+k kept); null keeps every
 //   DOF, and then x may hold anything at nodes of absent elements.
-//   kSmooth with dot_part: partials of b . y as well.
+//   kSmooth with dot.part: sum b . y.
 template <class T>
 void launch_fine_op(int mode, const Grid& g, const ModalConsts& mc, const T* ef,
                     const uint8_t* kept_node, const T* x, const T* b, const T* invdiag, T omega,
-                    T* y, double* dot_part, int* nblocks_out, cudaStream_t s);
+                    T* y, const SumOut& dot, cudaStream_t s);
 int fine_op_blocks(const Grid& g, bool fp64);  // upper bound of the partials any schedule writes
 
 // How the FP32 fine operator is scheduled on a grid (k_operator.cu): two packed
@@ -186,7 +205,7 @@ bool fine_schedule_known(const Grid& g);  // in the table, or an override is set
 void launch_fine_op_sched(const FineSchedule& fs, int mode, const Grid& g, const ModalConsts& c,
                           const float* ef, const uint8_t* kept_node, const float* x,
                           const float* b, const float* invdiag, float omega, float* y,
-                          double* dot_part, int* nblocks_out, cudaStream_t s);
+                          const SumOut& dot, cudaStream_t s);
 // Times every candidate schedule of the FP32 operator on the given buffers
 // (CUDA events on s) for the apply and, with b and invdiag, the residual and
 // smoothing modes; publishes the fastest per mode in the table for g (one sweep
@@ -224,23 +243,25 @@ void launch_fine_invdiag(const Grid& g, double kdiag, const double* ef, const ui
                          double* invdiag, cudaStream_t s);
 
 // ------------------------------------------------------------------ vectors
-// Deterministic reductions: a fixed grid of kRedBlocks blocks writes partials,
-// one block sums them in order.
-constexpr int kRedBlocks = 608;  // 4 x 152 SMs
-void launch_dot(const double* a, const double* b, int64_t n, double* part, double* out,
-                cudaStream_t s);
-void launch_dot_f(const float* a, const float* b, int64_t n, double* part, double* out,
-                  cudaStream_t s);
+// Deterministic reductions: a grid of red_blocks(n) blocks, fixed by n, and the
+// total by the block that ends last (SumOut).
+constexpr int kRedBlocks = 608;  // 4 x 152 SMs, the most
+int red_blocks(int64_t n);
+void launch_dot(const double* a, const double* b, int64_t n, const SumOut& o, cudaStream_t s);
+void launch_dot_f(const float* a, const float* b, int64_t n, const SumOut& o, cudaStream_t s);
 void launch_sum_partials(const double* part, int n, double* out, cudaStream_t s);
-// Partials of a . b (FP32 vectors) over kRedBlocks blocks, not yet summed.
-void launch_dot_partials_f(const float* a, const float* b, int64_t n, double* part,
-                           cudaStream_t s);
-// PCG pieces with scalars living in device memory (no host round trip).
-template <class T>
-void launch_cg_update_xr(T* x, T* r, const T* p, const T* ap, const double* rz,
-                         const double* pap, int64_t n, double* rr_part, cudaStream_t s);
-// The FP32 PCG update in two kernels (alpha = rz / pAp as launch_cg_update_xr
-// forms it, 0 on a breakdown): r -= alpha Ap with partials of r.r, and
+// PCG pieces with scalars living in device memory (no host round trip): x += alpha
+// p, r -= alpha Ap with alpha = rz / pAp (0 on a breakdown), sum of r.r; with x0
+// set, also x0 = omega invdiag .* r.
+void launch_cg_update_xr(double* x, double* r, const double* p, const double* ap,
+                         const double* rz, const double* pap, int64_t n, const SumOut& rr,
+                         cudaStream_t s, const double* invdiag = nullptr, double omega = 0.0,
+                         double* x0 = nullptr);
+// The FP32 PCG update in two kernels: r (and x0) with r.r, and x.
+void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const double* pap,
+                          int64_t n, const SumOut& rr, cudaStream_t s,
+                          const float* invdiag = nullptr, float omega = 0.0f,
+                          float* x0 = nullptr);
 // x += alpha p.
 // With x0 set, launch_cg_update_r_f also writes x0 = omega invdiag .* r.
 void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const double* pap,
@@ -250,7 +271,7 @@ void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const dou
 void launch_cg_update_x_f(float* x, const float* p, const double* rz, const double* pap,
                           int64_t n, cudaStream_t s);
 void launch_scale_mask(double* z, const double* r, const double* invdiag, int64_t n,
-                       double* rz_part, cudaStream_t s);
+                       const SumOut& rz, cudaStream_t s);
 template <class T>
 void launch_cg_update_p(T* p, const T* z, const double* rz_new, const double* rz_old, int64_t n,
                         cudaStream_t s);

@@ -60,11 +60,11 @@ void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, co
                    const T* b, const T* invdiag, T omega, T* y, cudaStream_t s,
                    ChebStep ch = ChebStep{});
 // lambda_max(D^-1 A) of a stencil level by `iters` power-iteration steps (v, w:
-// level-sized scratch), times `safety`, into lam[0] on the device.
-template <class T>
-void mg_lambda_max(const MgDims& d, const T* A, const uint8_t* act, const T* invdiag, T* v,
-                   T* w, int iters, double safety, double* part, double* nrm2, double* lam,
-                   cudaStream_t s);
+// level-sized scratch; part: partials, nrm2: two sums, count: a zero counter),
+// times `safety`, into lam[0] on the device.
+void mg_lambda_max(const MgDims& d, const float* A, const uint8_t* act, const float* invdiag,
+                   float* v, float* w, int iters, double safety, double* part, double* nrm2,
+                   unsigned* count, double* lam, cudaStream_t s);
 template <class T>
 void mg_jacobi_first(const T* b, const T* invdiag, T omega, int64_t n, T* x, cudaStream_t s);
 // The coarse level's first smoothing step from a zero iterate, taken by the

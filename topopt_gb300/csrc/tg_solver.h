@@ -96,7 +96,13 @@ class Solver {
   float* fused_coarse_vcycle();
   template <class T>
   bool inner_pcg(int max_it, double rel_tol, SolverStats& st, int* iters);
-  bool build_inner_graph();
+  struct LoopGraph;
+  template <class Body>
+  bool capture_loop(std::unique_ptr<LoopGraph>& slot, Body&& record);
+  void run_loop(const LoopGraph& ig, double thr, int first, int most, int* done, int* broke);
+  static constexpr int kSumSlots = 4;
+  // The sum of one launch: partials in part_, total in scal_[idx], counter `slot`.
+  SumOut sum_to(int idx, int slot) { return SumOut{part_.p, scal_.p + idx, cnt_.p + slot}; }
   double read_scalar(int idx);
   void read_scalars(int idx0, int n, double* out);
 
@@ -116,7 +122,8 @@ class Solver {
   int cheb_iters_ = 10;
   double cheb_safety_ = 1.1;
   DBuf<double> lam_;     // lambda_max per level
-  DBuf<double> pipart_;  // per level: the power iteration's partials and norm
+  DBuf<double> pipart_;  // per level: the power iteration's partials and norms
+  DBuf<unsigned> picnt_;
   std::vector<cudaStream_t> pi_streams_;  // per level, the power iterations' streams
   std::vector<cudaEvent_t> pi_events_;
   cudaEvent_t pi_fork_ = nullptr;
@@ -129,6 +136,7 @@ class Solver {
   DBuf<double> invdiag_, rhs_, x_, r_, z_, p_, ap_, t0_, t1_;
   DBuf<float> Ef_, invdiagf_, xf_, rf_, zf_, pf_, apf_, t0f_, t1f_;
   DBuf<double> part_, scal_;
+  DBuf<unsigned> cnt_;
   double* h_scal_ = nullptr;  // pinned
   int part_n_ = 0;
   // hierarchy
@@ -141,12 +149,11 @@ class Solver {
   int nc_ = 0;
   DBuf<int> cidx_, cdof_, chol_fail_;
   DBuf<double> chol_, chol_work_, chol_li_, chol_inv_;
-  // The mixed inner PCG loop as one CUDA graph: a conditional WHILE node whose
-  // body is one PCG iteration (V-cycle, update, apply) ending in a kernel that
-  // decides, on the device, whether another iteration runs.
-  struct InnerGraph;
-  std::unique_ptr<InnerGraph> ig_;
-  bool ig_failed_ = false, use_graph_ = true;
+  // The PCG loops (mixed inner, FP64 multigrid, FP64 Jacobi) as one CUDA graph
+  // each: a conditional WHILE node whose body is one iteration and whose last
+  // kernel decides, on the device, whether another one runs.
+  std::unique_ptr<LoopGraph> ig_, ig64_, igj_;
+  bool graph_failed_ = false, use_graph_ = true;
   DBuf<int> istate_;           // [0] iterations done, [1] budget, [2] breakdown
   // Level 1 of the FP32 V-cycle without its matrix: the coarse elements whose
   // matrix is not the children's sum (a Dirichlet or untouched fine DOF in a

@@ -106,10 +106,10 @@ FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const 
     FineSchedule best = default_fine_schedule(g);
     float best_ms = 1e30f;
     for (const FineSchedule& c : cands) {
-      launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, pp, nullptr, s);
+      launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, SumOut{pp}, s);
       TG_CUDA(cudaEventRecord(ea, s));
       for (int r = 0; r < reps; ++r)
-        launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, pp, nullptr, s);
+        launch_fine_op_sched(c, mode, g, mc, ef, kn, x, bb, dd, 0.6f, y, SumOut{pp}, s);
       TG_CUDA(cudaEventRecord(eb, s));
       TG_CUDA(cudaEventSynchronize(eb));
       float ms = 0.0f;
