@@ -86,205 +86,187 @@ __device__ __forceinline__ void kron_map(const T (&mw)[3][4], T (&v)[24]) {
   }
 }
 
-// One warp per coarse element; lane c < 24 owns column c of the coarse element
-// matrix (rows in corner-bit order, row = 3*corner + comp).  For every child,
-// X = S W (lane r = row r of S) then Y += W^T X (lane c = column c), with the
-// sparsity pattern of W uniform across the warp.  S is the child's matrix:
+// One block of eight warps per coarse element, a warp per child; lane c < 24 owns
+// column c of the child's share (rows in corner-bit order, row = 3*corner +
+// comp).  X = S W (lane r = row r of S), then Y = W^T X (lane c = column c), with
+// the sparsity pattern of W uniform across the warp.  S is the child's matrix:
 // level 1 -- f * Ke with inactive fine DOFs zeroed (or the precomputed
 // G_c = W_c^T Ke W_c times f when all 24 are active); deeper levels -- the stored,
-// already masked, child element matrix.  Rows/cols of inactive coarse DOFs are
-// zeroed at the end.
-// With skip set, level 1's elements with skip[ce] < 0 are left to
-// k_galerkin1_fast.
+// already masked, child element matrix.  The shares are added in child order;
+// rows/cols of inactive coarse DOFs are zeroed at the end.  (One warp walking its
+// element's children took eight times as long a chain: 110 us in FP64 and 25 in
+// FP32 on levels of any small size.)
+// With list set, only the nlist coarse elements it names (level 1's others are
+// k_galerkin1_fast's).
 template <class T, bool LEVEL1>
-__global__ void __launch_bounds__(128) k_galerkin(MgDims fd, MgDims cd, const T* __restrict__ ef,
+__global__ void __launch_bounds__(256) k_galerkin(MgDims fd, MgDims cd, const T* __restrict__ ef,
                                                   const uint8_t* __restrict__ fact,
                                                   const uint8_t* __restrict__ cact,
                                                   const T* __restrict__ Ke,
                                                   const T* __restrict__ G,
-                                                  const T* __restrict__ Kf,
-                                                  T* __restrict__ Kc,
-                                                  const int* __restrict__ skip) {
-  constexpr int NW = 4;
+                                                  const T* __restrict__ Kf, T* __restrict__ Kc,
+                                                  const int* __restrict__ list, int64_t nlist) {
   constexpr int LD = 25;  // padded row stride: row and column walks are bank-conflict free
-  // Level 1 in FP32: the 8 child blocks G_c live in shared memory (18 KB per CTA).
-  constexpr bool kSmemG = LEVEL1 && sizeof(T) == 4;
-  __shared__ T sS[NW][24 * LD];
-  __shared__ T sX[NW][24 * LD];
-  __shared__ T sG[kSmemG ? 8 * 576 : 1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T* S = sS[warp];
-  T* X = sX[warp];
-  if (kSmemG) {
-    for (int e = threadIdx.x; e < 8 * 576; e += blockDim.x) sG[e] = G[e];
-    __syncthreads();
-    G = sG;
-  }
-  const int64_t nce = int64_t(cd.ex) * cd.ey * cd.ez;
-  for (int64_t ce = blockIdx.x * int64_t(NW) + warp; ce < nce; ce += int64_t(gridDim.x) * NW) {
-    if (skip != nullptr && skip[ce] < 0) continue;  // warp-uniform
+  __shared__ T sX[8][24 * LD];
+  __shared__ bool s_have[8];
+  __shared__ T s_f[8];  // a child's factor: its modulus where X holds G_c, else 1
+  __shared__ unsigned s_cm;
+  const int ch = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T* X = sX[ch];
+  for (int64_t q = blockIdx.x; q < nlist; q += gridDim.x) {
+    const int64_t ce = list ? list[q] : q;
     const int I = int(ce % cd.ex), J = int((ce / cd.ex) % cd.ey),
               K = int(ce / (int64_t(cd.ex) * cd.ey));
     const int hm = cd.align ? ((2 * I + 1 == fd.ex) | ((2 * J + 1 == fd.ey) << 1) |
                                ((2 * K + 1 == fd.ez) << 2))
                             : 0;
-    T acc[24];
-#pragma unroll
-    for (int r = 0; r < 24; ++r) acc[r] = T(0);
-    // Level 1: the children's moduli (lane ch holds child ch's) and this lane's
-    // kept bit of every child (bit ch), all requested before the child loop.
-    T f_lane = T(0);
-    unsigned int kept_bits = 0;
-    if (LEVEL1) {
-      if (lane < 8) {
-        const int fi = 2 * I + cx(lane), fj = 2 * J + cy(lane), fk = 2 * K + cz(lane);
-        if (fi < fd.ex && fj < fd.ey && fk < fd.ez)
-          f_lane = ef[(int64_t(fk) * fd.ey + fj) * fd.ex + fi];
-      }
+    const int fi = 2 * I + cx(ch), fj = 2 * J + cy(ch), fk = 2 * K + cz(ch);
+    bool have = fi < fd.ex && fj < fd.ey && fk < fd.ez;
+    const int64_t fe = (int64_t(fk) * fd.ey + fj) * fd.ex + fi;
+    const int cc = lane / 3, comp = lane % 3;
+    T f = T(1);
+    unsigned m = 0xffffffu;
+    if (LEVEL1 && have) {
+      f = ef[fe];
+      have = f != T(0);
+      unsigned bit = 0;
       if (lane < 24) {
-        const int c = lane / 3, comp = lane % 3;
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          const int fi = 2 * I + cx(ch), fj = 2 * J + cy(ch), fk = 2 * K + cz(ch);
-          if (fi >= fd.ex || fj >= fd.ey || fk >= fd.ez) continue;
-          const int64_t node =
-              (int64_t(fk + cz(c)) * fd.nny + (fj + cy(c))) * fd.nnx + (fi + cx(c));
-          if (fact[3 * node + comp]) kept_bits |= 1u << ch;
-        }
+        const int64_t node =
+            (int64_t(fk + cz(cc)) * fd.nny + (fj + cy(cc))) * fd.nnx + (fi + cx(cc));
+        bit = fact[3 * node + comp] ? 1u << lane : 0u;
       }
+      m = __reduce_or_sync(0xffffffffu, bit);
     }
-    for (int ch = 0; ch < 8; ++ch) {
-      const int fi = 2 * I + cx(ch), fj = 2 * J + cy(ch), fk = 2 * K + cz(ch);
-      if (fi >= fd.ex || fj >= fd.ey || fk >= fd.ez) continue;
-      const int64_t fe = (int64_t(fk) * fd.ey + fj) * fd.ex + fi;
-      T f = T(1);
-      unsigned int m = 0xffffffu;
-      if (LEVEL1) {
-        f = __shfl_sync(0xffffffffu, f_lane, ch);
-        if (f == T(0)) continue;
-        m = __reduce_or_sync(0xffffffffu, ((kept_bits >> ch) & 1u) << lane);
-        if (m == 0xffffffu && hm == 0) {
-          if (lane < 24)
+    if (have) {  // warp-uniform
+      if (LEVEL1 && m == 0xffffffu && hm == 0) {
+        if (lane < 24)
 #pragma unroll
-            for (int r = 0; r < 24; ++r) acc[r] += f * G[ch * 576 + r * 24 + lane];
-          continue;
+          for (int r = 0; r < 24; ++r) X[r * LD + lane] = G[ch * 576 + r * 24 + lane];
+      } else {
+        // W = W_x (x) W_y (x) W_z on the corner index (times I3 on components):
+        // per axis a 2x2 map from the child's sub-corner bit to the parent's
+        // corner bit -- [[1,0],[1/2,1/2]] for child bit 0, [[1/2,1/2],[0,1]] for
+        // child bit 1, the identity on an aligned half element.  X = S W and
+        // Y = W^T X are three 2x2 passes each instead of a dense 8x8 product.
+        T mw[3][4];  // per axis: M[sc][t] as {m00, m01, m10, m11}; warp-uniform
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const bool half = (hm >> a) & 1, hi = (ch >> a) & 1;
+          mw[a][0] = half ? T(1) : (hi ? T(0.5) : T(1));
+          mw[a][1] = half ? T(0) : (hi ? T(0.5) : T(0));
+          mw[a][2] = half ? T(0) : (hi ? T(0) : T(0.5));
+          mw[a][3] = half ? T(1) : (hi ? T(1) : T(0.5));
         }
+        // Row `lane` of S: staged through X, so that global reads are whole lines.
         for (int e = lane; e < 576; e += 32) {
           const int r = e / 24, c2 = e % 24;
-          S[r * LD + c2] = ((m >> r) & 1u) && ((m >> c2) & 1u) ? f * Ke[e] : T(0);
+          if (LEVEL1)
+            X[r * LD + c2] = ((m >> r) & 1u) && ((m >> c2) & 1u) ? f * Ke[e] : T(0);
+          else
+            X[r * LD + c2] = Kf[fe * 576 + e];
         }
-      } else {
-        for (int e = lane; e < 576; e += 32) S[(e / 24) * LD + e % 24] = Kf[fe * 576 + e];
-      }
-      __syncwarp();
-      // W = W_x (x) W_y (x) W_z on the corner index (times I3 on components):
-      // per axis a 2x2 map from the child's sub-corner bit to the parent's
-      // corner bit -- [[1,0],[1/2,1/2]] for child bit 0, [[1/2,1/2],[0,1]] for
-      // child bit 1, the identity on an aligned half element.  X = S W and
-      // Y += W^T X are three 2x2 passes each instead of a dense 8x8 product.
-      T mw[3][4];  // per axis: M[sc][t] as {m00, m01, m10, m11}; warp-uniform
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const bool half = (hm >> a) & 1, hi = (ch >> a) & 1;
-        mw[a][0] = half ? T(1) : (hi ? T(0.5) : T(1));
-        mw[a][1] = half ? T(0) : (hi ? T(0.5) : T(0));
-        mw[a][2] = half ? T(0) : (hi ? T(0) : T(0.5));
-        mw[a][3] = half ? T(1) : (hi ? T(1) : T(0.5));
-      }
-      if (lane < 24) {  // X = S W: lane = row
+        __syncwarp();
         T v[24];
+        if (lane < 24) {  // X = S W: lane = row
 #pragma unroll
-        for (int j = 0; j < 24; ++j) v[j] = S[lane * LD + j];
-        kron_map(mw, v);
+          for (int j = 0; j < 24; ++j) v[j] = X[lane * LD + j];
+          kron_map(mw, v);
 #pragma unroll
-        for (int j = 0; j < 24; ++j) X[lane * LD + j] = v[j];
+          for (int j = 0; j < 24; ++j) X[lane * LD + j] = v[j];
+        }
+        __syncwarp();
+        if (lane < 24) {  // Y = W^T X: lane = column
+#pragma unroll
+          for (int j = 0; j < 24; ++j) v[j] = X[j * LD + lane];
+          kron_map(mw, v);
+#pragma unroll
+          for (int j = 0; j < 24; ++j) X[j * LD + lane] = v[j];
+        }
       }
-      __syncwarp();
-      if (lane < 24) {  // Y += W^T X: lane = column
-        T v[24];
-#pragma unroll
-        for (int j = 0; j < 24; ++j) v[j] = X[j * LD + lane];
-        kron_map(mw, v);
-#pragma unroll
-        for (int j = 0; j < 24; ++j) acc[j] += v[j];
+    }
+    if (lane == 0) {
+      s_have[ch] = have;
+      s_f[ch] = LEVEL1 && m == 0xffffffu && hm == 0 ? f : T(1);
+    }
+    if (ch == 0) {
+      unsigned cm = 0;
+      if (lane < 24) {
+        const int64_t node =
+            (int64_t(K + cz(cc)) * cd.nny + (J + cy(cc))) * cd.nnx + (I + cx(cc));
+        if (cact[3 * node + comp]) cm = 1u << lane;
       }
-      __syncwarp();
+      cm = __reduce_or_sync(0xffffffffu, cm);
+      if (lane == 0) s_cm = cm;
     }
-    unsigned int cm = 0;
-    if (lane < 24) {
-      const int c = lane / 3, comp = lane % 3;
-      const int64_t node = (int64_t(K + cz(c)) * cd.nny + (J + cy(c))) * cd.nnx + (I + cx(c));
-      if (cact[3 * node + comp]) cm = 1u << lane;
-    }
-    cm = __reduce_or_sync(0xffffffffu, cm);
-    if (lane < 24) {
-      const bool colk = (cm >> lane) & 1u;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 576; e += 256) {
+      const int r = e / 24, c = e % 24;
+      T acc = T(0);
 #pragma unroll
-      for (int r = 0; r < 24; ++r) Kc[ce * 576 + r * 24 + lane] = (colk && ((cm >> r) & 1u)) ? acc[r] : T(0);
+      for (int k = 0; k < 8; ++k)
+        if (s_have[k]) acc = fma(s_f[k], sX[k][r * LD + c], acc);
+      Kc[ce * 576 + e] = ((s_cm >> r) & 1u) && ((s_cm >> c) & 1u) ? acc : T(0);
     }
+    __syncthreads();
   }
 }
 
 // Node stencil from the element matrices around each node: the self block and
 // the forward blocks only.  Entry index q = (j*3 + c1)*3 + c2 with
-// j = d - 13, d = (dz+1)*9 + (dy+1)*3 + (dx+1) >= 13.  With A null only the
-// inverse diagonal is formed (the self block), from the same sums.
+// j = d - 13, d = (dz+1)*9 + (dy+1)*3 + (dx+1) >= 13.  One thread per node and
+// block (blockIdx.y = j): a thread that formed a node's 14 blocks one after
+// another took 20-50 us on the smallest levels.  With A null only the inverse
+// diagonal is formed (one row of blocks, j = 0), from the same sums.
 template <class T>
 __global__ void k_assemble_stencil(MgDims d, const T* __restrict__ Kel,
                                    const uint8_t* __restrict__ act, T* __restrict__ A,
                                    T* __restrict__ invdiag) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
+  const int j = blockIdx.y, di = 13 + j;
+  const int dx = di % 3 - 1, dy = (di / 3) % 3 - 1, dz = di / 9 - 1;
   for (int64_t n = blockIdx.x * int64_t(kThreads) + threadIdx.x; n < nn;
        n += int64_t(gridDim.x) * kThreads) {
     int a, b, c;
     node_abc(d, n, a, b, c);
     bool ra[3];
     for (int k = 0; k < 3; ++k) ra[k] = act[3 * n + k] != 0;
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int di = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
-          if (di < 13) continue;  // backward blocks: the neighbour's forward block, transposed
-          if (A == nullptr && di != 13) continue;
-          const int j = di - 13;
-          T blk[9];
+    T blk[9];
 #pragma unroll
-          for (int k = 0; k < 9; ++k) blk[k] = T(0);
-          // Elements containing both n and n+d: offsets ox in {-1,0} with the
-          // node at corner (-ox) and the neighbour at corner (-ox + dx) in [0,1].
-          for (int oz = -1; oz <= 0; ++oz) {
-            const int lz = -oz, mz = lz + dz;
-            if (mz < 0 || mz > 1) continue;
-            for (int oy = -1; oy <= 0; ++oy) {
-              const int ly = -oy, my = ly + dy;
-              if (my < 0 || my > 1) continue;
-              for (int ox = -1; ox <= 0; ++ox) {
-                const int lx = -ox, mx = lx + dx;
-                if (mx < 0 || mx > 1) continue;
-                const int ei = a + ox, ej = b + oy, ek = c + oz;
-                if (ei < 0 || ei >= d.ex || ej < 0 || ej >= d.ey || ek < 0 || ek >= d.ez) continue;
-                const int64_t e = (int64_t(ek) * d.ey + ej) * d.ex + ei;
-                const int ln = lx | (ly << 1) | (lz << 2), lm = mx | (my << 1) | (mz << 2);
-                const T* Ke = Kel + e * 576;
+    for (int k = 0; k < 9; ++k) blk[k] = T(0);
+    // Elements containing both n and n+d: offsets ox in {-1,0} with the
+    // node at corner (-ox) and the neighbour at corner (-ox + dx) in [0,1].
+    for (int oz = -1; oz <= 0; ++oz) {
+      const int lz = -oz, mz = lz + dz;
+      if (mz < 0 || mz > 1) continue;
+      for (int oy = -1; oy <= 0; ++oy) {
+        const int ly = -oy, my = ly + dy;
+        if (my < 0 || my > 1) continue;
+        for (int ox = -1; ox <= 0; ++ox) {
+          const int lx = -ox, mx = lx + dx;
+          if (mx < 0 || mx > 1) continue;
+          const int ei = a + ox, ej = b + oy, ek = c + oz;
+          if (ei < 0 || ei >= d.ex || ej < 0 || ej >= d.ey || ek < 0 || ek >= d.ez) continue;
+          const int64_t e = (int64_t(ek) * d.ey + ej) * d.ex + ei;
+          const int ln = lx | (ly << 1) | (lz << 2), lm = mx | (my << 1) | (mz << 2);
+          const T* Ke = Kel + e * 576;
 #pragma unroll
-                for (int c1 = 0; c1 < 3; ++c1)
+          for (int c1 = 0; c1 < 3; ++c1)
 #pragma unroll
-                  for (int c2 = 0; c2 < 3; ++c2) blk[c1 * 3 + c2] += Ke[(3 * ln + c1) * 24 + 3 * lm + c2];
-              }
-            }
-          }
-          if (A != nullptr)
-#pragma unroll
-            for (int c1 = 0; c1 < 3; ++c1)
-#pragma unroll
-              for (int c2 = 0; c2 < 3; ++c2)
-                A[int64_t(j * 9 + c1 * 3 + c2) * nn + n] = ra[c1] ? blk[c1 * 3 + c2] : T(0);
-          if (j == 0)
-            for (int k = 0; k < 3; ++k) {
-              const T dg = blk[k * 3 + k];
-              invdiag[3 * n + k] = (ra[k] && dg > T(0)) ? T(1) / dg : T(0);
-            }
+            for (int c2 = 0; c2 < 3; ++c2) blk[c1 * 3 + c2] += Ke[(3 * ln + c1) * 24 + 3 * lm + c2];
         }
+      }
+    }
+    if (A != nullptr)
+#pragma unroll
+      for (int c1 = 0; c1 < 3; ++c1)
+#pragma unroll
+        for (int c2 = 0; c2 < 3; ++c2)
+          A[int64_t(j * 9 + c1 * 3 + c2) * nn + n] = ra[c1] ? blk[c1 * 3 + c2] : T(0);
+    if (j == 0)
+      for (int k = 0; k < 3; ++k) {
+        const T dg = blk[k * 3 + k];
+        invdiag[3 * n + k] = (ra[k] && dg > T(0)) ? T(1) / dg : T(0);
+      }
   }
 }
 
@@ -719,28 +701,118 @@ __global__ void k_dense_from_stencil(MgDims d, const T* __restrict__ A,
                                      const int* __restrict__ cidx, int nc,
                                      double* __restrict__ D) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
+  const int j = blockIdx.y, di = 13 + j;
   for (int64_t n = blockIdx.x * int64_t(kThreads) + threadIdx.x; n < nn;
        n += int64_t(gridDim.x) * kThreads) {
     int a, b, c;
     node_abc(d, n, a, b, c);
-    for (int j = 0; j < 14; ++j) {
-      const int di = 13 + j;
-      const int i = a + di % 3 - 1, jj = b + (di / 3) % 3 - 1, k = c + di / 9 - 1;
-      if (i < 0 || i >= d.nnx || jj < 0 || jj >= d.nny || k >= d.nnz) continue;
-      const int64_t m = (int64_t(k) * d.nny + jj) * d.nnx + i;
-      for (int c1 = 0; c1 < 3; ++c1) {
-        const int row = cidx[3 * n + c1];
-        if (row < 0) continue;
-        for (int c2 = 0; c2 < 3; ++c2) {
-          const int col = cidx[3 * m + c2];
-          if (col < 0) continue;
-          const double v = double(A[int64_t(j * 9 + c1 * 3 + c2) * nn + n]);
-          D[int64_t(row) * nc + col] = v;
-          if (j > 0) D[int64_t(col) * nc + row] = v;
-        }
+    const int i = a + di % 3 - 1, jj = b + (di / 3) % 3 - 1, k = c + di / 9 - 1;
+    if (i < 0 || i >= d.nnx || jj < 0 || jj >= d.nny || k >= d.nnz) continue;
+    const int64_t m = (int64_t(k) * d.nny + jj) * d.nnx + i;
+    for (int c1 = 0; c1 < 3; ++c1) {
+      const int row = cidx[3 * n + c1];
+      if (row < 0) continue;
+      for (int c2 = 0; c2 < 3; ++c2) {
+        const int col = cidx[3 * m + c2];
+        if (col < 0) continue;
+        const double v = double(A[int64_t(j * 9 + c1 * 3 + c2) * nn + n]);
+        D[int64_t(row) * nc + col] = v;
+        if (j > 0) D[int64_t(col) * nc + row] = v;
       }
     }
   }
+}
+
+// Explicit inverse of the coarsest operator, for small coarsest levels (each
+// V-cycle then needs one dense matvec): block Gauss-Jordan, 32 pivots at a time,
+// from one buffer into another.  For pivot block K with P = M_KK^-1,
+//   M_ij <- M_ij - M_iK (P M_Kj),  M_iK <- -M_iK P,  M_Kj <- P M_Kj,  M_KK <- P.
+// The operator is symmetric positive definite, so its pivots are a Cholesky
+// factorisation's and need no exchange; one that is not positive sets *fail.
+// Two launches per block: the pivot block's inverse by one CTA, 32 dependent
+// steps of about 900 cycles (one FP64 division each), then every 16x16 tile of
+// the matrix.  A blocked Cholesky factor, its inverse by one warp per column and
+// their product took 510 us for 135 unknowns and 2.3 ms for 325.
+constexpr int kGjBlock = 32, kGjTile = 16;
+__global__ void __launch_bounds__(1024) k_gj_pivot(const double* __restrict__ M, int nc, int k0,
+                                                   double* __restrict__ P,
+                                                   int* __restrict__ fail) {
+  __shared__ double s[32][33];
+  __shared__ double inv;
+  const int nb = min(kGjBlock, nc - k0);
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const bool in = tx < nb && ty < nb;
+  double v = in ? M[int64_t(k0 + ty) * nc + k0 + tx] : (tx == ty ? 1.0 : 0.0);
+  auto reciprocal = [&] {  // of the pivot this thread holds
+    if (!(v > 0.0)) *fail = 1;
+    inv = v > 0.0 ? 1.0 / v : 1.0;
+  };
+  s[ty][tx] = v;
+  if (threadIdx.x == 0) reciprocal();
+  __syncthreads();
+  for (int k = 0; k < nb; ++k) {
+    // Row k of the new matrix, then everyone's update; the next pivot's
+    // reciprocal as soon as its entry is known.
+    const double p = inv, col = s[ty][k];
+    double row = 0.0;
+    if (ty == k) {
+      row = tx == k ? p : s[k][tx] * p;
+      s[k][tx] = row;
+    }
+    __syncthreads();
+    if (ty == k)
+      v = row;
+    else
+      v = tx == k ? -(col * p) : fma(-col, s[k][tx], v);
+    __syncthreads();  // row k and column k read
+    s[ty][tx] = v;
+    if (ty == k + 1 && tx == k + 1 && k + 1 < nb) reciprocal();
+    __syncthreads();
+  }
+  if (in) P[ty * kGjBlock + tx] = v;
+}
+
+__global__ void __launch_bounds__(256) k_gj_update(const double* __restrict__ M, int nc, int k0,
+                                                   const double* __restrict__ P,
+                                                   double* __restrict__ out) {
+  __shared__ double sP[32][33], sC[kGjTile][33], sR[32][kGjTile + 1], sT[32][kGjTile + 1];
+  const int nb = min(kGjBlock, nc - k0);
+  const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  for (int e = t; e < 32 * 32; e += 256) {
+    const int r = e >> 5, c = e & 31;
+    sP[r][c] = r < nb && c < nb ? P[r * kGjBlock + c] : 0.0;
+  }
+  for (int e = t; e < kGjTile * 32; e += 256) {
+    const int r = e >> 5, c = e & 31;  // column block K of this tile's rows
+    sC[r][c] = i0 + r < nc && c < nb ? M[int64_t(i0 + r) * nc + k0 + c] : 0.0;
+    const int rr = e >> 4, cc = e & 15;  // row block K of this tile's columns
+    sT[rr][cc] = rr < nb && j0 + cc < nc ? M[int64_t(k0 + rr) * nc + j0 + cc] : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // R = P M_Kj
+    const int r = ty + 16 * h;
+    double v = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) v = fma(sP[r][k], sT[k][tx], v);
+    sR[r][tx] = v;
+  }
+  __syncthreads();
+  const int i = i0 + ty, j = j0 + tx;
+  if (i >= nc || j >= nc) return;
+  const bool ik = i >= k0 && i < k0 + nb, jk = j >= k0 && j < k0 + nb;
+  double v;
+  if (ik && jk) {
+    v = sP[i - k0][j - k0];
+  } else if (ik) {
+    v = sR[i - k0][tx];
+  } else {
+    v = jk ? 0.0 : M[int64_t(i) * nc + j];
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) v = fma(-sC[ty][k], jk ? sP[k][j - k0] : sR[k][tx], v);
+  }
+  out[int64_t(i) * nc + j] = v;
 }
 
 // Blocked right-looking Cholesky, panel width 32.  Step 1: factor the diagonal
@@ -806,35 +878,6 @@ __global__ void k_chol_update(double* __restrict__ D, int nc, int k0) {
     for (int t = 0; t < nb; ++t) s += Li[yy][t] * Lj[tx][t];
     D[int64_t(i) * nc + j] -= s;
   }
-}
-
-// Explicit inverse of the coarsest operator from its Cholesky factor, for small
-// coarsest levels: thread j forms column j of L^-1 by forward substitution, then
-// Ainv = L^-T L^-1 (both FP64).  Each V-cycle then needs one dense matvec.
-// Column j of L^-1 by forward substitution, one warp per column: the inner
-// product of row i of L with the column's entries above i is split over the
-// lanes and reduced by shuffles, so a column costs nc short steps instead of a
-// serial O(nc^2) chain (the factor and the column stay in L2).
-__global__ void k_chol_invert_L(const double* __restrict__ L, int nc, double* __restrict__ Li) {
-  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (j >= nc) return;  // warp-uniform
-  for (int i = lane; i < j; i += 32) Li[int64_t(i) * nc + j] = 0.0;
-  for (int i = j; i < nc; ++i) {
-    double part = 0.0;
-    for (int k = j + lane; k < i; k += 32) part += L[int64_t(i) * nc + k] * Li[int64_t(k) * nc + j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) Li[int64_t(i) * nc + j] = ((i == j ? 1.0 : 0.0) - part) / L[int64_t(i) * nc + i];
-    __syncwarp();  // the new entry is read by every lane from the next row on
-  }
-}
-
-__global__ void k_chol_inverse(const double* __restrict__ Li, int nc, double* __restrict__ Ainv) {
-  const int i = blockIdx.y * 16 + threadIdx.y, j = blockIdx.x * 16 + threadIdx.x;
-  if (i >= nc || j >= nc) return;
-  double s = 0.0;
-  for (int k = max(i, j); k < nc; ++k) s += Li[int64_t(k) * nc + i] * Li[int64_t(k) * nc + j];
-  Ainv[int64_t(i) * nc + j] = s;
 }
 
 // x = Ainv b on the compact numbering, gathered from / scattered to the level
@@ -950,20 +993,23 @@ __global__ void __launch_bounds__(576) k_galerkin1_fast(MgDims fd, MgDims cd,
 template <class T>
 void mg_galerkin_level1(const MgDims& fd, const MgDims& cd, const T* ef, const uint8_t* fact,
                         const uint8_t* cact, const T* Ke, const T* G, T* Kc, cudaStream_t s,
-                        const int* spos) {
+                        const int* spos, const int* slist, int nspec) {
   const int64_t nce = int64_t(cd.ex) * cd.ey * cd.ez;
-  const int* skip = nullptr;
+  const int* list = nullptr;
+  int64_t n = nce;
   if constexpr (sizeof(T) == 4) {
     if (spos != nullptr) {
       const int64_t steps = (nce + kGalFastBatch - 1) / kGalFastBatch;
       const int nb = int(std::min<int64_t>(steps, 152 * 6));
       k_galerkin1_fast<<<nb, 576, 0, s>>>(fd, cd, ef, spos, G, Kc);
       TG_LAUNCH_CHECK();
-      skip = spos;
+      list = slist;
+      n = nspec;
     }
   }
-  k_galerkin<T, true><<<nblk(nce, 4), 128, 0, s>>>(fd, cd, ef, fact, cact, Ke, G, nullptr, Kc,
-                                                   skip);
+  if (n == 0) return;
+  k_galerkin<T, true><<<nblk(n, 1), 256, 0, s>>>(fd, cd, ef, fact, cact, Ke, G, nullptr, Kc, list,
+                                                 n);
   TG_LAUNCH_CHECK();
 }
 
@@ -971,8 +1017,8 @@ template <class T>
 void mg_galerkin_coarse(const MgDims& fd, const MgDims& cd, const T* Kf, const uint8_t* cact,
                         T* Kc, cudaStream_t s) {
   const int64_t nce = int64_t(cd.ex) * cd.ey * cd.ez;
-  k_galerkin<T, false><<<nblk(nce, 4), 128, 0, s>>>(fd, cd, nullptr, nullptr, cact, nullptr,
-                                                    nullptr, Kf, Kc, nullptr);
+  k_galerkin<T, false><<<nblk(nce, 1), 256, 0, s>>>(fd, cd, nullptr, nullptr, cact, nullptr,
+                                                    nullptr, Kf, Kc, nullptr, nce);
   TG_LAUNCH_CHECK();
 }
 
@@ -980,7 +1026,8 @@ template <class T>
 void mg_assemble_stencil(const MgDims& d, const T* Kel, const uint8_t* act, T* A, T* invdiag,
                          cudaStream_t s) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
-  k_assemble_stencil<T><<<nblk(nn), kThreads, 0, s>>>(d, Kel, act, A, invdiag);
+  k_assemble_stencil<T><<<dim3(unsigned(nblk(nn)), A != nullptr ? 14 : 1), kThreads, 0, s>>>(
+      d, Kel, act, A, invdiag);
   TG_LAUNCH_CHECK();
 }
 
@@ -1079,7 +1126,7 @@ void mg_dense_from_stencil(const MgDims& d, const T* A, const int* cidx, int nc,
                            cudaStream_t s) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
   TG_CUDA(cudaMemsetAsync(D, 0, sizeof(double) * size_t(nc) * nc, s));
-  k_dense_from_stencil<T><<<nblk(nn), kThreads, 0, s>>>(d, A, cidx, nc, D);
+  k_dense_from_stencil<T><<<dim3(unsigned(nblk(nn)), 14), kThreads, 0, s>>>(d, A, cidx, nc, D);
   TG_LAUNCH_CHECK();
 }
 
@@ -1097,12 +1144,21 @@ void mg_cholesky(double* D, int nc, int* fail, cudaStream_t s) {
   }
 }
 
-void mg_chol_inverse(const double* L, int nc, double* Li, double* Ainv, cudaStream_t s) {
-  k_chol_invert_L<<<(nc + 3) / 4, 128, 0, s>>>(L, nc, Li);  // a warp per column
-  TG_LAUNCH_CHECK();
-  const dim3 grid((nc + 15) / 16, (nc + 15) / 16);
-  k_chol_inverse<<<grid, dim3(16, 16), 0, s>>>(Li, nc, Ainv);
-  TG_LAUNCH_CHECK();
+double* mg_dense_start(int nc, double* a, double* inv) {
+  return ((nc + kGjBlock - 1) / kGjBlock) & 1 ? a : inv;
+}
+
+void mg_dense_inverse(int nc, double* a, double* inv, double* pivot, int* fail, cudaStream_t s) {
+  double* src = mg_dense_start(nc, a, inv);
+  double* dst = src == a ? inv : a;
+  const unsigned tiles = unsigned((nc + kGjTile - 1) / kGjTile);
+  for (int k0 = 0; k0 < nc; k0 += kGjBlock) {
+    k_gj_pivot<<<1, 1024, 0, s>>>(src, nc, k0, pivot, fail);
+    TG_LAUNCH_CHECK();
+    k_gj_update<<<dim3(tiles, tiles), 256, 0, s>>>(src, nc, k0, pivot, dst);
+    TG_LAUNCH_CHECK();
+    std::swap(src, dst);
+  }
 }
 
 template <class T>
@@ -1133,7 +1189,7 @@ void mg_chol_solve(const double* L, int nc, const int* cidx, int64_t ndof, const
                                        const T*, T*, cudaStream_t);                           \
   template void mg_galerkin_level1<T>(const MgDims&, const MgDims&, const T*, const uint8_t*,  \
                                       const uint8_t*, const T*, const T*, T*, cudaStream_t,   \
-                                      const int*);                                            \
+                                      const int*, const int*, int);                           \
   template void mg_galerkin_coarse<T>(const MgDims&, const MgDims&, const T*, const uint8_t*,  \
                                       T*, cudaStream_t);                                      \
   template void mg_assemble_stencil<T>(const MgDims&, const T*, const uint8_t*, T*, T*,       \

@@ -410,7 +410,7 @@ size_t Solver::device_bytes() const {
   for (const DBuf<double>* d : {&invdiag_, &rhs_, &x_, &r_, &z_, &p_, &ap_, &t0_, &t1_, &part_,
                                 &scal_, &keb_, &G_, &chol_, &chol_work_})
     b += d->bytes();
-  b += chol_li_.bytes() + chol_inv_.bytes() + cdof_.bytes();
+  b += gj_pivot_.bytes() + chol_inv_.bytes() + cdof_.bytes();
   for (const DBuf<float>* d : {&Ef_, &invdiagf_, &xf_, &rf_, &zf_, &pf_, &apf_, &t0f_, &t1f_})
     b += d->bytes();
   for (const auto& L : levels_) b += L->bytes();
@@ -498,7 +498,7 @@ void Solver::build_structure() {
   cdof_.alloc(size_t(nc_));
   TG_CUDA(cudaMemcpyAsync(cdof_.p, cdof.data(), cdof_.bytes(), cudaMemcpyHostToDevice, s_));
   if (nc_ <= kMaxInverseDof) {
-    chol_li_.alloc(size_t(nc_) * nc_);
+    gj_pivot_.alloc(1024);
     chol_inv_.alloc(size_t(nc_) * nc_);
   }
   chol_.alloc(size_t(nc_) * nc_);
@@ -790,8 +790,8 @@ const float* pick<float>(const DBuf<double>&, const DBuf<float>& f) {
 }
 
 // Galerkin hierarchy in precision T from the current element factors, then the
-// FP64 dense Cholesky factor of the coarsest level.  Returns false when the
-// factorisation meets a non-positive pivot (the caller falls back).
+// coarsest level's FP64 inverse (small levels) or dense Cholesky factor.  Returns
+// false when that meets a non-positive pivot (the caller falls back).
 template <class T>
 bool Solver::build_numeric() {
   const Grid& g = fp_.g;
@@ -806,7 +806,8 @@ bool Solver::build_numeric() {
                             pick<T>(G_, Gf_), L.Ke<T>(), s_,
                             sizeof(T) == 4 && l1_mf_ && level1_galerkin_fast_enabled()
                                 ? spos1_.p
-                                : nullptr);
+                                : nullptr,
+                            slist1_.p, nspec1_);
     else
       mg_galerkin_coarse<T>(pd, L.d, levels_[l - 1]->Ke<T>(), L.act.p, L.Ke<T>(), s_);
     // The matrix-free level 1 needs only its inverse diagonal; the assembled
@@ -848,13 +849,18 @@ bool Solver::build_numeric() {
     }
   }
   Level& C = *levels_.back();
-  mg_dense_from_stencil<T>(C.d, C.Am<T>(), cidx_.p, nc_, chol_.p, s_);
   TG_CUDA(cudaMemsetAsync(chol_fail_.p, 0, sizeof(int), s_));
-  mg_cholesky(chol_.p, nc_, chol_fail_.p, s_);
+  if (chol_inv_.p) {
+    mg_dense_from_stencil<T>(C.d, C.Am<T>(), cidx_.p, nc_,
+                             mg_dense_start(nc_, chol_.p, chol_inv_.p), s_);
+    mg_dense_inverse(nc_, chol_.p, chol_inv_.p, gj_pivot_.p, chol_fail_.p, s_);
+  } else {
+    mg_dense_from_stencil<T>(C.d, C.Am<T>(), cidx_.p, nc_, chol_.p, s_);
+    mg_cholesky(chol_.p, nc_, chol_fail_.p, s_);
+  }
   int fail = 0;
   TG_CUDA(cudaMemcpyAsync(&fail, chol_fail_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
   TG_CUDA(cudaStreamSynchronize(s_));
-  if (fail == 0 && chol_inv_.p) mg_chol_inverse(chol_.p, nc_, chol_li_.p, chol_inv_.p, s_);
   numeric_[sizeof(T) == 8 ? 1 : 0] = (fail == 0);
   return fail == 0;
 }

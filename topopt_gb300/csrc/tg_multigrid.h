@@ -27,11 +27,12 @@ struct MgDims {
 
 // spos (FP32, optional): per coarse element, < 0 on the fast path (sum_c f_c G_c;
 // the level-1 operator's special-element positions), where a
-// bandwidth-bound kernel forms the matrix.
+// bandwidth-bound kernel forms the matrix and the general one only the nspec
+// elements of slist.
 template <class T>
 void mg_galerkin_level1(const MgDims& fd, const MgDims& cd, const T* ef, const uint8_t* fact,
                         const uint8_t* cact, const T* Ke, const T* G, T* Kc, cudaStream_t s,
-                        const int* spos = nullptr);
+                        const int* spos = nullptr, const int* slist = nullptr, int nspec = 0);
 template <class T>
 void mg_galerkin_coarse(const MgDims& fd, const MgDims& cd, const T* Kf, const uint8_t* cact,
                         T* Kc, cudaStream_t s);
@@ -90,8 +91,12 @@ template <class T>
 void mg_dense_from_stencil(const MgDims& d, const T* A, const int* cidx, int nc, double* D,
                            cudaStream_t s);
 void mg_cholesky(double* D, int nc, int* fail, cudaStream_t s);
-// Explicit inverse of the coarsest operator from its factor (small levels).
-void mg_chol_inverse(const double* L, int nc, double* Li, double* Ainv, cudaStream_t s);
+// Explicit inverse of the coarsest operator (small levels): the dense matrix is in
+// mg_dense_start(nc, a, inv) -- one of the two buffers -- and its inverse comes
+// out in inv.  pivot: 1024 scratch values; *fail is set by a pivot that is not
+// positive.
+double* mg_dense_start(int nc, double* a, double* inv);
+void mg_dense_inverse(int nc, double* a, double* inv, double* pivot, int* fail, cudaStream_t s);
 // x = Ainv b over the compact numbering (cidx: dof -> compact, cdof: compact -> dof).
 template <class T>
 void mg_coarse_inv_apply(const double* Ainv, int nc, const int* cidx, const int* cdof,

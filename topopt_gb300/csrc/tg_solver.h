@@ -148,7 +148,7 @@ class Solver {
   int64_t fine_matvecs_ = 0, lowp_matvecs_ = 0;
   int nc_ = 0;
   DBuf<int> cidx_, cdof_, chol_fail_;
-  DBuf<double> chol_, chol_work_, chol_li_, chol_inv_;
+  DBuf<double> chol_, chol_work_, gj_pivot_, chol_inv_;
   // The PCG loops (mixed inner, FP64 multigrid, FP64 Jacobi) as one CUDA graph
   // each: a conditional WHILE node whose body is one iteration and whose last
   // kernel decides, on the device, whether another one runs.
