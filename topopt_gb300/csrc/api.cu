@@ -253,11 +253,13 @@ struct FilterState {
 };
 
 // ------------------------------------------------------------ OC update
-// Candidate fields of one projected bisection pass: up to kOcMulti, at most
-// 128 MB of them.
+// Candidate fields of one projected bisection pass, at most 128 MB of them.  Eight
+// (16 would fit the sums): a pass is FP64-bound from a few thousand voxels on, and
+// half of the longer path behind a prediction is evaluated for nothing.
+constexpr int kProjMulti = 8;
 int projected_candidates(int64_t nv) {
   const int64_t cap = (int64_t(128) << 20) / (8 * std::max<int64_t>(nv, 1));
-  return int(std::max<int64_t>(1, std::min<int64_t>(kOcMulti, cap)));
+  return int(std::max<int64_t>(1, std::min<int64_t>(kProjMulti, cap)));
 }
 
 struct OcState {
@@ -268,6 +270,7 @@ struct OcState {
   double radius = 1.5;
   DBuf<uint64_t> part, total;
   DBuf<int> inexact;
+  DBuf<unsigned> count;  // CTAs done, per candidate of a pass
   uint64_t* h_total = nullptr;  // pinned: 3 limbs + flag
   std::vector<double> h_xp;
   double* h_v = nullptr;  // pinned: kOcMulti candidate volumes
@@ -282,10 +285,12 @@ struct OcState {
     kproj = projected_candidates(g.nv);
     cand.alloc(size_t(kproj) * size_t(g.nv));
   }
-  void init(const Grid& g, cudaStream_t) {
+  void init(const Grid& g, cudaStream_t s) {
     for (DBuf<double>* d : {&dcf, &dvf, &xp, &sq, &lo, &hi, &dvd}) d->alloc(size_t(g.nv));
     vpart.alloc(size_t(kRedBlocks) * kOcMulti);
     vsum.alloc(kOcMulti);
+    count.alloc(kOcMulti);
+    TG_CUDA(cudaMemsetAsync(count.p, 0, count.bytes(), s));
     h_v = static_cast<double*>(pinned_scalars(kOcMulti * sizeof(double)));
     part.alloc(size_t(3 * exact_sum_blocks()));
     total.alloc(3);
@@ -299,7 +304,7 @@ struct OcState {
   size_t bytes() const {
     return dcf.bytes() + dvf.bytes() + xp.bytes() + sq.bytes() + lo.bytes() + hi.bytes() +
            dvd.bytes() + vpart.bytes() + vsum.bytes() + part.bytes() + total.bytes() + inexact.bytes() +
-           cand.bytes();
+           count.bytes() + cand.bytes();
   }
 };
 
@@ -342,6 +347,75 @@ bool volume_exceeds(OcState& oc, const Grid& g, const uint8_t* act,
   return v > target;
 }
 
+// The values a bisection has evaluated ahead, by the multiplier they belong to.
+struct Evaluated {
+  std::vector<std::pair<double, double>> at;  // (lambda, value)
+  void add(double lam, double v) { at.emplace_back(lam, v); }
+  bool find(double lam, double* v) const {
+    for (const auto& kv : at)
+      if (kv.first == lam) {
+        *v = kv.second;
+        return true;
+      }
+    return false;
+  }
+};
+
+// The multipliers a doubling loop at l2 tests next, as many as a pass takes; the
+// first pass spends half of them on the halvings that the bisection of (0, 1) starts
+// with if the value at 1 is small enough.
+std::vector<double> bracket_ahead(double l2, int kmax) {
+  std::vector<double> c;
+  const int up = l2 == 1.0 && kmax > 1 ? (kmax + 1) / 2 : kmax;
+  for (double t = l2; int(c.size()) < up && t < 1e30; t *= 2.0) c.push_back(t);
+  if (up < kmax)
+    for (double t = 0.5; int(c.size()) < kmax; t *= 0.5) c.push_back(t);
+  return c;
+}
+
+// The midpoints a bisection of (l1, l2) tests next, by its own arithmetic, on its way
+// to where the values known so far place the crossing of `target` (they fall with
+// the multiplier): to 0 while nothing is known at l1, else to the inverse
+// interpolation of log(lambda) through the interval's ends and the nearest value
+// outside.  A wrong prediction costs the rest of its pass and narrows the interval
+// for the next.  All paths at once instead (a binary tree) is four levels in 16
+// evaluations, seven passes an update; this way it is four.  With the passes' own
+// kernels an update went from 0.6 to 0.2 ms (60x20x20), from 2.45 to 1.86 ms
+// (256x128x128), and projected from 1.1 to 0.26 ms (48x8x8).
+template <class Open>
+std::vector<double> bisect_ahead(const Evaluated& known, double l1, double l2, double target,
+                                 int kmax, const Open& open) {
+  double aim = 0.0, v1 = 0.0, v2 = 0.0;
+  if (l1 > 0.0 && known.find(l1, &v1) && known.find(l2, &v2)) {
+    const double y1 = std::log(l1), y2 = std::log(l2);
+    double y = y1 + (y2 - y1) * (v1 - target) / (v1 - v2);
+    double y3 = 0.0, v3 = 0.0, gap = INFINITY;
+    for (const auto& kv : known.at) {
+      if (!(kv.first > 0.0) || (kv.first >= l1 && kv.first <= l2)) continue;
+      const double yk = std::log(kv.first), d = std::max(y1 - yk, yk - y2);
+      if (d < gap) gap = d, y3 = yk, v3 = kv.second;
+    }
+    // The three in Newton's form; kept where it stays inside the interval.
+    const double s = (y2 - y1) / (v2 - v1), c = ((y3 - y2) / (v3 - v2) - s) / (v3 - v1);
+    const double q = y1 + (target - v1) * (s + (target - v2) * c);
+    if (q > y1 && q < y2) y = q;
+    if (!(y > y1 && y < y2)) y = 0.5 * (y1 + y2);
+    aim = std::exp(y);
+  }
+  std::vector<double> c;
+  for (int it = 0; it < 100 && int(c.size()) < kmax && open(l1, l2); ++it) {
+    const double m = 0.5 * (l1 + l2);
+    double v = 0.0;
+    bool right = aim > m;
+    if (known.find(m, &v))
+      right = v > target;
+    else
+      c.push_back(m);
+    (right ? l1 : l2) = m;
+  }
+  return c;
+}
+
 // oc_update (simp.cpp:948-1025) on device-resident fields; dvf must hold the
 // filtered unit volume sensitivity.  Each bisection branch is first decided from
 // the fast linear volume sum_n dv_n x~_n(lambda) (k_oc_volume), whose distance to
@@ -370,41 +444,32 @@ void oc_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_t
   // below the n u of the reference's own sequential sum.
   const double eps =
       (n + 2.0 * (m + 1.0) + 12.0 + n / (double(kRedBlocks) * 256.0) + 64.0 + 8192.0) * u * 1.01;
-  // Fast volumes are computed ahead, kmax lambdas per pass over the fields: the
-  // next doublings while bracketing, the next levels of the bisection tree
-  // (breadth first) while bisecting.  Every branch is still decided one at a
-  // time, in the reference's order, from the volume of exactly the lambda the
-  // sequential loop would test, so the speculation changes no decision.  A
-  // candidate costs a few FP64 operations per voxel: on large grids the pass is
-  // FP64-bound, and 4 per pass (two bisection levels and one more midpoint)
-  // wastes less work than 16 (four levels, of which one path is used).
-  const int kmax = g.nv > (int64_t(1) << 20) ? 4 : kOcMulti;
-  std::vector<std::pair<double, double>> known;  // (lambda, fast volume)
-  auto lookup = [&](double lam, double* V) {
-    for (const auto& kv : known)
-      if (kv.first == lam) {
-        *V = kv.second;
-        return true;
-      }
-    return false;
-  };
+  // Fast volumes are computed ahead, kmax lambdas per pass over the fields
+  // (bracket_ahead, bisect_ahead).  Every branch is still decided one at a time, in
+  // the reference's order, from the volume of exactly the lambda the sequential loop
+  // would test, so the speculation changes no decision.  On large grids a pass is
+  // bound by its double-float arithmetic and its reads alike, and 8 lambdas take half
+  // the time of 16; a small grid's pass is its launch and the round trip to the host.
+  const int kmax = g.nv > (int64_t(1) << 20) ? 8 : kOcMulti;
+  const auto open = [](double l1, double l2) { return (l2 - l1) > 1e-6 * (l1 + l2); };
+  Evaluated known;  // fast volumes
   auto batch = [&](const std::vector<double>& lams) {
     OcCands cs;
     cs.k = int(std::min<size_t>(lams.size(), size_t(kmax)));
     for (int k = 0; k < cs.k; ++k) cs.c[k] = 1.0 / std::sqrt(lams[size_t(k)]);
     launch_oc_volume_multi(oc.sq.p, oc.lo.p, oc.hi.p, oc.dvd.p, g.nv, cs, oc.vpart.p, oc.vsum.p,
-                           s);
+                           oc.count.p, s);
     TG_CUDA(cudaMemcpyAsync(oc.h_v, oc.vsum.p, sizeof(double) * cs.k, cudaMemcpyDeviceToHost, s));
     TG_CUDA(cudaStreamSynchronize(s));
     ++oc.passes;
-    for (int k = 0; k < cs.k; ++k) known.emplace_back(lams[size_t(k)], oc.h_v[k]);
+    for (int k = 0; k < cs.k; ++k) known.add(lams[size_t(k)], oc.h_v[k]);
   };
   auto eval = [&](double lam) {
     ++oc.evals;
     double V = 0.0;
-    if (!lookup(lam, &V)) {
+    if (!known.find(lam, &V)) {
       batch({lam});
-      lookup(lam, &V);
+      known.find(lam, &V);
     }
     const double bound = eps * V / (1.0 - eps) + 1e-300;
     if (std::isfinite(V)) {
@@ -425,34 +490,13 @@ void oc_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_t
   double l1 = 0.0, l2 = 1.0;
   double Vtmp = 0.0;
   while (l2 < 1e30) {
-    if (!lookup(l2, &Vtmp)) {
-      std::vector<double> c;
-      for (double t = l2; int(c.size()) < kmax && t < 1e30; t *= 2.0) c.push_back(t);
-      batch(c);
-    }
+    if (!known.find(l2, &Vtmp)) batch(bracket_ahead(l2, kmax));
     if (!eval(l2)) break;
     l2 *= 2.0;
   }
-  for (int it = 0; it < 100 && (l2 - l1) > 1e-6 * (l1 + l2); ++it) {
+  for (int it = 0; it < 100 && open(l1, l2); ++it) {
     const double lmid = 0.5 * (l1 + l2);
-    if (!lookup(lmid, &Vtmp)) {
-      // The midpoints the next bisection steps can reach, breadth first,
-      // computed with the loop's own arithmetic.
-      std::vector<double> c;
-      std::vector<std::pair<double, double>> lv{{l1, l2}};
-      while (!lv.empty() && int(c.size()) < kmax) {
-        std::vector<std::pair<double, double>> nx;
-        for (const auto& iv : lv) {
-          if (int(c.size()) >= kmax) break;
-          const double m = 0.5 * (iv.first + iv.second);
-          c.push_back(m);
-          nx.emplace_back(iv.first, m);
-          nx.emplace_back(m, iv.second);
-        }
-        lv.swap(nx);
-      }
-      batch(c);
-    }
+    if (!known.find(lmid, &Vtmp)) batch(bisect_ahead(known, l1, l2, target, kmax, open));
     if (eval(lmid))
       l1 = lmid;
     else
@@ -483,15 +527,8 @@ void oc_update_projected_device(OcState& oc, FilterState& fs, const Grid& g, con
   fs.adj(g, act, oc.lo.p, oc.dcf.p, s);
   fs.adj(g, act, oc.sq.p, oc.dvf.p, s);
   const double target = volfrac * double(oc.n_solid);
-  std::vector<std::pair<double, double>> known;  // (lambda, projected volume)
-  auto lookup = [&](double lam, double* V) {
-    for (const auto& kv : known)
-      if (kv.first == lam) {
-        *V = kv.second;
-        return true;
-      }
-    return false;
-  };
+  const auto open = [](double l1, double l2) { return (l2 - l1) > 1e-6 * (l1 + l2); };
+  Evaluated known;  // projected volumes
   auto batch = [&](const std::vector<double>& lams) {
     ProjLambdas ls;
     ls.k = int(std::min<size_t>(lams.size(), size_t(oc.kproj)));
@@ -499,51 +536,31 @@ void oc_update_projected_device(OcState& oc, FilterState& fs, const Grid& g, con
     launch_oc_candidates_projected(x, oc.dcf.p, oc.dvf.p, act, g.nv, ls, move, rho_min, oc.carry,
                                    oc.cand.p, s);
     launch_proj_volume(g, fs.st_dev, fs.st.n, act, fs.hs.p, oc.cand.p, ls.k, beta, eta,
-                       oc.vpart.p, oc.vsum.p, s);
+                       oc.vpart.p, oc.vsum.p, oc.count.p, s);
     TG_CUDA(cudaMemcpyAsync(oc.h_v, oc.vsum.p, sizeof(double) * ls.k, cudaMemcpyDeviceToHost, s));
     TG_CUDA(cudaStreamSynchronize(s));
     ++oc.passes;
-    for (int k = 0; k < ls.k; ++k) known.emplace_back(ls.lam[k], oc.h_v[k]);
+    for (int k = 0; k < ls.k; ++k) known.add(ls.lam[k], oc.h_v[k]);
   };
   auto exceeds = [&](double lam) {
     ++oc.evals;
     double V = 0.0;
-    if (!lookup(lam, &V)) {
+    if (!known.find(lam, &V)) {
       batch({lam});
-      lookup(lam, &V);
+      known.find(lam, &V);
     }
     return V > target;
   };
   double l1 = 0.0, l2 = 1.0, Vtmp = 0.0;
   while (l2 < 1e30) {
-    if (!lookup(l2, &Vtmp)) {
-      std::vector<double> c;
-      for (double t = l2; int(c.size()) < oc.kproj && t < 1e30; t *= 2.0) c.push_back(t);
-      batch(c);
-    }
+    if (!known.find(l2, &Vtmp)) batch(bracket_ahead(l2, oc.kproj));
     if (!exceeds(l2)) break;
     l2 *= 2.0;
   }
-  for (int it = 0; it < 100 && (l2 - l1) > 1e-6 * (l1 + l2); ++it) {
+  for (int it = 0; it < 100 && open(l1, l2); ++it) {
     const double lmid = 0.5 * (l1 + l2);
-    if (!lookup(lmid, &Vtmp)) {
-      // Midpoints of the next bisection levels, breadth first, as many as one
-      // pass holds (the loop's own arithmetic).
-      std::vector<double> c;
-      std::vector<std::pair<double, double>> lv{{l1, l2}};
-      while (!lv.empty() && int(c.size()) < oc.kproj) {
-        std::vector<std::pair<double, double>> nx;
-        for (const auto& iv : lv) {
-          if (int(c.size()) >= oc.kproj) break;
-          const double m = 0.5 * (iv.first + iv.second);
-          c.push_back(m);
-          nx.emplace_back(iv.first, m);
-          nx.emplace_back(m, iv.second);
-        }
-        lv.swap(nx);
-      }
-      batch(c);
-    }
+    if (!known.find(lmid, &Vtmp))
+      batch(bisect_ahead(known, l1, l2, target, oc.kproj, open));
     if (exceeds(lmid))
       l1 = lmid;
     else
@@ -574,36 +591,29 @@ void mma_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_
   const double vol = exact_volume(oc, g, act, xphys, &exact, s);
   const double g0 = vol - volfrac * double(oc.n_solid);
   launch_mma_prepare(m, x, oc.dcf.p, oc.dvf.p, act, g.nv, iter, move, rho_min, scale.p,
-                     oc.vpart.p, oc.vsum.p, s);
+                     oc.vpart.p, oc.vsum.p, oc.count.p, s);
   TG_CUDA(cudaMemcpyAsync(oc.h_v, oc.vsum.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   TG_CUDA(cudaStreamSynchronize(s));
   const double b = -g0 + oc.h_v[0];
-  std::vector<std::pair<double, double>> known;  // (lambda, constraint sum)
-  auto lookup = [&](double lam, double* v) {
-    for (const auto& kv : known)
-      if (kv.first == lam) {
-        *v = kv.second;
-        return true;
-      }
-    return false;
-  };
-  const int kmax = g.nv > (int64_t(1) << 22) ? 4 : kOcMulti;
+  Evaluated known;  // constraint sums
+  const int kmax = 8;  // an FP64-bound pass, like the projected volumes'
+  const auto open = [](double l1, double l2) { return (l2 - l1) > 1e-9 * (1.0 + l1 + l2); };
   auto batch = [&](const std::vector<double>& lams) {
     ProjLambdas ls;
     ls.k = int(std::min<size_t>(lams.size(), size_t(kmax)));
     for (int k = 0; k < ls.k; ++k) ls.lam[k] = lams[size_t(k)];
-    launch_mma_dual(m, act, g.nv, ls, oc.vpart.p, oc.vsum.p, s);
+    launch_mma_dual(m, act, g.nv, ls, oc.vpart.p, oc.vsum.p, oc.count.p, s);
     TG_CUDA(cudaMemcpyAsync(oc.h_v, oc.vsum.p, sizeof(double) * ls.k, cudaMemcpyDeviceToHost, s));
     TG_CUDA(cudaStreamSynchronize(s));
     ++oc.passes;
-    for (int k = 0; k < ls.k; ++k) known.emplace_back(ls.lam[k], oc.h_v[k]);
+    for (int k = 0; k < ls.k; ++k) known.add(ls.lam[k], oc.h_v[k]);
   };
   auto positive = [&](double lam) {  // gval(candidate(lam)) > 0
     ++oc.evals;
     double v = 0.0;
-    if (!lookup(lam, &v)) {
+    if (!known.find(lam, &v)) {
       batch({lam});
-      lookup(lam, &v);
+      known.find(lam, &v);
     }
     return (v - b) > 0.0;
   };
@@ -617,7 +627,7 @@ void mma_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_
   if (positive(0.0)) {
     double l1 = 0.0, l2 = 1.0;
     while (l2 < 1e30) {
-      if (!lookup(l2, &tmp)) {
+      if (!known.find(l2, &tmp)) {
         std::vector<double> c;
         for (double t = l2; int(c.size()) < kmax && t < 1e30; t *= 2.0) c.push_back(t);
         batch(c);
@@ -625,24 +635,10 @@ void mma_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_
       if (!positive(l2)) break;
       l2 *= 2.0;
     }
-    for (int it = 0; it < 100 && (l2 - l1) > 1e-9 * (1.0 + l1 + l2); ++it) {
+    for (int it = 0; it < 100 && open(l1, l2); ++it) {
       const double lmid = 0.5 * (l1 + l2);
-      if (!lookup(lmid, &tmp)) {
-        std::vector<double> c;
-        std::vector<std::pair<double, double>> lv{{l1, l2}};
-        while (!lv.empty() && int(c.size()) < kmax) {
-          std::vector<std::pair<double, double>> nx;
-          for (const auto& iv : lv) {
-            if (int(c.size()) >= kmax) break;
-            const double mm = 0.5 * (iv.first + iv.second);
-            c.push_back(mm);
-            nx.emplace_back(iv.first, mm);
-            nx.emplace_back(mm, iv.second);
-          }
-          lv.swap(nx);
-        }
-        batch(c);
-      }
+      if (!known.find(lmid, &tmp))
+        batch(bisect_ahead(known, l1, l2, b, kmax, open));
       if (positive(lmid))
         l1 = lmid;
       else

@@ -19,10 +19,12 @@
 // scatter adds them in.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "tg_df.h"
 #include "tg_internal.h"
+#include "tg_reduce.h"
 
 namespace tg {
 
@@ -403,16 +405,36 @@ __device__ __forceinline__ bool df_less(df a, df b) {
   return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
 }
 
-// The linear volume sum_e dv_e clamp(sq_e c, lo_e, hi_e) for up to kOcMulti
-// candidates c = 1/sqrt(lambda) in one pass over the fields, in double-float
-// arithmetic on the FP32 pipe (tg_df.h; ~2^-46 relative per operation, all
-// terms positive), each candidate summed in a fixed per-thread order, then the
-// FP64 trees.  These volumes only decide bisection branches under a certified
-// bound that includes this arithmetic's error.
+// Of each two lanes' 2 M candidates a lane keeps M, both lanes' parts added.
+template <int M>
+__device__ __forceinline__ void fold_half(df* a, int lane, int off) {
+  const bool upper = (lane & off) != 0;
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    const df mine = upper ? a[j + M] : a[j], give = upper ? a[j] : a[j + M];
+    a[j] = mine + df(__shfl_xor_sync(0xffffffffu, give.hi, off),
+                     __shfl_xor_sync(0xffffffffu, give.lo, off));
+  }
+}
+
+// The linear volume sum_e dv_e clamp(sq_e c, lo_e, hi_e) for up to K candidates
+// c = 1/sqrt(lambda) in one pass over the fields, in double-float arithmetic on the
+// FP32 pipe (tg_df.h; ~2^-46 relative per operation, all terms positive).  These
+// volumes only decide bisection branches under a certified bound that includes this
+// arithmetic's error.  On small grids the sum over the block bounds the pass: K FP64
+// trees are K x 10 dependent adds of 64 cycles.  Here a warp's lanes exchange halves
+// of their candidates, so that the K sums take about K double-float adds, FP64 adds
+// up only the eight warps' totals, and the CTA that ends last adds up the CTAs'
+// shares.
 template <int K>
 __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
     const df* __restrict__ sq, const df* __restrict__ lo, const df* __restrict__ hi,
-    const df* __restrict__ dvd, int64_t n, OcCandsDF cs, double* __restrict__ part) {
+    const df* __restrict__ dvd, int64_t n, OcCandsDF cs, double* __restrict__ part,
+    double* __restrict__ out, unsigned* __restrict__ count) {
+  static_assert(K == 8 || K == 16, "a warp's lanes exchange K candidates down to one");
+  constexpr int kWarps = kThreads / 32, kLanes = 32 / K;  // lanes that end with one candidate
+  __shared__ double share[kWarps][K];
+  __shared__ bool last;
   df acc[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) acc[k] = df(0.0f, 0.0f);
@@ -428,21 +450,46 @@ __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
       acc[k] = acc[k] + d * xt;
     }
   }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  fold_half<K / 2>(acc, lane, 16);
+  fold_half<K / 4>(acc, lane, 8);
+  fold_half<K / 8>(acc, lane, 4);
+  if constexpr (K == 16) fold_half<1>(acc, lane, 2);
+  df v = acc[0];
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (k >= cs.k) break;  // cs.k is uniform over the block
-    const double v = block_sum256(df_to_double(acc[k]));
-    if (threadIdx.x == 0) part[k * gridDim.x + blockIdx.x] = v;
+  for (int off = kLanes / 2; off > 0; off >>= 1)
+    v = v + df(__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off));
+  if (lane % kLanes == 0) share[wid][lane / kLanes] = df_to_double(v);
+  __syncthreads();
+  if (threadIdx.x < unsigned(cs.k)) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) s += share[w][threadIdx.x];
+    part[threadIdx.x * gridDim.x + blockIdx.x] = s;
+    __threadfence();
   }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = wid; k < cs.k; k += kWarps) {
+    double s = 0.0;
+    for (unsigned i = lane; i < gridDim.x; i += 32) s += __ldcg(part + k * gridDim.x + i);
+    s = warp_sum(s);
+    if (lane == 0) out[k] = s;
+  }
+  if (threadIdx.x == 0) *count = 0u;
 }
 
-// out[k] = sum of part[k][0..n) -- block k, the k_sum_partials tree.
-__global__ void k_sum_partials_multi(const double* __restrict__ part, int n,
-                                     double* __restrict__ out) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += kThreads) s += part[blockIdx.x * n + i];
-  s = block_sum256(s);
-  if (threadIdx.x == 0) out[blockIdx.x] = s;
+// The sum of v over the CTAs of one candidate (blockIdx.y) into out[candidate].
+__device__ __forceinline__ void candidate_sum(double v, double* part, double* out,
+                                              unsigned* count) {
+  SumOut o{};
+  o.part = part + blockIdx.y * gridDim.x;
+  o.out = out + blockIdx.y;
+  o.count = count + blockIdx.y;
+  grid_sum(v, o, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------------------ projection
@@ -498,78 +545,63 @@ __global__ void k_proj_chain(const double* __restrict__ xtilde, const double* __
 // B = -dc / (lambda dv) with UNCLAMPED dv, a non-finite B holds the voxel
 // (B = 1), B < 0 -> 0; x sqrt(B) clamped to the move window.  Candidate j goes
 // to cand + j * n.
+// A thread per voxel and candidate (blockIdx.y): a division and a root in FP64 a
+// candidate are the cost, and a thread that walked over them left a small grid's SMs
+// with a warp or two each (48x8x8, 16 candidates: 26 us).
 __global__ void k_oc_candidates_projected(const double* __restrict__ x,
                                           const double* __restrict__ dcf,
                                           const double* __restrict__ dvf,
                                           const uint8_t* __restrict__ act, int64_t n,
                                           ProjLambdas ls, double move, double rho_min, int carry,
                                           double* __restrict__ cand) {
+  const int j = blockIdx.y;
+  const double lam = ls.lam[j];
   for (int64_t e = blockIdx.x * int64_t(kThreads) + threadIdx.x; e < n;
        e += int64_t(gridDim.x) * kThreads) {
     const double xe = x[e];
-    if (!act[e]) {
-      const double v = carry ? xe : 0.0;
-      for (int j = 0; j < ls.k; ++j) cand[j * n + e] = v;
-      continue;
-    }
-    const double mdc = -dcf[e], dv = dvf[e];
-    const double xm = __dsub_rn(xe, move), xp = __dadd_rn(xe, move);
-    const double lo = (rho_min < xm) ? xm : rho_min;
-    const double hi = (xp < 1.0) ? xp : 1.0;
-    for (int j = 0; j < ls.k; ++j) {
-      double be = __ddiv_rn(mdc, __dmul_rn(ls.lam[j], dv));
+    double xt = carry ? xe : 0.0;
+    if (act[e]) {
+      const double xm = __dsub_rn(xe, move), xp = __dadd_rn(xe, move);
+      const double lo = (rho_min < xm) ? xm : rho_min;
+      const double hi = (xp < 1.0) ? xp : 1.0;
+      double be = __ddiv_rn(-dcf[e], __dmul_rn(lam, dvf[e]));
       if (!isfinite(be)) be = 1.0;
       if (be < 0.0) be = 0.0;
-      double xt = __dmul_rn(xe, __dsqrt_rn(be));
+      xt = __dmul_rn(xe, __dsqrt_rn(be));
       if (xt < lo) xt = lo;
       if (xt > hi) xt = hi;
-      cand[j * n + e] = xt;
     }
+    cand[j * n + e] = xt;
   }
 }
 
-// proj_vol (simp.cpp:1707-1716) of k candidates in one pass: for every design
-// voxel, the density filter of each candidate (the k_filter_fwd arithmetic,
-// neighbour bookkeeping shared by the k fields), projected, summed per block.
-template <int K>
-__global__ void __launch_bounds__(kThreads) k_proj_volume(GridDev g, const StencilEntry* __restrict__ st,
-                                                          int ns, const uint8_t* __restrict__ act,
-                                                          const double* __restrict__ hs,
-                                                          const double* __restrict__ cand, int k,
-                                                          ProjConsts c, double* __restrict__ part) {
+// proj_vol (simp.cpp:1707-1716) of the candidates: for every design voxel, the
+// density filter of the candidate (the k_filter_fwd arithmetic), projected, summed.
+// A thread per voxel and candidate (blockIdx.y), for the same reason: about a hundred
+// FP64 instructions each.
+__global__ void __launch_bounds__(kThreads) k_proj_volume(
+    GridDev g, const StencilEntry* __restrict__ st, int ns, const uint8_t* __restrict__ act,
+    const double* __restrict__ hs, const double* __restrict__ cand, ProjConsts c,
+    double* __restrict__ part, double* __restrict__ out, unsigned* __restrict__ count) {
   const int64_t n = int64_t(g.nx) * g.ny * g.nz;
-  double vol[K];
-#pragma unroll
-  for (int j = 0; j < K; ++j) vol[j] = 0.0;
+  const double* xc = cand + blockIdx.y * n;
+  double vol = 0.0;
   for (int64_t e = blockIdx.x * int64_t(kThreads) + threadIdx.x; e < n;
        e += int64_t(gridDim.x) * kThreads) {
     if (!act[e]) continue;
-    const double h = hs[e];
     int i, jy, kz;
     vox_ijk(g, e, i, jy, kz);
-    double acc[K];
-#pragma unroll
-    for (int j = 0; j < K; ++j) acc[j] = 0.0;
+    double acc = 0.0;
     for (int q = 0; q < ns; ++q) {
       const int ii = i + st[q].di, jj = jy + st[q].dj, kk = kz + st[q].dk;
       if (!in_grid(g, ii, jj, kk)) continue;
       const int64_t nb = (int64_t(kk) * g.ny + jj) * g.nx + ii;
       if (!act[nb]) continue;
-      const double w = st[q].w;
-#pragma unroll
-      for (int j = 0; j < K; ++j)
-        if (j < k) acc[j] = __dadd_rn(acc[j], __dmul_rn(w, cand[j * n + nb]));
+      acc = __dadd_rn(acc, __dmul_rn(st[q].w, xc[nb]));
     }
-#pragma unroll
-    for (int j = 0; j < K; ++j)
-      if (j < k) vol[j] += proj_value(c, __ddiv_rn(acc[j], h));
+    vol += proj_value(c, __ddiv_rn(acc, hs[e]));
   }
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    if (j >= k) break;  // k is uniform over the block
-    const double v = block_sum256(vol[j]);
-    if (threadIdx.x == 0) part[j * gridDim.x + blockIdx.x] = v;
-  }
+  candidate_sum(vol, part, out, count);
 }
 
 // ------------------------------------------------------------------ MMA
@@ -602,8 +634,7 @@ __global__ void k_mma_prepare(const double* __restrict__ x, const double* __rest
                               const double* __restrict__ xold1, const double* __restrict__ xold2,
                               double* __restrict__ p0, double* __restrict__ q0,
                               double* __restrict__ p1, double* __restrict__ q1,
-                              double* __restrict__ al, double* __restrict__ be,
-                              double* __restrict__ part) {
+                              double* __restrict__ al, double* __restrict__ be, SumOut sum) {
   const double scale = __longlong_as_double((long long)*scale_bits);
   const double xr = __dsub_rn(c.xmax, c.xmin);
   const double reg = __ddiv_rn(1e-5, xr);
@@ -662,8 +693,7 @@ __global__ void k_mma_prepare(const double* __restrict__ x, const double* __rest
     al[e] = lo;
     be[e] = hi;
   }
-  const double v = block_sum256(tsum);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
+  grid_sum(tsum, sum, blockIdx.x, gridDim.x);
 }
 
 __device__ __forceinline__ double mma_candidate(double lam, double p0, double q0, double p1,
@@ -677,35 +707,25 @@ __device__ __forceinline__ double mma_candidate(double lam, double p0, double q0
   return xt;
 }
 
-// The dual's constraint sums sum_e p1/(U - x(lambda)) + q1/(x(lambda) - L) for
-// up to K multipliers in one pass over the coefficients.
-template <int K>
+// The dual's constraint sums sum_e p1/(U - x(lambda)) + q1/(x(lambda) - L), a
+// thread per voxel and multiplier (blockIdx.y): two roots and three divisions in FP64
+// each, against nine loads that the other multipliers' CTAs find in the L2.
 __global__ void __launch_bounds__(kThreads) k_mma_dual(
     const double* __restrict__ p0, const double* __restrict__ q0, const double* __restrict__ p1,
     const double* __restrict__ q1, const double* __restrict__ low, const double* __restrict__ upp,
     const double* __restrict__ al, const double* __restrict__ be, const uint8_t* __restrict__ act,
-    int64_t n, ProjLambdas ls, double* __restrict__ part) {
-  double acc[K];
-#pragma unroll
-  for (int j = 0; j < K; ++j) acc[j] = 0.0;
+    int64_t n, ProjLambdas ls, double* __restrict__ part, double* __restrict__ out,
+    unsigned* __restrict__ count) {
+  const double lam = ls.lam[blockIdx.y];
+  double acc = 0.0;
   for (int64_t e = blockIdx.x * int64_t(kThreads) + threadIdx.x; e < n;
        e += int64_t(gridDim.x) * kThreads) {
     if (!act[e]) continue;
-    const double a0 = p0[e], b0 = q0[e], a1 = p1[e], b1 = q1[e], L = low[e], U = upp[e];
-    const double lo = al[e], hi = be[e];
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      if (j >= ls.k) break;
-      const double xt = mma_candidate(ls.lam[j], a0, b0, a1, b1, L, U, lo, hi);
-      acc[j] += __dadd_rn(__ddiv_rn(a1, __dsub_rn(U, xt)), __ddiv_rn(b1, __dsub_rn(xt, L)));
-    }
+    const double a1 = p1[e], b1 = q1[e], L = low[e], U = upp[e];
+    const double xt = mma_candidate(lam, p0[e], q0[e], a1, b1, L, U, al[e], be[e]);
+    acc += __dadd_rn(__ddiv_rn(a1, __dsub_rn(U, xt)), __ddiv_rn(b1, __dsub_rn(xt, L)));
   }
-#pragma unroll
-  for (int j = 0; j < K; ++j) {
-    if (j >= ls.k) break;
-    const double v = block_sum256(acc[j]);
-    if (threadIdx.x == 0) part[j * gridDim.x + blockIdx.x] = v;
-  }
+  candidate_sum(acc, part, out, count);
 }
 
 __global__ void k_mma_candidate(const double* __restrict__ p0, const double* __restrict__ q0,
@@ -985,9 +1005,23 @@ void launch_mask_pins(const uint8_t* eff, int64_t n, double* xphys, cudaStream_t
 
 int exact_sum_blocks() { return kRedBlocks; }
 
+namespace {
+// CTAs of a pass over the voxels: two voxels a thread, so that a small grid's sums
+// are few, and at most kRedBlocks (the scratch; 4 CTAs an SM).
+int pass_blocks(int64_t n) {
+  return int(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + 2 * kThreads - 1) / (2 * kThreads))));
+}
+// The same where the pass is FP64-bound and has a grid row a candidate: one voxel a
+// thread.
+dim3 candidate_grid(int64_t n, int k) {
+  return dim3(unsigned(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + kThreads - 1) / kThreads))),
+              unsigned(k));
+}
+}  // namespace
+
 void launch_oc_volume_multi(const double* sq, const double* lo, const double* hi,
                             const double* dvd, int64_t n, const OcCands& cs, double* part,
-                            double* out, cudaStream_t s) {
+                            double* out, unsigned* count, cudaStream_t s) {
   // sq, lo, hi, dvd hold double-float pairs (written by launch_oc_prepare).
   OcCandsDF cd;
   cd.k = cs.k;
@@ -996,12 +1030,11 @@ void launch_oc_volume_multi(const double* sq, const double* lo, const double* hi
   const df* l = reinterpret_cast<const df*>(lo);
   const df* h = reinterpret_cast<const df*>(hi);
   const df* d = reinterpret_cast<const df*>(dvd);
-  if (cs.k <= 4)
-    k_oc_volume_multi<4><<<kRedBlocks, kThreads, 0, s>>>(a, l, h, d, n, cd, part);
+  const int nb = pass_blocks(n);
+  if (cs.k <= 8)
+    k_oc_volume_multi<8><<<nb, kThreads, 0, s>>>(a, l, h, d, n, cd, part, out, count);
   else
-    k_oc_volume_multi<kOcMulti><<<kRedBlocks, kThreads, 0, s>>>(a, l, h, d, n, cd, part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials_multi<<<cs.k, kThreads, 0, s>>>(part, kRedBlocks, out);
+    k_oc_volume_multi<kOcMulti><<<nb, kThreads, 0, s>>>(a, l, h, d, n, cd, part, out, count);
   TG_LAUNCH_CHECK();
 }
 
@@ -1039,54 +1072,43 @@ void launch_oc_candidates_projected(const double* x, const double* dcf, const do
                                     const uint8_t* act, int64_t n, const ProjLambdas& ls,
                                     double move, double rho_min, bool carry, double* cand,
                                     cudaStream_t s) {
-  k_oc_candidates_projected<<<grid_blocks(n), kThreads, 0, s>>>(x, dcf, dvf, act, n, ls, move,
+  k_oc_candidates_projected<<<dim3(grid_blocks(n), ls.k), kThreads, 0, s>>>(x, dcf, dvf, act, n, ls, move,
                                                                 rho_min, carry ? 1 : 0, cand);
   TG_LAUNCH_CHECK();
 }
 
 void launch_proj_volume(const Grid& g, const void* st, int ns, const uint8_t* act,
                         const double* hs, const double* cand, int k, double beta, double eta,
-                        double* part, double* out, cudaStream_t s) {
-  const auto* se = static_cast<const StencilEntry*>(st);
-  const ProjConsts c = proj_consts(beta, eta);
-  if (k <= 1)
-    k_proj_volume<1><<<kRedBlocks, kThreads, 0, s>>>(dev(g), se, ns, act, hs, cand, k, c, part);
-  else if (k <= 4)
-    k_proj_volume<4><<<kRedBlocks, kThreads, 0, s>>>(dev(g), se, ns, act, hs, cand, k, c, part);
-  else
-    k_proj_volume<kOcMulti><<<kRedBlocks, kThreads, 0, s>>>(dev(g), se, ns, act, hs, cand, k, c,
-                                                            part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials_multi<<<k, kThreads, 0, s>>>(part, kRedBlocks, out);
+                        double* part, double* out, unsigned* count, cudaStream_t s) {
+  k_proj_volume<<<candidate_grid(g.nv, k), kThreads, 0, s>>>(
+      dev(g), static_cast<const StencilEntry*>(st), ns, act, hs, cand, proj_consts(beta, eta),
+      part, out, count);
   TG_LAUNCH_CHECK();
 }
 
 void launch_mma_prepare(const MmaFields& m, const double* x, const double* dcf, const double* dvf,
                         const uint8_t* act, int64_t n, int iter, double move, double xmin,
-                        uint64_t* scale_bits, double* part, double* tsum, cudaStream_t s) {
+                        uint64_t* scale_bits, double* part, double* tsum, unsigned* count,
+                        cudaStream_t s) {
   TG_CUDA(cudaMemsetAsync(scale_bits, 0, sizeof(uint64_t), s));
   k_absmax_design<<<kRedBlocks, kThreads, 0, s>>>(dcf, act, n,
                                                   reinterpret_cast<unsigned long long*>(scale_bits));
   TG_LAUNCH_CHECK();
   const MmaConsts c{xmin, 1.0, move, iter};
-  k_mma_prepare<<<kRedBlocks, kThreads, 0, s>>>(
+  SumOut sum{};
+  sum.part = part;
+  sum.out = tsum;
+  sum.count = count;
+  k_mma_prepare<<<pass_blocks(n), kThreads, 0, s>>>(
       x, dcf, dvf, act, n, c, reinterpret_cast<const unsigned long long*>(scale_bits), m.low,
-      m.upp, m.xold1, m.xold2, m.p0, m.q0, m.p1, m.q1, m.al, m.be, part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials_multi<<<1, kThreads, 0, s>>>(part, kRedBlocks, tsum);
+      m.upp, m.xold1, m.xold2, m.p0, m.q0, m.p1, m.q1, m.al, m.be, sum);
   TG_LAUNCH_CHECK();
 }
 
 void launch_mma_dual(const MmaFields& m, const uint8_t* act, int64_t n, const ProjLambdas& ls,
-                     double* part, double* out, cudaStream_t s) {
-  if (ls.k <= 4)
-    k_mma_dual<4><<<kRedBlocks, kThreads, 0, s>>>(m.p0, m.q0, m.p1, m.q1, m.low, m.upp, m.al, m.be,
-                                                  act, n, ls, part);
-  else
-    k_mma_dual<kOcMulti><<<kRedBlocks, kThreads, 0, s>>>(m.p0, m.q0, m.p1, m.q1, m.low, m.upp,
-                                                         m.al, m.be, act, n, ls, part);
-  TG_LAUNCH_CHECK();
-  k_sum_partials_multi<<<ls.k, kThreads, 0, s>>>(part, kRedBlocks, out);
+                     double* part, double* out, unsigned* count, cudaStream_t s) {
+  k_mma_dual<<<candidate_grid(n, ls.k), kThreads, 0, s>>>(m.p0, m.q0, m.p1, m.q1, m.low, m.upp,
+                                                          m.al, m.be, act, n, ls, part, out, count);
   TG_LAUNCH_CHECK();
 }
 

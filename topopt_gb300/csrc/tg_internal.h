@@ -327,10 +327,11 @@ struct OcCandsDF {
 };
 // out[k] = sum_e dv_e clamp(sq_e c_k, lo_e, hi_e) in double-float arithmetic;
 // sq, lo, hi, dvd are the double-float fields launch_oc_prepare writes (8 bytes
-// per voxel each, in double-sized buffers); part holds k * kRedBlocks partials.
+// per voxel each, in double-sized buffers); part holds k * kRedBlocks partials and
+// count kOcMulti zeros, which every pass leaves zero.
 void launch_oc_volume_multi(const double* sq, const double* lo, const double* hi,
                             const double* dvd, int64_t n, const OcCands& cs, double* part,
-                            double* out, cudaStream_t s);
+                            double* out, unsigned* count, cudaStream_t s);
 void launch_oc_candidate(const double* x, const double* dcf, const double* dvf,
                          const uint8_t* act, int64_t n, double lambda, double move,
                          double rho_min, bool carry, double* xnew, cudaStream_t s);
@@ -352,10 +353,10 @@ void launch_oc_candidates_projected(const double* x, const double* dcf, const do
                                     double move, double rho_min, bool carry, double* cand,
                                     cudaStream_t s);
 // out[j] = sum over design voxels of heaviside_project(filter(cand_j)), j < k;
-// part holds k * kRedBlocks partials.
+// part and count as above.
 void launch_proj_volume(const Grid& g, const void* st, int ns, const uint8_t* act,
                         const double* hs, const double* cand, int k, double beta, double eta,
-                        double* part, double* out, cudaStream_t s);
+                        double* part, double* out, unsigned* count, cudaStream_t s);
 // MMA (mma_joint.cpp): the per-voxel fields of one run's subproblem.
 struct MmaFields {
   double *low, *upp, *xold1, *xold2, *p0, *q0, *p1, *q1, *al, *be;
@@ -364,10 +365,11 @@ struct MmaFields {
 // sum over the design set of p1/(U - x) + q1/(x - L).  scale_bits: 1 scratch word.
 void launch_mma_prepare(const MmaFields& m, const double* x, const double* dcf, const double* dvf,
                         const uint8_t* act, int64_t n, int iter, double move, double xmin,
-                        uint64_t* scale_bits, double* part, double* tsum, cudaStream_t s);
+                        uint64_t* scale_bits, double* part, double* tsum, unsigned* count,
+                        cudaStream_t s);
 // out[j] = the dual's constraint sum at ls.lam[j], j < ls.k.
 void launch_mma_dual(const MmaFields& m, const uint8_t* act, int64_t n, const ProjLambdas& ls,
-                     double* part, double* out, cudaStream_t s);
+                     double* part, double* out, unsigned* count, cudaStream_t s);
 // x_new(lambda) on the design set, 0 elsewhere.
 void launch_mma_candidate(const MmaFields& m, const uint8_t* act, int64_t n, double lam,
                           double* xnew, cudaStream_t s);
