@@ -688,6 +688,32 @@ FineSchedule default_fine_schedule(const Grid& g) {
 
 int fine_schedule_shapes() { return kNumShapes; }
 
+// The schedules worth measuring on g: of every tile shape with z-chunks of about 8 to
+// 64 node layers, the sixteen that the cost model puts first (its error against
+// measured times is a few percent; the sixteenth is beyond that).
+std::vector<FineSchedule> fine_schedule_candidates(const Grid& g) {
+  std::vector<std::pair<double, FineSchedule>> all;
+  for (int sh = 0; sh < kNumShapes; ++sh) {
+    int last = 0;
+    for (int target : {64, 43, 33, 26, 22, 16, 13, 11, 8}) {
+      const int chunks = std::max(1, (g.nnz + target - 1) / target);
+      const MarchTile t{kShapeWarps[sh], std::max(kTunedMinKz, (g.nnz + chunks - 1) / chunks)};
+      if (t.kz == last) continue;
+      last = t.kz;
+      FineSchedule s;
+      s.shape = sh;
+      s.kz = t.kz;
+      all.emplace_back(march_cost<float2>(t, march_grid<float2>(g.nnx, g.nny, g.nnz, 1, false, t)),
+                       s);
+    }
+  }
+  std::stable_sort(all.begin(), all.end(),
+                   [](const auto& a, const auto& b) { return a.first < b.first; });
+  std::vector<FineSchedule> out;
+  for (size_t i = 0; i < all.size() && i < 16; ++i) out.push_back(all[i].second);
+  return out;
+}
+
 bool fine_schedule_valid(const FineSchedule& s) {
   if (s.kind == FineSchedule::kPencil) return true;
   return s.kind == FineSchedule::kColumn && s.shape >= 0 && s.shape < kNumShapes &&

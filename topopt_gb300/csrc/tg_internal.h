@@ -195,6 +195,7 @@ struct FineSchedule {
 };
 FineSchedule default_fine_schedule(const Grid& g);
 int fine_schedule_shapes();
+std::vector<FineSchedule> fine_schedule_candidates(const Grid& g);
 bool fine_schedule_valid(const FineSchedule& s);
 // The schedule the FP32 operator uses on g: a process-wide override when one is
 // set, else the table entry for g's dimensions (tune.cu), else the default.
@@ -206,7 +207,7 @@ void launch_fine_op_sched(const FineSchedule& fs, int mode, const Grid& g, const
                           const float* ef, const uint8_t* kept_node, const float* x,
                           const float* b, const float* invdiag, float omega, float* y,
                           const SumOut& dot, cudaStream_t s);
-// Times every candidate schedule of the FP32 operator on the given buffers
+// Times the candidate schedules of the FP32 operator on the given buffers
 // (CUDA events on s) for the apply and, with b and invdiag, the residual and
 // smoothing modes; publishes the fastest per mode in the table for g (one sweep
 // at a time; a grid already in the table is not measured again) and returns

@@ -62,9 +62,10 @@ bool fine_schedule_known(const Grid& g) {
   return g_have_override || g_sched.count(std::make_tuple(g.nx, g.ny, g.nz, int(kApply))) != 0;
 }
 
-// The measured sweep: every column tile shape with z-chunks of about 8 .. 33
-// node layers, and the one-row kernel, each launched once untimed and then
-// timed over `reps` back-to-back launches, for each of the three modes as the
+// The measured sweep: the schedules that the cost model ranks first, each launched
+// once untimed and then timed over `reps` back-to-back launches (192 launches in all;
+// every tile shape with every chunk length took 688, 35 ms of a 192x96x96 grid's
+// first solve), for each of the three modes as the
 // mixed solve runs them: the apply with the kept mask and the p.Ap partials,
 // the residual, and the smoothing sweep with its b.y partials (b, invdiag:
 // any finite vectors).  The fastest per mode goes into the table for g's
@@ -77,24 +78,7 @@ FineSchedule autotune_fine_schedule(const Grid& g, const ModalConsts& mc, const 
                                     const float* invdiag, int reps) {
   std::lock_guard<std::mutex> tune_lock(g_tune_mu);
   if (fine_schedule_known(g)) return fine_schedule_for(g, kApply);
-  std::vector<FineSchedule> cands;
-  FineSchedule pencil;
-  pencil.kind = FineSchedule::kPencil;
-  cands.push_back(pencil);
-  std::vector<int> kzs;
-  for (int target : {8, 11, 13, 16, 22, 26, 33}) {
-    const int chunks = std::max(1, (g.nnz + target - 1) / target);
-    const int kz = std::max(8, (g.nnz + chunks - 1) / chunks);
-    if (std::find(kzs.begin(), kzs.end(), kz) == kzs.end()) kzs.push_back(kz);
-  }
-  for (int sh = 0; sh < fine_schedule_shapes(); ++sh)
-    for (int kz : kzs) {
-      FineSchedule c;
-      c.kind = FineSchedule::kColumn;
-      c.shape = sh;
-      c.kz = kz;
-      cands.push_back(c);
-    }
+  const std::vector<FineSchedule> cands = fine_schedule_candidates(g);
   EventPair ev;
   const cudaEvent_t ea = ev.a, eb = ev.b;
   std::vector<std::pair<int, FineSchedule>> chosen;
