@@ -1,0 +1,37 @@
+"""Solves whose last smoothed level is applied as a dense matrix, at the edges of that
+form: 3, 5 and 7 columns a CTA, its largest level (1,050 DOFs on 26x8x8) and the first
+beyond it (28x8x8), odd grids with both coarsenings, and a void pocket, against the
+CPU's Jacobi-PCG.  Both solve to 1e-12 of the right-hand side; the condition numbers
+of these grids (about 1e4) leave 1e-8 of the displacement."""
+import numpy as np
+import pytest
+
+from oracle.oracle import cantilever
+from test_oracle_mg import smooth_modulus
+
+pytestmark = pytest.mark.gpu
+
+CASES = [((8, 8, 8), False), ((12, 8, 8), False), ((24, 8, 8), False), ((26, 8, 8), False),
+         ((28, 8, 8), False), ((11, 7, 9), False), ((40, 16, 16), True)]
+
+
+@pytest.mark.parametrize("coarsening", [1, 2])
+@pytest.mark.parametrize("dims,voids", CASES)
+def test_dense_cycle_solve(tg, port, dims, voids, coarsening):
+    nx, ny, nz = dims
+    solid = None
+    if voids:
+        s = np.ones((nz, ny, nx), np.uint8)
+        s[4:10, 4:10, 10:20] = 0
+        solid = s.ravel()
+    o = cantilever(nx, ny, nz, solid=solid)
+    pb = tg.Problem(nx, ny, nz, 1.0, solid, list(zip(o.bc_node, o.bc_comp, o.bc_val)),
+                    list(zip(o.ld_node, o.ld_comp, o.ld_val)))
+    f = smooth_modulus(*dims)
+    ue, _, _ = port.solve_cg(o, f, tol=1e-12)
+    for prec in (0, tg.PREC_MIXED):
+        u, info = tg.fea_solve_mgcg_matfree(pb, f, tolerance=1e-12, max_iterations=2000,
+                                            options=tg.SolveOptions(precision=prec,
+                                                                    coarsening=coarsening))
+        assert info.converged and info.mg_levels >= 3
+        assert np.abs(u - ue).max() <= 1e-8 * np.abs(ue).max()

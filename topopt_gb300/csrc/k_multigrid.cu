@@ -26,11 +26,13 @@
 // Half the bytes of the full 243-entry stencil, the bound of the coarse apply.
 #include <cuda_runtime.h>
 
+#include "tg_df.h"
 #include "tg_internal.h"
 #include "tg_multigrid.h"
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <utility>
 
 namespace tg {
@@ -880,23 +882,40 @@ __global__ void k_chol_update(double* __restrict__ D, int nc, int k0) {
   }
 }
 
+// An FP32 value as FP64: by integer operations where it is normal or zero, since the
+// conversion is an FP64-pipe instruction like the multiply-add it feeds.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu, sign = u & 0x80000000u;
+  if (m == 0u) return __hiloint2double(int(sign), 0);
+  if (m - 0x00800000u >= 0x7f000000u) return double(v);  // denormal, infinite, NaN
+  return __hiloint2double(int(sign | ((m >> 3) + (896u << 20))), int(u << 29));
+}
+
 // x = Ainv b on the compact numbering, gathered from / scattered to the level
-// vector; one warp per row of Ainv.
+// vector (cidx and cdof null: Ainv is over the level's own numbering); one warp per
+// row of Ainv.  Each lane's products are one chain of FP64 multiply-adds, 64 cycles
+// a link on its scheduler, so a warp takes one row and the rows are spread over all
+// SMs; the matrix comes from the L2, eight loads ahead of the chain.
+constexpr int kRowWarps = 4;
 template <class T>
-__global__ void k_coarse_inv_apply(const double* __restrict__ Ainv, int nc,
-                                   const int* __restrict__ cidx, const int* __restrict__ cdof,
-                                   int64_t ndof, const T* __restrict__ b, T* __restrict__ x) {
+__global__ void __launch_bounds__(32 * kRowWarps) k_coarse_inv_apply(
+    const double* __restrict__ Ainv, int nc, const int* __restrict__ cidx,
+    const int* __restrict__ cdof, int64_t ndof, const T* __restrict__ b, T* __restrict__ x) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int64_t dd = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; dd < ndof;
-       dd += int64_t(gridDim.x) * blockDim.x)
-    if (cidx[dd] < 0) x[dd] = T(0);
+  if (cidx != nullptr)
+    for (int64_t dd = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; dd < ndof;
+         dd += int64_t(gridDim.x) * blockDim.x)
+      if (cidx[dd] < 0) x[dd] = T(0);
   for (int r = warp; r < nc; r += nwarps) {
+    const double* row = Ainv + int64_t(r) * nc;
     double s = 0.0;
-    for (int k = lane; k < nc; k += 32) s += Ainv[int64_t(r) * nc + k] * double(b[cdof[k]]);
+#pragma unroll 8
+    for (int k = lane; k < nc; k += 32) s += row[k] * widen(b[cdof != nullptr ? cdof[k] : k]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) x[cdof[r]] = T(s);
+    if (lane == 0) x[cdof != nullptr ? cdof[r] : r] = T(s);
   }
 }
 
@@ -1164,7 +1183,8 @@ void mg_dense_inverse(int nc, double* a, double* inv, double* pivot, int* fail, 
 template <class T>
 void mg_coarse_inv_apply(const double* Ainv, int nc, const int* cidx, const int* cdof,
                          int64_t ndof, const T* b, T* x, cudaStream_t s) {
-  k_coarse_inv_apply<T><<<std::max(1, std::min(152, (nc + 7) / 8)), 256, 0, s>>>(Ainv, nc, cidx, cdof, ndof, b, x);
+  const int nb = std::max(1, std::min(152 * 4, (nc + kRowWarps - 1) / kRowWarps));
+  k_coarse_inv_apply<T><<<nb, 32 * kRowWarps, 0, s>>>(Ainv, nc, cidx, cdof, ndof, b, x);
   TG_LAUNCH_CHECK();
 }
 
@@ -1175,7 +1195,259 @@ void mg_chol_solve(const double* L, int nc, const int* cidx, int64_t ndof, const
   TG_LAUNCH_CHECK();
 }
 
+// ------------------------------------------- the last smoothed level, dense
+// One V-cycle of the last smoothed level (its smoothing steps, the transfers and the
+// coarsest solve) is a linear map of the level's right-hand side.  Launch by launch
+// it is five dependent kernels of a few hundred rows (damped Jacobi, one sweep a side)
+// or eleven (Chebyshev of degree four), 3-4 us each, in every V-cycle; as a dense
+// matrix it is one product (FP64 675 DOFs: 3.6 MB from the L2, an FP64 multiply-add an
+// entry; per iteration 86 -> 80 us at 24x8x8 FP64, 73 -> 68 at 60x20x20 mixed, 244 ->
+// 224 at 128x64x64 mixed, Chebyshev).  This kernel forms the matrix once per hierarchy: column j
+// is the cycle applied to the unit vector e_j.  Columns are independent, so a CTA
+// takes NC of them through the whole cycle with its vectors in shared memory, and each
+// stencil entry that it reads (coalesced, from the L2) serves NC columns.  FP64
+// hierarchies are formed in FP64, FP32 ones in double-float arithmetic: their matrix
+// is kept in FP64, as the coarsest inverse is.
+namespace {
+
+__device__ __forceinline__ double cy_mad(double a, double x, double acc) {
+  return __fma_rn(a, x, acc);
+}
+__device__ __forceinline__ df cy_mad(float a, df x, df acc) {
+  const float p = __fmul_rn(a, x.hi);
+  return acc + df(p, __fmaf_rn(a, x.lo, __fmaf_rn(a, x.hi, -p)));
+}
+__device__ __forceinline__ df cy_mad(df a, df x, df acc) { return acc + a * x; }
+__device__ __forceinline__ double cy_sub(double a, double b) { return a - b; }
+__device__ __forceinline__ df cy_sub(df a, df b) { return a - b; }
+template <class C>
+__device__ __forceinline__ C cy_const(float v);
+template <>
+__device__ __forceinline__ double cy_const<double>(float v) {
+  return double(v);
+}
+template <>
+__device__ __forceinline__ df cy_const<df>(float v) {
+  return df(v, 0.0f);
+}
+__device__ __forceinline__ void cy_load(double v, double& c) { c = v; }
+__device__ __forceinline__ void cy_load(double v, df& c) { c = df_split(v); }
+__device__ __forceinline__ double cy_store(double v) { return v; }
+__device__ __forceinline__ double cy_store(df v) { return df_to_double(v); }
+
+// Row r of node (a, bb, c) of the stencil times NC columns x (n apart).
+template <class T, class C, int NC>
+__device__ __forceinline__ void stencil_columns(const MgDims& d, const T* __restrict__ A,
+                                                const C* x, int n, int a, int bb, int c, int r,
+                                                C (&s)[NC]) {
+  const int nn = d.nnx * d.nny * d.nnz, sy = d.nnx, sz = d.nnx * d.nny;
+  const int node = c * sz + bb * sy + a;
+  const T* An = A + node + int64_t(3 * r) * nn;
+  auto block = [&](const T* e, int64_t step, int m) {
+    const T a0 = e[0], a1 = e[step], a2 = e[2 * step];
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const C* v = x + q * n + 3 * m;
+      s[q] = cy_mad(a2, v[2], cy_mad(a1, v[1], cy_mad(a0, v[0], s[q])));
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < NC; ++q) s[q] = cy_const<C>(0.0f);
+  block(An, nn, node);
+#pragma unroll 1
+  for (int j = 1; j < 14; ++j) {
+    const int di = 13 + j;
+    const int dx = di % 3 - 1, dy = (di / 3) % 3 - 1, dz = di / 9 - 1;
+    const int off = dz * sz + dy * sy + dx;
+    if ((a + dx) < d.nnx && (a + dx) >= 0 && (bb + dy) < d.nny && (bb + dy) >= 0 &&
+        (c + dz) < d.nnz)
+      block(An + int64_t(j * 9) * nn, nn, node + off);
+    if ((a - dx) >= 0 && (a - dx) < d.nnx && (bb - dy) >= 0 && (bb - dy) < d.nny && (c - dz) >= 0)
+      block(A + int64_t(j * 9 + r) * nn + (node - off), 3 * int64_t(nn), node - off);
+  }
+}
+
+constexpr int kCycleThreads = 768;
+
+// Smoothing: Chebyshev of degree cheb_m (> 0; coef) or `sweeps` damped-Jacobi steps a
+// side, as the V-cycle's.  M is row-major over the level's n DOFs.
+template <class T, class C, int NC>
+__global__ void __launch_bounds__(kCycleThreads, 1) k_cycle_columns(
+    MgDims d, MgDims cd, const T* __restrict__ A, const uint8_t* __restrict__ act,
+    const T* __restrict__ dinv, const float* __restrict__ coef, int cheb_m, int sweeps, T omega,
+    const double* __restrict__ Ainv, int nc, const int* __restrict__ cidx,
+    const int* __restrict__ cdof, double* __restrict__ M) {
+  extern __shared__ double2 cycle_smem[];
+  const int nodes = d.nnx * d.nny * d.nnz, n = 3 * nodes;
+  C* x = reinterpret_cast<C*>(cycle_smem);
+  C* y = x + NC * n;
+  C* rc = y + NC * n;
+  C* ec = rc + NC * nc;
+  C* dir = ec + NC * nc;  // Chebyshev only
+  const int j0 = blockIdx.x * NC, items = ((nodes + 31) / 32) * 96;
+  const C zero = cy_const<C>(0.0f);
+  // One item is a (node, row) pair, a component per warp.
+  auto each_row = [&](auto&& f) {
+    for (int it = threadIdx.x; it < items; it += blockDim.x) {
+      const int node = (it / 96) * 32 + (it & 31), r = (it / 32) % 3;
+      if (node >= nodes) continue;
+      const int a = node % d.nnx, b = (node / d.nnx) % d.nny, c = node / (d.nnx * d.nny);
+      f(a, b, c, r, 3 * node + r);
+    }
+  };
+  // dinv (e_j - s), the preconditioned residual of column q at DOF i.
+  auto dres = [&](int i, int q, T dv, C s) {
+    return cy_mad(dv, cy_sub(cy_const<C>(i == j0 + q ? 1.0f : 0.0f), s), zero);
+  };
+  auto step = [&](int k) {  // one smoothing step from x into y, then swapped
+    each_row([&](int a, int b, int c, int r, int i) {
+      C s[NC];
+      stencil_columns<T, C, NC>(d, A, x, n, a, b, c, r, s);
+      const bool ac = act[i] != 0;
+      const T dv = dinv[i];
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        C out = zero;
+        if (cheb_m > 0) {
+          C dn = zero;
+          if (ac) {
+            const C res = dres(i, q, dv, s[q]);
+            dn = k == 0 ? cy_mad(cy_const<C>(coef[0]), res, zero)
+                        : cy_mad(cy_const<C>(coef[2 * k]), dir[q * n + i],
+                                 cy_mad(cy_const<C>(coef[2 * k + 1]), res, zero));
+            out = x[q * n + i] + dn;
+          }
+          dir[q * n + i] = dn;
+        } else if (ac) {
+          out = cy_mad(omega, dres(i, q, dv, s[q]), x[q * n + i]);
+        }
+        y[q * n + i] = out;
+      }
+    });
+    __syncthreads();
+    C* t = x;
+    x = y;
+    y = t;
+  };
+  // The first step, from zero: only DOF j of column j is not zero.
+  for (int i = threadIdx.x; i < NC * n; i += blockDim.x) {
+    const int q = i / n, dof = i - q * n;
+    C v = zero;
+    if (dof == j0 + q && act[dof]) {
+      v = dres(dof, q, dinv[dof], zero);
+      v = cheb_m > 0 ? cy_mad(cy_const<C>(coef[0]), v, zero) : cy_mad(omega, v, zero);
+    }
+    x[i] = v;
+    if (cheb_m > 0) dir[i] = v;
+  }
+  __syncthreads();
+  const int steps = cheb_m > 0 ? cheb_m : sweeps;
+  for (int k = 1; k < steps; ++k) step(k);
+  each_row([&](int a, int b, int c, int r, int i) {
+    C s[NC];
+    stencil_columns<T, C, NC>(d, A, x, n, a, b, c, r, s);
+    const bool ac = act[i] != 0;
+#pragma unroll
+    for (int q = 0; q < NC; ++q)
+      y[q * n + i] =
+          ac ? cy_sub(cy_const<C>(i == j0 + q ? 1.0f : 0.0f), s[q]) : zero;
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i < NC * nc; i += blockDim.x) {  // restriction
+    const int q = i / nc, dof = cdof[i - q * nc], k = dof % 3, cn = dof / 3;
+    const int a = cn % cd.nnx, b = (cn / cd.nnx) % cd.nny, c = cn / (cd.nnx * cd.nny);
+    float wx[3], wy[3], wz[3];
+    axis_weights<float>(a, d.ex, d.nnx, cd.align, wx);
+    axis_weights<float>(b, d.ey, d.nny, cd.align, wy);
+    axis_weights<float>(c, d.ez, d.nnz, cd.align, wz);
+    C s = zero;
+    for (int p = 0; p < 27; ++p) {
+      const int dx = p % 3, dy = (p / 3) % 3, dz = p / 9;
+      const float w = wx[dx] * wy[dy] * wz[dz];
+      if (w == 0.0f) continue;  // beyond the grid
+      const int m = ((2 * c + dz - 1) * d.nny + 2 * b + dy - 1) * d.nnx + 2 * a + dx - 1;
+      s = cy_mad(cy_const<C>(w), y[q * n + 3 * m + k], s);
+    }
+    rc[i] = s;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < NC * nc; i += blockDim.x) {  // coarsest solve
+    const int q = i / nc, k = i - q * nc;
+    C s = zero;
+    for (int m = 0; m < nc; ++m) {
+      C v;
+      cy_load(Ainv[int64_t(m) * nc + k], v);
+      s = cy_mad(v, rc[q * nc + m], s);
+    }
+    ec[i] = s;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < NC * n; i += blockDim.x) {  // prolongation
+    const int q = i / n, dof = i - q * n, k = dof % 3, node = dof / 3;
+    if (!act[dof]) continue;
+    const int a = node % d.nnx, b = (node / d.nnx) % d.nny, c = node / (d.nnx * d.nny);
+    const bool ta = tail_node(a, d.ex, cd.align), tb = tail_node(b, d.ey, cd.align),
+               tc = tail_node(c, d.ez, cd.align);
+    const bool ha = (a & 1) && !ta, hb = (b & 1) && !tb, hc = (c & 1) && !tc;
+    const float w = (ha ? 0.5f : 1.0f) * (hb ? 0.5f : 1.0f) * (hc ? 0.5f : 1.0f);
+    C s = x[i];
+    for (int p = 0; p < 8; ++p) {
+      const int dx = p & 1, dy = (p >> 1) & 1, dz = p >> 2;
+      if ((dx && !ha) || (dy && !hb) || (dz && !hc)) continue;
+      const int ia = (ta ? (a + 1) >> 1 : a >> 1) + dx, ib = (tb ? (b + 1) >> 1 : b >> 1) + dy,
+                ic = (tc ? (c + 1) >> 1 : c >> 1) + dz;
+      if (ia >= cd.nnx || ib >= cd.nny || ic >= cd.nnz) continue;
+      const int e = cidx[3 * ((ic * cd.nny + ib) * cd.nnx + ia) + k];
+      if (e >= 0) s = cy_mad(cy_const<C>(w), ec[q * nc + e], s);
+    }
+    x[i] = s;
+  }
+  __syncthreads();
+  for (int k = 0; k < steps; ++k) step(k);
+  for (int i = threadIdx.x; i < NC * n; i += blockDim.x) {
+    const int dof = i / NC, q = i - dof * NC;
+    if (j0 + q < n) M[int64_t(dof) * n + j0 + q] = cy_store(x[q * n + dof]);
+  }
+}
+
+// Columns of a CTA: the fewest that put every column on an SM of its own at once.
+int cycle_columns(int64_t ndof) { return ndof <= 3 * 152 ? 3 : ndof <= 5 * 152 ? 5 : 7; }
+size_t cycle_bytes(int64_t ndof, int nc, bool cheb) {
+  return 8 * size_t(cycle_columns(ndof)) * (size_t(ndof) * (cheb ? 3 : 2) + 2 * size_t(nc));
+}
+
+}  // namespace
+
+bool mg_dense_cycle_fits(int64_t ndof, int nc, bool cheb) {
+  return ndof <= kDenseCycleDof && cycle_bytes(ndof, nc, cheb) <= size_t(227) * 1024;
+}
+
+template <class T>
+void mg_dense_cycle(const MgDims& d, const MgDims& cd, const T* A, const uint8_t* act,
+                    const T* dinv, const float* coef, int cheb_m, int sweeps, T omega,
+                    const double* Ainv, int nc, const int* cidx, const int* cdof, double* M,
+                    cudaStream_t s) {
+  using C = typename std::conditional<sizeof(T) == 8, double, df>::type;
+  const int64_t nodes = int64_t(d.nnx) * d.nny * d.nnz, ndof = 3 * nodes;
+  const size_t sm = cycle_bytes(ndof, nc, cheb_m > 0);
+  const int threads = int(std::min<int64_t>(kCycleThreads, (nodes + 31) / 32 * 96));
+  auto run = [&](auto kernel, int cols) {
+    TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    kernel<<<unsigned((ndof + cols - 1) / cols), threads, sm, s>>>(
+        d, cd, A, act, dinv, coef, cheb_m, sweeps, omega, Ainv, nc, cidx, cdof, M);
+    TG_LAUNCH_CHECK();
+  };
+  switch (cycle_columns(ndof)) {
+    case 3: run(k_cycle_columns<T, C, 3>, 3); break;
+    case 5: run(k_cycle_columns<T, C, 5>, 5); break;
+    default: run(k_cycle_columns<T, C, 7>, 7);
+  }
+}
+
 #define TG_INST(T)                                                                            \
+  template void mg_dense_cycle<T>(const MgDims&, const MgDims&, const T*, const uint8_t*,     \
+                                  const T*, const float*, int, int, T, const double*, int,    \
+                                  const int*, const int*, double*, cudaStream_t);             \
   template void mg_stencil_op<T>(int, const MgDims&, const T*, const uint8_t*, const T*,      \
                                  const T*, const T*, T, T*, cudaStream_t, ChebStep);          \
   template void mg_jacobi_first<T>(const T*, const T*, T, int64_t, T*, cudaStream_t);         \
@@ -1341,20 +1613,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_coarse_vcycle(FusedCoarse 
         if (F.act[3 * n + k]) xf[3 * n + k] = __ldcg(xf + 3 * n + k) + s[k];
     }
   };
-  auto coarsest = [&]() {  // x = A^-1 b over the compact numbering, a warp per row
+  // x = A^-1 b over the compact numbering, or the last smoothed level's dense cycle
+  // over its own (cidx and cdof null), a warp per row.
+  auto coarsest = [&]() {
     const FusedLevel& L = fc.L[top];
     const int64_t ndof = 3 * int64_t(L.d.nnx) * L.d.nny * L.d.nnz;
     for (int64_t dd = tid; dd < ndof; dd += nthreads)
-      if (fc.cidx[dd] < 0) L.xp[dd] = 0.0f;
+      if (fc.cidx != nullptr && fc.cidx[dd] < 0) L.xp[dd] = 0.0f;
     const int lane = threadIdx.x & 31;
     const int64_t warp = tid >> 5, nwarps = nthreads >> 5;
     for (int64_t row = warp; row < fc.nc; row += nwarps) {
       double s = 0.0;
       for (int k = lane; k < fc.nc; k += 32)
-        s += fc.Ainv[row * fc.nc + k] * double(__ldcg(L.b + fc.cdof[k]));
+        s += fc.Ainv[row * fc.nc + k] * double(__ldcg(L.b + (fc.cdof != nullptr ? fc.cdof[k] : k)));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-      if (lane == 0) L.xp[fc.cdof[row]] = float(s);
+      if (lane == 0) L.xp[fc.cdof != nullptr ? fc.cdof[row] : row] = float(s);
     }
     cur[top] = 0;
   };

@@ -410,7 +410,7 @@ size_t Solver::device_bytes() const {
   for (const DBuf<double>* d : {&invdiag_, &rhs_, &x_, &r_, &z_, &p_, &ap_, &t0_, &t1_, &part_,
                                 &scal_, &keb_, &G_, &chol_, &chol_work_})
     b += d->bytes();
-  b += gj_pivot_.bytes() + chol_inv_.bytes() + cdof_.bytes();
+  b += gj_pivot_.bytes() + chol_inv_.bytes() + dense_.bytes() + cdof_.bytes();
   for (const DBuf<float>* d : {&Ef_, &invdiagf_, &xf_, &rf_, &zf_, &pf_, &apf_, &t0f_, &t1f_})
     b += d->bytes();
   for (const auto& L : levels_) b += L->bytes();
@@ -500,6 +500,16 @@ void Solver::build_structure() {
   if (nc_ <= kMaxInverseDof) {
     gj_pivot_.alloc(1024);
     chol_inv_.alloc(size_t(nc_) * nc_);
+  }
+  // The last smoothed level in the form of its dense cycle, with the coarsest inverse.
+  dense_level_ = 0;
+  if (levels_.size() >= 2 && nc_ <= kMaxInverseDof) {
+    const size_t l = levels_.size() - 1;
+    const int64_t nd = levels_[l - 1]->ndof;
+    if (mg_dense_cycle_fits(nd, nc_, mixed_ && cheb_m_ > 0)) {
+      dense_level_ = l;
+      dense_.alloc(size_t(nd * nd));
+    }
   }
   chol_.alloc(size_t(nc_) * nc_);
   chol_work_.alloc(size_t(nc_));
@@ -601,7 +611,7 @@ void Solver::build_structure() {
   if (mixed_ && side_level_ > 0) ensure_side();
   fused_level_ = 0;
   if (mixed_ && coarse_fused_enabled() && chol_inv_.p != nullptr) {
-    for (size_t l = 2; l < levels_.size(); ++l) {
+    for (size_t l = 2; l < (dense_level_ ? dense_level_ : levels_.size()); ++l) {
       const MgDims& d = levels_[l - 1]->d;
       if (int64_t(d.nnx) * d.nny * d.nnz <= kFusedMaxNodes) {
         if (levels_.size() - (l - 1) <= size_t(kFusedMaxLevels)) fused_level_ = l;
@@ -812,7 +822,7 @@ bool Solver::build_numeric() {
       mg_galerkin_coarse<T>(pd, L.d, levels_[l - 1]->Ke<T>(), L.act.p, L.Ke<T>(), s_);
     // The matrix-free level 1 needs only its inverse diagonal; the assembled
     // stencil (275 MB on the 256x128x128 cantilever) is formed on demand (level1_stencil()).
-    const bool diag_only = sizeof(T) == 4 && l == 0 && l1_mf_;
+    const bool diag_only = sizeof(T) == 4 && l == 0 && l1_mf_ && dense_level_ != 1;
     mg_assemble_stencil<T>(L.d, L.Ke<T>(), L.act.p, diag_only ? nullptr : L.Am<T>(), L.Dinv<T>(),
                            s_);
     if (sizeof(T) == 4 && l == 0) l1_stencil_ok_ = !diag_only;
@@ -854,6 +864,14 @@ bool Solver::build_numeric() {
     mg_dense_from_stencil<T>(C.d, C.Am<T>(), cidx_.p, nc_,
                              mg_dense_start(nc_, chol_.p, chol_inv_.p), s_);
     mg_dense_inverse(nc_, chol_.p, chol_inv_.p, gj_pivot_.p, chol_fail_.p, s_);
+    if (dense_level_ > 0) {
+      Level& L = *levels_[dense_level_ - 1];
+      const bool cheb = sizeof(T) == 4 && cheb_m_ > 0 && dense_level_ >= 2;
+      mg_dense_cycle<T>(L.d, C.d, L.Am<T>(), L.act.p, L.Dinv<T>(),
+                        cheb ? chc_.p + kChebCoefStride * (dense_level_ - 1) : nullptr,
+                        cheb ? cheb_m_ : 0, sweeps_, T(omega_), chol_inv_.p, nc_, cidx_.p,
+                        cdof_.p, dense_.p, s_);
+    }
   } else {
     mg_dense_from_stencil<T>(C.d, C.Am<T>(), cidx_.p, nc_, chol_.p, s_);
     mg_cholesky(chol_.p, nc_, chol_fail_.p, s_);
@@ -870,6 +888,7 @@ template <class T>
 FirstStep<T> Solver::first_step(size_t l) {
   FirstStep<T> f;
   if (l >= levels_.size()) return f;  // the coarsest: solved, not smoothed
+  if (l == dense_level_) return f;    // its dense cycle starts from the right-hand side
   if constexpr (sizeof(T) == 4) {
     if (l == fused_level_) return f;  // the fused launch takes its own first step
   }
@@ -956,6 +975,11 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
   if constexpr (sizeof(T) == 4) {
     if (l == side_level_ && pending_x_) side.on = fork_x();
   }
+  if (l == dense_level_) {
+    mg_coarse_inv_apply<T>(dense_.p, int(L.ndof), nullptr, nullptr, L.ndof, L.B<T>(), L.X<T>(),
+                           s_);
+    return L.X<T>();
+  }
   if (l == levels_.size()) {
     if (chol_inv_.p)
       mg_coarse_inv_apply<T>(chol_inv_.p, nc_, cidx_.p, cdof_.p, L.ndof, L.B<T>(), L.X<T>(), s_);
@@ -1030,7 +1054,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
 float* Solver::fused_coarse_vcycle() {
   FusedCoarse fc;
   const size_t first = fused_level_ - 1;  // levels_ index of the first fused level
-  fc.nlev = int(levels_.size() - first);
+  fc.nlev = int((dense_level_ ? dense_level_ : levels_.size()) - first);
   for (int i = 0; i < fc.nlev; ++i) {
     Level& L = *levels_[first + size_t(i)];
     FusedLevel& F = fc.L[i];
@@ -1047,10 +1071,10 @@ float* Solver::fused_coarse_vcycle() {
   fc.cheb_m = cheb_m_;
   fc.sweeps = sweeps_;
   fc.omega = float(omega_);
-  fc.Ainv = chol_inv_.p;
-  fc.nc = nc_;
-  fc.cidx = cidx_.p;
-  fc.cdof = cdof_.p;
+  fc.Ainv = dense_level_ ? dense_.p : chol_inv_.p;
+  fc.nc = dense_level_ ? int(levels_[dense_level_ - 1]->ndof) : nc_;
+  fc.cidx = dense_level_ ? nullptr : cidx_.p;
+  fc.cdof = dense_level_ ? nullptr : cdof_.p;
   mg_coarse_vcycle_fused(fc, s_);
   // Chebyshev: 2 cheb_m toggles per level (even); Jacobi: the first sweep in
   // place, then 2 sweeps - 1 toggles (odd).

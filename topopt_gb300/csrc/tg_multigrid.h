@@ -97,10 +97,22 @@ void mg_cholesky(double* D, int nc, int* fail, cudaStream_t s);
 // positive.
 double* mg_dense_start(int nc, double* a, double* inv);
 void mg_dense_inverse(int nc, double* a, double* inv, double* pivot, int* fail, cudaStream_t s);
-// x = Ainv b over the compact numbering (cidx: dof -> compact, cdof: compact -> dof).
+// x = Ainv b over the compact numbering (cidx: dof -> compact, cdof: compact -> dof;
+// both null: the level's own).
 template <class T>
 void mg_coarse_inv_apply(const double* Ainv, int nc, const int* cidx, const int* cdof,
                          int64_t ndof, const T* b, T* x, cudaStream_t s);
+// The last smoothed level's V-cycle (smoothing, transfers, coarsest solve with Ainv)
+// as a dense matrix over its DOFs, row-major in M: up to kDenseCycleDof DOFs, if the
+// build's vectors fit in shared memory.  Applied by mg_coarse_inv_apply with null
+// index maps.
+constexpr int64_t kDenseCycleDof = 7 * 152;
+bool mg_dense_cycle_fits(int64_t ndof, int nc, bool cheb);
+template <class T>
+void mg_dense_cycle(const MgDims& d, const MgDims& cd, const T* A, const uint8_t* act,
+                    const T* dinv, const float* coef, int cheb_m, int sweeps, T omega,
+                    const double* Ainv, int nc, const int* cidx, const int* cdof, double* M,
+                    cudaStream_t s);
 template <class T>
 void mg_chol_solve(const double* L, int nc, const int* cidx, int64_t ndof, const T* b, T* x,
                    double* work, cudaStream_t s);
@@ -108,7 +120,8 @@ void mg_chol_solve(const double* L, int nc, const int* cidx, int64_t ndof, const
 // The small levels of the FP32 V-cycle in one launch of one thread-block cluster
 // (k_multigrid.cu).  L[0] is the first fused level (its right-hand side b set by
 // the finer level's restriction), L[nlev-1] the coarsest (solved with the dense
-// inverse Ainv over the compact numbering cidx/cdof).  Each smoothed level has
+// inverse Ainv over the compact numbering cidx/cdof) or the level whose cycle is a
+// dense matrix (Ainv, with null index maps).  Each smoothed level has
 // two iterate buffers: xp (the iterate on entry, as the launch-by-launch
 // V-cycle's X) and xq; smoothing is Chebyshev of degree cheb_m (> 0, direction
 // chd, coefficient table coef on the device) or damped Jacobi with `sweeps` sweeps per

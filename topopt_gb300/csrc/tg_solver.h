@@ -149,6 +149,9 @@ class Solver {
   int nc_ = 0;
   DBuf<int> cidx_, cdof_, chol_fail_;
   DBuf<double> chol_, chol_work_, gj_pivot_, chol_inv_;
+  // The last smoothed level's V-cycle as a dense matrix (0: none).
+  size_t dense_level_ = 0;
+  DBuf<double> dense_;
   // The PCG loops (mixed inner, FP64 multigrid, FP64 Jacobi) as one CUDA graph
   // each: a conditional WHILE node whose body is one iteration and whose last
   // kernel decides, on the device, whether another one runs.
