@@ -443,12 +443,13 @@ __global__ void __launch_bounds__(kStencilThreads) k_stencil_op(MgDims d, const 
 // before the row's, so they overlap.
 constexpr int kSplitThreads = 384;
 // Up to here the four threads win.  FP32, bound by memory latency: 3.1-3.6 us
-// against 6.4-7.5 on 225 to 9,537 nodes, 14.8 against 14.1 on 70,785.  FP64, bound
+// against 6.4-7.5 on 225 to 9,537 nodes, 10.3 both on 30,625, 14.8 against 14.1 on
+// 70,785.  FP64, bound
 // by its units: 7-10 us against 21 on 225 to 4,225 nodes, 19-26 against 30 on
 // 30,625.
 template <class T>
 constexpr int64_t split_max_nodes() {
-  return sizeof(T) == 8 ? 100000 : 16384;
+  return sizeof(T) == 8 ? 100000 : 32768;
 }
 
 template <class T, int MODE>

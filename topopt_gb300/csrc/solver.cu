@@ -36,6 +36,12 @@ const double kXi[8] = {-1, +1, +1, -1, -1, +1, +1, -1};
 const double kEta[8] = {-1, -1, +1, +1, -1, -1, +1, +1};
 const double kZeta[8] = {-1, -1, -1, -1, +1, +1, +1, +1};
 constexpr int kMaxCoarseDof = 8192;   // dense coarsest factor <= 512 MB
+// Level 1 of the FP32 V-cycle is applied from its assembled stencil up to here and
+// matrix-free above.  The stencil is one launch that reads 1 KB a node from the L2, the
+// matrix-free form two with little to read: 6.2 against 10.3 us on 3,751 to 9,537
+// nodes, 10.3 against 12.3 on 30,625, 14.7 against 14.4 on 43,904, 17.1 against 15.2
+// on 70,785, 177 against 41 on 545,025.
+constexpr int64_t kLevel1AssembledNodes = 32768;
 constexpr int kMaxInverseDof = 512;   // explicit coarsest inverse up to here
 constexpr int64_t kAutotuneMinVoxels = int64_t(1) << 20;  // FP32 schedule measured from here
 
@@ -553,6 +559,7 @@ void Solver::build_structure() {
   TG_CUDA(cudaMemcpyAsync(kebf_.p, kbf.data(), kebf_.bytes(), cudaMemcpyHostToDevice, s_));
   TG_CUDA(cudaMemcpyAsync(Gf_.p, Gf.data(), Gf_.bytes(), cudaMemcpyHostToDevice, s_));
   l1_mf_ = mixed_ && level1_matfree_enabled();
+  l1_assembled_ = !l1_mf_ || dense_level_ == 1 || levels_[0]->nn <= kLevel1AssembledNodes;
   if (l1_mf_) {
     // Coarse elements of level 1 off the sum_c E_c G_c fast path.
     const Level& L1 = *levels_[0];
@@ -820,9 +827,10 @@ bool Solver::build_numeric() {
                             slist1_.p, nspec1_);
     else
       mg_galerkin_coarse<T>(pd, L.d, levels_[l - 1]->Ke<T>(), L.act.p, L.Ke<T>(), s_);
-    // The matrix-free level 1 needs only its inverse diagonal; the assembled
-    // stencil (275 MB on the 256x128x128 cantilever) is formed on demand (level1_stencil()).
-    const bool diag_only = sizeof(T) == 4 && l == 0 && l1_mf_ && dense_level_ != 1;
+    // The matrix-free level 1 needs only its inverse diagonal; where the V-cycle
+    // applies it, the assembled stencil (275 MB on the 256x128x128 cantilever) is
+    // formed on demand (level1_stencil()).
+    const bool diag_only = sizeof(T) == 4 && l == 0 && !l1_assembled_;
     mg_assemble_stencil<T>(L.d, L.Ke<T>(), L.act.p, diag_only ? nullptr : L.Am<T>(), L.Dinv<T>(),
                            s_);
     if (sizeof(T) == 4 && l == 0) l1_stencil_ok_ = !diag_only;
@@ -994,7 +1002,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
   const T w = T(omega_);
   auto op = [&](int mode) {
     if constexpr (sizeof(T) == 4) {
-      if (l == 1 && l1_mf_) {
+      if (l == 1 && !l1_assembled_) {
         level1_op(mode, L, float(w));
         return;
       }

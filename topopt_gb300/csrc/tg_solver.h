@@ -158,11 +158,12 @@ class Solver {
   std::unique_ptr<LoopGraph> ig_, ig64_, igj_;
   bool graph_failed_ = false, use_graph_ = true;
   DBuf<int> istate_;           // [0] iterations done, [1] budget, [2] breakdown
-  // Level 1 of the FP32 V-cycle without its matrix: the coarse elements whose
-  // matrix is not the children's sum (a Dirichlet or untouched fine DOF in a
-  // solid child, an inactive coarse DOF or a half element), applied from their
-  // stored matrices; the level's activity as 3 bits per node.
-  bool l1_mf_ = false;
+  // Level 1 of the FP32 V-cycle without its matrix (l1_mf_: prepared; used unless
+  // l1_assembled_): the coarse elements whose matrix is not the children's sum (a
+  // Dirichlet or untouched fine DOF in a solid child, an inactive coarse DOF or a
+  // half element), applied from their stored matrices; the level's activity as 3
+  // bits per node.
+  bool l1_mf_ = false, l1_assembled_ = true;
   int nspec1_ = 0;
   DBuf<int> spos1_, slist1_;  // per coarse element: position in slist1_ or -1
   DBuf<float> yspec1_;        // their outputs, nspec1_ x 24
