@@ -228,6 +228,12 @@ __global__ void k_axpy_scaled_f2d(double* __restrict__ y, const float* __restric
     y[i] += sc * double(x[i]);
 }
 
+__global__ void k_scatter(double* __restrict__ v, const int64_t* __restrict__ at,
+                          const double* __restrict__ val, int64_t n) {
+  const int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x;
+  if (i < n) v[at[i]] = val[i];
+}
+
 template <class T>
 __global__ void k_fill(T* __restrict__ a, T v, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
@@ -395,6 +401,10 @@ void launch_axpy_scaled_f2d(double* y, const float* x, const double* nrm2, int64
 template <class T>
 void launch_fill(T* a, T v, int64_t n, cudaStream_t s) {
   k_fill<T><<<stream_blocks(n), kThreads, 0, s>>>(a, v, n);
+  TG_LAUNCH_CHECK();
+}
+void launch_scatter(double* v, const int64_t* at, const double* val, int64_t n, cudaStream_t s) {
+  k_scatter<<<unsigned((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(v, at, val, n);
   TG_LAUNCH_CHECK();
 }
 template void launch_fill<double>(double*, double, int64_t, cudaStream_t);

@@ -282,6 +282,8 @@ void launch_axpy_scaled_f2d(double* y, const float* x, const double* nrm2, int64
                             cudaStream_t s);
 template <class T>
 void launch_fill(T* a, T v, int64_t n, cudaStream_t s);
+// v[at[i]] = val[i], i < n (distinct places).
+void launch_scatter(double* v, const int64_t* at, const double* val, int64_t n, cudaStream_t s);
 void launch_copy_d2f(float* dst, const double* src, int64_t n, cudaStream_t s);
 void launch_axpy_f2d(double* y, const float* x, int64_t n, cudaStream_t s);
 void launch_sub_mask(double* r, const double* b, const double* ax, const uint8_t* kept, int64_t n,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "tg_internal.h"
@@ -24,9 +25,10 @@ struct FineProblem {
   std::vector<uint8_t> elem_h;     // element exists (solid and active) [nv]
   std::vector<uint8_t> kept_h;     // [ndof]
   std::vector<uint8_t> kept_node_h;  // [nnodes] kept bits per node (bit k: DOF 3n+k)
-  std::vector<double> f_h;         // load vector [ndof]
-  std::vector<double> up_h;        // prescribed field [ndof]
-  std::vector<uint8_t> fixed_h;    // Dirichlet mask [ndof]
+  std::vector<uint8_t> fixed_node_h;  // [nnodes] Dirichlet bits per node
+  // The load vector's and the prescribed field's entries, one per DOF.
+  std::vector<std::pair<int64_t, double>> f_entries, up_entries;
+  bool fixed(int64_t dof) const { return (fixed_node_h[size_t(dof / 3)] >> (dof % 3)) & 1; }
   bool nonzero_bc = false;
   int64_t ng = 0, n_free = 0;
   DBuf<uint8_t> elem, kept, kept_node;
