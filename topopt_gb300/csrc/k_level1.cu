@@ -34,6 +34,7 @@
 #include <atomic>
 
 #include "tg_internal.h"
+#include "tg_launch.h"
 #include "tg_march.h"
 #include "tg_multigrid.h"
 
@@ -140,10 +141,11 @@ __device__ __forceinline__ void parent_stress(const ModalT<float>& mc, const flo
 template <int MODE>
 __global__ void __launch_bounds__(32 * kMaxWarps, 1)
     k_level1_march(MgDims fd, MgDims cd, ModalT<float> mc, int KZ, int nss,
-                   const float* __restrict__ ef, const uint8_t* __restrict__ an,
-                   const int* __restrict__ spos, const float* __restrict__ yspec,
-                   const float* __restrict__ x, const float* __restrict__ b,
-                   const float* __restrict__ invdiag, float omega, float* __restrict__ y) {
+                   const float* ef, const uint8_t* __restrict__ an,
+                   const int* __restrict__ spos, const float* yspec,
+                   const float* x, const float* b,
+                   const float* invdiag, float omega, float* __restrict__ y) {
+  let_next_start();
   extern __shared__ __align__(16) unsigned char l1_smem[];
   float* const xs = reinterpret_cast<float*>(l1_smem);  // [2][W][6][32]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
     }
   }
   const unsigned so = ev ? 4u * unsigned(ey * cd.ex + ex) : 0u;
+  wait_for_previous();
   // Step s: node layer ez + 1 of x, everything else of layer ez.
   auto copy_step = [&](int s) {
     const int ez = z0 - 1 + s;
@@ -361,8 +364,9 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
 __global__ void __launch_bounds__(256) k_level1_special(MgDims cd, int nspec,
                                                         const int* __restrict__ list,
                                                         const float* __restrict__ Kel,
-                                                        const float* __restrict__ x,
+                                                        const float* x,
                                                         float* __restrict__ yspec) {
+  behind_previous();
   const int lane = threadIdx.x & 31;
   const int p = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (p >= nspec) return;
@@ -437,8 +441,8 @@ void launch(const Tile& t, const MgDims& fd, const MgDims& cd, const ModalConsts
     done.store(true);
   }
   const int nss = (cd.nny + t.W - 2) / (t.W - 1);
-  k_level1_march<MODE><<<tile_grid(cd, t), 32 * t.W, t.W * per_warp, s>>>(
-      fd, cd, to_modal<float>(c), t.kz, nss, ef, an, spos, yspec, x, b, invdiag, omega, y);
+  launch_behind(k_level1_march<MODE>, tile_grid(cd, t), 32 * t.W, t.W * per_warp, s, fd, cd,
+                to_modal<float>(c), t.kz, nss, ef, an, spos, yspec, x, b, invdiag, omega, y);
   TG_LAUNCH_CHECK();
 }
 
@@ -449,7 +453,7 @@ void mg_level1_op(int mode, const MgDims& fd, const MgDims& cd, const ModalConst
                   int nspec, const float* Kel, const float* x, const float* b,
                   const float* invdiag, float omega, float* y, float* yspec, cudaStream_t s) {
   if (nspec > 0) {
-    k_level1_special<<<(nspec + 7) / 8, 256, 0, s>>>(cd, nspec, slist, Kel, x, yspec);
+    launch_behind(k_level1_special, (nspec + 7) / 8, 256, 0, s, cd, nspec, slist, Kel, x, yspec);
     TG_LAUNCH_CHECK();
   }
   const int* sp = nspec > 0 ? spos : nullptr;

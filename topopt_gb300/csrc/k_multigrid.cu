@@ -28,6 +28,7 @@
 
 #include "tg_df.h"
 #include "tg_internal.h"
+#include "tg_launch.h"
 #include "tg_multigrid.h"
 
 #include <algorithm>
@@ -326,43 +327,64 @@ __device__ __forceinline__ double add_block(double s, double a0, double x0, doub
   return on ? t : s;
 }
 
-// Part `part` (0..3) of row r of node (a, bb, c) of a stored symmetric stencil
-// times x.  The row is the self block (term 0) plus, for j = 1..13, forward
-// block j (neighbour n + off_j) and the transposed forward block of neighbour
-// n - off_j; part q accumulates the terms j = q, q + 4, ... in increasing j (part
-// 0 starts from the self term), and the row is ((p0 + p1) + p2) + p3.  Four
-// parts let four threads share a row on the small levels, where a row's ~160
-// loads in one thread are a chain of dependent memory round trips -- and, in
-// FP64, its 81 multiply-adds a chain of 64 cycles each.
-template <class T, bool COH>
-__device__ __forceinline__ T stencil_part(const MgDims& d, const T* __restrict__ A, const T* x,
-                                          int a, int bb, int c, int r, int part) {
+// The matrix entries of a part and the nodes that they meet (n itself beyond the grid);
+// slot t is block j = 4 t + part (block 0, the self block, has no transposed partner).
+template <class T>
+struct StencilPart {
+  T f[4][3], b[4][3];
+  int m[4], p[4];
+  bool fin[4], bin[4];
+};
+template <class T>
+__device__ __forceinline__ void stencil_entries(const MgDims& d, const T* __restrict__ A, int a,
+                                                int bb, int c, int r, int part,
+                                                StencilPart<T>& w) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
-  const int64_t sy = d.nnx, sz = int64_t(d.nnx) * d.nny;
-  const int64_t n = c * sz + bb * sy + a;
+  const int sy = d.nnx, sz = d.nnx * d.nny, n = c * sz + bb * sy + a;
   const T* An = A + n + int64_t(3 * r) * nn;  // row r of the self block
-  T s = T(0);
-  if (part == 0)
-    s = add_block(T(0), An[0], vload<T, COH>(x + 3 * n), An[nn], vload<T, COH>(x + 3 * n + 1),
-                  An[2 * nn], vload<T, COH>(x + 3 * n + 2), true);
 #pragma unroll
-  for (int j = 1; j < 14; ++j) {
-    if ((j & 3) != part) continue;
+  for (int t = 0; t < 4; ++t) {
+    const int j = 4 * t + part;
+    if (j >= 14) continue;
     const int di = 13 + j;
     const int dx = di % 3 - 1, dy = (di / 3) % 3 - 1, dz = di / 9 - 1;
-    const int64_t off = dz * sz + dy * sy + dx;
-    const bool fin = (a + dx) < d.nnx && (a + dx) >= 0 && (bb + dy) < d.nny && (bb + dy) >= 0 &&
-                     (c + dz) < d.nnz;
-    const bool bin = (a - dx) >= 0 && (a - dx) < d.nnx && (bb - dy) >= 0 && (bb - dy) < d.nny &&
-                     (c - dz) >= 0;
-    const int64_t m = fin ? n + off : n;
-    const int64_t p = bin ? n - off : n;
+    const int off = dz * sz + dy * sy + dx;
+    w.fin[t] = (a + dx) < d.nnx && (a + dx) >= 0 && (bb + dy) < d.nny && (bb + dy) >= 0 &&
+               (c + dz) < d.nnz;
+    w.bin[t] = j > 0 && (a - dx) >= 0 && (a - dx) < d.nnx && (bb - dy) >= 0 &&
+               (bb - dy) < d.nny && (c - dz) >= 0;
+    w.m[t] = w.fin[t] ? n + off : n;
+    w.p[t] = w.bin[t] ? n - off : n;
     const T* Af = An + int64_t(j * 9) * nn;
-    const T* Ab = A + int64_t(j * 9 + r) * nn + p;
-    s = add_block(s, Af[0], vload<T, COH>(x + 3 * m), Af[nn], vload<T, COH>(x + 3 * m + 1),
-                  Af[2 * nn], vload<T, COH>(x + 3 * m + 2), fin);
-    s = add_block(s, Ab[0], vload<T, COH>(x + 3 * p), Ab[3 * nn], vload<T, COH>(x + 3 * p + 1),
-                  Ab[6 * nn], vload<T, COH>(x + 3 * p + 2), bin);
+    const T* Ab = A + int64_t(j * 9 + r) * nn + w.p[t];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      w.f[t][e] = Af[e * nn];
+      w.b[t][e] = Ab[3 * e * nn];
+    }
+  }
+}
+
+// Part `part` (0..3) of row r of a node of a stored symmetric stencil times x.  The row
+// is the self block (term 0) plus, for j = 1..13, forward block j (neighbour n + off_j)
+// and the transposed forward block of neighbour n - off_j; part q accumulates the terms
+// j = q, q + 4, ... in increasing j, and the row is ((p0 + p1) + p2) + p3.  Four parts
+// let four threads share a row on the small levels, where a row's ~160 loads in one
+// thread are a chain of dependent memory round trips -- and, in FP64, its 81
+// multiply-adds a chain of 64 cycles each.
+template <class T, bool COH>
+__device__ __forceinline__ T stencil_part(const StencilPart<T>& w, int part, const T* x) {
+  T s = T(0);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const int j = 4 * t + part;
+    if (j >= 14) continue;
+    const T *xm = x + 3 * int64_t(w.m[t]), *xp = x + 3 * int64_t(w.p[t]);
+    s = add_block(s, w.f[t][0], vload<T, COH>(xm), w.f[t][1], vload<T, COH>(xm + 1), w.f[t][2],
+                  vload<T, COH>(xm + 2), w.fin[t]);
+    if (j > 0)
+      s = add_block(s, w.b[t][0], vload<T, COH>(xp), w.b[t][1], vload<T, COH>(xp + 1), w.b[t][2],
+                    vload<T, COH>(xp + 2), w.bin[t]);
   }
   return s;
 }
@@ -373,7 +395,11 @@ __device__ __forceinline__ T stencil_row(const MgDims& d, const T* __restrict__ 
                                          int a, int bb, int c, int r) {
   T p[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) p[q] = stencil_part<T, COH>(d, A, x, a, bb, c, r, q);
+  for (int q = 0; q < 4; ++q) {
+    StencilPart<T> w;
+    stencil_entries(d, A, a, bb, c, r, q, w);
+    p[q] = stencil_part<T, COH>(w, q, x);
+  }
   return ((p[0] + p[1]) + p[2]) + p[3];
 }
 
@@ -408,10 +434,11 @@ constexpr int kStencilThreads = 192;
 template <class T, int MODE>
 __global__ void __launch_bounds__(kStencilThreads) k_stencil_op(MgDims d, const T* __restrict__ A,
                                                     const uint8_t* __restrict__ act,
-                                                    const T* __restrict__ x,
-                                                    const T* __restrict__ b,
+                                                    const T* x,
+                                                    const T* b,
                                                     const T* __restrict__ invdiag, T omega,
                                                     T* __restrict__ y, ChebStep ch) {
+  behind_previous();
   // 192 threads: two chunks of 32 consecutive nodes (in x-fastest order, across
   // row ends) x 3 components, one component per warp, so a warp's stencil and
   // vector reads are coalesced and no lane idles at the odd row lengths
@@ -439,25 +466,28 @@ __global__ void __launch_bounds__(kStencilThreads) k_stencil_op(MgDims d, const 
 // The stencil kernels on small levels: four threads per (node, row), one
 // part of the row each (stencil_part), combined in shared memory in the order
 // stencil_row uses, so both kernels give the same bits.  384 threads: 32
-// consecutive nodes x 3 rows x 4 parts.  The update's vector reads are issued
-// before the row's, so they overlap.
+// consecutive nodes x 3 rows x 4 parts.  A launch is a chain of round trips to the L2:
+// the matrix entries are read before the wait for the previous kernel, so that behind
+// it only the vectors' remain (24 launches of a 128x64x64 iteration: 224 -> 204 us
+// with the other kernels of the chain launched that way too).
 constexpr int kSplitThreads = 384;
-// Up to here the four threads win.  FP32, bound by memory latency: 3.1-3.6 us
-// against 6.4-7.5 on 225 to 9,537 nodes, 10.3 both on 30,625, 14.8 against 14.1 on
-// 70,785.  FP64, bound
-// by its units: 7-10 us against 21 on 225 to 4,225 nodes, 19-26 against 30 on
-// 30,625.
+// Up to here the four threads win.  FP32, bound by memory latency (a solve of many
+// steps, launched behind one another): 2.4-3.6 us against 6.4-7.5 on 225 to 9,537 nodes,
+// 14.4 against 15.0 ms for a solve whose level 1 has 26,400, 12.3 against 10.4 us on
+// 30,625.  FP64, bound by its units: 7-10 us against 21 on 225 to 4,225 nodes, 19-26
+// against 30 on 30,625.
 template <class T>
 constexpr int64_t split_max_nodes() {
-  return sizeof(T) == 8 ? 100000 : 32768;
+  return sizeof(T) == 8 ? 100000 : 28672;
 }
 
 template <class T, int MODE>
-__global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
+__global__ void __launch_bounds__(kSplitThreads, 2) k_stencil_split(
     MgDims d, const T* __restrict__ A, const uint8_t* __restrict__ act,
-    const T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ invdiag,
+    const T* x, const T* b, const T* __restrict__ invdiag,
     T omega, T* __restrict__ y, ChebStep ch) {
   __shared__ T parts[3][3][32];
+  let_next_start();
   const int t = threadIdx.x, q = t / 96, r = (t / 32) % 3, lane = t & 31;
   const int64_t n = int64_t(blockIdx.x) * 32 + lane;
   const bool valid = n < int64_t(d.nnx) * d.nny * d.nnz;
@@ -465,19 +495,23 @@ __global__ void __launch_bounds__(kSplitThreads) k_stencil_split(
   T* dir = static_cast<T*>(ch.dir_);
   bool ac = false;
   T xv = T(0), bv = T(0), dv = T(0), dprev = T(0);
-  if (q == 0 && valid) {
-    ac = act[dof] != 0;
-    if (MODE == kSmooth || MODE == kCheb) xv = x[dof];
-    if (MODE != kApply && MODE != kDinvA) bv = b[dof];
-    if (MODE == kSmooth || MODE == kCheb || MODE == kDinvA) dv = invdiag[dof];
-    if (MODE == kCheb && ch.step > 0) dprev = dir[dof];
-  }
-  T p = T(0);
+  StencilPart<T> w;
   if (valid) {
     int a, bb, c;
     node_abc(d, n, a, bb, c);
-    p = stencil_part<T, false>(d, A, x, a, bb, c, r, q);
+    stencil_entries(d, A, a, bb, c, r, q, w);
+    if (q == 0) {
+      ac = act[dof] != 0;
+      if (MODE == kSmooth || MODE == kCheb || MODE == kDinvA) dv = invdiag[dof];
+    }
   }
+  wait_for_previous();
+  if (q == 0 && valid) {
+    if (MODE == kSmooth || MODE == kCheb) xv = x[dof];
+    if (MODE != kApply && MODE != kDinvA) bv = b[dof];
+    if (MODE == kCheb && ch.step > 0) dprev = dir[dof];
+  }
+  const T p = valid ? stencil_part<T, false>(w, q, x) : T(0);
   if (q > 0) parts[q - 1][r][lane] = p;
   __syncthreads();
   if (q != 0 || !valid) return;
@@ -650,16 +684,18 @@ constexpr int kRestrictThreads = 128;
 // step from zero.
 template <class T>
 __global__ void __launch_bounds__(kRestrictThreads) k_restrict(MgDims fd, MgDims cd, RowDiv rd,
-                                                               const T* __restrict__ rf,
+                                                               const T* rf,
                                                                const uint8_t* __restrict__ cact,
                                                                T* __restrict__ bc,
                                                                FirstStep<T> first) {
+  let_next_start();
   const unsigned id = blockIdx.x * unsigned(kRestrictThreads) + threadIdx.x;
   const int c = blockIdx.y;
   if (id >= rd.len * unsigned(cd.nny)) return;
   const int b = int(row_of(rd, id)), e = int(id - unsigned(b) * rd.len), a = e / 3, k = e - 3 * a;
   const int64_t dof = int64_t(c) * rd.len * cd.nny + id;
   const bool ac = cact[dof] != 0;
+  wait_for_previous();
   const T s = restrict_dof<T, false>(fd, cd, rf, a, b, c, k);
   const T bv = ac ? s : T(0);
   bc[dof] = bv;
@@ -678,16 +714,18 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(MgDims fd, MgDims
 // took 79 us against 33 on 257x129x129 nodes.
 template <class T>
 __global__ void __launch_bounds__(256) k_prolong_add(MgDims fd, MgDims cd,
-                                                     const T* __restrict__ ec,
+                                                     const T* ec,
                                                      const uint8_t* __restrict__ fact,
-                                                     T* __restrict__ xf) {
+                                                     T* xf) {
+  let_next_start();
   const int a = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y * 8 + threadIdx.y, c = blockIdx.z;
   if (a >= fd.nnx || b >= fd.nny) return;
   const int64_t n = (int64_t(c) * fd.nny + b) * fd.nnx + a;
   // The iterate and the mask are read unconditionally, in parallel with the
   // coarse values: a read under the mask's branch would wait for the mask first.
-  const T x0 = xf[3 * n], x1 = xf[3 * n + 1], x2 = xf[3 * n + 2];
   const bool f0 = fact[3 * n] != 0, f1 = fact[3 * n + 1] != 0, f2 = fact[3 * n + 2] != 0;
+  wait_for_previous();
+  const T x0 = xf[3 * n], x1 = xf[3 * n + 1], x2 = xf[3 * n + 2];
   T s[3];
   prolong_node<T, false>(fd, cd, ec, a, b, c, s);
   if (f0) xf[3 * n] = x0 + s[0];
@@ -897,14 +935,28 @@ __device__ __forceinline__ double widen(float v) {
 // vector (cidx and cdof null: Ainv is over the level's own numbering); one warp per
 // row of Ainv.  Each lane's products are one chain of FP64 multiply-adds, 64 cycles
 // a link on its scheduler, so a warp takes one row and the rows are spread over all
-// SMs; the matrix comes from the L2, eight loads ahead of the chain.
+// SMs.
 constexpr int kRowWarps = 4;
 template <class T>
 __global__ void __launch_bounds__(32 * kRowWarps) k_coarse_inv_apply(
     const double* __restrict__ Ainv, int nc, const int* __restrict__ cidx,
-    const int* __restrict__ cdof, int64_t ndof, const T* __restrict__ b, T* __restrict__ x) {
+    const int* __restrict__ cdof, int64_t ndof, const T* b, T* __restrict__ x) {
+  let_next_start();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  // The matrix is read kAhead entries a lane at a time, those of the warp's first row
+  // before the previous kernel has ended.
+  constexpr int kAhead = 12;
+  double m[kAhead];
+  auto fetch = [&](const double* row, int k0) {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const int k = k0 + 32 * i;
+      m[i] = k < nc ? row[k] : 0.0;
+    }
+  };
+  if (warp < nc) fetch(Ainv + int64_t(warp) * nc, lane);
+  wait_for_previous();
   if (cidx != nullptr)
     for (int64_t dd = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; dd < ndof;
          dd += int64_t(gridDim.x) * blockDim.x)
@@ -912,8 +964,14 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_coarse_inv_apply(
   for (int r = warp; r < nc; r += nwarps) {
     const double* row = Ainv + int64_t(r) * nc;
     double s = 0.0;
-#pragma unroll 8
-    for (int k = lane; k < nc; k += 32) s += row[k] * widen(b[cdof != nullptr ? cdof[k] : k]);
+    for (int k0 = lane; k0 < nc; k0 += 32 * kAhead) {
+      if (r != warp || k0 != lane) fetch(row, k0);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int k = k0 + 32 * i;
+        if (k < nc) s += m[i] * widen(b[cdof != nullptr ? cdof[k] : k]);
+      }
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) x[cdof != nullptr ? cdof[r] : r] = T(s);
@@ -1059,42 +1117,32 @@ void mg_to_float(const double* src, float* dst, int64_t n, cudaStream_t s) {
 template <class T>
 void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, const T* x,
                    const T* b, const T* invdiag, T omega, T* y, cudaStream_t s,
-                   ChebStep ch) {
+                   ChebStep ch, bool settled) {
   const int64_t nn = int64_t(d.nnx) * d.nny * d.nnz;
-  if (nn <= split_max_nodes<T>()) {
-    const unsigned ns = unsigned((nn + 31) / 32);
-    if (mode == kApply)
-      k_stencil_split<T, kApply><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
-                                                              ch);
-    else if (mode == kResidual)
-      k_stencil_split<T, kResidual><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega,
-                                                                 y, ch);
-    else if (mode == kDinvA)
-      k_stencil_split<T, kDinvA><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
-                                                              ch);
-    else if (mode == kCheb)
-      k_stencil_split<T, kCheb><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
-                                                             ch);
+  auto run = [&](auto kernel, unsigned blocks, int threads) {
+    if (settled)
+      launch_behind_if_spread<T>(kernel, blocks, threads, 0, s, d, A, act, x, b, invdiag, omega, y,
+                                 ch);
     else
-      k_stencil_split<T, kSmooth><<<ns, kSplitThreads, 0, s>>>(d, A, act, x, b, invdiag, omega, y,
-                                                               ch);
+      kernel<<<blocks, threads, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
     TG_LAUNCH_CHECK();
-    return;
+  };
+  auto pick = [&](auto m) {
+    constexpr int MODE = decltype(m)::value;
+    if (nn <= split_max_nodes<T>())
+      run(k_stencil_split<T, MODE>, unsigned((nn + 31) / 32), kSplitThreads);
+    else
+      run(k_stencil_op<T, MODE>,
+          unsigned(((nn + 31) / 32 * 96 + kStencilThreads - 1) / kStencilThreads),
+          kStencilThreads);
+  };
+  switch (mode) {
+    case kApply: pick(std::integral_constant<int, kApply>{}); break;
+    case kResidual: pick(std::integral_constant<int, kResidual>{}); break;
+    case kDinvA: pick(std::integral_constant<int, kDinvA>{}); break;
+    case kCheb: pick(std::integral_constant<int, kCheb>{}); break;
+    default: pick(std::integral_constant<int, kSmooth>{});
   }
-  const int64_t items = (nn + 31) / 32 * 96;
-  const unsigned nb = unsigned((items + kStencilThreads - 1) / kStencilThreads);
-  const unsigned nt = kStencilThreads;
-  if (mode == kApply)
-    k_stencil_op<T, kApply><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-  else if (mode == kResidual)
-    k_stencil_op<T, kResidual><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-  else if (mode == kDinvA)
-    k_stencil_op<T, kDinvA><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-  else if (mode == kCheb)
-    k_stencil_op<T, kCheb><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-  else
-    k_stencil_op<T, kSmooth><<<nb, nt, 0, s>>>(d, A, act, x, b, invdiag, omega, y, ch);
-  TG_LAUNCH_CHECK();
 }
 
 void mg_cheb_table(const double* lam, double ratio, int m, float* coef, cudaStream_t s) {
@@ -1129,15 +1177,19 @@ template <class T>
 void mg_restrict(const MgDims& fd, const MgDims& cd, const T* rf, const uint8_t* cact, T* bc,
                  cudaStream_t s, FirstStep<T> first) {
   const dim3 grid((3 * cd.nnx * cd.nny + kRestrictThreads - 1) / kRestrictThreads, cd.nnz);
-  k_restrict<T><<<grid, kRestrictThreads, 0, s>>>(fd, cd, row_div(cd.nnx), rf, cact, bc, first);
+  launch_behind_if_spread<T>(k_restrict<T>, grid, kRestrictThreads, 0, s, fd, cd, row_div(cd.nnx),
+                             rf, cact, bc, first);
   TG_LAUNCH_CHECK();
 }
 
 template <class T>
 void mg_prolong_add(const MgDims& fd, const MgDims& cd, const T* ec, const uint8_t* fact, T* xf,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool joined) {
   const dim3 grid((fd.nnx + 31) / 32, (fd.nny + 7) / 8, fd.nnz);
-  k_prolong_add<T><<<grid, dim3(32, 8), 0, s>>>(fd, cd, ec, fact, xf);
+  if (joined)
+    k_prolong_add<T><<<grid, dim3(32, 8), 0, s>>>(fd, cd, ec, fact, xf);
+  else
+    launch_behind_if_spread<T>(k_prolong_add<T>, grid, dim3(32, 8), 0, s, fd, cd, ec, fact, xf);
   TG_LAUNCH_CHECK();
 }
 
@@ -1185,7 +1237,8 @@ template <class T>
 void mg_coarse_inv_apply(const double* Ainv, int nc, const int* cidx, const int* cdof,
                          int64_t ndof, const T* b, T* x, cudaStream_t s) {
   const int nb = std::max(1, std::min(152 * 4, (nc + kRowWarps - 1) / kRowWarps));
-  k_coarse_inv_apply<T><<<nb, 32 * kRowWarps, 0, s>>>(Ainv, nc, cidx, cdof, ndof, b, x);
+  launch_behind_if_spread<double>(k_coarse_inv_apply<T>, nb, 32 * kRowWarps, 0, s, Ainv, nc, cidx,
+                                  cdof, ndof, b, x);
   TG_LAUNCH_CHECK();
 }
 
@@ -1450,12 +1503,12 @@ void mg_dense_cycle(const MgDims& d, const MgDims& cd, const T* A, const uint8_t
                                   const T*, const float*, int, int, T, const double*, int,    \
                                   const int*, const int*, double*, cudaStream_t);             \
   template void mg_stencil_op<T>(int, const MgDims&, const T*, const uint8_t*, const T*,      \
-                                 const T*, const T*, T, T*, cudaStream_t, ChebStep);          \
+                                 const T*, const T*, T, T*, cudaStream_t, ChebStep, bool);    \
   template void mg_jacobi_first<T>(const T*, const T*, T, int64_t, T*, cudaStream_t);         \
   template void mg_restrict<T>(const MgDims&, const MgDims&, const T*, const uint8_t*, T*,    \
                                cudaStream_t, FirstStep<T>);                                   \
   template void mg_prolong_add<T>(const MgDims&, const MgDims&, const T*, const uint8_t*, T*, \
-                                  cudaStream_t);                                              \
+                                  cudaStream_t, bool);                                        \
   template void mg_chol_solve<T>(const double*, int, const int*, int64_t, const T*, T*,       \
                                  double*, cudaStream_t);                                      \
   template void mg_coarse_inv_apply<T>(const double*, int, const int*, const int*, int64_t,    \

@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "tg_internal.h"
+#include "tg_launch.h"
 #include "tg_march.h"
 #include "tg_reduce.h"
 
@@ -137,10 +138,11 @@ __host__ __device__ constexpr int slot_words() {
 template <class V, class T, int MODE, bool PER>
 __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
     k_fine_march(GridDev g, ModalT<typename RowsOf<V>::S> mc, int KZ, int nss,
-                 const T* __restrict__ ef, const uint8_t* __restrict__ kn,
-                 const T* __restrict__ x, const T* __restrict__ b, const T* __restrict__ invdiag,
+                 const T* ef, const uint8_t* __restrict__ kn,
+                 const T* x, const T* b, const T* invdiag,
                  T omega, T* __restrict__ y, SumOut dot, int guard,
                  BatchDev bd) {
+  let_next_start();
   using S = typename RowsOf<V>::S;
   constexpr int R = RowsOf<V>::R;
   constexpr bool kXtra = !PER && std::is_same<S, double>::value;  // lane 31 loads its neighbour
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
   const int rows = W * R - 1;
   if constexpr (PER) {
+    wait_for_previous();
     const int bi = blockIdx.z, cell = bi / bd.nrhs;
     if (bd.run != nullptr && bd.run[bi] != 1) return;  // uniform over the CTA
     x += bi * bd.sx;
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
       }
     }
   }
+  if constexpr (!PER) wait_for_previous();
   // The copies of step s: node layer ez + 1, factors, b and diagonal of layer ez.
   auto copy_step = [&](int s) {
     if constexpr (kPipe) {
@@ -634,8 +638,13 @@ void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalCo
   // Only the public apply takes values at nodes of absent elements; within the
   // solver (a kept mask) they are zeros.
   const int guard = kn == nullptr ? 1 : 0;
-  k_fine_march<V, T, MODE, PER><<<grid, 32 * t.W, smem, s>>>(
-      gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b, invdiag, omega, y, dot, guard, bd);
+  auto kernel = k_fine_march<V, T, MODE, PER>;
+  if constexpr (sizeof(T) == 4)
+    launch_behind(kernel, grid, 32 * t.W, smem, s, gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b,
+                  invdiag, omega, y, dot, guard, bd);
+  else  // the SMs' FP64 units (or double-float arithmetic) bound it: see tg_launch.h
+    kernel<<<grid, 32 * t.W, smem, s>>>(gd, to_modal<S>(c), t.kz, nss, ef, kn, x, b, invdiag,
+                                        omega, y, dot, guard, bd);
   TG_LAUNCH_CHECK();
 }
 

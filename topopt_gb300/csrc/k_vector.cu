@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "tg_internal.h"
+#include "tg_launch.h"
 #include "tg_reduce.h"
 
 namespace tg {
@@ -88,11 +89,12 @@ __global__ void k_max_partials(const double* __restrict__ part, int n, double* _
 // x += alpha p; r -= alpha Ap with alpha = rz / pAp; sum of r.r (FP64).  With x0
 // set, also x0 = omega invdiag .* r.  The FP64 PCG's update; the FP32 inner PCG
 // runs it as two kernels below.
-__global__ void k_cg_update_xr(double* __restrict__ x, double* __restrict__ r,
-                               const double* __restrict__ p, const double* __restrict__ ap,
-                               const double* __restrict__ rz, const double* __restrict__ pap,
-                               int64_t n, const double* __restrict__ invdiag, double omega,
-                               double* __restrict__ x0, SumOut o) {
+__global__ void k_cg_update_xr(double* x, double* r,
+                               const double* p, const double* ap,
+                               const double* rz, const double* pap,
+                               int64_t n, const double* invdiag, double omega,
+                               double* x0, SumOut o) {
+  behind_previous();
   // A non-positive or non-finite pAp is a breakdown the host reports; leave the
   // iterate untouched so the last good x survives.
   const double pp = *pap;
@@ -100,10 +102,13 @@ __global__ void k_cg_update_xr(double* __restrict__ x, double* __restrict__ r,
   double t = 0.0;
   for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
        i += int64_t(gridDim.x) * kThreads) {
-    x[i] += a * p[i];
-    const double ri = r[i] - a * ap[i];
+    // All loads before the first store.
+    const double xv = x[i], pv = p[i], rv = r[i], qv = ap[i];
+    const double dv = x0 != nullptr ? invdiag[i] : 0.0;
+    x[i] = xv + a * pv;
+    const double ri = rv - a * qv;
     r[i] = ri;
-    if (x0 != nullptr) x0[i] = omega * invdiag[i] * ri;
+    if (x0 != nullptr) x0[i] = omega * dv * ri;
     t += ri * ri;
   }
   grid_sum(t, o, int(blockIdx.x), int(gridDim.x));
@@ -119,10 +124,11 @@ __device__ __forceinline__ float cg_alpha_f(const double* rz, const double* pap)
 }
 // With x0 set, also x0 = omega invdiag .* r (the next V-cycle's first smoothing
 // sweep from zero, as k_jacobi_first computes it).
-__global__ void k_cg_update_r_f(float* __restrict__ r, const float* __restrict__ ap,
-                                const double* __restrict__ rz, const double* __restrict__ pap,
-                                int64_t n, const float* __restrict__ invdiag, float omega,
-                                float* __restrict__ x0, SumOut o) {
+__global__ void k_cg_update_r_f(float* r, const float* ap,
+                                const double* rz, const double* pap,
+                                int64_t n, const float* invdiag, float omega,
+                                float* x0, SumOut o) {
+  behind_previous();
   const float af = cg_alpha_f(rz, pap);
   const int64_t n4 = n >> 2;
   float4* r4 = reinterpret_cast<float4*>(r);
@@ -134,14 +140,13 @@ __global__ void k_cg_update_r_f(float* __restrict__ r, const float* __restrict__
        i += int64_t(gridDim.x) * kThreads) {
     float4 rv = r4[i];
     const float4 qv = a4[i];
+    const float4 dv = x0 != nullptr ? d4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     rv.x -= af * qv.x; rv.y -= af * qv.y; rv.z -= af * qv.z; rv.w -= af * qv.w;
     r4[i] = rv;
     tf += rv.x * rv.x + rv.y * rv.y + rv.z * rv.z + rv.w * rv.w;
-    if (x0 != nullptr) {
-      const float4 dv = d4[i];
+    if (x0 != nullptr)
       x4[i] = make_float4(omega * dv.x * rv.x, omega * dv.y * rv.y, omega * dv.z * rv.z,
                           omega * dv.w * rv.w);
-    }
   }
   float t = tf;
   for (int64_t i = (n4 << 2) + blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
@@ -187,9 +192,10 @@ __global__ void k_scale_mask(double* __restrict__ z, const double* __restrict__ 
 
 // p = z + beta p, beta = rz_new / rz_old.
 template <class T>
-__global__ void k_cg_update_p(T* __restrict__ p, const T* __restrict__ z,
-                              const double* __restrict__ rz_new, const double* __restrict__ rz_old,
+__global__ void k_cg_update_p(T* p, const T* z,
+                              const double* rz_new, const double* rz_old,
                               int64_t n) {
+  behind_previous();
   const T beta = T(*rz_new / *rz_old);
   int64_t i0 = 0;
   if (std::is_same<T, float>::value) {
@@ -352,15 +358,16 @@ void launch_sum_partials(const double* part, int n, double* out, cudaStream_t s)
 void launch_cg_update_xr(double* x, double* r, const double* p, const double* ap,
                          const double* rz, const double* pap, int64_t n, const SumOut& rr,
                          cudaStream_t s, const double* invdiag, double omega, double* x0) {
-  k_cg_update_xr<<<red_blocks(n), kThreads, 0, s>>>(x, r, p, ap, rz, pap, n, invdiag, omega, x0,
-                                                    rr);
+  launch_behind(k_cg_update_xr, red_blocks(n), kThreads, 0, s, x, r, p, ap, rz, pap, n, invdiag,
+                omega, x0, rr);
   TG_LAUNCH_CHECK();
 }
 
 void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const double* pap,
                           int64_t n, const SumOut& rr, cudaStream_t s, const float* invdiag,
                           float omega, float* x0) {
-  k_cg_update_r_f<<<red_blocks(n), kThreads, 0, s>>>(r, ap, rz, pap, n, invdiag, omega, x0, rr);
+  launch_behind(k_cg_update_r_f, red_blocks(n), kThreads, 0, s, r, ap, rz, pap, n, invdiag, omega,
+                x0, rr);
   TG_LAUNCH_CHECK();
 }
 void launch_cg_update_x_f(float* x, const float* p, const double* rz, const double* pap,
@@ -378,7 +385,7 @@ void launch_scale_mask(double* z, const double* r, const double* invdiag, int64_
 template <class T>
 void launch_cg_update_p(T* p, const T* z, const double* rz_new, const double* rz_old, int64_t n,
                         cudaStream_t s) {
-  k_cg_update_p<T><<<red_blocks(n), kThreads, 0, s>>>(p, z, rz_new, rz_old, n);
+  launch_behind(k_cg_update_p<T>, red_blocks(n), kThreads, 0, s, p, z, rz_new, rz_old, n);
   TG_LAUNCH_CHECK();
 }
 template void launch_cg_update_p<double>(double*, const double*, const double*, const double*,

@@ -39,9 +39,9 @@ const double kZeta[8] = {-1, -1, -1, -1, +1, +1, +1, +1};
 constexpr int kMaxCoarseDof = 8192;   // dense coarsest factor <= 512 MB
 // Level 1 of the FP32 V-cycle is applied from its assembled stencil up to here and
 // matrix-free above.  The stencil is one launch that reads 1 KB a node from the L2, the
-// matrix-free form two with little to read: 6.2 against 10.3 us on 3,751 to 9,537
-// nodes, 10.3 against 12.3 on 30,625, 14.7 against 14.4 on 43,904, 17.1 against 15.2
-// on 70,785, 177 against 41 on 545,025.
+// matrix-free form two with little to read: 4.1 against 6.5 us on 3,751 nodes, 6.2
+// against 7.4 on 9,537, 10.3 against 14.9 on 30,625, 14.5 against 13.9 on 43,904, 105
+// against 40 on 545,025.
 constexpr int64_t kLevel1AssembledNodes = 32768;
 constexpr int kMaxInverseDof = 512;   // explicit coarsest inverse up to here
 constexpr int64_t kAutotuneMinVoxels = int64_t(1) << 20;  // FP32 schedule measured from here
@@ -1005,6 +1005,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
   }
   Level& N = *levels_[l];
   const T w = T(omega_);
+  const bool joined = sizeof(T) == 4 && l + 1 == side_level_;  // behind the next level's join
   auto op = [&](int mode) {
     if constexpr (sizeof(T) == 4) {
       if (l == 1 && !l1_assembled_) {
@@ -1013,7 +1014,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
       }
     }
     mg_stencil_op<T>(mode, L.d, L.Am<T>(), L.act.p, L.X<T>(), L.B<T>(), L.Dinv<T>(), w, L.R<T>(),
-                     s_);
+                     s_, ChebStep{}, true);
   };
   if (sizeof(T) == 4 && cheb_m_ > 0 && l >= 2) {
     // Mixed form, levels >= 2: a degree-cheb_m_ Chebyshev polynomial in D^-1 A
@@ -1023,7 +1024,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
       for (int k = k0; k < cheb_m_; ++k) {
         ch.step = k;
         mg_stencil_op<T>(kCheb, L.d, L.Am<T>(), L.act.p, L.X<T>(), L.B<T>(), L.Dinv<T>(), w,
-                         L.R<T>(), s_, ch);
+                         L.R<T>(), s_, ch, true);
         std::swap(L.X<T>(), L.R<T>());
       }
     };
@@ -1038,7 +1039,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
     const FirstStep<T> fs = first_step<T>(l + 1);
     mg_restrict<T>(L.d, N.d, L.R<T>(), N.act.p, N.B<T>(), s_, fs);
     T* ec = vcycle_level<T>(l + 1, fs.kind != 0);
-    mg_prolong_add<T>(L.d, N.d, ec, L.act.p, L.X<T>(), s_);
+    mg_prolong_add<T>(L.d, N.d, ec, L.act.p, L.X<T>(), s_, joined);
     cheb(0);
     return L.X<T>();
   }
@@ -1053,7 +1054,7 @@ T* Solver::vcycle_level(size_t l, bool first_done) {
   const FirstStep<T> fs = first_step<T>(l + 1);
   mg_restrict<T>(L.d, N.d, L.R<T>(), N.act.p, N.B<T>(), s_, fs);
   T* ec = vcycle_level<T>(l + 1, fs.kind != 0);
-  mg_prolong_add<T>(L.d, N.d, ec, L.act.p, L.X<T>(), s_);
+  mg_prolong_add<T>(L.d, N.d, ec, L.act.p, L.X<T>(), s_, joined);
   for (int k = 0; k < sweeps_; ++k) {
     op(kSmooth);
     std::swap(L.X<T>(), L.R<T>());
@@ -1128,7 +1129,7 @@ T* Solver::vcycle(const T* b, double* bz, bool x0_ready) {
   const FirstStep<T> fs = first_step<T>(1);
   mg_restrict<T>(fd, N.d, r, N.act.p, N.B<T>(), s_, fs);
   T* ec = vcycle_level<T>(1, fs.kind != 0);
-  mg_prolong_add<T>(fd, N.d, ec, fp_.kept.p, x, s_);
+  mg_prolong_add<T>(fd, N.d, ec, fp_.kept.p, x, s_, sizeof(T) == 4 && side_level_ == 1);
   for (int k = 0; k < sweeps_; ++k) smooth(k == sweeps_ - 1);
   (sizeof(T) == 4 ? lowp_matvecs_ : fine_matvecs_) += 2 * sweeps_;
   return x;

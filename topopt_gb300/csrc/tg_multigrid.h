@@ -56,10 +56,12 @@ struct ChebStep {
 // its FP32 rate).
 constexpr int kChebCoefStride = 16;  // up to 8 steps
 void mg_cheb_table(const double* lam, double ratio, int m, float* coef, cudaStream_t s);
+// settled: the host has waited for the kernels that form A, act and invdiag, so that
+// they may be read while the previous kernel of the stream still runs.
 template <class T>
 void mg_stencil_op(int mode, const MgDims& d, const T* A, const uint8_t* act, const T* x,
                    const T* b, const T* invdiag, T omega, T* y, cudaStream_t s,
-                   ChebStep ch = ChebStep{});
+                   ChebStep ch = ChebStep{}, bool settled = false);
 // lambda_max(D^-1 A) of a stencil level by `iters` power-iteration steps (v, w:
 // level-sized scratch; part: partials, nrm2: two sums, count: a zero counter),
 // times `safety`, into lam[0] on the device.
@@ -84,9 +86,10 @@ struct FirstStep {
 template <class T>
 void mg_restrict(const MgDims& fd, const MgDims& cd, const T* rf, const uint8_t* cact, T* bc,
                  cudaStream_t s, FirstStep<T> first = FirstStep<T>{});
+// joined: the stream has just waited for another one.
 template <class T>
 void mg_prolong_add(const MgDims& fd, const MgDims& cd, const T* ec, const uint8_t* fact, T* xf,
-                    cudaStream_t s);
+                    cudaStream_t s, bool joined = false);
 template <class T>
 void mg_dense_from_stencil(const MgDims& d, const T* A, const int* cidx, int nc, double* D,
                            cudaStream_t s);
