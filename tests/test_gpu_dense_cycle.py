@@ -35,3 +35,20 @@ def test_dense_cycle_solve(tg, port, dims, voids, coarsening):
                                                                     coarsening=coarsening))
         assert info.converged and info.mg_levels >= 3
         assert np.abs(u - ue).max() <= 1e-8 * np.abs(ue).max()
+
+
+def test_dense_cycles_from_many_threads(tg):
+    """Hierarchies with dense levels of different sizes built at the same time: each
+    solve is the one it is alone, bit for bit."""
+    from concurrent.futures import ThreadPoolExecutor
+    dims = [(8, 8, 8), (12, 8, 8), (16, 8, 8), (20, 8, 8), (24, 8, 8), (26, 8, 8)]
+    jobs = [(tg.Problem.cantilever(*d), smooth_modulus(*d)) for d in dims]
+
+    def solve(i):
+        pb, f = jobs[i % len(jobs)]
+        return tg.fea_solve_mgcg_matfree(pb, f, tolerance=1e-6)[0]
+
+    alone = [solve(i) for i in range(len(jobs))]
+    with ThreadPoolExecutor(6) as pool:
+        for i, u in enumerate(pool.map(solve, range(60))):
+            assert np.array_equal(u, alone[i % len(jobs)])

@@ -1464,6 +1464,7 @@ __global__ void __launch_bounds__(kCycleThreads, 1) k_cycle_columns(
   }
 }
 
+constexpr size_t kCycleSmem = size_t(227) * 1024;
 // Columns of a CTA: the fewest that put every column on an SM of its own at once.
 int cycle_columns(int64_t ndof) { return ndof <= 3 * 152 ? 3 : ndof <= 5 * 152 ? 5 : 7; }
 size_t cycle_bytes(int64_t ndof, int nc, bool cheb) {
@@ -1473,7 +1474,7 @@ size_t cycle_bytes(int64_t ndof, int nc, bool cheb) {
 }  // namespace
 
 bool mg_dense_cycle_fits(int64_t ndof, int nc, bool cheb) {
-  return ndof <= kDenseCycleDof && cycle_bytes(ndof, nc, cheb) <= size_t(227) * 1024;
+  return ndof <= kDenseCycleDof && cycle_bytes(ndof, nc, cheb) <= kCycleSmem;
 }
 
 template <class T>
@@ -1486,7 +1487,10 @@ void mg_dense_cycle(const MgDims& d, const MgDims& cd, const T* A, const uint8_t
   const size_t sm = cycle_bytes(ndof, nc, cheb_m > 0);
   const int threads = int(std::min<int64_t>(kCycleThreads, (nodes + 31) / 32 * 96));
   auto run = [&](auto kernel, int cols) {
-    TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    // The same value from every thread: a level's own size could fall short of what
+    // another job is about to launch with.
+    TG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kCycleSmem)));
     kernel<<<unsigned((ndof + cols - 1) / cols), threads, sm, s>>>(
         d, cd, A, act, dinv, coef, cheb_m, sweeps, omega, Ainv, nc, cidx, cdof, M);
     TG_LAUNCH_CHECK();
