@@ -1,7 +1,7 @@
 """Solves whose last smoothed level is applied as a dense matrix, at the edges of that
 form: 3, 5 and 7 columns a CTA, its largest level (1,050 DOFs on 26x8x8) and the first
-beyond it (28x8x8), odd grids with both coarsenings, and a void pocket, against the
-CPU's Jacobi-PCG.  Both solve to 1e-12 of the right-hand side; the condition numbers
+beyond it (28x8x8), odd grids with both coarsenings, a void pocket, and coarsest
+levels with an inverse of 702 and 1,269 DOFs, against the CPU's Jacobi-PCG.  Both solve to 1e-12 of the right-hand side; the condition numbers
 of these grids (about 1e4) leave 1e-8 of the displacement."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ from test_oracle_mg import smooth_modulus
 pytestmark = pytest.mark.gpu
 
 CASES = [((8, 8, 8), False), ((12, 8, 8), False), ((24, 8, 8), False), ((26, 8, 8), False),
-         ((28, 8, 8), False), ((11, 7, 9), False), ((40, 16, 16), True)]
+         ((28, 8, 8), False), ((11, 7, 9), False), ((40, 16, 16), True),
+         ((100, 8, 8), False), ((60, 30, 8), False)]
 
 
 @pytest.mark.parametrize("coarsening", [1, 2])

@@ -780,6 +780,10 @@ __global__ void __launch_bounds__(1024) k_gj_pivot(const double* __restrict__ M,
                                                    int* __restrict__ fail) {
   __shared__ double s[32][33];
   __shared__ double inv;
+  // An earlier block met a pivot that is not positive: the inverse will not be used.
+  const bool failed = *fail != 0;
+  __syncthreads();  // before this block's own verdict
+  if (failed) return;
   const int nb = min(kGjBlock, nc - k0);
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const bool in = tx < nb && ty < nb;
@@ -813,21 +817,23 @@ __global__ void __launch_bounds__(1024) k_gj_pivot(const double* __restrict__ M,
   if (in) P[ty * kGjBlock + tx] = v;
 }
 
+// `tall` tiles of one column each, whose R = P M_Kj is formed once: two thirds of a
+// single tile's multiply-adds.
 __global__ void __launch_bounds__(256) k_gj_update(const double* __restrict__ M, int nc, int k0,
                                                    const double* __restrict__ P,
-                                                   double* __restrict__ out) {
+                                                   double* __restrict__ out, int tall,
+                                                   const int* __restrict__ fail) {
+  if (*fail != 0) return;
   __shared__ double sP[32][33], sC[kGjTile][33], sR[32][kGjTile + 1], sT[32][kGjTile + 1];
   const int nb = min(kGjBlock, nc - k0);
-  const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+  const int j0 = blockIdx.x * kGjTile;
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   for (int e = t; e < 32 * 32; e += 256) {
     const int r = e >> 5, c = e & 31;
     sP[r][c] = r < nb && c < nb ? P[r * kGjBlock + c] : 0.0;
   }
   for (int e = t; e < kGjTile * 32; e += 256) {
-    const int r = e >> 5, c = e & 31;  // column block K of this tile's rows
-    sC[r][c] = i0 + r < nc && c < nb ? M[int64_t(i0 + r) * nc + k0 + c] : 0.0;
-    const int rr = e >> 4, cc = e & 15;  // row block K of this tile's columns
+    const int rr = e >> 4, cc = e & 15;  // row block K of these columns
     sT[rr][cc] = rr < nb && j0 + cc < nc ? M[int64_t(k0 + rr) * nc + j0 + cc] : 0.0;
   }
   __syncthreads();
@@ -839,21 +845,32 @@ __global__ void __launch_bounds__(256) k_gj_update(const double* __restrict__ M,
     for (int k = 0; k < 32; ++k) v = fma(sP[r][k], sT[k][tx], v);
     sR[r][tx] = v;
   }
-  __syncthreads();
-  const int i = i0 + ty, j = j0 + tx;
-  if (i >= nc || j >= nc) return;
-  const bool ik = i >= k0 && i < k0 + nb, jk = j >= k0 && j < k0 + nb;
-  double v;
-  if (ik && jk) {
-    v = sP[i - k0][j - k0];
-  } else if (ik) {
-    v = sR[i - k0][tx];
-  } else {
-    v = jk ? 0.0 : M[int64_t(i) * nc + j];
+  const int j = j0 + tx;
+  const bool jk = j >= k0 && j < k0 + nb;
+  for (int q = 0; q < tall; ++q) {
+    const int i0 = (blockIdx.y * tall + q) * kGjTile;
+    if (i0 >= nc) break;  // uniform over the CTA
+    __syncthreads();      // R formed, the last tile's C read
+    for (int e = t; e < kGjTile * 32; e += 256) {
+      const int r = e >> 5, c = e & 31;  // column block K of this tile's rows
+      sC[r][c] = i0 + r < nc && c < nb ? M[int64_t(i0 + r) * nc + k0 + c] : 0.0;
+    }
+    __syncthreads();
+    const int i = i0 + ty;
+    if (i >= nc || j >= nc) continue;
+    const bool ik = i >= k0 && i < k0 + nb;
+    double v;
+    if (ik && jk) {
+      v = sP[i - k0][j - k0];
+    } else if (ik) {
+      v = sR[i - k0][tx];
+    } else {
+      v = jk ? 0.0 : M[int64_t(i) * nc + j];
 #pragma unroll 8
-    for (int k = 0; k < 32; ++k) v = fma(-sC[ty][k], jk ? sP[k][j - k0] : sR[k][tx], v);
+      for (int k = 0; k < 32; ++k) v = fma(-sC[ty][k], jk ? sP[k][j - k0] : sR[k][tx], v);
+    }
+    out[int64_t(i) * nc + j] = v;
   }
-  out[int64_t(i) * nc + j] = v;
 }
 
 // Blocked right-looking Cholesky, panel width 32.  Step 1: factor the diagonal
@@ -1224,10 +1241,12 @@ void mg_dense_inverse(int nc, double* a, double* inv, double* pivot, int* fail, 
   double* src = mg_dense_start(nc, a, inv);
   double* dst = src == a ? inv : a;
   const unsigned tiles = unsigned((nc + kGjTile - 1) / kGjTile);
+  const unsigned tall = std::max(1u, std::min(8u, tiles * tiles / (4 * 152)));  // 4 CTAs an SM
   for (int k0 = 0; k0 < nc; k0 += kGjBlock) {
     k_gj_pivot<<<1, 1024, 0, s>>>(src, nc, k0, pivot, fail);
     TG_LAUNCH_CHECK();
-    k_gj_update<<<dim3(tiles, tiles), 256, 0, s>>>(src, nc, k0, pivot, dst);
+    k_gj_update<<<dim3(tiles, (tiles + tall - 1) / tall), 256, 0, s>>>(src, nc, k0, pivot, dst,
+                                                                      int(tall), fail);
     TG_LAUNCH_CHECK();
     std::swap(src, dst);
   }

@@ -43,7 +43,13 @@ constexpr int kMaxCoarseDof = 8192;   // dense coarsest factor <= 512 MB
 // against 7.4 on 9,537, 10.3 against 14.9 on 30,625, 14.5 against 13.9 on 43,904, 105
 // against 40 on 545,025.
 constexpr int64_t kLevel1AssembledNodes = 32768;
-constexpr int kMaxInverseDof = 512;   // explicit coarsest inverse up to here
+// Explicit coarsest inverse up to here.  Substitution with the Cholesky factor is a
+// chain of 2 nc steps in one CTA, 1 ms an application at 612 DOFs and 4.4 at 1,755,
+// where the product with the inverse is 4 to 9 us; forming the inverse takes as long as
+// the factor up to 891 DOFs and 13.7 ms against 7.9 at 1,755 (solves of 17 to 25
+// iterations: 124x16x22 mixed 26 -> 4.4 ms, 256x16x16 mixed 45 -> 6.6, 512x16x16 FP64
+// 85 -> 21).  The two matrices take 64 MB at the limit.
+constexpr int kMaxInverseDof = 2048;
 constexpr int64_t kAutotuneMinVoxels = int64_t(1) << 20;  // FP32 schedule measured from here
 
 MgDims dims_of(int ex, int ey, int ez) { return MgDims{ex, ey, ez, ex + 1, ey + 1, ez + 1}; }
