@@ -100,16 +100,50 @@ __global__ void k_cg_update_xr(double* x, double* r,
   const double pp = *pap;
   const double a = (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
   double t = 0.0;
-  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * kThreads) {
-    // All loads before the first store.
-    const double xv = x[i], pv = p[i], rv = r[i], qv = ap[i];
-    const double dv = x0 != nullptr ? invdiag[i] : 0.0;
-    x[i] = xv + a * pv;
-    const double ri = rv - a * qv;
-    r[i] = ri;
-    if (x0 != nullptr) x0[i] = omega * dv * ri;
-    t += ri * ri;
+  const bool next = x0 != nullptr;
+  auto one = [&](double& xv, double pv, double& rv, double qv, double dv) {
+    xv += a * pv;
+    rv -= a * qv;
+    t += rv * rv;
+    return omega * dv * rv;
+  };
+  // Pairs, two a round: all of a round's loads before its first store, since the
+  // compiler may not move them past one.
+  const int64_t n2 = n >> 1, step = int64_t(gridDim.x) * kThreads;
+  double2 *x2 = reinterpret_cast<double2*>(x), *r2 = reinterpret_cast<double2*>(r),
+          *z2 = reinterpret_cast<double2*>(x0);
+  const double2 *p2 = reinterpret_cast<const double2*>(p),
+                *q2 = reinterpret_cast<const double2*>(ap),
+                *d2 = reinterpret_cast<const double2*>(invdiag);
+  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n2; i += 2 * step) {
+    const int64_t j[2] = {i, i + step};
+    double2 xv[2], pv[2], rv[2], qv[2], dv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= n2) continue;
+      xv[u] = x2[j[u]];
+      pv[u] = p2[j[u]];
+      rv[u] = r2[j[u]];
+      qv[u] = q2[j[u]];
+      dv[u] = next ? d2[j[u]] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= n2) continue;
+      double2 zv;
+      zv.x = one(xv[u].x, pv[u].x, rv[u].x, qv[u].x, dv[u].x);
+      zv.y = one(xv[u].y, pv[u].y, rv[u].y, qv[u].y, dv[u].y);
+      x2[j[u]] = xv[u];
+      r2[j[u]] = rv[u];
+      if (next) z2[j[u]] = zv;
+    }
+  }
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+    double xv = x[n - 1], rv = r[n - 1];
+    const double zv = one(xv, p[n - 1], rv, ap[n - 1], next ? invdiag[n - 1] : 0.0);
+    x[n - 1] = xv;
+    r[n - 1] = rv;
+    if (next) x0[n - 1] = zv;
   }
   grid_sum(t, o, int(blockIdx.x), int(gridDim.x));
 }
@@ -136,17 +170,30 @@ __global__ void k_cg_update_r_f(float* r, const float* ap,
   const float4* d4 = reinterpret_cast<const float4*>(invdiag);
   float4* x4 = reinterpret_cast<float4*>(x0);
   float tf = 0.0f;
-  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n4;
-       i += int64_t(gridDim.x) * kThreads) {
-    float4 rv = r4[i];
-    const float4 qv = a4[i];
-    const float4 dv = x0 != nullptr ? d4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    rv.x -= af * qv.x; rv.y -= af * qv.y; rv.z -= af * qv.z; rv.w -= af * qv.w;
-    r4[i] = rv;
-    tf += rv.x * rv.x + rv.y * rv.y + rv.z * rv.z + rv.w * rv.w;
-    if (x0 != nullptr)
-      x4[i] = make_float4(omega * dv.x * rv.x, omega * dv.y * rv.y, omega * dv.z * rv.z,
-                          omega * dv.w * rv.w);
+  const int64_t step = int64_t(gridDim.x) * kThreads;
+  // Two a round: all of a round's loads before its first store, since the compiler may
+  // not move them past one.
+  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n4; i += 2 * step) {
+    const int64_t j[2] = {i, i + step};
+    float4 rv[2], qv[2], dv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= n4) continue;
+      rv[u] = r4[j[u]];
+      qv[u] = a4[j[u]];
+      dv[u] = x0 != nullptr ? d4[j[u]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= n4) continue;
+      float4& v = rv[u];
+      v.x -= af * qv[u].x; v.y -= af * qv[u].y; v.z -= af * qv[u].z; v.w -= af * qv[u].w;
+      r4[j[u]] = v;
+      tf += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+      if (x0 != nullptr)
+        x4[j[u]] = make_float4(omega * dv[u].x * v.x, omega * dv[u].y * v.y,
+                               omega * dv[u].z * v.z, omega * dv[u].w * v.w);
+    }
   }
   float t = tf;
   for (int64_t i = (n4 << 2) + blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
@@ -197,23 +244,31 @@ __global__ void k_cg_update_p(T* p, const T* z,
                               int64_t n) {
   behind_previous();
   const T beta = T(*rz_new / *rz_old);
-  int64_t i0 = 0;
-  if (std::is_same<T, float>::value) {
-    const int64_t n4 = n >> 2;
-    float4* p4 = reinterpret_cast<float4*>(p);
-    const float4* z4 = reinterpret_cast<const float4*>(z);
-    const float b = float(beta);
-    for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n4;
-         i += int64_t(gridDim.x) * kThreads) {
-      float4 pv = p4[i];
-      const float4 zv = z4[i];
-      pv.x = zv.x + b * pv.x; pv.y = zv.y + b * pv.y; pv.z = zv.z + b * pv.z; pv.w = zv.w + b * pv.w;
-      p4[i] = pv;
+  // 16 bytes at a time, two a round, as in the updates above.
+  using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
+  constexpr int kPer = int(sizeof(V) / sizeof(T));
+  const int64_t nv = n / kPer, step = int64_t(gridDim.x) * kThreads;
+  V* pw = reinterpret_cast<V*>(p);
+  const V* zw = reinterpret_cast<const V*>(z);
+  for (int64_t i = blockIdx.x * int64_t(kThreads) + threadIdx.x; i < nv; i += 2 * step) {
+    const int64_t j[2] = {i, i + step};
+    V pv[2], zv[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= nv) continue;
+      pv[u] = pw[j[u]];
+      zv[u] = zw[j[u]];
     }
-    i0 = n4 << 2;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (j[u] >= nv) continue;
+      T *a = reinterpret_cast<T*>(pv + u), *b = reinterpret_cast<T*>(zv + u);
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) a[k] = b[k] + beta * a[k];
+      pw[j[u]] = pv[u];
+    }
   }
-  for (int64_t i = i0 + blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n;
-       i += int64_t(gridDim.x) * kThreads)
+  for (int64_t i = nv * kPer + blockIdx.x * int64_t(kThreads) + threadIdx.x; i < n; i += step)
     p[i] = z[i] + beta * p[i];
 }
 
