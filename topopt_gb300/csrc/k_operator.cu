@@ -527,6 +527,182 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
 }
 
 // ------------------------------------------------------------------ schedules
+constexpr int kSplitMaxRows = 5;  // element rows a CTA: 43 KB of shared memory
+namespace {
+
+// The FP64 operator with a warp per element row and component.  On a small grid the
+// marching kernel's time is its chain: a warp instruction on FP64 takes 64 cycles of its
+// scheduler whatever waits, a step has 150 of them, and a 24x8x8 grid has 66 rows of
+// lanes for 608 schedulers.  The transforms of the three displacement components do not
+// meet except in the modal stresses, so here three warps take one component each and
+// exchange their modes in shared memory: 66 instructions a step and warp.  24x8x8 and
+// 48x8x8: 14.5 -> 10.3 us, bound now by the six warps of a CTA on one SM's FP64 units.
+// A row takes 198 instructions instead of 150, so the marching kernel keeps the grids
+// that fill the SMs: its best tile takes 26.7 us against 28.8 on 60x20x20, 43.1 against
+// 45.2 on 60x36x28, 110.7 against 137 on 96x48x48.
+template <int MODE>
+__global__ void __launch_bounds__(96 * kSplitMaxRows, 1)
+    k_fine_split(GridDev g, ModalT<double> mc, int KZ, int nss, const double* ef,
+                 const uint8_t* __restrict__ kn, const double* x, const double* b,
+                 const double* invdiag, double omega, double* y, SumOut dot, int guard) {
+  let_next_start();
+  constexpr int kOwn = 31;
+  extern __shared__ __align__(16) unsigned char march_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, w = wid / 3, k = wid - 3 * w;
+  const int W = blockDim.x / 96, rows = W - 1;
+  double* const xs = reinterpret_cast<double*>(march_smem);  // [2][W][3][2][32]
+  double* const us = xs + 2 * W * 192 + w * (21 * 32) + lane;  // [3][7][32] of this row
+  const int q = blockIdx.x * kOwn - 1 + lane;
+  const int ss = q > 0 ? q / g.nnx : 0, ex = q - ss * g.nnx;
+  const bool own_x = lane >= 1 && ss < nss;
+  const int rl = lane < 31 ? lane + 1 : lane, ll = lane > 0 ? lane - 1 : lane;
+  const int ey = ss * rows - 1 + w;  // element row ey, node rows ey and ey + 1
+  const bool vx = ex >= 0 && ss < nss;
+  const int plane = g.nnx * g.nny, eplane = g.nx * g.ny;
+  const int no[2] = {g.nnx * ey + ex, g.nnx * (ey + 1) + ex};
+  const bool rv[2] = {vx && ey >= 0 && ey < g.nny, vx && ey + 1 < g.nny};
+  const bool own = own_x && w < W - 1 && ey + 1 < g.nny;
+  const bool ev = vx && ex < g.nx && ey >= 0 && ey < g.ny;
+  const int eo = ey * g.nx + ex, z0 = blockIdx.y * KZ;
+  const bool far = lane == 31 && ex + 1 < g.nnx;  // its right neighbour has no lane
+  wait_for_previous();
+
+  auto load_layer = [&](int c, double (&r)[2], double (&e)[2]) {
+    const bool vc = c >= 0 && c < g.nnz;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool ok = vc && rv[i];
+      const double* xn = x + 3 * (plane * c + no[i]) + k;
+      r[i] = ok ? xn[0] : 0.0;
+      e[i] = ok && far ? xn[3] : 0.0;
+    }
+  };
+  auto load_f = [&](int c) { return c >= 0 && c < g.nz && ev ? ef[eplane * c + eo] : 0.0; };
+  auto face = [&](const double (&r)[2], const double (&e)[2], double (&F)[4]) {
+    double nb[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      nb[i] = shfl_at(r[i], rl);
+      nb[i] = lane == 31 ? e[i] : nb[i];
+    }
+    face_modes<double, double>(r, nb, F);
+  };
+  auto load_kb = [&](int s) -> unsigned {
+    const int ez = z0 - 1 + s;
+    return kn == nullptr ? 7u : (s >= 1 && ez < g.nnz && own ? unsigned(kn[plane * ez + no[1]]) : 0u);
+  };
+
+  const int s0 = z0 == 0 ? 1 : 0;
+  double raw[2], rext[2], Fc[4], pend[4] = {0.0, 0.0, 0.0, 0.0};
+  load_layer(z0 - 1 + s0, raw, rext);
+  face(raw, rext, Fc);
+  double keep = raw[1];
+  load_layer(z0 + s0, raw, rext);
+  double fn = load_f(z0 - 1 + s0);
+  unsigned kbn = load_kb(s0);
+  double dsum = 0.0;
+#pragma unroll 1
+  for (int s = s0; s <= KZ; ++s) {
+    const int ez = z0 - 1 + s;
+    if (ez > g.nnz - 1) break;  // uniform: the last chunk ends with the grid
+    const bool out = s >= 1 && own;
+    const unsigned kb = kbn;
+    if (s < KZ) kbn = load_kb(s + 1);
+    const int at1 = 3 * (plane * ez + no[1]) + k;
+    const double bv = MODE != kApply && out ? b[at1] : 0.0;
+    const double dv = MODE == kSmooth && out ? invdiag[at1] : 0.0;
+    const double f = fn;
+    double Fn[4];
+    face(raw, rext, Fn);
+    const double knext = raw[1];
+    if (s < KZ) {
+      load_layer(ez + 2, raw, rext);
+      fn = load_f(ez + 1);
+    }
+    double u[8];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      if (m > 0) u[m] = Fn[m] + Fc[m];
+      u[m | 4] = Fn[m] - Fc[m];
+    }
+#pragma unroll
+    for (int m = 1; m < 8; ++m) us[(k * 7 + m - 1) * 32] = u[m];
+    asm volatile("bar.sync %0, 96;" ::"r"(1 + w) : "memory");
+    // modal_stress (tg_march.h) for component K alone: its axis' mode A, the others' B
+    // and C.
+    auto stress = [&](auto kc) {
+      constexpr int K = decltype(kc)::value, KB = (K + 1) % 3, KC = (K + 2) % 3;
+      constexpr int A = 1 << K, B = 1 << KB, C = 1 << KC;
+      auto o = [&](int comp, int m) { return comp == K ? u[m] : us[(comp * 7 + m - 1) * 32]; };
+      const double m0 = mc.M0 * f, m02 = mc.M02 * f, l0 = mc.L0 * f, l1 = mc.L1 * f,
+                   m1 = mc.M1 * f, lm2 = mc.LM2 * f;
+      const double tr = l0 * ((o(0, 1) + o(1, 2)) + o(2, 4));
+      const double sh = m1 * ((o(2, 3) + o(1, 5)) + o(0, 6));
+      const double tb = l1 * (u[A | B] + o(KC, B | C)), tc = l1 * (u[A | C] + o(KB, B | C));
+      const double ub = m0 * (u[B] + o(KB, A)), uc = m0 * (u[C] + o(KC, A));
+      u[A] = mad(m02, u[A], tr);
+      u[B] = ub;
+      u[C] = uc;
+      u[A | B] = mad(m0, u[A | B], tb);
+      u[A | C] = mad(m0, u[A | C], tc);
+      u[B | C] = mad(m1, u[B | C], sh);
+      u[7] = lm2 * u[7];
+    };
+    if (k == 0)
+      stress(std::integral_constant<int, 0>{});
+    else if (k == 1)
+      stress(std::integral_constant<int, 1>{});
+    else
+      stress(std::integral_constant<int, 2>{});
+    if (guard) {
+#pragma unroll
+      for (int m = 1; m < 8; ++m) u[m] = f != 0.0 ? u[m] : 0.0;
+    }
+    // Back in z and y, as in the marching kernel.
+    double P[4];
+    P[0] = pend[0] - u[4];
+    pend[0] = u[4];
+#pragma unroll
+    for (int m = 1; m < 4; ++m) {
+      P[m] = pend[m] + (u[m] - u[m | 4]);
+      pend[m] = u[m] + u[m | 4];
+    }
+    double* const buf = xs + (s & 1) * (W * 192);
+    buf[w * 192 + (2 * k) * 32 + lane] = P[0] - P[2];
+    buf[w * 192 + (2 * k + 1) * 32 + lane] = P[1] - P[3];
+    const double up0 = P[0] + P[2], up1 = P[1] + P[3];
+    __syncthreads();  // the rows' exchange, and every row's modes are read
+    if (w < W - 1) {
+      const double r0 = up0 + buf[(w + 1) * 192 + (2 * k) * 32 + lane];
+      const double r1 = up1 + buf[(w + 1) * 192 + (2 * k + 1) * 32 + lane];
+      const double ax = (r0 - r1) + shfl_at(r0 + r1, ll);
+      if (out) {
+        const bool kk = ((kb >> k) & 1u) != 0u;
+        double v;
+        if constexpr (MODE == kApply) {
+          v = kk ? ax : 0.0;
+          dsum += keep * v;
+        } else if constexpr (MODE == kResidual) {
+          v = kk ? bv - ax : 0.0;
+        } else {
+          v = kk ? keep + omega * dv * (bv - ax) : 0.0;
+          dsum += bv * v;
+        }
+        y[at1] = v;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) Fc[m] = Fn[m];
+    keep = knext;
+  }
+  if constexpr (MODE != kResidual) {
+    if (dot.part != nullptr)
+      grid_sum(dsum, dot, int(blockIdx.y * gridDim.x + blockIdx.x), int(gridDim.x * gridDim.y));
+  }
+}
+
+}  // namespace
+
 namespace {
 
 struct MarchTile {
@@ -615,6 +791,47 @@ MarchTile march_tile(int nnx, int nny, int nnz, int nsys, bool per) {
   return best;
 }
 
+// The FP64 operator's kernel and tile on a grid: whichever the model puts first.  A row
+// of the split kernel is 1.3 times the FP64 work of the marching kernel's, and about
+// half its chain.
+struct Fp64Plan {
+  bool split;
+  MarchTile t;
+};
+Fp64Plan fp64_plan(int nnx, int nny, int nnz) {
+  constexpr double kBusy = 3800.0, kChain = 5200.0, kStart = 4000.0;
+  Fp64Plan best{false, march_tile<double>(nnx, nny, nnz, 1, false)};
+  double cost = march_cost<double>(best.t, march_grid<double>(nnx, nny, nnz, 1, false, best.t));
+  for (int W = 2; W <= kSplitMaxRows; ++W)
+    for (int target : {1, 2, 3, 4, 6, 8, 11, 16}) {
+      const int chunks = (nnz + target - 1) / target;
+      const MarchTile t{W, (nnz + chunks - 1) / chunks};
+      const dim3 d = march_grid<double>(nnx, nny, nnz, 1, false, t);
+      const double per_sm = double((int64_t(d.x) * d.y + kSms - 1) / kSms);
+      const double rounds = std::ceil(per_sm / std::max(1, 7 / W));
+      const double c = std::max(per_sm * W * (t.kz + 1) * kBusy, rounds * (t.kz + 1) * kChain) +
+                       rounds * kStart;
+      if (c < cost) {
+        cost = c;
+        best = Fp64Plan{true, t};
+      }
+      if (target >= nnz) break;
+    }
+  return best;
+}
+
+template <int MODE>
+void launch_split(const GridDev& gd, const MarchTile& t, const ModalConsts& c, const double* ef,
+                  const uint8_t* kn, const double* x, const double* b, const double* invdiag,
+                  double omega, double* y, const SumOut& dot, cudaStream_t s) {
+  const dim3 grid = march_grid<double>(gd.nnx, gd.nny, gd.nnz, 1, false, t);
+  const int nss = (gd.nny + t.W - 2) / (t.W - 1);
+  const size_t smem = size_t(t.W) * (2 * 192 + 21 * 32) * sizeof(double);
+  k_fine_split<MODE><<<grid, 96 * t.W, smem, s>>>(gd, to_modal<double>(c), t.kz, nss, ef, kn, x, b,
+                                                 invdiag, omega, y, dot, kn == nullptr ? 1 : 0);
+  TG_LAUNCH_CHECK();
+}
+
 template <class V, class T, int MODE, bool PER>
 void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalConsts& c,
                   const T* ef, const uint8_t* kn, const T* x, const T* b, const T* invdiag,
@@ -675,7 +892,7 @@ int blocks_of(const dim3& d) { return int(d.x * d.y); }
 int fine_op_blocks(const Grid& g, bool fp64) {
   if (fp64)
     return blocks_of(march_grid<double>(g.nnx, g.nny, g.nnz, 1, false,
-                                        march_tile<double>(g.nnx, g.nny, g.nnz, 1, false)));
+                                        fp64_plan(g.nnx, g.nny, g.nnz).t));
   int n = std::max(blocks_of(march_grid<float2>(g.nnx, g.nny, g.nnz, 1, false,
                                                 march_tile<float2>(g.nnx, g.nny, g.nnz, 1, false))),
                    blocks_of(march_grid<float>(g.nnx, g.nny, g.nnz, 1, false,
@@ -737,8 +954,16 @@ void launch_fine_op(int mode, const Grid& g, const ModalConsts& c, const T* ef, 
     launch_fine_op_sched(fine_schedule_for(g, mode), mode, g, c, ef, kn, x, b, invdiag, omega, y,
                          dot, s);
   } else {
-    launch_march_mode<double, double>(mode, g, march_tile<double>(g.nnx, g.nny, g.nnz, 1, false),
-                                      c, ef, kn, x, b, invdiag, omega, y, dot, s);
+    const Fp64Plan p = fp64_plan(g.nnx, g.nny, g.nnz);
+    const GridDev gd{g.nx, g.ny, g.nz, g.nnx, g.nny, g.nnz};
+    if (!p.split)
+      launch_march_mode<double, double>(mode, g, p.t, c, ef, kn, x, b, invdiag, omega, y, dot, s);
+    else if (mode == kApply)
+      launch_split<kApply>(gd, p.t, c, ef, kn, x, b, invdiag, omega, y, dot, s);
+    else if (mode == kResidual)
+      launch_split<kResidual>(gd, p.t, c, ef, kn, x, b, invdiag, omega, y, SumOut{}, s);
+    else
+      launch_split<kSmooth>(gd, p.t, c, ef, kn, x, b, invdiag, omega, y, dot, s);
   }
 }
 
