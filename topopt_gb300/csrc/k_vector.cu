@@ -86,6 +86,20 @@ __global__ void k_max_partials(const double* __restrict__ part, int n, double* _
   if (threadIdx.x == 0) *out = s;
 }
 
+// A scalar of the step (an FP64 division) by one warp for the whole block: each warp
+// that divides takes the SM's FP64 units ten or more times for 19 cycles, 3 us of a
+// kernel with 32 warps on every SM.
+template <class F>
+__device__ __forceinline__ double block_scalar(const F& f) {
+  __shared__ double s;
+  if (threadIdx.x < 32) {
+    const double v = f();
+    if (threadIdx.x == 0) s = v;
+  }
+  __syncthreads();
+  return s;
+}
+
 // x += alpha p; r -= alpha Ap with alpha = rz / pAp; sum of r.r (FP64).  With x0
 // set, also x0 = omega invdiag .* r.  The FP64 PCG's update; the FP32 inner PCG
 // runs it as two kernels below.
@@ -97,8 +111,10 @@ __global__ void k_cg_update_xr(double* x, double* r,
   behind_previous();
   // A non-positive or non-finite pAp is a breakdown the host reports; leave the
   // iterate untouched so the last good x survives.
-  const double pp = *pap;
-  const double a = (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
+  const double a = block_scalar([&] {
+    const double pp = *pap;
+    return (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
+  });
   double t = 0.0;
   const bool next = x0 != nullptr;
   auto one = [&](double& xv, double pv, double& rv, double qv, double dv) {
@@ -153,8 +169,10 @@ __global__ void k_cg_update_xr(double* x, double* r,
 // which the solver runs later, beside the next V-cycle's coarse levels
 // (nothing in the loop reads x).
 __device__ __forceinline__ float cg_alpha_f(const double* rz, const double* pap) {
-  const double pp = *pap;
-  return float((pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0);
+  return float(block_scalar([&] {
+    const double pp = *pap;
+    return (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
+  }));
 }
 // With x0 set, also x0 = omega invdiag .* r (the next V-cycle's first smoothing
 // sweep from zero, as k_jacobi_first computes it).
@@ -243,7 +261,7 @@ __global__ void k_cg_update_p(T* p, const T* z,
                               const double* rz_new, const double* rz_old,
                               int64_t n) {
   behind_previous();
-  const T beta = T(*rz_new / *rz_old);
+  const T beta = T(block_scalar([&] { return *rz_new / *rz_old; }));
   // 16 bytes at a time, two a round, as in the updates above.
   using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
   constexpr int kPer = int(sizeof(V) / sizeof(T));
