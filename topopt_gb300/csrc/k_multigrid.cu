@@ -712,11 +712,10 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(MgDims fd, MgDims
 // Prolongation + correction: x_f += P e_c on active fine DOFs.  One thread per
 // fine node on a 3D grid: a thread per DOF repeats the node's index arithmetic and
 // took 79 us against 33 on 257x129x129 nodes.
-template <class T>
 __global__ void __launch_bounds__(256) k_prolong_add(MgDims fd, MgDims cd,
-                                                     const T* ec,
+                                                     const double* ec,
                                                      const uint8_t* __restrict__ fact,
-                                                     T* xf) {
+                                                     double* xf) {
   let_next_start();
   const int a = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y * 8 + threadIdx.y, c = blockIdx.z;
   if (a >= fd.nnx || b >= fd.nny) return;
@@ -725,12 +724,77 @@ __global__ void __launch_bounds__(256) k_prolong_add(MgDims fd, MgDims cd,
   // coarse values: a read under the mask's branch would wait for the mask first.
   const bool f0 = fact[3 * n] != 0, f1 = fact[3 * n + 1] != 0, f2 = fact[3 * n + 2] != 0;
   wait_for_previous();
-  const T x0 = xf[3 * n], x1 = xf[3 * n + 1], x2 = xf[3 * n + 2];
-  T s[3];
-  prolong_node<T, false>(fd, cd, ec, a, b, c, s);
+  const double x0 = xf[3 * n], x1 = xf[3 * n + 1], x2 = xf[3 * n + 2];
+  double s[3];
+  prolong_node<double, false>(fd, cd, ec, a, b, c, s);
   if (f0) xf[3 * n] = x0 + s[0];
   if (f1) xf[3 * n + 1] = x1 + s[1];
   if (f2) xf[3 * n + 2] = x2 + s[2];
+}
+
+// The same for FP32, a thread per two fine nodes, (a, b) of layers 2 cz and 2 cz + 1:
+// the loads that one node leaves in flight are too few to reach the memory's rate
+// (257x129x129 nodes: 33 us for 108 MB), and the two share the coarse layer between
+// them.  Each node's sum is prolong_node's, in its order.  256x128x128 solves 36.3 ->
+// 35.8 ms, 128x64x64 10.43 -> 10.26.  In FP64, where an absent neighbour's products
+// cost what they cost, it is the slower one (60x36x28 33.2 -> 33.7 ms).
+__global__ void __launch_bounds__(256) k_prolong_pair(MgDims fd, MgDims cd, const float* ec,
+                                                     const uint8_t* __restrict__ fact, float* xf) {
+  let_next_start();
+  const int a = blockIdx.x * 32 + threadIdx.x, b = blockIdx.y * 8 + threadIdx.y, cz = blockIdx.z;
+  if (a >= fd.nnx || b >= fd.nny) return;
+  const bool ta = tail_node(a, fd.ex, cd.align), tb = tail_node(b, fd.ey, cd.align);
+  const int na = (a & 1) && !ta ? 2 : 1, nb = (b & 1) && !tb ? 2 : 1;
+  const int ia = ta ? (a + 1) >> 1 : a >> 1, ib = tb ? (b + 1) >> 1 : b >> 1;
+  const int64_t layer = int64_t(fd.nnx) * fd.nny, n = (2 * cz) * layer + int64_t(b) * fd.nnx + a;
+  const bool two = 2 * cz + 1 < fd.nnz;
+  const bool tail = two && tail_node(2 * cz + 1, fd.ez, cd.align);  // at coarse layer cz + 1
+  bool on[2][3];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) on[q][k] = (q == 0 || two) && fact[3 * (n + q * layer) + k] != 0;
+  wait_for_previous();
+  // The iterate is read unconditionally, with the coarse values: a read under the
+  // mask's branch would wait for the mask first.
+  float xv[2][3], e[2][2][2][3];
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) xv[q][k] = q == 0 || two ? xf[3 * (n + q * layer) + k] : 0.0f;
+#pragma unroll
+  for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+    for (int yy = 0; yy < 2; ++yy)
+#pragma unroll
+      for (int xx = 0; xx < 2; ++xx) {
+        const bool in = xx < na && yy < nb && (zz == 0 || two) && ia + xx < cd.nnx &&
+                        ib + yy < cd.nny && cz + zz < cd.nnz;
+        const float* p = ec + 3 * ((int64_t(cz + zz) * cd.nny + ib + yy) * cd.nnx + ia + xx);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) e[zz][yy][xx][k] = in ? p[k] : 0.0f;
+      }
+  const float wxy = (na == 2 ? 0.5f : 1.0f) * (nb == 2 ? 0.5f : 1.0f);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    if (q == 1 && !two) continue;
+    const bool both = q == 1 && !tail;
+    const float w = wxy * (both ? 0.5f : 1.0f);
+    float s[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int zz = 0; zz < 2; ++zz) {
+      if (!both && zz != (q == 1 ? 1 : 0)) continue;
+#pragma unroll
+      for (int yy = 0; yy < 2; ++yy)
+#pragma unroll
+        for (int xx = 0; xx < 2; ++xx)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) s[k] += w * e[zz][yy][xx][k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (on[q][k]) xf[3 * (n + q * layer) + k] = xv[q][k] + s[k];
+  }
 }
 
 // ---------------------------------------------------------- coarsest solve
@@ -1202,11 +1266,17 @@ void mg_restrict(const MgDims& fd, const MgDims& cd, const T* rf, const uint8_t*
 template <class T>
 void mg_prolong_add(const MgDims& fd, const MgDims& cd, const T* ec, const uint8_t* fact, T* xf,
                     cudaStream_t s, bool joined) {
-  const dim3 grid((fd.nnx + 31) / 32, (fd.nny + 7) / 8, fd.nnz);
-  if (joined)
-    k_prolong_add<T><<<grid, dim3(32, 8), 0, s>>>(fd, cd, ec, fact, xf);
+  const unsigned gx = unsigned(fd.nnx + 31) / 32, gy = unsigned(fd.nny + 7) / 8;
+  auto run = [&](auto kernel, dim3 grid) {
+    if (joined)
+      kernel<<<grid, dim3(32, 8), 0, s>>>(fd, cd, ec, fact, xf);
+    else
+      launch_behind_if_spread<T>(kernel, grid, dim3(32, 8), 0, s, fd, cd, ec, fact, xf);
+  };
+  if constexpr (sizeof(T) == 4)
+    run(k_prolong_pair, dim3(gx, gy, unsigned(fd.nnz + 1) / 2));
   else
-    launch_behind_if_spread<T>(k_prolong_add<T>, grid, dim3(32, 8), 0, s, fd, cd, ec, fact, xf);
+    run(k_prolong_add, dim3(gx, gy, unsigned(fd.nnz)));
   TG_LAUNCH_CHECK();
 }
 
