@@ -73,7 +73,7 @@ def peaks():
 def committed_traffic(nx, ny, nz):
     """DRAM bytes per launch of the FP32 fine operator from the committed ncu
     capture of the same workload (profiles/), or None."""
-    path = os.path.join(ROOT, "profiles", f"fine_op_fp32_column_{nx}x{ny}x{nz}.txt")
+    path = os.path.join(ROOT, "profiles", f"fine_op_fp32_{nx}x{ny}x{nz}.txt")
     try:
         with open(path) as f:
             for line in f:
@@ -392,8 +392,8 @@ def run_ours(args, world, rank, local, pg):
         "fp64_operator": {"ms_per_launch": m["op_fp64_ms"],
                           "reference_flops_per_launch": fp64_alg_flops,
                           "reference_equiv_tflops": fp64_alg_flops / (m["op_fp64_ms"] * 1e-3) / 1e12,
-                          "executed_fp64_ops_per_element": 212,
-                          "executed_tflops": 212 * nv / (m["op_fp64_ms"] * 1e-3) / 1e12,
+                          "executed_fp64_ops_per_element": 141,
+                          "executed_tflops": 141 * nv / (m["op_fp64_ms"] * 1e-3) / 1e12,
                           "fp64_fma_peak_tflops": fp64_peak, "fp32_fma_peak_tflops": fp32_peak},
         "forms": forms, "mixed_vs_fp64": acc,
     }
@@ -563,7 +563,7 @@ def run_homog(args):
                                "read back (per cell)"}
     line["roofline"] = None
     line["roofline_note"] = ("the batched periodic operator runs inside the lock-step solve only; "
-                             "its kernel is the pencil operator of the FP64 form (see the headline "
+                             "its kernel is the periodic form of the fine operator (see the headline "
                              "line for the fine operator's roofline)")
     if not args.no_cpu:
         port = oracle_port()

@@ -725,9 +725,10 @@ int tg_job_check_level1(tg_job* job, double* rel_diff);
 /* Kernels this library has launched in the process so far. */
 int64_t tg_kernel_launches(void);
 /* Level 1 of the mixed form's V-cycle: on (default) the Galerkin operator is
- * applied without a matrix, from the fine moduli (the name is historical: it was
- * a tensor-core kernel); off, as the assembled FP32 node stencil.  Applies to
- * solvers created afterwards. */
+ * applied without a matrix, from the fine moduli, where it has more than 32,768
+ * nodes (the name is historical: it was a tensor-core kernel); off, and on smaller
+ * levels always, as the assembled FP32 node stencil, which is faster there.  Applies
+ * to solvers created afterwards. */
 int tg_set_level1_tc(int32_t on);
 /* Level 1's Galerkin matrices in the mixed form with the matrix-free level 1:
  * on (default) the fast-path elements' matrices (sum_c E_c G_c) come

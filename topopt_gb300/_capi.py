@@ -959,9 +959,10 @@ APPLY_L1_STENCIL, APPLY_L1_TC = 3, 4
 
 
 def set_level1_tc(on: bool):
-    """Level 1 of the mixed V-cycle without a matrix, from the fine moduli (True,
-    default), or as the assembled FP32 stencil (False), for solvers created
-    afterwards.  (The name is historical: it was a tensor-core kernel.)"""
+    """Level 1 of the mixed V-cycle, where it has more than 32,768 nodes, without a
+    matrix, from the fine moduli (True, default), or as the assembled FP32 stencil
+    (False; smaller levels always), for solvers created afterwards.  (The name is
+    historical: it was a tensor-core kernel.)"""
     _check(lib().tg_set_level1_tc(int(bool(on))))
 
 
