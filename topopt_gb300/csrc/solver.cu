@@ -355,14 +355,16 @@ Solver::Solver(const FineProblem& fp, const tg_solve_options& opt, cudaStream_t 
   df_residual_ = opt.mixed_residual != TG_RESIDUAL_FP64;
   mixed_ = opt.precision == TG_PREC_MIXED;
   // Coarse levels >= 2 of the FP32 V-cycle: Chebyshev by default from 20,000 elements
-  // up, of degree 3 below 200,000 and 4 above, damped Jacobi on smaller grids.  A step
-  // of a small level costs 2 to 3 us, a fine level's part of an iteration 20 to 300:
-  // eight design iterations take 0.78 to 0.94 of their time with Jacobi from 48x24x24 to
-  // 108x62x28, 1.00 to 1.03 at 32x16x16 (at 1e-6; 0.96 to 0.99 at 1e-10); degree 4 takes
-  // 1.02 to 1.05 times degree 3 on 60x36x28 to 80x40x40 and 0.97 on 128x64x64.
+  // up, of degree 3 below 60,000 and 4 above, damped Jacobi on smaller grids.  A step of
+  // a small level costs 2 to 3 us, a fine level's part of an iteration 20 to 300: eight
+  // design iterations take 0.78 to 0.94 of their time with Jacobi from 48x24x24 to
+  // 108x62x28, 1.00 to 1.03 at 32x16x16 (at 1e-6; 0.96 to 0.99 at 1e-10).  Degree 4
+  // takes 1.02 to 1.05 times degree 3 there, but 0.75 to 0.94 in single solves of 24
+  // strongly graded designs each at 60x36x28, 80x40x40, 96x40x24 and 108x62x28, where it
+  // also falls back to FP64 less often (1.04 at 48x24x24), and 0.97 at 128x64x64.
   const bool cheb = opt.coarse_smoother == TG_SMOOTHER_CHEBYSHEV ||
                     (opt.coarse_smoother == TG_SMOOTHER_AUTO && fp.g.nv >= 20000);
-  const bool four = opt.coarse_smoother == TG_SMOOTHER_CHEBYSHEV || fp.g.nv >= 200000;
+  const bool four = opt.coarse_smoother == TG_SMOOTHER_CHEBYSHEV || fp.g.nv >= 60000;
   cheb_m_ = mixed_ && cheb ? (four ? 4 : 3) : 0;
   const size_t n = size_t(fp.g.ndof);
   for (DBuf<double>* b : {&invdiag_, &rhs_, &x_, &r_, &z_, &p_, &ap_, &t0_, &t1_}) b->alloc(n);
