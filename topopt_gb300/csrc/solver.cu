@@ -1278,27 +1278,30 @@ bool Solver::mgpcg(double tol, int max_it, bool warm, SolverStats& st) {
     if (k > 1) next_p();
     apply_update(k > 1, LoopCond{});
     ++fine_matvecs_;
+    bool graph = false;
+    if (k == 1 && max_it > 1 && use_graph_) {
+      // The capture, while the device works on this iteration.
+      if (ig64_ && ig64_->E != E_) ig64_.reset();
+      graph = ig64_ || capture_loop(ig64_, [&](cudaGraphConditionalHandle h) {
+                next_p();
+                apply_update(true, LoopCond{h, scal_.p + 1, scal_.p + 11, istate_.p});
+              });
+    }
     double sc[2];
     read_scalars(1, 2, sc);
     if (!(sc[0] > 0.0) || !std::isfinite(sc[0])) return false;
     st.iterations = k;
     st.residual = std::sqrt(sc[1]) / bnorm;
     if (std::sqrt(sc[1]) <= threshold) return finish(sc[1]);
-    if (k == 1 && max_it > 1 && use_graph_) {
+    if (graph) {
       // Iterations 2.. on the device: one graph launch, one read-back.
-      if (ig64_ && ig64_->E != E_) ig64_.reset();
-      if (ig64_ || capture_loop(ig64_, [&](cudaGraphConditionalHandle h) {
-            next_p();
-            apply_update(true, LoopCond{h, scal_.p + 1, scal_.p + 11, istate_.p});
-          })) {
-        int done = 0, broke = 0;
-        run_loop(*ig64_, threshold, 1, max_it, &done, &broke);
-        const int64_t runs = int64_t(done - 1) + broke;  // body executions
-        add_kernel_launches(runs * ig64_->body_launches);
-        fine_matvecs_ += (2 * sweeps_ + 1) * runs;
-        st.iterations = done;
-        return finish(h_scal_[2]) && !broke;
-      }
+      int done = 0, broke = 0;
+      run_loop(*ig64_, threshold, 1, max_it, &done, &broke);
+      const int64_t runs = int64_t(done - 1) + broke;  // body executions
+      add_kernel_launches(runs * ig64_->body_launches);
+      fine_matvecs_ += (2 * sweeps_ + 1) * runs;
+      st.iterations = done;
+      return finish(h_scal_[2]) && !broke;
     }
   }
   return false;
@@ -1315,8 +1318,6 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
   launch_dot_f(rf_.p, rf_.p, n, sum_to(10, 0), s_);
   float* z = vcycle<float>(rf_.p, scal_.p + 6);
   TG_CUDA(cudaMemcpyAsync(pf_.p, z, size_t(n) * sizeof(float), cudaMemcpyDeviceToDevice, s_));
-  const double b2 = read_scalar(10);
-  const double thr = rel_tol * std::sqrt(b2);
   // p.Ap into scal_[7] (and rz_new, scal_[9], into rz, scal_[6]), then r with r.r
   // into scal_[8].  x += alpha p when p is next overwritten or at exit (flush_x),
   // or on the side stream beside the next V-cycle's coarse levels (fork_x).
@@ -1339,12 +1340,23 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
     launch_cg_update_p<float>(pf_.p, zn, scal_.p + 9, scal_.p + 6, n, s_);
   };
   *iters = 0;
+  double thr = 0.0;
   for (int k = 1; k <= max_it; ++k) {
     if (k > 1) next_p();
     apply_update(k > 1, LoopCond{});
     ++lowp_matvecs_;
-    double sc[2];
-    read_scalars(7, 2, sc);
+    // The first solve's capture, while the device works on this iteration.
+    const bool graph =
+        k == 1 && max_it > 1 && use_graph_ &&
+        (ig_ || capture_loop(ig_, [&](cudaGraphConditionalHandle h) {
+           pending_x_ = true;  // every body execution starts with the last one's x update
+           next_p();
+           apply_update(true, LoopCond{h, scal_.p + 7, scal_.p + 11, istate_.p});
+         }));
+    pending_x_ = true;
+    double sc[4];
+    read_scalars(7, k == 1 ? 4 : 2, sc);
+    if (k == 1) thr = rel_tol * std::sqrt(sc[3]);  // r.r at the start, in scal_[10]
     if (!(sc[0] > 0.0) || !std::isfinite(sc[0])) {  // breakdown: alpha = 0, x and r untouched
       flush_x();
       ++st.inner_breakdowns;
@@ -1355,15 +1367,10 @@ bool Solver::inner_pcg<float>(int max_it, double rel_tol, SolverStats& st, int* 
       flush_x();
       return true;
     }
-    if (k == 1 && max_it > 1 && use_graph_ &&
-        (ig_ || capture_loop(ig_, [&](cudaGraphConditionalHandle h) {
-           pending_x_ = true;  // every body execution starts with the last one's x update
-           next_p();
-           apply_update(true, LoopCond{h, scal_.p + 7, scal_.p + 11, istate_.p});
-         }))) {
-      // Iterations 2.. on the device: one graph launch, one read-back.
+    if (graph) {
+      // Iterations 2.. on the device: one graph launch, one read-back; the last body
+      // execution's x update runs behind the graph.
       int done = 0, broke = 0;
-      pending_x_ = true;  // the last body execution's x update, run behind the graph
       run_loop(*ig_, thr, 1, max_it, &done, &broke);
       const int64_t runs = int64_t(done - 1) + broke;  // body executions
       add_kernel_launches(runs * ig_->body_launches);
