@@ -20,8 +20,9 @@
 // multiply-adds; on the tensor cores (three TF32 products for FP32 accuracy) they
 // were bound by each batch's chain stage -> MMA -> commit -> read back: 66 us on
 // the 256x128x128 cantilever's level 1 and 43-53 us on small ones (24x8x8 to
-// 128x64x64); this kernel with its pre-pass takes 41 us there, and 10-15 us on
-// those (17 us and 142 us for the assembled stencil on the two largest).
+// 128x64x64); this kernel with its pre-pass takes 40 us there, and 6-17 us on
+// those.  The assembled stencil takes 105 us there and 16.5 at 128x64x64, but 4 to
+// 10 up to 32,768 nodes, where the V-cycle uses it instead.
 //
 // Coarse elements that touch a Dirichlet DOF, an inactive coarse DOF or an odd
 // axis's half element use their stored matrix: a pre-pass (one warp per element)
