@@ -103,11 +103,14 @@ __device__ __forceinline__ double block_scalar(const F& f) {
 // x += alpha p; r -= alpha Ap with alpha = rz / pAp; sum of r.r (FP64).  With x0
 // set, also x0 = omega invdiag .* r.  The FP64 PCG's update; the FP32 inner PCG
 // runs it as two kernels below.
+// NEXT: 0 as it is, 1 with x0, 2 with x0 and r.x0 (a template, since an FP64 product that
+// nobody reads still takes its 19 cycles of the SM).
+template <int NEXT>
 __global__ void k_cg_update_xr(double* x, double* r,
                                const double* p, const double* ap,
                                const double* rz, const double* pap,
                                int64_t n, const double* invdiag, double omega,
-                               double* x0, SumOut o) {
+                               double* x0, SumOut o, SumOut oz) {
   behind_previous();
   // A non-positive or non-finite pAp is a breakdown the host reports; leave the
   // iterate untouched so the last good x survives.
@@ -115,13 +118,15 @@ __global__ void k_cg_update_xr(double* x, double* r,
     const double pp = *pap;
     return (pp > 0.0 && isfinite(pp)) ? *rz / pp : 0.0;
   });
-  double t = 0.0;
-  const bool next = x0 != nullptr;
+  double t = 0.0, tz = 0.0;
+  constexpr bool next = NEXT > 0;
   auto one = [&](double& xv, double pv, double& rv, double qv, double dv) {
     xv += a * pv;
     rv -= a * qv;
     t += rv * rv;
-    return omega * dv * rv;
+    const double zv = next ? omega * dv * rv : 0.0;
+    if constexpr (NEXT == 2) tz += rv * zv;
+    return zv;
   };
   // Pairs, two a round: all of a round's loads before its first store, since the
   // compiler may not move them past one.
@@ -161,6 +166,7 @@ __global__ void k_cg_update_xr(double* x, double* r,
     r[n - 1] = rv;
     if (next) x0[n - 1] = zv;
   }
+  if constexpr (NEXT == 2) grid_sum(tz, oz, int(blockIdx.x), int(gridDim.x));
   grid_sum(t, o, int(blockIdx.x), int(gridDim.x));
 }
 
@@ -434,9 +440,13 @@ void launch_sum_partials(const double* part, int n, double* out, cudaStream_t s)
 
 void launch_cg_update_xr(double* x, double* r, const double* p, const double* ap,
                          const double* rz, const double* pap, int64_t n, const SumOut& rr,
-                         cudaStream_t s, const double* invdiag, double omega, double* x0) {
-  launch_behind(k_cg_update_xr, red_blocks(n), kThreads, 0, s, x, r, p, ap, rz, pap, n, invdiag,
-                omega, x0, rr);
+                         cudaStream_t s, const double* invdiag, double omega, double* x0,
+                         const SumOut& r_x0) {
+  auto kernel = x0 == nullptr          ? k_cg_update_xr<0>
+                : r_x0.part == nullptr ? k_cg_update_xr<1>
+                                       : k_cg_update_xr<2>;
+  launch_behind(kernel, red_blocks(n), kThreads, 0, s, x, r, p, ap, rz, pap, n, invdiag, omega, x0,
+                rr, r_x0);
   TG_LAUNCH_CHECK();
 }
 

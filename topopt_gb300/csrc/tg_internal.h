@@ -253,11 +253,11 @@ void launch_dot_f(const float* a, const float* b, int64_t n, const SumOut& o, cu
 void launch_sum_partials(const double* part, int n, double* out, cudaStream_t s);
 // PCG pieces with scalars living in device memory (no host round trip): x += alpha
 // p, r -= alpha Ap with alpha = rz / pAp (0 on a breakdown), sum of r.r; with x0
-// set, also x0 = omega invdiag .* r.
+// set, also x0 = omega invdiag .* r, and with r_x0 its sum r.x0.
 void launch_cg_update_xr(double* x, double* r, const double* p, const double* ap,
                          const double* rz, const double* pap, int64_t n, const SumOut& rr,
                          cudaStream_t s, const double* invdiag = nullptr, double omega = 0.0,
-                         double* x0 = nullptr);
+                         double* x0 = nullptr, const SumOut& r_x0 = SumOut{});
 // The FP32 PCG update in two kernels: r (and x0) with r.r, and x.
 void launch_cg_update_r_f(float* r, const float* ap, const double* rz, const double* pap,
                           int64_t n, const SumOut& rr, cudaStream_t s,
