@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
     // Writes node row i of layer ez from its x-modes r[k][2].
     auto finish = [&](int i, const S (&r)[3][2]) {
       S nd = czero<S>();
-      T* const yl = at(y + 3 * int64_t(oz), unsigned(3 * sizeof(T)) * unsigned(no[i]));
+      T* const yl = at(y + 3 * int64_t(oz), node_bytes<T, sizeof(T) == 4>(no[i]));
       if constexpr (kPipe) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "tg_df.h"
+#include "tg_index.h"
 #include "tg_internal.h"
 
 namespace tg {
@@ -190,12 +191,6 @@ __device__ __forceinline__ df shfl_at(df v, int l) {
 constexpr int kDepth = 3;      // layers copied ahead
 constexpr int kRowWords = 96;  // a copied row: 32 nodes x 3 components
 
-// base (the same for every lane) + an unsigned byte offset: one address operand.
-template <class P>
-__device__ __forceinline__ P* at(P* base, unsigned bytes) {
-  using B = typename std::conditional<std::is_const<P>::value, const char, char>::type;
-  return reinterpret_cast<P*>(reinterpret_cast<B*>(base) + bytes);
-}
 __device__ __forceinline__ void copy_word(unsigned dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
