@@ -38,3 +38,29 @@ def test_fp64_layer_beyond_32_bits(tg):
         assert (got[:, r:r + PERIOD] - want).abs().max() < bound, r
     del got
     torch.cuda.empty_cache()
+
+
+def test_fp32_periodic_layer_beyond_32_bits(tg):
+    """A periodic cell of 20,000 x 18,000 x 1: 360,000,000 nodes of 12 bytes.  FP32
+    schedules are held to 2e-6."""
+    import torch
+    from native import I, ModalConsts, call
+    nx, ny = 20000, 18000
+    gen = torch.Generator("cuda").manual_seed(6)
+    ef = torch.rand(1, PERIOD, nx, device="cuda", generator=gen) + 1e-3
+    x = torch.randn(1, PERIOD, nx, 3, device="cuda", generator=gen)
+
+    def apply(rows):
+        y = torch.full((1, rows, nx, 3), torch.nan, device="cuda")
+        call(tg, "_ZN2tg18launch_periodic_opIfEEviiiiRKNS_11ModalConstsEPKT_PKhS6_S6_PS4_Pdii"
+             "PKiP11CUstream_st", I(0), I(nx), I(rows), I(1), ModalConsts(), repeats(torch, ef, rows),
+             None, repeats(torch, x, rows), None, y, None, I(1), I(1), None, None)
+        return y
+
+    want = apply(PERIOD)
+    bound = 2e-6 * want.abs().max()
+    got = apply(ny)
+    for r in range(0, ny, PERIOD):
+        assert (got[:, r:r + PERIOD] - want).abs().max() < bound, r
+    del got
+    torch.cuda.empty_cache()

@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
     // Writes node row i of layer ez from its x-modes r[k][2].
     auto finish = [&](int i, const S (&r)[3][2]) {
       S nd = czero<S>();
-      T* const yl = at(y + 3 * int64_t(oz), node_bytes<T, sizeof(T) == 4>(no[i]));
+      T* const yl = at(y + 3 * int64_t(oz), node_bytes<T, kPipe>(no[i]));
       if constexpr (kPipe) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -1004,20 +1004,31 @@ template void launch_fine_op<float>(int, const Grid&, const ModalConsts&, const 
 // (kApply) receives one partial of x.y per CTA, the CTAs of a system
 // contiguous: periodic_op_blocks<T>() per system.
 namespace {
-template <class T>
-using PerV = typename std::conditional<std::is_same<T, float>::value, float2, double>::type;
 // One tile per cell size, whatever the batch, so that a system's partial sums
 // and with them its iterates do not depend on who else runs: the tile of four
 // cells' worth of strains, between a single cell's and a full GPU's.
 constexpr int kTileSystems = 24;
-template <class T>
+template <class V>
 MarchTile periodic_tile(int nx, int ny, int nz) {
-  return march_tile<PerV<T>>(nx, ny, nz, kTileSystems, true);
+  return march_tile<V>(nx, ny, nz, kTileSystems, true);
+}
+// f of a value of the type that the cell's rows are carried in: FP32 rows in pairs,
+// whose offsets within a layer are 32 bits, unless the layer is too large for that (one
+// of more than 357,913,941 nodes, a cell of a single one).
+template <class T, class F>
+auto periodic_rows(int nx, int ny, F&& f) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (narrow_layer(int64_t(nx) * ny)) return f(float2{});
+  }
+  return f(T{});
 }
 }  // namespace
 template <class T>
 int periodic_op_blocks(int nx, int ny, int nz) {
-  return blocks_of(march_grid<PerV<T>>(nx, ny, nz, 1, true, periodic_tile<T>(nx, ny, nz)));
+  return periodic_rows<T>(nx, ny, [&](auto v) {
+    using V = decltype(v);
+    return blocks_of(march_grid<V>(nx, ny, nz, 1, true, periodic_tile<V>(nx, ny, nz)));
+  });
 }
 template int periodic_op_blocks<double>(int, int, int);
 template int periodic_op_blocks<float>(int, int, int);
@@ -1026,17 +1037,19 @@ template <class T>
 void launch_periodic_op(int mode, int nx, int ny, int nz, const ModalConsts& c, const T* ef,
                         const uint8_t* kn, const T* x, const T* b, T* y, double* dot_part,
                         int nsys, int nrhs, const int* run, cudaStream_t s) {
-  using V = PerV<T>;
   const GridDev gd{nx, ny, nz, nx, ny, nz};
   const int64_t nv = int64_t(nx) * ny * nz;
-  const MarchTile t = periodic_tile<T>(nx, ny, nz);
   const BatchDev bd{nrhs, 3 * nv, nv, run, periodic_flat(nx) ? 1 : 0};
-  if (mode == kApply)
-    launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
-                                     SumOut{dot_part}, bd, s);
-  else
-    launch_march<V, T, kResidual, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
-                                        SumOut{}, bd, s);
+  periodic_rows<T>(nx, ny, [&](auto v) {
+    using V = decltype(v);
+    const MarchTile t = periodic_tile<V>(nx, ny, nz);
+    if (mode == kApply)
+      launch_march<V, T, kApply, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
+                                       SumOut{dot_part}, bd, s);
+    else
+      launch_march<V, T, kResidual, true>(gd, t, nsys, c, ef, kn, x, b, nullptr, T(0), y,
+                                          SumOut{}, bd, s);
+  });
 }
 template void launch_periodic_op<double>(int, int, int, int, const ModalConsts&, const double*,
                                          const uint8_t*, const double*, const double*, double*,

@@ -22,10 +22,14 @@ TG_HD P* at(P* base, O bytes) {
   return reinterpret_cast<P*>(reinterpret_cast<B*>(base) + bytes);
 }
 
+// Whether FP32 may address the nodes of a layer, 12 bytes each, by 32-bit byte offsets.
+// Every layer of a bounded grid: DOF indices fit 32 bits, so one (of at least two) has
+// at most 357,913,941 nodes.  A periodic cell's single layer may have twice as many.
+TG_HD bool narrow_layer(int64_t nodes) { return 12 * nodes <= int64_t(1) << 32; }
+
 // Bytes from a layer's first node to node `no` of a vector of T, three components a
-// node: 32 bits with kNarrow, which FP32 on a bounded grid may use -- DOF indices fit 32
-// bits, so a layer (of at least two) has at most 357,913,941 nodes of 12 bytes.  FP64's
-// 24 bytes pass 2^32 from the 178,956,971st node on.
+// node, in 32 bits with kNarrow.  FP64's 24 bytes pass 2^32 from the 178,956,971st node
+// on.
 template <class T, bool kNarrow>
 TG_HD auto node_bytes(int no) {
   using B = typename std::conditional<kNarrow, unsigned, int64_t>::type;
