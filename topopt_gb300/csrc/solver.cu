@@ -17,10 +17,9 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
-#include <system_error>
-#include <thread>
 #include <unordered_map>
 
+#include "tg_host_parallel.h"
 #include "tg_solver.h"
 
 namespace tg {
@@ -106,38 +105,6 @@ void hex8_ke(double E, double nu, double h, double* ke) {
 }
 
 // ------------------------------------------------------------- FineProblem
-// fn(lo, hi, part) over [0, n) split across host threads.  The loops it runs are byte
-// and integer work with per-part results combined exactly, so the outcome does not
-// depend on the split.  Serial where the whole is less than 2^20 nodes' worth: starting
-// sixteen threads took 0.5 to 1.8 ms, a loop over 200,000 nodes 0.2.
-template <class F>
-static void host_parallel(int64_t n, int64_t nodes, F&& fn) {
-  const unsigned hc = std::thread::hardware_concurrency();
-  const int nt = int(std::max(1u, std::min(16u, hc)));
-  if (nodes < (int64_t(1) << 20) || nt == 1) {
-    fn(0, n, 0);
-    return;
-  }
-  std::vector<std::thread> th;
-  th.reserve(size_t(nt));
-  const int64_t chunk = (n + nt - 1) / nt;
-  int t = 0;
-  for (; t < nt; ++t) {
-    const int64_t lo = t * chunk, hi = std::min(n, lo + chunk);
-    if (lo >= hi) continue;
-    try {
-      th.emplace_back([&fn, lo, hi, t] { fn(lo, hi, t); });
-    } catch (const std::system_error&) {
-      break;  // no thread to be had (many jobs building at once): the rest runs here
-    }
-  }
-  for (; t < nt; ++t) {
-    const int64_t lo = t * chunk, hi = std::min(n, lo + chunk);
-    if (lo < hi) fn(lo, hi, t);
-  }
-  for (std::thread& x : th) x.join();
-}
-
 // v = 0 but for the listed entries (one per DOF).
 static void scatter_entries(const DBuf<double>& v,
                             const std::vector<std::pair<int64_t, double>>& list, cudaStream_t s) {
@@ -211,7 +178,7 @@ void FineProblem::build(const tg_grid& grid, double poisson, const tg_dirichlet_
   // neighbours.
   kept_h.resize(size_t(g.ndof));
   kept_node_h.resize(size_t(g.nnodes));
-  int64_t kept_part[16] = {};
+  int64_t kept_part[kHostParts] = {};
   host_parallel(int64_t(g.nny) * g.nnz, g.nnodes, [&](int64_t lo, int64_t hi, int part) {
     std::vector<uint8_t> row(size_t(g.nx) + 2, 0);
     int64_t nk = 0;
