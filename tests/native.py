@@ -34,6 +34,14 @@ class SumOut(C.Structure):
                 ("cond", LoopCond)]
 
 
+class MgDims(C.Structure):
+    """A level's extents (tg_multigrid.h)."""
+    _fields_ = [(n, I) for n in ("ex", "ey", "ez", "nnx", "nny", "nnz", "align")]
+
+    def __init__(self, ex, ey, ez, align=0):
+        super().__init__(ex, ey, ez, ex + 1, ey + 1, ez + 1, align)
+
+
 def ptr(t):
     return None if t is None else P(t.data_ptr())
 

@@ -24,7 +24,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <type_traits>
 
@@ -842,15 +841,11 @@ void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalCo
   const size_t smem = size_t(2) * t.W * 192 * sizeof(S) +
                       (RowsOf<V>::R == 2 ? size_t(t.W) * (kDepth + 1) * slot_words<MODE>() * 4 : 0);
   if constexpr (RowsOf<V>::R == 2) {
-    // More than the default 48 KB: once per process and mode (any thread may be
-    // first; the attribute is the same).
-    static std::atomic<bool> done{false};
-    if (!done.load()) {
-      constexpr int most = RowsOf<V>::kMaxWarps * (2 * 192 + (kDepth + 1) * slot_words<MODE>()) * 4;
-      TG_CUDA(cudaFuncSetAttribute(k_fine_march<V, T, MODE, PER>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-      done.store(true);
-    }
+    // More than the default 48 KB.  On every call, since the limit belongs to the kernel
+    // in the current device's context, and the same value from every thread.
+    constexpr int most = RowsOf<V>::kMaxWarps * (2 * 192 + (kDepth + 1) * slot_words<MODE>()) * 4;
+    TG_CUDA(cudaFuncSetAttribute(k_fine_march<V, T, MODE, PER>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, most));
   }
   // Only the public apply takes values at nodes of absent elements; within the
   // solver (a kept mask) they are zeros.
