@@ -18,7 +18,8 @@
 // converged system freezes (its own iteration count and iterate are exactly what
 // a solo solve would give).  Mixed precision: FP64 iterative refinement (FP64
 // residual b - A x) around lock-step FP32 Jacobi-PCG inner solves on the
-// unit-norm residual, FP64 dot products throughout.  The CH sum is evaluated as
+// unit-norm residual; the dot products that alpha and beta take across a system are as
+// accurate as FP64 sums.  The CH sum is evaluated as
 //   CH[I][J] = (n_solid chi0_I^T ke chi0_J - F_I . chi_J) / |Y|,
 // the same sum regrouped: sum_e chi0_I^T ke chi_J,e = F_I . chi_J.
 #include <cuda_runtime.h>
@@ -31,6 +32,7 @@
 #include <vector>
 
 #include "tg_solver.h"
+#include "tg_sum3.h"
 
 namespace tg {
 namespace {
@@ -115,17 +117,26 @@ __device__ __forceinline__ double bred(double v, double* sh) {
   return s;
 }
 
-// Running sums of r.r and r.(D^-1 r).  FP64 data: FP64.  FP32 data: each product
-// exact as a value and its rounding error (one FMA), accumulated as an unevaluated
-// FP32 pair (Knuth's TwoSum; the errors in the low part), about 2^-46 relative.
-// Alpha and beta, rounded to FP32, and the iteration counts come out the same as
-// from FP64 sums, whose five instructions per DOF on units 58 times slower took
-// twice the operator's time (24 systems of 32^3: 34 us against 17).
+// A power of two that brings the inverse diagonal to at most 1, and its inverse.
+struct RzScale {
+  float up = 1.0f;
+  double down = 1.0;
+};
+
+// Running sums of r.r and r.(D^-1 r).  FP64 data: FP64.  FP32 data: every product
+// exactly, as FP32 values, in sums of three FP32 values each (tg_sum3.h); FP64 from the
+// warps' totals on.  FP64 sums of FP32 products take five instructions per DOF on units
+// 64 times slower, twice the operator's time (24 systems of 32^3: 34 us against 17).
+// Of 98,304 products they are off by up to 2^-52 of the sum, the sums of three by 2^-68
+// before their one rounding to FP64 (sums of two, 2^-45, would not do:
+// tests/test_sum3.py).  D^-1 is scaled to at most 1, exactly, so that no modulus takes
+// the products' errors out of FP32's range.
 template <class T>
 struct RrRz;
 template <>
 struct RrRz<double> {
   double a = 0.0, b = 0.0;
+  __device__ __forceinline__ explicit RrRz(const RzScale&) {}
   __device__ __forceinline__ void add(double v, double iv) {
     a += v * v;
     b += v * (iv * v);
@@ -141,38 +152,47 @@ struct RrRz<double> {
 };
 template <>
 struct RrRz<float> {
-  float ah = 0.0f, al = 0.0f, bh = 0.0f, bl = 0.0f;
-  __device__ __forceinline__ void add(float v, float iv) {
-    const float p = __fmul_rn(v, v), pe = __fmaf_rn(v, v, -p);
-    const df s = two_sum(ah, p);
-    ah = s.hi;
-    al = __fadd_rn(al, __fadd_rn(s.lo, pe));
-    const float q = __fmul_rn(iv, v), qe = __fmaf_rn(iv, v, -q);
-    const float m = __fmul_rn(q, v), me = __fmaf_rn(qe, v, __fmaf_rn(q, v, -m));
-    const df t = two_sum(bh, m);
-    bh = t.hi;
-    bl = __fadd_rn(bl, __fadd_rn(t.lo, me));
+  Sum3<float2> a{}, b{};  // the DOFs of even and odd place in a run of four
+  RzScale sc;
+  __device__ __forceinline__ explicit RrRz(const RzScale& s) : sc(s) {}
+  __device__ __forceinline__ void add(float2 v, float2 iv) {
+    sum3_square(a, v);
+    sum3_weighted_square(b, vmul(iv, make_float2(sc.up, sc.up)), v);
   }
-  // Across the warp as pairs too (an FP64 addition holds its scheduler 64 cycles),
-  // then one FP64 sum over the warps.
+  __device__ __forceinline__ void add(float v, float iv) {
+    add(make_float2(v, 0.0f), make_float2(iv, 0.0f));
+  }
+  // Across the warp as sums of three too (an FP64 addition holds its scheduler 64
+  // cycles), r.r in the first half and r.(D^-1 r) in the second; then sixteen lanes turn
+  // the eight warps' totals to FP64 and add them up.
   __device__ __forceinline__ void store(double* prr, double* prz, double* sh) const {
-    df a = quick_two_sum(ah, al), b = quick_two_sum(bh, bl);
+    constexpr int kW = kT / 32;
+    static_assert(kW == 8, "eight lanes a sum");
+    float* const tot = reinterpret_cast<float*>(sh);  // [2][kW][3]
+    Sum3<float2> s = sum3_join(
+        Sum3<float2>{make_float2(a.h.x, b.h.x), make_float2(a.m.x, b.m.x), make_float2(a.l.x, b.l.x)},
+        Sum3<float2>{make_float2(a.h.y, b.h.y), make_float2(a.m.y, b.m.y), make_float2(a.l.y, b.l.y)});
+    auto from = [](float2 v, int o) {
+      return make_float2(__shfl_down_sync(0xffffffffu, v.x, o),
+                         __shfl_down_sync(0xffffffffu, v.y, o));
+    };
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a = a + df(__shfl_down_sync(0xffffffffu, a.hi, o), __shfl_down_sync(0xffffffffu, a.lo, o));
-      b = b + df(__shfl_down_sync(0xffffffffu, b.hi, o), __shfl_down_sync(0xffffffffu, b.lo, o));
-    }
+    for (int o = 16; o > 0; o >>= 1)
+      s = sum3_join(s, Sum3<float2>{from(s.h, o), from(s.m, o), from(s.l, o)});
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) {
-      sh[wid] = df_to_double(a);
-      sh[kT / 32 + wid] = df_to_double(b);
+      float *t0 = tot + 3 * wid, *t1 = tot + 3 * (kW + wid);
+      t0[0] = s.h.x, t0[1] = s.m.x, t0[2] = s.l.x;
+      t1[0] = s.h.y, t1[1] = s.m.y, t1[2] = s.l.y;
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
-      double t = 0.0;
-      for (int q = 0; q < kT / 32; ++q) t += sh[threadIdx.x * (kT / 32) + q];
-      *(threadIdx.x == 0 ? prr : prz) = t;
-    }
+    if (wid != 0) return;
+    const float* t = tot + 3 * (lane & 15);
+    double v = sum3_total(t[0], t[1], t[2]);
+#pragma unroll
+    for (int o = kW / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, kW);
+    if (lane == 0) *prr = v;
+    if (lane == kW) *prz = v * sc.down;
   }
 };
 
@@ -191,12 +211,13 @@ __device__ __forceinline__ void share(int64_t nd, F4&& f4, F1&& f1) {
 // rr = r.r, rz = r.(D^-1 r) per system.
 template <class T>
 __global__ void k_b_rr_rz(const T* __restrict__ R, const T* __restrict__ invd, int64_t nd,
-                          int nrhs, double* __restrict__ prr, double* __restrict__ prz) {
+                          int nrhs, RzScale sc, double* __restrict__ prr,
+                          double* __restrict__ prz) {
   __shared__ double sh[32];
   const int bi = blockIdx.y, P = gridDim.x;
   const T* r = R + bi * nd;
   const T* iv = invd + (bi / nrhs) * nd;
-  RrRz<T> acc;
+  RrRz<T> acc(sc);
   for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd; d += int64_t(P) * kT)
     acc.add(r[d], iv[d]);
   acc.store(prr + int64_t(bi) * P + blockIdx.x, prz + int64_t(bi) * P + blockIdx.x, sh);
@@ -297,17 +318,18 @@ __global__ void k_b_init(int B, const double* __restrict__ rr, const double* __r
 
 // x += alpha p, r -= alpha t for iterating systems (alpha = absNew / p.Ap, p.Ap the
 // sum of the operator's npap partials, kept in pap), with the partials of r.r and
-// r.(D^-1 r) of the updated residual.
+// r.(D^-1 r) of the updated residual.  Five CTAs an SM, at the price of 40 bytes spilled
+// in FP32: 32 cells of 32^3 82.6 -> 81.0 ms.
 template <class T>
-__global__ void __launch_bounds__(kT) k_b_xr(T* __restrict__ X, T* __restrict__ R,
+__global__ void __launch_bounds__(kT, 5) k_b_xr(T* __restrict__ X, T* __restrict__ R,
                                              const T* __restrict__ Pv, const T* __restrict__ Tv,
                                              const T* __restrict__ invd, int64_t nd, int nrhs,
                                              const double* __restrict__ absn,
                                              const double* __restrict__ ppap, int npap,
                                              double* __restrict__ pap,
-                                             const int* __restrict__ act,
+                                             const int* __restrict__ act, RzScale sc,
                                              double* __restrict__ prr, double* __restrict__ prz) {
-  __shared__ double sh[32];
+  __shared__ double sh[32];  // [2][kT / 32][3] floats in FP32
   __shared__ double s_pa;
   const int bi = blockIdx.y, P = gridDim.x;
   if (act[bi] != 1) return;  // uniform over the CTA; its partials are not read
@@ -326,7 +348,7 @@ __global__ void __launch_bounds__(kT) k_b_xr(T* __restrict__ X, T* __restrict__ 
   T* r = R + bi * nd;
   const T* p = Pv + bi * nd;
   const T* t = Tv + bi * nd;
-  RrRz<T> acc;
+  RrRz<T> acc(sc);
   share<T>(
       nd,
       [&](int64_t q) {
@@ -339,10 +361,10 @@ __global__ void __launch_bounds__(kT) k_b_xr(T* __restrict__ X, T* __restrict__ 
         rv.x -= al * tv.x; rv.y -= al * tv.y; rv.z -= al * tv.z; rv.w -= al * tv.w;
         reinterpret_cast<float4*>(x)[q] = xv;
         reinterpret_cast<float4*>(r)[q] = rv;
-        acc.add(T(rv.x), T(dv.x));
-        acc.add(T(rv.y), T(dv.y));
-        acc.add(T(rv.z), T(dv.z));
-        acc.add(T(rv.w), T(dv.w));
+        if constexpr (sizeof(T) == 4) {
+          acc.add(make_float2(rv.x, rv.y), make_float2(dv.x, dv.y));
+          acc.add(make_float2(rv.z, rv.w), make_float2(dv.z, dv.w));
+        }
       },
       [&](int64_t d) {
         x[d] += alpha * p[d];
@@ -485,6 +507,7 @@ struct Batch {
   int64_t nd;
   ModalConsts mc;
   const uint8_t* kept;
+  RzScale rzs;
   cudaStream_t s;
   DBuf<double> prr, prz, ppap, rr, rz, pap, thr, rhs2, absn, rn;
   DBuf<int> act, it, nact, run, nrun;  // absn, act and it: two buffers of B, used in turn
@@ -521,7 +544,7 @@ struct Batch {
           const int* runp, const double* r64) {
     k_b_begin<T><<<g2(), kT, 0, s>>>(r64, rn.p, invd, nd, nrhs, runp, X, R, Pv);
     TG_LAUNCH_CHECK();
-    k_b_rr_rz<T><<<g2(), kT, 0, s>>>(R, invd, nd, nrhs, prr.p, prz.p);
+    k_b_rr_rz<T><<<g2(), kT, 0, s>>>(R, invd, nd, nrhs, rzs, prr.p, prz.p);
     TG_LAUNCH_CHECK();
     k_bsum<<<wb(), 256, 0, s>>>(prr.p, P, B, rr.p, prz.p, rz.p);
     TG_LAUNCH_CHECK();
@@ -536,7 +559,7 @@ struct Batch {
       launch_periodic_op<T>(kApply, nx, ny, nz, mc, ef, kept, Pv, nullptr, Tv, ppap.p, B, nrhs,
                             act.p + in, s);
       k_b_xr<T><<<g2(), kT, 0, s>>>(X, R, Pv, Tv, invd, nd, nrhs, absn.p + in, ppap.p, Pop, pap.p,
-                                    act.p + in, prr.p, prz.p);
+                                    act.p + in, rzs, prr.p, prz.p);
       TG_LAUNCH_CHECK();
       k_b_p<T><<<g2(), kT, 0, s>>>(Pv, R, invd, nd, nrhs, prr.p, prz.p, P, thr.p, pap.p, max_it,
                                    act.p + in, act.p + out, absn.p + in, absn.p + out, it.p + in,
@@ -648,6 +671,10 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
     bt.mc = ModalConsts::make(poisson, spacing);
     bt.mc.kdiag = ke[0];
     bt.s = s;
+    // D^-1's entries are 1 / (n kdiag E), n = 1 .. 8.
+    const int ex = std::min(126, std::max(-126, std::ilogb(ke[0] * youngs_modulus)));
+    bt.rzs.up = float(std::ldexp(1.0, ex));
+    bt.rzs.down = std::ldexp(1.0, -ex);
     // All cells together: solving them a group at a time, so that a group's CG
     // vectors stay in L2, measured slower (32 cells of 32^3: 109 ms in groups of 8,
     // 96 in groups of 16, 80 at once) -- the launches of a group are too short to
@@ -716,7 +743,7 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
       k_to_f32<<<nb_cell, kT, 0, s>>>(invd.p, invd32.p, ncell * nd);
       TG_LAUNCH_CHECK();
       // |b|^2 and the outer threshold tol^2 |b|^2.
-      k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
+      k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.rzs, bt.prr.p, bt.prz.p);
       TG_LAUNCH_CHECK();
       k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, b2.p, nullptr, nullptr);
       TG_LAUNCH_CHECK();
@@ -733,7 +760,7 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
         if (ref > 0)
           launch_periodic_op<double>(kResidual, nx, ny, nz, bt.mc, ef.p, kept.p, X.p, Bv.p, R.p,
                                      nullptr, B, nrhs, bt.run.p, s);
-        k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
+        k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.rzs, bt.prr.p, bt.prz.p);
         TG_LAUNCH_CHECK();
         k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, bt.rr.p, nullptr, nullptr);
         TG_LAUNCH_CHECK();
