@@ -17,12 +17,8 @@ COUNTER = """
 static int calls = 0;
 extern "C" int limit_calls() { return calls; }
 extern "C" int cudaFuncSetAttribute(const void* f, int attr, int value) {
-<<<<<<< Updated upstream
   static auto real = (int (*)(const void*, int, int))dlsym(
       dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD), "cudaFuncSetAttribute");
-=======
-  static auto real = (int (*)(const void*, int, int))dlsym(RTLD_NEXT, "cudaFuncSetAttribute");
->>>>>>> Stashed changes
   if (attr == 8) ++calls;  // cudaFuncAttributeMaxDynamicSharedMemorySize
   return real(f, attr, value);
 }
