@@ -440,8 +440,8 @@ void oc_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_t
   const double m = double(fs.st.n);
   // + 8192 u: the fast pass runs in double-float arithmetic -- the split of its
   // four FP64 inputs (2^-49 each), the product, clamp and accumulation (~2^-46
-  // relative per operation over a per-thread run of a few dozen terms) -- far
-  // below the n u of the reference's own sequential sum.
+  // relative per operation over a per-thread run of n / (608 * 256) terms; the sums
+  // over threads are FP64) -- far below the n u of the reference's own sequential sum.
   const double eps =
       (n + 2.0 * (m + 1.0) + 12.0 + n / (double(kRedBlocks) * 256.0) + 64.0 + 8192.0) * u * 1.01;
   // Fast volumes are computed ahead, kmax lambdas per pass over the fields

@@ -1002,16 +1002,6 @@ __global__ void k_chol_update(double* __restrict__ D, int nc, int k0) {
   }
 }
 
-// An FP32 value as FP64: by integer operations where it is normal or zero, since the
-// conversion is an FP64-pipe instruction like the multiply-add it feeds.
-__device__ __forceinline__ double widen(double v) { return v; }
-__device__ __forceinline__ double widen(float v) {
-  const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu, sign = u & 0x80000000u;
-  if (m == 0u) return __hiloint2double(int(sign), 0);
-  if (m - 0x00800000u >= 0x7f000000u) return double(v);  // denormal, infinite, NaN
-  return __hiloint2double(int(sign | ((m >> 3) + (896u << 20))), int(u << 29));
-}
-
 // x = Ainv b on the compact numbering, gathered from / scattered to the level
 // vector (cidx and cdof null: Ainv is over the level's own numbering); one warp per
 // row of Ainv.  Each lane's products are one chain of FP64 multiply-adds, 64 cycles

@@ -405,15 +405,14 @@ __device__ __forceinline__ bool df_less(df a, df b) {
   return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
 }
 
-// Of each two lanes' 2 M candidates a lane keeps M, both lanes' parts added.
+// Of each two lanes' 2 M candidates a lane keeps M, both lanes' parts added in FP64.
 template <int M>
-__device__ __forceinline__ void fold_half(df* a, int lane, int off) {
+__device__ __forceinline__ void fold_half(double* a, int lane, int off) {
   const bool upper = (lane & off) != 0;
 #pragma unroll
   for (int j = 0; j < M; ++j) {
-    const df mine = upper ? a[j + M] : a[j], give = upper ? a[j] : a[j + M];
-    a[j] = mine + df(__shfl_xor_sync(0xffffffffu, give.hi, off),
-                     __shfl_xor_sync(0xffffffffu, give.lo, off));
+    const double mine = upper ? a[j + M] : a[j], give = upper ? a[j] : a[j + M];
+    a[j] = mine + __shfl_xor_sync(0xffffffffu, give, off);
   }
 }
 
@@ -421,11 +420,11 @@ __device__ __forceinline__ void fold_half(df* a, int lane, int off) {
 // c = 1/sqrt(lambda) in one pass over the fields, in double-float arithmetic on the
 // FP32 pipe (tg_df.h; ~2^-46 relative per operation, all terms positive).  These
 // volumes only decide bisection branches under a certified bound that includes this
-// arithmetic's error.  On small grids the sum over the block bounds the pass: K FP64
-// trees are K x 10 dependent adds of 64 cycles.  Here a warp's lanes exchange halves
-// of their candidates, so that the K sums take about K double-float adds, FP64 adds
-// up only the eight warps' totals, and the CTA that ends last adds up the CTAs'
-// shares.
+// arithmetic's error; from a thread's own run on the sums are FP64.  On small grids the
+// sum over the block bounds the pass: K FP64 trees are K x 10 dependent adds of 64
+// cycles.  Here a warp's lanes exchange halves of their candidates, so that the K sums
+// take 2 K adds, the eight warps' totals one each, and the CTA that ends last adds up
+// the CTAs' shares.
 template <int K>
 __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
     const df* __restrict__ sq, const df* __restrict__ lo, const df* __restrict__ hi,
@@ -451,15 +450,17 @@ __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
     }
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  fold_half<K / 2>(acc, lane, 16);
-  fold_half<K / 4>(acc, lane, 8);
-  fold_half<K / 8>(acc, lane, 4);
-  if constexpr (K == 16) fold_half<1>(acc, lane, 2);
-  df v = acc[0];
+  double sum[K];
 #pragma unroll
-  for (int off = kLanes / 2; off > 0; off >>= 1)
-    v = v + df(__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off));
-  if (lane % kLanes == 0) share[wid][lane / kLanes] = df_to_double(v);
+  for (int k = 0; k < K; ++k) sum[k] = widen(acc[k].hi) + widen(acc[k].lo);
+  fold_half<K / 2>(sum, lane, 16);
+  fold_half<K / 4>(sum, lane, 8);
+  fold_half<K / 8>(sum, lane, 4);
+  if constexpr (K == 16) fold_half<1>(sum, lane, 2);
+  double v = sum[0];
+#pragma unroll
+  for (int off = kLanes / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if (lane % kLanes == 0) share[wid][lane / kLanes] = v;
   __syncthreads();
   if (threadIdx.x < unsigned(cs.k)) {
     double s = 0.0;
@@ -1006,17 +1007,13 @@ void launch_mask_pins(const uint8_t* eff, int64_t n, double* xphys, cudaStream_t
 int exact_sum_blocks() { return kRedBlocks; }
 
 namespace {
-// CTAs of a pass over the voxels: two voxels a thread, so that a small grid's sums
-// are few, and at most kRedBlocks (the scratch; 4 CTAs an SM).
+// CTAs of a pass over the voxels: one voxel a thread, and at most kRedBlocks (the
+// scratch; 4 CTAs an SM).
 int pass_blocks(int64_t n) {
-  return int(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + 2 * kThreads - 1) / (2 * kThreads))));
+  return int(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + kThreads - 1) / kThreads)));
 }
-// The same where the pass is FP64-bound and has a grid row a candidate: one voxel a
-// thread.
-dim3 candidate_grid(int64_t n, int k) {
-  return dim3(unsigned(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + kThreads - 1) / kThreads))),
-              unsigned(k));
-}
+// The same with a grid row a candidate.
+dim3 candidate_grid(int64_t n, int k) { return dim3(unsigned(pass_blocks(n)), unsigned(k)); }
 }  // namespace
 
 void launch_oc_volume_multi(const double* sq, const double* lo, const double* hi,

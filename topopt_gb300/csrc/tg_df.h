@@ -50,6 +50,15 @@ __device__ __forceinline__ df df_split(double v) {
   if (e == 0u) return df(0.0f, 0.0f);
   return df_from(v);
 }
+// An FP32 value as FP64: by integer operations where it is normal or zero, since the
+// conversion is an FP64-pipe instruction like the multiply-add it feeds.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+  const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu, sign = u & 0x80000000u;
+  if (m == 0u) return __hiloint2double(int(sign), 0);
+  if (m - 0x00800000u >= 0x7f000000u) return double(v);  // denormal, infinite, NaN
+  return __hiloint2double(int(sign | ((m >> 3) + (896u << 20))), int(u << 29));
+}
 #endif
 __host__ __device__ __forceinline__ double df_to_double(df a) {
   return double(a.hi) + double(a.lo);
