@@ -429,7 +429,8 @@ void launch_dot(const double* a, const double* b, int64_t n, const SumOut& o, cu
 }
 
 void launch_dot_f(const float* a, const float* b, int64_t n, const SumOut& o, cudaStream_t s) {
-  k_dot<float><<<red_blocks(n), kThreads, 0, s>>>(a, b, n, o);
+  // One term a thread as far as the grid goes (155,648): a thread's run is FP32.
+  k_dot<float><<<stream_blocks(n), kThreads, 0, s>>>(a, b, n, o);
   TG_LAUNCH_CHECK();
 }
 
