@@ -718,9 +718,9 @@ int tg_filter_noalloc(int32_t nx, int32_t ny, int32_t nz, const uint8_t* d_tags,
  * mixed job (TG_APPLY_L1_STENCIL, TG_APPLY_L1_TC), over `reps` back-to-back
  * launches timed with CUDA events on the job's stream. */
 int tg_job_time_operator(tg_job* job, int32_t precision, int32_t reps, double* avg_ms);
-/* The level-1 operator of a mixed job's V-cycle on its current design, applied
- * to a seeded vector by the assembled FP32 stencil and by the matrix-free
- * operator: max |difference| / max |stencil result|. */
+/* The level-1 operator of a mixed job's V-cycle on its current design, as product,
+ * residual and smoothing sweep of seeded vectors, by the assembled FP32 stencil and by
+ * the matrix-free operator: the largest of max |difference| / max |stencil result|. */
 int tg_job_check_level1(tg_job* job, double* rel_diff);
 /* Kernels this library has launched in the process so far. */
 int64_t tg_kernel_launches(void);

@@ -1157,8 +1157,9 @@ class SimpJob:
         return x, xp
 
     def check_level1(self):
-        """Level-1 operator, matrix-free against the assembled FP32 stencil on a
-        seeded vector: max |difference| / max |stencil result|."""
+        """Level-1 operator (product, residual and smoothing sweep of seeded vectors),
+        matrix-free against the assembled FP32 stencil: the largest of
+        max |difference| / max |stencil result|."""
         d = C.c_double(0.0)
         _check(lib().tg_job_check_level1(self._h, C.byref(d)))
         return d.value

@@ -656,28 +656,41 @@ double Solver::check_level1() {
   level1_stencil();
   Level& L = *levels_[0];
   const size_t n = size_t(L.ndof);
-  std::vector<float> xh(n), a(n), bq(n);
+  std::vector<float> x(n), b(n), want(n), got(n);
   uint64_t h = 0x9E3779B97F4A7C15ull;
-  for (size_t i = 0; i < n; ++i) {
+  auto seeded = [&] {  // uniform in [-1/2, 1/2)
     h ^= h << 13;
     h ^= h >> 7;
     h ^= h << 17;
-    xh[i] = L.act_h[i] ? float(double(h >> 11) * (1.0 / 9007199254740992.0) - 0.5) : 0.0f;
+    return float(double(h >> 11) * (1.0 / 9007199254740992.0) - 0.5);
+  };
+  for (size_t i = 0; i < n; ++i) x[i] = L.act_h[i] ? seeded() : 0.0f;
+  TG_CUDA(cudaMemcpyAsync(L.X<float>(), x.data(), n * sizeof(float), cudaMemcpyHostToDevice, s_));
+  auto result = [&](std::vector<float>& v) {
+    TG_CUDA(cudaMemcpyAsync(v.data(), L.R<float>(), n * sizeof(float), cudaMemcpyDeviceToHost, s_));
+    TG_CUDA(cudaStreamSynchronize(s_));
+  };
+  double worst = 0.0;
+  for (int mode : {int(kApply), int(kResidual), int(kSmooth)}) {
+    mg_stencil_op<float>(mode, L.d, L.Am<float>(), L.act.p, L.X<float>(), L.B<float>(),
+                         L.Dinv<float>(), float(omega_), L.R<float>(), s_);
+    result(want);
+    level1_op(mode, L, float(omega_));
+    result(got);
+    double dmax = 0.0, amax = 0.0;
+    for (size_t i = 0; i < n; ++i) {
+      dmax = std::max(dmax, std::fabs(double(want[i]) - double(got[i])));
+      amax = std::max(amax, std::fabs(double(want[i])));
+    }
+    worst = std::max(worst, amax > 0.0 ? dmax / amax : dmax);
+    if (mode == kApply) {
+      // A right-hand side of the product's size everywhere, whatever the moduli there.
+      for (size_t i = 0; i < n; ++i) b[i] = 2.0f * seeded() * want[i];
+      TG_CUDA(cudaMemcpyAsync(L.B<float>(), b.data(), n * sizeof(float), cudaMemcpyHostToDevice,
+                              s_));
+    }
   }
-  TG_CUDA(cudaMemcpyAsync(L.X<float>(), xh.data(), n * sizeof(float), cudaMemcpyHostToDevice, s_));
-  mg_stencil_op<float>(kApply, L.d, L.Am<float>(), L.act.p, L.X<float>(), L.B<float>(),
-                       L.Dinv<float>(), 0.0f, L.R<float>(), s_);
-  TG_CUDA(cudaMemcpyAsync(a.data(), L.R<float>(), n * sizeof(float), cudaMemcpyDeviceToHost, s_));
-  TG_CUDA(cudaStreamSynchronize(s_));
-  level1_op(kApply, L, 0.0f);
-  TG_CUDA(cudaMemcpyAsync(bq.data(), L.R<float>(), n * sizeof(float), cudaMemcpyDeviceToHost, s_));
-  TG_CUDA(cudaStreamSynchronize(s_));
-  double dmax = 0.0, amax = 0.0;
-  for (size_t i = 0; i < n; ++i) {
-    dmax = std::max(dmax, std::fabs(double(a[i]) - double(bq[i])));
-    amax = std::max(amax, std::fabs(double(a[i])));
-  }
-  return amax > 0.0 ? dmax / amax : dmax;
+  return worst;
 }
 
 double Solver::time_operator(int form, int reps) {

@@ -73,8 +73,9 @@ class Solver {
   // Time `reps` fine-operator launches (FP64 or FP32) on the current factors.
   // form: 0 FP64, 1 FP32, 2 the double-float residual kernel.
   double time_operator(int form, int reps);
-  // Level 1 of the FP32 V-cycle applied to a seeded vector by the assembled
-  // stencil and by the matrix-free operator: max |difference| / max |stencil|.
+  // Level 1 of the FP32 V-cycle on seeded vectors by the assembled stencil and by the
+  // matrix-free operator, as product, residual and smoothing sweep: the largest of
+  // max |difference| / max |stencil|.
   double check_level1();
   size_t device_bytes() const;
   int levels() const { return int(levels_.size()) + 1; }
