@@ -1472,9 +1472,9 @@ bool Solver::jacobi_pcg(double tol, int max_it, bool warm, SolverStats& st) {
     return st.residual <= tol;
   }
   launch_scale_mask(p_.p, r_.p, invdiag_.p, n, sum_to(0, 3), s_);
-  // z = D^-1 r and r.z ride in the update that has r in registers while a thread holds
-  // one entry (red_blocks): 29.6 -> 28.5 us an iteration at 24x8x8, 46.9 -> 45.8 at
-  // 60x20x20.  Beyond, where the kernels are bound by their FP64 work, a launch of their
+  // z = D^-1 r and r.z ride in the update that has r in registers up to a CTA per SM of
+  // four entries a thread (red_blocks): 29.6 -> 28.5 us an iteration at 24x8x8, 46.9 ->
+  // 45.8 at 60x20x20.  Beyond, where the kernels are bound by their FP64 work, a launch of their
   // own is the faster one (96x48x48: 141.6 against 142.7).
   const bool with_r = n <= int64_t(152) * 1024;
   auto apply_update = [&](bool next, const LoopCond& cond) {
