@@ -1,5 +1,5 @@
-"""The volume pass of the OC bisection adds its threads' double-float terms up in FP64:
-terms whose sums need all of FP64's 53 bits, five more than a double-float has, come out
+"""The volume pass of the OC bisection adds its threads' double-float terms up to FP64's
+accuracy: terms whose sums need all of FP64's 53 bits, five more than a double-float has, come out
 exactly, on one warp's voxels and on one CTA's, for both candidate counts.  GPU only."""
 import ctypes as C
 

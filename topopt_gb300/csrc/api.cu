@@ -379,8 +379,9 @@ std::vector<double> bracket_ahead(double l2, int kmax) {
 // interpolation of log(lambda) through the interval's ends and the nearest value
 // outside.  A wrong prediction costs the rest of its pass and narrows the interval
 // for the next.  All paths at once instead (a binary tree) is four levels in 16
-// evaluations, seven passes an update; this way it is four.  With the passes' own
-// kernels an update went from 0.6 to 0.2 ms (60x20x20), from 2.45 to 1.86 ms
+// evaluations, seven passes an update of a small grid and 17 (of four evaluations) on
+// 256x128x128; this way it is four, and seven of eight evaluations there.  With the
+// passes' own kernels an update went from 0.6 to 0.2 ms (60x20x20), from 2.45 to 1.86 ms
 // (256x128x128), and projected from 1.1 to 0.26 ms (48x8x8).
 template <class Open>
 std::vector<double> bisect_ahead(const Evaluated& known, double l1, double l2, double target,
@@ -441,7 +442,8 @@ void oc_update_device(OcState& oc, FilterState& fs, const Grid& g, const uint8_t
   // + 8192 u: the fast pass runs in double-float arithmetic -- the split of its
   // four FP64 inputs (2^-49 each), the product, clamp and accumulation (~2^-46
   // relative per operation over a per-thread run of n / (608 * 256) terms; the sums
-  // over threads are FP64) -- far below the n u of the reference's own sequential sum.
+  // over threads have FP64's accuracy) -- far below the n u of the reference's own
+  // sequential sum.
   const double eps =
       (n + 2.0 * (m + 1.0) + 12.0 + n / (double(kRedBlocks) * 256.0) + 64.0 + 8192.0) * u * 1.01;
   // Fast volumes are computed ahead, kmax lambdas per pass over the fields

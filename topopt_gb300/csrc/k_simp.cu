@@ -25,6 +25,7 @@
 #include "tg_df.h"
 #include "tg_internal.h"
 #include "tg_reduce.h"
+#include "tg_sum3.h"
 
 namespace tg {
 
@@ -405,14 +406,18 @@ __device__ __forceinline__ bool df_less(df a, df b) {
   return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo);
 }
 
-// Of each two lanes' 2 M candidates a lane keeps M, both lanes' parts added in FP64.
+// Of each two lanes' 2 M pairs of candidates a lane keeps M, both lanes' parts added.
 template <int M>
-__device__ __forceinline__ void fold_half(double* a, int lane, int off) {
+__device__ __forceinline__ void fold_half(Sum3<float2>* a, int lane, int off) {
   const bool upper = (lane & off) != 0;
+  auto from = [off](float2 v) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, off),
+                       __shfl_xor_sync(0xffffffffu, v.y, off));
+  };
 #pragma unroll
   for (int j = 0; j < M; ++j) {
-    const double mine = upper ? a[j + M] : a[j], give = upper ? a[j] : a[j + M];
-    a[j] = mine + __shfl_xor_sync(0xffffffffu, give, off);
+    const Sum3<float2> mine = upper ? a[j + M] : a[j], give = upper ? a[j] : a[j + M];
+    a[j] = sum3_join(mine, Sum3<float2>{from(give.h), from(give.m), from(give.l)});
   }
 }
 
@@ -420,11 +425,13 @@ __device__ __forceinline__ void fold_half(double* a, int lane, int off) {
 // c = 1/sqrt(lambda) in one pass over the fields, in double-float arithmetic on the
 // FP32 pipe (tg_df.h; ~2^-46 relative per operation, all terms positive).  These
 // volumes only decide bisection branches under a certified bound that includes this
-// arithmetic's error; from a thread's own run on the sums are FP64.  On small grids the
-// sum over the block bounds the pass: K FP64 trees are K x 10 dependent adds of 64
-// cycles.  Here a warp's lanes exchange halves of their candidates, so that the K sums
-// take 2 K adds, the eight warps' totals one each, and the CTA that ends last adds up
-// the CTAs' shares.
+// arithmetic's error; beyond a thread's own run the sums have FP64's accuracy.  On small
+// grids the sum over the block bounds the pass: K FP64 trees are K x 10 dependent adds of
+// 64 cycles.  Here a warp's lanes exchange halves of their candidates, so that the K sums
+// take about K additions, two candidates' at a time as sums of three FP32 values
+// (tg_sum3.h); the last two of a lane are FP64, the eight warps' totals one addition
+// each, and the CTA that ends last adds up the CTAs' shares.  (In FP64 from the start,
+// 2 K additions a warp: 31 us a pass of 16 on 200,000 voxels.)
 template <int K>
 __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
     const df* __restrict__ sq, const df* __restrict__ lo, const df* __restrict__ hi,
@@ -450,14 +457,18 @@ __global__ void __launch_bounds__(kThreads) k_oc_volume_multi(
     }
   }
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double sum[K];
+  Sum3<float2> sum[K / 2];
 #pragma unroll
-  for (int k = 0; k < K; ++k) sum[k] = widen(acc[k].hi) + widen(acc[k].lo);
-  fold_half<K / 2>(sum, lane, 16);
-  fold_half<K / 4>(sum, lane, 8);
-  fold_half<K / 8>(sum, lane, 4);
-  if constexpr (K == 16) fold_half<1>(sum, lane, 2);
-  double v = sum[0];
+  for (int k = 0; k < K; k += 2)
+    sum[k / 2] = Sum3<float2>{make_float2(acc[k].hi, acc[k + 1].hi),
+                              make_float2(acc[k].lo, acc[k + 1].lo), make_float2(0.0f, 0.0f)};
+  fold_half<K / 4>(sum, lane, 16);
+  fold_half<K / 8>(sum, lane, 8);
+  if constexpr (K == 16) fold_half<1>(sum, lane, 4);
+  const double even = widen(sum[0].h.x) + (widen(sum[0].m.x) + widen(sum[0].l.x));
+  const double odd = widen(sum[0].h.y) + (widen(sum[0].m.y) + widen(sum[0].l.y));
+  const bool upper = (lane & kLanes) != 0;
+  double v = (upper ? odd : even) + __shfl_xor_sync(0xffffffffu, upper ? even : odd, kLanes);
 #pragma unroll
   for (int off = kLanes / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   if (lane % kLanes == 0) share[wid][lane / kLanes] = v;
