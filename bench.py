@@ -259,7 +259,7 @@ def workload_config(args):
             "elements": args.nx * args.ny * args.nz,
             "dofs": 3 * (args.nx + 1) * (args.ny + 1) * (args.nz + 1),
             "volfrac": 0.3, "rmin": 1.5, "move": 0.2, "penal": 3, "cg_tol": 1e-8,
-            "solver": "MG-PCG (Galerkin, damped Jacobi 1+1, dense Cholesky coarsest)",
+            "solver": "MG-PCG (Galerkin, damped Jacobi 1+1, dense direct coarsest)",
             "l2": "inputs larger than L2 (no flush)", "parallelism": "replicas"}
 
 

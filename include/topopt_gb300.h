@@ -746,7 +746,10 @@ int tg_set_coarse_fused(int32_t on);
  * one element row per thread (the FP64 form's schedule, its tile chosen by a
  * cost model); kind 1: two element rows per thread in paired FP32 instructions,
  * with 2, 3, 4, 5, 6, 8, 10 or 12 warps per CTA for `shape` 0 .. 7 and `kz` >= 8
- * node layers per CTA.  The setting overrides the per-grid, per-mode table (apply, residual,
+ * node layers per CTA.  A shape's number means a tile of this version: earlier
+ * ones gave other tiles to the numbers 0 .. 7 (Y x W element rows and warps of a
+ * kernel that is gone), so a number stored with one of them selects another tile
+ * here.  The setting overrides the per-grid, per-mode table (apply, residual,
  * smoothing; measured on the first large mixed job of a grid) for every later
  * FP32 launch in the process; kind < 0 clears it.  Results of every schedule
  * agree to FP32 rounding. */

@@ -6,7 +6,8 @@
 //   P0 and A1 = P0^T A0 P0 :1408-1446, galerkin_a1_from_prolong :1543-1899
 //   levels 2.. (Galerkin)  :557-697 (build_hierarchy)
 //   jacobi_sweep, v_cycle  :780-817, mf_jacobi_sweep / mf_v_cycle :1128-1160
-//   coarsest direct solve  SimplicialLDLT :690-695 -> here a dense Cholesky
+//   coarsest direct solve  SimplicialLDLT :690-695 -> here a dense FP64 inverse, or
+//     (above 2,048 DOFs) a Cholesky factor
 //
 // Coarse operators are Galerkin, formed element by element: a coarse element's
 // 24x24 matrix is the sum over its (up to) eight children of W^T K_child W, with
