@@ -341,6 +341,10 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
 #pragma unroll
     for (int m = 0; m < 4; ++m) pend[k][m] = vset<V>(czero<S>());
   S dsum = czero<S>();
+  // Periodic FP32: a thread's share of p.Ap in runs of eight layers (16 nodes with two
+  // rows), the runs added up as a double-float, since a march takes up to 64 layers.
+  constexpr bool kRuns = PER && MODE == kApply && std::is_same<S, float>::value;
+  df druns(0.0f, 0.0f);
 
   // Two steps per pass: this layer's faces become the last layer's without moves.
 #pragma unroll(kPipe ? 2 : 1)
@@ -508,6 +512,12 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
         }
       finish(R, r2);
     }
+    if constexpr (kRuns) {
+      if ((s & 7) == 0) {
+        druns = druns + df(dsum, 0.0f);
+        dsum = 0.0f;
+      }
+    }
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -518,8 +528,13 @@ __global__ void __launch_bounds__(32 * RowsOf<V>::kMaxWarps, 1)
       for (int k = 0; k < 3; ++k) keep[i][k] = knext[i][k];
   }
   if constexpr (MODE != kResidual) {
+    double share;
+    if constexpr (kRuns)
+      share = df_to_double(druns + df(dsum, 0.0f));
+    else
+      share = double(store_t(dsum));
     if (dot.part != nullptr)
-      grid_sum(double(store_t(dsum)), dot,
+      grid_sum(share, dot,
                int((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x),
                int(gridDim.x * gridDim.y));
   }
