@@ -434,9 +434,7 @@ void launch(const Tile& t, const MgDims& fd, const MgDims& cd, const ModalConsts
             const float* x, const float* b, const float* invdiag, float omega, float* y,
             cudaStream_t s) {
   const size_t per_warp = (2 * 192 + (kDepth + 1) * slot_words1<MODE>()) * sizeof(float);
-  // On every call: the limit belongs to the kernel in the current device's context.
-  TG_CUDA(cudaFuncSetAttribute(k_level1_march<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(kMaxWarps * per_warp)));
+  allow_shared<k_level1_march<MODE>>(int(kMaxWarps * per_warp));
   const int nss = (cd.nny + t.W - 2) / (t.W - 1);
   launch_behind(k_level1_march<MODE>, tile_grid(cd, t), 32 * t.W, t.W * per_warp, s, fd, cd,
                 to_modal<float>(c), t.kz, nss, ef, an, spos, yspec, x, b, invdiag, omega, y);

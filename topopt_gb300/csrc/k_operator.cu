@@ -856,11 +856,9 @@ void launch_march(const GridDev& gd, const MarchTile& t, int nsys, const ModalCo
   const size_t smem = size_t(2) * t.W * 192 * sizeof(S) +
                       (RowsOf<V>::R == 2 ? size_t(t.W) * (kDepth + 1) * slot_words<MODE>() * 4 : 0);
   if constexpr (RowsOf<V>::R == 2) {
-    // More than the default 48 KB.  On every call, since the limit belongs to the kernel
-    // in the current device's context, and the same value from every thread.
-    constexpr int most = RowsOf<V>::kMaxWarps * (2 * 192 + (kDepth + 1) * slot_words<MODE>()) * 4;
-    TG_CUDA(cudaFuncSetAttribute(k_fine_march<V, T, MODE, PER>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    // More than the default 48 KB.
+    allow_shared<k_fine_march<V, T, MODE, PER>>(
+        RowsOf<V>::kMaxWarps * (2 * 192 + (kDepth + 1) * slot_words<MODE>()) * 4);
   }
   // Only the public apply takes values at nodes of absent elements; within the
   // solver (a kept mask) they are zeros.
