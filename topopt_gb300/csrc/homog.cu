@@ -117,26 +117,18 @@ __device__ __forceinline__ double bred(double v, double* sh) {
   return s;
 }
 
-// A power of two that brings the inverse diagonal to at most 1, and its inverse.
-struct RzScale {
-  float up = 1.0f;
-  double down = 1.0;
-};
-
 // Running sums of r.r and r.(D^-1 r).  FP64 data: FP64.  FP32 data: every product
 // exactly, as FP32 values, in sums of three FP32 values each (tg_sum3.h); FP64 from the
 // warps' totals on.  FP64 sums of FP32 products take five instructions per DOF on units
 // 64 times slower, twice the operator's time (24 systems of 32^3: 34 us against 17).
 // Of 98,304 products they are off by up to 2^-52 of the sum, the sums of three by 2^-68
 // before their one rounding to FP64 (sums of two, 2^-45, would not do:
-// tests/test_sum3.py).  D^-1 is scaled to at most 1, exactly, so that no modulus takes
-// the products' errors out of FP32's range.
+// tests/test_sum3.py).
 template <class T>
 struct RrRz;
 template <>
 struct RrRz<double> {
   double a = 0.0, b = 0.0;
-  __device__ __forceinline__ explicit RrRz(const RzScale&) {}
   __device__ __forceinline__ void add(double v, double iv) {
     a += v * v;
     b += v * (iv * v);
@@ -153,11 +145,9 @@ struct RrRz<double> {
 template <>
 struct RrRz<float> {
   Sum3<float2> a{}, b{};  // the DOFs of even and odd place in a run of four
-  RzScale sc;
-  __device__ __forceinline__ explicit RrRz(const RzScale& s) : sc(s) {}
   __device__ __forceinline__ void add(float2 v, float2 iv) {
     sum3_square(a, v);
-    sum3_weighted_square(b, vmul(iv, make_float2(sc.up, sc.up)), v);
+    sum3_weighted_square(b, iv, v);
   }
   __device__ __forceinline__ void add(float v, float iv) {
     add(make_float2(v, 0.0f), make_float2(iv, 0.0f));
@@ -192,7 +182,7 @@ struct RrRz<float> {
 #pragma unroll
     for (int o = kW / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, kW);
     if (lane == 0) *prr = v;
-    if (lane == kW) *prz = v * sc.down;
+    if (lane == kW) *prz = v;
   }
 };
 
@@ -211,13 +201,12 @@ __device__ __forceinline__ void share(int64_t nd, F4&& f4, F1&& f1) {
 // rr = r.r, rz = r.(D^-1 r) per system.
 template <class T>
 __global__ void k_b_rr_rz(const T* __restrict__ R, const T* __restrict__ invd, int64_t nd,
-                          int nrhs, RzScale sc, double* __restrict__ prr,
-                          double* __restrict__ prz) {
+                          int nrhs, double* __restrict__ prr, double* __restrict__ prz) {
   __shared__ double sh[32];
   const int bi = blockIdx.y, P = gridDim.x;
   const T* r = R + bi * nd;
   const T* iv = invd + (bi / nrhs) * nd;
-  RrRz<T> acc(sc);
+  RrRz<T> acc;
   for (int64_t d = blockIdx.x * int64_t(kT) + threadIdx.x; d < nd; d += int64_t(P) * kT)
     acc.add(r[d], iv[d]);
   acc.store(prr + int64_t(bi) * P + blockIdx.x, prz + int64_t(bi) * P + blockIdx.x, sh);
@@ -327,7 +316,7 @@ __global__ void __launch_bounds__(kT, 5) k_b_xr(T* __restrict__ X, T* __restrict
                                              const double* __restrict__ absn,
                                              const double* __restrict__ ppap, int npap,
                                              double* __restrict__ pap,
-                                             const int* __restrict__ act, RzScale sc,
+                                             const int* __restrict__ act,
                                              double* __restrict__ prr, double* __restrict__ prz) {
   __shared__ double sh[32];  // [2][kT / 32][3] floats in FP32
   __shared__ double s_pa;
@@ -348,7 +337,7 @@ __global__ void __launch_bounds__(kT, 5) k_b_xr(T* __restrict__ X, T* __restrict
   T* r = R + bi * nd;
   const T* p = Pv + bi * nd;
   const T* t = Tv + bi * nd;
-  RrRz<T> acc(sc);
+  RrRz<T> acc;
   share<T>(
       nd,
       [&](int64_t q) {
@@ -475,9 +464,10 @@ __global__ void k_b_refine(int B, const double* __restrict__ rr, const double* _
   if (go) atomicAdd(nrun, 1);
 }
 
-__global__ void k_to_f32(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
+__global__ void k_to_f32(const double* __restrict__ a, double scale, float* __restrict__ b,
+                         int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(kT) + threadIdx.x; i < n; i += int64_t(gridDim.x) * kT)
-    b[i] = float(a[i]);
+    b[i] = float(a[i] * scale);
 }
 
 // Partials of F[cell][I] . X[bi] for I = 0..5 (grid.z = I).
@@ -507,7 +497,6 @@ struct Batch {
   int64_t nd;
   ModalConsts mc;
   const uint8_t* kept;
-  RzScale rzs;
   cudaStream_t s;
   DBuf<double> prr, prz, ppap, rr, rz, pap, thr, rhs2, absn, rn;
   DBuf<int> act, it, nact, run, nrun;  // absn, act and it: two buffers of B, used in turn
@@ -544,7 +533,7 @@ struct Batch {
           const int* runp, const double* r64) {
     k_b_begin<T><<<g2(), kT, 0, s>>>(r64, rn.p, invd, nd, nrhs, runp, X, R, Pv);
     TG_LAUNCH_CHECK();
-    k_b_rr_rz<T><<<g2(), kT, 0, s>>>(R, invd, nd, nrhs, rzs, prr.p, prz.p);
+    k_b_rr_rz<T><<<g2(), kT, 0, s>>>(R, invd, nd, nrhs, prr.p, prz.p);
     TG_LAUNCH_CHECK();
     k_bsum<<<wb(), 256, 0, s>>>(prr.p, P, B, rr.p, prz.p, rz.p);
     TG_LAUNCH_CHECK();
@@ -559,7 +548,7 @@ struct Batch {
       launch_periodic_op<T>(kApply, nx, ny, nz, mc, ef, kept, Pv, nullptr, Tv, ppap.p, B, nrhs,
                             act.p + in, s);
       k_b_xr<T><<<g2(), kT, 0, s>>>(X, R, Pv, Tv, invd, nd, nrhs, absn.p + in, ppap.p, Pop, pap.p,
-                                    act.p + in, rzs, prr.p, prz.p);
+                                    act.p + in, prr.p, prz.p);
       TG_LAUNCH_CHECK();
       k_b_p<T><<<g2(), kT, 0, s>>>(Pv, R, invd, nd, nrhs, prr.p, prz.p, P, thr.p, pap.p, max_it,
                                    act.p + in, act.p + out, absn.p + in, absn.p + out, it.p + in,
@@ -671,10 +660,6 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
     bt.mc = ModalConsts::make(poisson, spacing);
     bt.mc.kdiag = ke[0];
     bt.s = s;
-    // D^-1's entries are 1 / (n kdiag E), n = 1 .. 8.
-    const int ex = std::min(126, std::max(-126, std::ilogb(ke[0] * youngs_modulus)));
-    bt.rzs.up = float(std::ldexp(1.0, ex));
-    bt.rzs.down = std::ldexp(1.0, -ex);
     // All cells together: solving them a group at a time, so that a group's CG
     // vectors stay in L2, measured slower (32 cells of 32^3: 109 ms in groups of 8,
     // 96 in groups of 16, 80 at once) -- the launches of a group are too short to
@@ -738,12 +723,17 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
           all_ok = false;
     } else {
       // FP64 refinement around FP32 inner solves (relative 1e-3 each).
-      k_to_f32<<<nb_cell, kT, 0, s>>>(ef.p, eff32.p, ncell * np);
+      k_to_f32<<<nb_cell, kT, 0, s>>>(ef.p, 1.0, eff32.p, ncell * np);
       TG_LAUNCH_CHECK();
-      k_to_f32<<<nb_cell, kT, 0, s>>>(invd.p, invd32.p, ncell * nd);
+      // The preconditioner's scale is free: a power of two in D^-1 is one in p and its
+      // inverse in alpha, exactly.  This one, about the modulus' root, leaves the terms of
+      // p.Ap the size of the residual's squares, and those of r.(D^-1 r), with the products'
+      // errors that their sums take in, far inside FP32's range.
+      const double root = std::ldexp(1.0, std::ilogb(ke[0] * youngs_modulus) / 2);
+      k_to_f32<<<nb_cell, kT, 0, s>>>(invd.p, root, invd32.p, ncell * nd);
       TG_LAUNCH_CHECK();
       // |b|^2 and the outer threshold tol^2 |b|^2.
-      k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.rzs, bt.prr.p, bt.prz.p);
+      k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
       TG_LAUNCH_CHECK();
       k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, b2.p, nullptr, nullptr);
       TG_LAUNCH_CHECK();
@@ -760,7 +750,7 @@ extern "C" int tg_homogenize(int32_t ncell, int32_t nx, int32_t ny, int32_t nz, 
         if (ref > 0)
           launch_periodic_op<double>(kResidual, nx, ny, nz, bt.mc, ef.p, kept.p, X.p, Bv.p, R.p,
                                      nullptr, B, nrhs, bt.run.p, s);
-        k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.rzs, bt.prr.p, bt.prz.p);
+        k_b_rr_rz<double><<<bt.g2(), kT, 0, s>>>(R.p, invd.p, nd, nrhs, bt.prr.p, bt.prz.p);
         TG_LAUNCH_CHECK();
         k_bsum<<<bt.wb(), 256, 0, s>>>(bt.prr.p, P, B, bt.rr.p, nullptr, nullptr);
         TG_LAUNCH_CHECK();
